@@ -6,20 +6,26 @@
 // integer arithmetic and one single-precision approximation instruction, leaving the FP64 unit to the
 // products of the solvers.
 //
-// Method (Newton's iteration in fixed point followed by an exact remainder correction, as in Brent and
-// Zimmermann, "Modern Computer Arithmetic" (2010), sections 3.4 and 3.5):
-//   division a / b: with mantissas A, B (53-bit integers, A scaled so that B <= A < 2B), R ~ 2^61 / b for
-//     b = B / 2^53 in [1/2, 1) from the single-precision reciprocal, refined by two Newton steps
-//     R <- R + R (1 - b R); the estimate Q = A R / 2^61 of floor(A 2^53 / B) is within 2 units, and the
-//     remainder A 2^53 - Q B, exact in 64-bit two's complement because it is small, corrects it. The
-//     last bit of Q and whether the remainder vanishes give the rounding.
-//   square root of x: with the mantissa M (53-bit integer, doubled when the exponent is odd) and
-//     m = M / 2^52 in [1, 4), Y ~ 2^62 / sqrt(m) from the single-precision reciprocal square root, refined by
-//     two Newton steps Y <- Y + Y (1 - m Y^2) / 2; S = M Y / 2^61 estimates floor(sqrt(M 2^54)) within 2
-//     units and the remainder M 2^54 - S^2 corrects it. A square root never falls halfway between two
-//     doubles, so the last bit of S alone decides the rounding.
-// Zeros, infinities, NaNs, subnormal operands and results outside the normal range are passed to the
-// hardware operation, which handles them by definition; ordinary operands never take that branch.
+// Method (a Newton-type step in fixed point followed by an exact remainder test, as in Brent and Zimmermann,
+// "Modern Computer Arithmetic" (2010), sections 3.4 and 3.5), laid out for a short dependency chain: one
+// higher-order step in place of two Newton steps, 32 x 32 -> 64-bit multiply-adds in place of full 64-bit high
+// products, and one correction of the last place in place of four.
+//   division a / b: with mantissas A, B (53-bit integers, A scaled so that B <= A < 2B) and b = B / 2^53 in
+//     [1/2, 1), r0 ~ 1 / b is the single-precision reciprocal. eps = 1 - b r0 is exact (a low 64-bit product),
+//     and 1 / b = r0 (1 + eps + eps^2 + eps^3 + ...); the truncated series leaves eps^4 (below 2^-70 even for
+//     starting points 40 units off). A r with 8 bits below the last place, biased down, gives the rounded
+//     quotient or one less, and the sign of the exact remainder at the halfway point decides.
+//   square root of x: with the mantissa M (53-bit integer, doubled when the exponent is odd) and m = M / 2^52 in
+//     [1, 4), y0 ~ 1 / sqrt(m) is the single-precision reciprocal square root, eps = 1 - m y0^2,
+//     1 / sqrt(m) = y0 (1 + eps / 2 + 3 eps^2 / 8 + 5 eps^3 / 16 + ...), and M y with 7 bits below the last place
+//     gives the rounded root or one less; the sign of M 2^52 - (k + 1/2)^2 decides.
+// Neither a quotient of normal numbers nor a square root falls halfway between two doubles.
+// Cycles on GB300, one warp alone (latency) / per operation of a sub-partition's six warps (throughput): division
+// 325 / 152, square root 420 / 159; with two Newton steps and four corrections 496 / 258 and 559 / 269; the FP64
+// unit's own sequences 641 / 635 and 599 / 572.
+// Infinities, NaNs, subnormal operands, zero divisors and results outside the normal range are passed to the
+// hardware operation, which handles them by definition. Zero dividends and square roots of zero, which the
+// solvers meet all the time, stay on the fast path: a warp with one such lane would otherwise run both.
 //
 // Every function is __host__ __device__: on the host the single-precision approximation is the exact
 // reciprocal (optionally perturbed by a test), so the same integer steps can be compared against the host's
@@ -44,9 +50,13 @@ namespace ipipe {
 constexpr uint64_t kMant = (uint64_t(1) << 52) - 1;
 constexpr uint64_t kHidden = uint64_t(1) << 52;
 
+// The device moves between a double and its bits are opaque to the optimiser, which would otherwise turn tests and
+// sign changes written on the bits back into FP64 comparisons and negations (each an FP64 instruction).
 BG_HD uint64_t to_bits(double x) {
 #ifdef __CUDA_ARCH__
-  return (uint64_t)__double_as_longlong(x);
+  uint64_t u;
+  asm("mov.b64 %0, %1;" : "=l"(u) : "d"(x));
+  return u;
 #else
   uint64_t u;
   std::memcpy(&u, &x, 8);
@@ -55,7 +65,9 @@ BG_HD uint64_t to_bits(double x) {
 }
 BG_HD double from_bits(uint64_t u) {
 #ifdef __CUDA_ARCH__
-  return __longlong_as_double((long long)u);
+  double x;
+  asm("mov.b64 %0, %1;" : "=d"(x) : "l"(u));
+  return x;
 #else
   double x;
   std::memcpy(&x, &u, 8);
@@ -125,94 +137,79 @@ BG_HD float rsqrt_approx(float x) {
 #endif
 }
 
-// v * 2^s as an integer, for a float v in [1/4, 4) and s >= 26 (v's 24-bit significand shifted into place)
-BG_HD uint64_t fixed_of(float v, int s) {
+// v 2^(150 - f) as an integer, for a float v whose exponent field is f, f + 1 or f + 2
+BG_HD uint32_t fixed_of(float v, uint32_t f) {
   const uint32_t u = fbits(v);
-  const uint64_t sig = (uint64_t)((u & 0x7FFFFFu) | 0x800000u);
-  return sig << (int)(((u >> 23) & 0xFFu) - 150u + (uint32_t)s);
+  return ((u & 0x7FFFFFu) | 0x800000u) << ((u >> 23) - f);
+}
+BG_HD uint64_t mul_wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+BG_HD uint32_t lo32(uint64_t v) { return (uint32_t)v; }
+BG_HD uint32_t hi32(uint64_t v) { return (uint32_t)(v >> 32); }
+BG_HD int32_t mulhi_s(int32_t a, int32_t b) { return (int32_t)(((int64_t)a * b) >> 32); }
+// (a b) >> 64 without the low halves' product: low by at most two units
+BG_HD uint64_t mulhi_est(uint64_t a, uint64_t b) {
+  const uint64_t m1 = mul_wide(hi32(a), lo32(b)), m2 = mul_wide(lo32(a), hi32(b));
+  return mul_wide(hi32(a), hi32(b)) + hi32(m1) + hi32(m2);
+}
+// (s r) >> 32 for a signed s, |s| < 2^62, and r < 2^26
+BG_HD int64_t mul_shift32(int64_t s, uint32_t r) {
+  return (int64_t)(int32_t)(s >> 32) * (int64_t)r + (int64_t)hi32(mul_wide((uint32_t)s, r));
 }
 
-// Correctly rounded a / b when a, b are normal and the quotient is normal; `ok` false otherwise (the
-// returned value is then meaningless).
+// Correctly rounded a / b when b is normal and a is zero, or a and the quotient are normal; `ok` false otherwise
+// (the returned value is then meaningless).
 BG_HD double div_core(uint64_t ua, uint64_t ub, bool& ok) {
   const uint32_t ea = (uint32_t)(ua >> 52) & 0x7FFu, eb = (uint32_t)(ub >> 52) & 0x7FFu;
   uint64_t A = (ua & kMant) | kHidden;
   const uint64_t B = (ub & kMant) | kHidden;
-  int e = (int)ea - (int)eb + 1023;
   const bool lt = A < B;
-  A <<= lt ? 1 : 0;
-  e -= lt ? 1 : 0;
-  ok = (ea - 1u < 2046u) && (eb - 1u < 2046u) && (e >= 1) && (e <= 2045);
-  // b = B / 2^53 in [1/2, 1), truncated to 24 bits as a float
-  const float bf = bitsf(0x3F000000u | (uint32_t)((B >> 29) & 0x7FFFFFu));
-  uint64_t R = fixed_of(rcp_approx(bf), 61);  // ~ 2^61 / b, in (2^60, 2^62]
-  const uint64_t Bs = B << 11;                 // b 2^64
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int64_t E = (int64_t)((uint64_t(1) << 61) - umulhi(Bs, R));  // 2^61 (1 - b R / 2^61)
-    R = (uint64_t)((int64_t)R + smulhi((int64_t)R, E * 8));
-  }
-  uint64_t Q = umulhi(A << 3, R);  // ~ floor(A 2^53 / B), in [2^53, 2^54)
-  int64_t rem = (int64_t)((A << 53) - Q * B);
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const bool lo = rem < 0;
-    Q -= lo ? 1 : 0;
-    rem += lo ? (int64_t)B : 0;
-  }
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const bool hi = rem >= (int64_t)B;
-    Q += hi ? 1 : 0;
-    rem -= hi ? (int64_t)B : 0;
-  }
-  uint64_t mant = Q >> 1;
-  const bool up = (Q & 1) && (rem != 0 || (mant & 1));
-  mant += up ? 1 : 0;
-  const bool carry = mant >> 53;
-  mant >>= carry ? 1 : 0;
-  e += carry ? 1 : 0;
-  return from_bits(((ua ^ ub) & (uint64_t(1) << 63)) | ((uint64_t)e << 52) | (mant & kMant));
+  A <<= lt ? 1 : 0;  // A / B in [1, 2)
+  const int e = (int)ea - (int)eb + 1023 - (lt ? 1 : 0);
+  const uint64_t sign = (ua ^ ub) & (uint64_t(1) << 63);
+  const bool zero = (ua << 1) == 0;
+  ok = (eb - 1u < 2046u) && (zero || ((ea - 1u < 2046u) && (e >= 1) && (e <= 2045)));
+  // r0 ~ 1 / b for b = B / 2^53 in [1/2, 1) from the leading 24 bits, as R0 / 2^24 (r0 from just below 1 to 2)
+  const uint32_t R0 = fixed_of(rcp_approx(bitsf(0x3F000000u | (uint32_t)((B >> 29) & 0x7FFFFFu))), 126u);
+  // eps = 1 - b r0, exact at 2^-77: the product's bits from 2^77 up are those of 1
+  const int64_t E = -(int64_t)(B * R0);
+  const int32_t Eh = (int32_t)(E >> 32);                // eps 2^45
+  const int64_t e2 = (int64_t)Eh * Eh;                  // eps^2 2^90
+  const int32_t e3 = mulhi_s((int32_t)(e2 >> 25), Eh);  // eps^3 2^78
+  // r = r0 (1 + eps + eps^2 + eps^3) as R / 2^62
+  const uint64_t R = ((uint64_t)R0 << 38) + (uint64_t)(mul_shift32(E + (e2 >> 13) + (e3 >> 1), R0) >> 7);
+  // the rounded quotient or one less: q = A r 2^7 carries 8 bits below the last place, within 8 units
+  const uint64_t m = (mulhi_est(A << 9, R) + (128 - 8)) >> 8;
+  const int64_t rem = (int64_t)((A << 53) - (2 * m + 1) * B);  // sign of A / B - (m + 1/2); never a tie
+  const uint64_t mant = m + (rem > 0 ? 1 : 0);                 // in [2^52, 2^53)
+  return from_bits(zero ? sign : (sign | ((uint64_t)(uint32_t)(e - 1) << 52)) + mant);
 }
 
-// Correctly rounded sqrt(x) for a positive normal x; `ok` false otherwise.
+// Correctly rounded sqrt(x) for a positive normal x or a zero; `ok` false otherwise.
 BG_HD double sqrt_core(uint64_t ux, bool& ok) {
   const uint32_t ex = (uint32_t)(ux >> 52);  // sign included: negative x fails the range test
-  ok = ex - 1u < 2046u;
-  int u = (int)ex - 1023;
-  const bool odd = u & 1;
-  const uint64_t M = ((ux & kMant) | kHidden) << (odd ? 1 : 0);  // [2^52, 2^54)
-  u -= odd ? 1 : 0;
-  // m = M / 2^52 in [1, 4), truncated to 24 bits as a float
-  const float mf = odd ? bitsf(0x40000000u | (uint32_t)((M >> 30) & 0x7FFFFFu))
-                       : bitsf(0x3F800000u | (uint32_t)((M >> 29) & 0x7FFFFFu));
-  uint64_t Y = fixed_of(rsqrt_approx(mf), 62);  // ~ 2^62 / sqrt(m), in (2^60, 2^62]
-  const uint64_t Ms = M << 10;                   // m 2^62
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const uint64_t Y2 = umulhi(Y, Y);                                   // y^2 2^60
-    const int64_t E = (int64_t)((uint64_t(1) << 58) - umulhi(Ms, Y2));  // 2^58 (1 - m y^2)
-    Y = (uint64_t)((int64_t)Y + smulhi((int64_t)Y, E * 32));
-  }
-  uint64_t S = umulhi(M << 3, Y);  // ~ floor(sqrt(M 2^54)), in [2^53, 2^54)
-  int64_t rem = (int64_t)((M << 54) - S * S);
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const bool lo = rem < 0;
-    S -= lo ? 1 : 0;
-    rem += lo ? (int64_t)(2 * S + 1) : 0;
-  }
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const bool hi = rem > (int64_t)(2 * S);
-    rem -= hi ? (int64_t)(2 * S + 1) : 0;
-    S += hi ? 1 : 0;
-  }
-  uint64_t mant = (S >> 1) + (S & 1);
-  const bool carry = mant >> 53;
-  mant >>= carry ? 1 : 0;
-  u += carry ? 2 : 0;
-  return from_bits((uint64_t)(u / 2 + 1023) << 52 | (mant & kMant));
+  const bool zero = (ux << 1) == 0;
+  ok = zero || ex - 1u < 2046u;
+  const bool odd = !(ex & 1u);  // the unbiased exponent ex - 1023 is odd
+  const uint64_t M = ((ux & kMant) | kHidden) << (odd ? 1 : 0);  // m = M / 2^52 in [1, 4)
+  // y0 ~ 1 / sqrt(m) from the leading 24 bits, as Y0 / 2^25 (y0 from just below 1/2 to 1)
+  const uint32_t Y0 = fixed_of(
+      rsqrt_approx(bitsf((odd ? 0x40000000u : 0x3F800000u) | (uint32_t)((ux >> 29) & 0x7FFFFFu))), 125u);
+  // eps = 1 - m y0^2 at 2^-70 (the product's last 32 bits dropped)
+  const uint64_t Z = mul_wide(Y0, Y0);
+  const uint64_t P = hi32(mul_wide(lo32(M), lo32(Z))) + mul_wide(lo32(M), hi32(Z)) + mul_wide(hi32(M), lo32(Z)) +
+                     ((uint64_t)(hi32(M) * hi32(Z)) << 32);
+  const int64_t E = -(int64_t)P;
+  const int32_t Eh = (int32_t)(E >> 26);                // eps 2^44
+  const int64_t e2 = (int64_t)Eh * Eh;                  // eps^2 2^88
+  const int32_t e3 = mulhi_s((int32_t)(e2 >> 25), Eh);  // eps^3 2^75
+  // y = y0 (1 + eps / 2 + 3 eps^2 / 8 + 5 eps^3 / 16) as Y / 2^62; the sum in brackets less 1 at 2^-69
+  const int64_t S = (E >> 2) + ((3 * e2) >> 22) + ((5 * e3) >> 10);
+  const uint64_t Y = ((uint64_t)Y0 << 37) + (uint64_t)mul_shift32(S, Y0);
+  // the rounded root or one less: M y 2^7 carries 7 bits below the last place, within 4 units
+  const uint64_t m = (mulhi_est(M << 9, Y) + (64 - 4)) >> 7;
+  const int64_t rem = (int64_t)((M << 52) - m * (m + 1));  // positive when sqrt(M 2^52) > m + 1/2; never a tie
+  const uint64_t mant = m + (rem > 0 ? 1 : 0);
+  return from_bits(zero ? ux : ((uint64_t)((ex + 1021u - (odd ? 1u : 0u)) >> 1) << 52) + mant);
 }
 
 // The hardware operations for the operands outside the fast domain, behind a call that the compiler cannot

@@ -56,7 +56,6 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_gs_flow(GSArgs a, int par
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   __shared__ double sB[kGSFlowWarps][32][12];
   __shared__ int sJ[kGSFlowWarps][32];
-  __shared__ double sHq[kGSFlowWarps][16];
   const unsigned tag = ld_acquire_u32(a.flow + 1);
   const int ntiles = (a.n + kGSTile - 1) / kGSTile;
   for (;;) {
@@ -117,7 +116,7 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_gs_flow(GSArgs a, int par
     for (int e = 0; e < 9; ++e) A[e] = a.local[9 * (size_t)i + e];
     double ldx[3] = {-lx[0], -lx[1], -lx[2]};
     const double sc = a.scaling[i];
-    const bool ok = law_solve_local<true>(a.desaxce != 0, a.strat, A, lb, lx, a.mu[i], sc, sHq[w]);
+    const bool ok = law_solve_local<true>(a.desaxce != 0, a.strat, A, lb, lx, a.mu[i], sc);
     if (lane == 0) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) ldx[k] = ldx[k] + lx[k];
@@ -240,7 +239,6 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_pgs_flow(GSArgs a, int pa
   // the whole warp works on its contact, as in k_gs_flow: lanes 0-2 form one component of lb each, every lane
   // runs the same local solve, lanes 0..d-1 update one dof of Mx each
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __shared__ double sHq[kGSFlowWarps][16];
   const unsigned tag = ld_acquire_u32(a.flow + 1);
   const int ntiles = (a.n + kGSTile - 1) / kGSTile;
   const int d = a.d;
@@ -285,7 +283,7 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_pgs_flow(GSArgs a, int pa
                           __shfl_sync(0xffffffffu, lbr, 2)};
     double ldx[3] = {-lx[0], -lx[1], -lx[2]};
     const double sc = a.scaling[i];
-    const bool ok = law_solve_local<true>(a.desaxce != 0, a.strat, A, lb, lx, a.mu[i], sc, sHq[w]);
+    const bool ok = law_solve_local<true>(a.desaxce != 0, a.strat, A, lb, lx, a.mu[i], sc);
 #pragma unroll
     for (int k = 0; k < 3; ++k) ldx[k] = ldx[k] + lx[k];
     if (!ok) {

@@ -33,6 +33,28 @@ constexpr double kLocalTol = 1.8189894035458565e-12;      // pow(eps, 0.75) == 2
 BG_HD bool is_zero(double s) {
   return (ipipe::to_bits(s) & ~(uint64_t(1) << 63)) < ipipe::to_bits(kEps);
 }
+// Signs and comparisons on the bits: as FP64 operations each would take the FP64 unit for as long as an addition
+// (an explicit negation too; one folded into a sum, product or FMA is free).
+constexpr uint64_t kSign = uint64_t(1) << 63, kInfBits = uint64_t(0x7FF) << 52;
+BG_HD uint64_t abs_bits(double v) { return ipipe::to_bits(v) & ~kSign; }
+BG_HD double neg(double v) { return ipipe::from_bits(ipipe::to_bits(v) ^ kSign); }
+BG_HD double absd(double v) { return ipipe::from_bits(abs_bits(v)); }
+BG_HD bool nonzero(double v) { return abs_bits(v) != 0; }  // v != 0.0
+BG_HD bool negative(double v) {                             // v < 0.0
+  const uint64_t u = ipipe::to_bits(v);
+  return u > kSign && u <= (kSign | kInfBits);
+}
+// a <= t and a < t for a >= 0 (or NaN) and any t
+BG_HD bool leq_from_zero(double a, double t) {
+  const uint64_t ut = ipipe::to_bits(ipipe::plus_zero(t));  // a negative t has a larger bit pattern than infinity
+  return ut <= kInfBits && ipipe::to_bits(a) <= ut;
+}
+BG_HD bool less_from_zero(double a, double t) {
+  const uint64_t ut = ipipe::to_bits(t);
+  return ut <= kInfBits && abs_bits(a) < ut;
+}
+// v > 0 ? v : 0
+BG_HD double positive_part(double v) { return ipipe::to_bits(v) <= kInfBits ? v : 0.0; }
 BG_HD double dmax(double a, double b) { return (a < b) ? b : a; }
 BG_HD double dmin(double a, double b) { return (b < a) ? b : a; }
 BG_HD double dot3(const double* a, const double* b) { return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0])); }
@@ -48,6 +70,19 @@ BG_HD void matvec3(const double* A, const double* x, double* y) {
 // Full-pivoting LU for n = 2, 3 (FullPivLU semantics: complete pivoting, first maximum in row-major
 // order, elimination stops at an exactly zero pivot, pivots below eps*n*|p0| count as zero in solve)
 // ------------------------------------------------------------------------------------------------
+// |v| as an integer that orders like it; -1 for NaN, which no comparison with |v| accepts
+BG_HD int64_t magnitude(double v) {
+  const uint64_t u = abs_bits(v);
+  return u <= kInfBits ? (int64_t)u : -1;
+}
+BG_HD void swap_if(bool on, double& a, double& b) {
+  const double t = a;
+  a = on ? b : a;
+  b = on ? t : b;
+}
+
+// The pivot search, the tests and the exchanges are integer and select operations on registers (every index is a
+// compile-time one): FP64 comparisons would each take the FP64 unit for as long as an addition.
 template <int N>
 struct SmallLU {
   double lu[N * N];
@@ -59,38 +94,51 @@ struct SmallLU {
 #pragma unroll
     for (int k = 0; k < N * N; ++k) lu[k] = A[k];
     int nonzero = N;
+#pragma unroll
     for (int k = 0; k < N; ++k) {
+      rowt[k] = colt[k] = k;
+      inv_piv[k] = 0.0;
+      if (nonzero < N) continue;
       int pi = k, pj = k;
-      double best = -1.0;
+      int64_t best = -1;
+#pragma unroll
       for (int i = k; i < N; ++i)
+#pragma unroll
         for (int j = k; j < N; ++j) {
-          const double a = fabs(lu[i * N + j]);
+          const int64_t a = magnitude(lu[i * N + j]);
           if (a > best) { best = a; pi = i; pj = j; }
         }
+      if (best == 0) {
+        nonzero = k;
+        continue;
+      }
       rowt[k] = pi;
       colt[k] = pj;
-      if (best == 0.0) {
-        nonzero = k;
-        for (int kk = k; kk < N; ++kk) { rowt[kk] = kk; colt[kk] = kk; }
-        break;
-      }
-      if (pi != k)
-        for (int j = 0; j < N; ++j) { const double t = lu[k * N + j]; lu[k * N + j] = lu[pi * N + j]; lu[pi * N + j] = t; }
-      if (pj != k)
-        for (int i = 0; i < N; ++i) { const double t = lu[i * N + k]; lu[i * N + k] = lu[i * N + pj]; lu[i * N + pj] = t; }
-      const double inv = 1.0 / lu[k * N + k];
+#pragma unroll
+      for (int i = k + 1; i < N; ++i)
+#pragma unroll
+        for (int j = 0; j < N; ++j) swap_if(pi == i, lu[k * N + j], lu[i * N + j]);
+#pragma unroll
+      for (int j = k + 1; j < N; ++j)
+#pragma unroll
+        for (int i = 0; i < N; ++i) swap_if(pj == j, lu[i * N + k], lu[i * N + j]);
+      const double inv = ipipe::div_rn(1.0, lu[k * N + k]);
       inv_piv[k] = inv;
+#pragma unroll
       for (int i = k + 1; i < N; ++i) lu[i * N + k] *= inv;
+#pragma unroll
       for (int i = k + 1; i < N; ++i) {
         const double l = lu[i * N + k];
+#pragma unroll
         for (int j = k + 1; j < N; ++j) lu[i * N + j] = fma(-l, lu[k * N + j], lu[i * N + j]);
       }
     }
     rank = 0;
     if (nonzero > 0) {
-      const double thr = kEps * (double)N * fabs(lu[0]);
-      for (int k = 0; k < nonzero; ++k)
-        if (fabs(lu[k * N + k]) > thr) ++rank;
+      const uint64_t thr = abs_bits(kEps * (double)N * fabs(lu[0]));
+#pragma unroll
+      for (int k = 0; k < N; ++k)
+        if (k < nonzero && magnitude(lu[k * N + k]) >= 0 && abs_bits(lu[k * N + k]) > thr) ++rank;
     }
   }
 
@@ -98,15 +146,29 @@ struct SmallLU {
     double c[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) c[i] = b[i];
-    for (int k = 0; k < N; ++k) { const int p = rowt[k]; if (p != k) { const double t = c[k]; c[k] = c[p]; c[p] = t; } }
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int i = k + 1; i < N; ++i) swap_if(rowt[k] == i, c[k], c[i]);
+#pragma unroll
     for (int i = 1; i < N; ++i)
+#pragma unroll
       for (int j = 0; j < i; ++j) c[i] = fma(-lu[i * N + j], c[j], c[i]);
-    for (int i = rank - 1; i >= 0; --i) {
-      for (int j = i + 1; j < rank; ++j) c[i] = fma(-lu[i * N + j], c[j], c[i]);
+#pragma unroll
+    for (int i = N - 1; i >= 0; --i) {
+      if (i >= rank) continue;
+#pragma unroll
+      for (int j = i + 1; j < N; ++j)
+        if (j < rank) c[i] = fma(-lu[i * N + j], c[j], c[i]);
       c[i] = c[i] * inv_piv[i];
     }
-    for (int i = rank; i < N; ++i) c[i] = 0.0;
-    for (int k = N - 1; k >= 0; --k) { const int p = colt[k]; if (p != k) { const double t = c[k]; c[k] = c[p]; c[p] = t; } }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (i >= rank) c[i] = 0.0;
+#pragma unroll
+    for (int k = N - 1; k >= 0; --k)
+#pragma unroll
+      for (int j = k + 1; j < N; ++j) swap_if(colt[k] == j, c[k], c[j]);
 #pragma unroll
     for (int i = 0; i < N; ++i) x[i] = c[i];
   }
@@ -245,64 +307,86 @@ BG_HD int hessenberg_eigenvalues(double* a, int n, double* wr, double* wi) {
 }
 
 #ifdef __CUDACC__
-// hessenberg_eigenvalues run by a whole (converged) warp on a matrix in the warp's shared memory. Every lane
-// holds the same scalars and follows the same control flow; the independent operations of a step run on
-// different lanes of one instruction: the deflation tests of every row, the three (or five) divisions by the
-// scale (or by s and p), the three squares of the norm, one column of the row modification, one row of the
-// column modification. On GB300 an FP64 instruction occupies the sub-partition's FP64 unit for the same time
-// with one active lane or many, so a step costs a fraction of the scalar chain. Each value goes through the
-// same operations in the same order as in the scalar version, so the eigenvalues are identical.
+// hessenberg_eigenvalues run by a whole (converged) warp, the matrix in registers: lane 4 i + j (and its copy 16
+// lanes on) holds element (i, j), lane q of a group of four returns eigenvalue q. Every lane holds the same scalars
+// and follows the same control flow; the independent operations of a step run on different lanes of one
+// instruction: the deflation tests of every row, the three (or five) divisions by the scale (or by s and p), the
+// three squares of the norm, the row and the column modification of every element. On GB300 an FP64 instruction
+// occupies the sub-partition's FP64 unit for the same time with one active lane or many, so a step costs a
+// fraction of the scalar chain. Each value goes through the same operations in the same order as in the scalar
+// version, so the eigenvalues are identical.
+//
+// Bound by the latency of that chain (one contact's solve on the critical path of the sweep). Divisions and square
+// roots, half of it on the FP64 unit, run on the integer pipe; the sign, zero and equality tests are integer
+// comparisons; elements are exchanged by shuffles (no shared memory and its barriers).
 __device__ __forceinline__ double warp_bcast(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ bool nonnegative(double v) { return ipipe::to_bits(v) <= kSign; }  // v >= 0 (not NaN)
+// a == b for a, b >= 0 (or NaN, which equals nothing)
+__device__ __forceinline__ bool equal_nonneg(double a, double b) {
+  return ipipe::to_bits(a) == ipipe::to_bits(b) && abs_bits(a) <= kInfBits;
+}
 
-__device__ inline int hessenberg_eigenvalues_warp(double* a, int n, double* wr, double* wi) {
-#define BG_A(i, j) a[(i) * n + (j)]
+__device__ inline int hessenberg_eigenvalues_warp(double av, int n, double& wr, double& wi) {
   const int lane = threadIdx.x & 31;
-  double anorm = 0.0;
-  for (int i = 0; i < n; ++i)
-    for (int j = (i > 0 ? i - 1 : 0); j < n; ++j) anorm += fabs(BG_A(i, j));
+  const int row = (lane >> 2) & 3, col = lane & 3;
+  const double a0 = av;
+  auto at = [&](int i, int j) { return __shfl_sync(0xffffffffu, av, 4 * i + j); };
   int nn = n - 1;
   double t = 0.0;
   int total = 0;
+  wr = wi = 0.0;
   while (nn >= 0) {
     int its = 0, l;
     for (;;) {
-      {  // lane c tests l = c + 1; the scalar search stops at the largest l that passes (0 when none does)
-        const int L = lane + 1;
-        bool pass = false;
-        if (L <= nn) {
-          double s = fabs(BG_A(L - 1, L - 1)) + fabs(BG_A(L, L));
-          if (s == 0.0) s = anorm;
-          pass = fabs(BG_A(L, L - 1)) + s == s;
+      {  // lane group c tests l = c + 1; the scalar search stops at the largest l that passes (0 when none does)
+        const int L = min(col + 1, 3);
+        const double d0 = at(L - 1, L - 1), d1 = at(L, L), sub = at(L, L - 1);
+        double s = fabs(d0) + fabs(d1);
+        if (__any_sync(0xffffffffu, lane < nn && !nonzero(s))) {  // rare: the norm of the initial matrix, in the scalar order
+          double anorm = 0.0;
+          for (int i = 0; i < n; ++i)
+            for (int j = (i > 0 ? i - 1 : 0); j < n; ++j) anorm += fabs(__shfl_sync(0xffffffffu, a0, 4 * i + j));
+          if (!nonzero(s)) s = anorm;
         }
+        const bool pass = lane < nn && equal_nonneg(fabs(sub) + s, s);
         const unsigned m = __ballot_sync(0xffffffffu, pass);
         l = m ? 32 - __clz((int)m) : 0;
-        __syncwarp();
-        if (l >= 1 && lane == 0) BG_A(l, l - 1) = 0.0;
-        __syncwarp();
+        if (l >= 1 && row == l && col == l - 1) av = 0.0;
       }
-      double x = BG_A(nn, nn);
+      double x = at(nn, nn);
       if (l == nn) {
-        wr[nn] = x + t;
-        wi[nn] = 0.0;
+        if (col == nn) {
+          wr = x + t;
+          wi = 0.0;
+        }
         --nn;
         break;
       }
-      double y = BG_A(nn - 1, nn - 1);
-      double w = BG_A(nn, nn - 1) * BG_A(nn - 1, nn);
+      double y = at(nn - 1, nn - 1);
+      double w = at(nn, nn - 1) * at(nn - 1, nn);
       if (l == nn - 1) {
         const double p = 0.5 * (y - x);
         const double q = p * p + w;
-        double z = sqrt(fabs(q));
+        double z = ipipe::sqrt_rn(absd(q));
         x += t;
-        if (q >= 0.0) {
-          z = p + (p >= 0.0 ? fabs(z) : -fabs(z));
-          wr[nn - 1] = wr[nn] = x + z;
-          if (z != 0.0) wr[nn] = x - w / z;
-          wi[nn - 1] = wi[nn] = 0.0;
+        double w0, w1, i0, i1;
+        if (nonnegative(q)) {
+          z = p + (nonnegative(p) ? z : neg(z));
+          w0 = w1 = x + z;
+          if (nonzero(z)) w1 = x - ipipe::div_rn(w, z);
+          i0 = i1 = 0.0;
         } else {
-          wr[nn - 1] = wr[nn] = x + p;
-          wi[nn - 1] = -z;
-          wi[nn] = z;
+          w0 = w1 = x + p;
+          i0 = neg(z);
+          i1 = z;
+        }
+        if (col == nn - 1) {
+          wr = w0;
+          wi = i0;
+        }
+        if (col == nn) {
+          wr = w1;
+          wi = i1;
         }
         nn -= 2;
         break;
@@ -310,163 +394,136 @@ __device__ inline int hessenberg_eigenvalues_warp(double* a, int n, double* wr, 
       if (its == 30 || total >= 40 * n) return -1;
       if (its == 10 || its == 20) {
         t += x;
-        __syncwarp();
-        if (lane <= nn) BG_A(lane, lane) -= x;
-        __syncwarp();
-        const double s = fabs(BG_A(nn, nn - 1)) + fabs(BG_A(nn - 1, nn - 2));
+        if (row == col && row <= nn) av -= x;
+        const double s = fabs(at(nn, nn - 1)) + fabs(at(nn - 1, nn - 2));
         x = y = 0.75 * s;
         w = -0.4375 * s * s;
       }
       ++its;
       ++total;
       int m;
-      double p = 0, q = 0, r = 0, z;
+      double p, q, r;
       {
         // The scalar search tries m = nn - 2, nn - 3, ..., l and stops at the first m that passes its test (m = l
-        // always does). Candidate values do not depend on one another: lane group g (lanes 3g..3g+2) evaluates
-        // m = nn - 2 - g, lane 3g + c normalising component c; the search's m is the first group that passes.
-        const int g = lane / 3, c = lane - 3 * g;
-        const bool valid = lane < 30 && nn - 2 - g >= l;
+        // always does); n <= 4 leaves at most the two candidates nn - 2 and nn - 3. Their values do not depend on
+        // one another: lane group g (lanes 4g .. 4g + 3) evaluates m = nn - 2 - g, lane 4g + c normalising
+        // component c; the search's m is the first group that passes.
+        const int g = (lane >> 2) & 1, c = lane & 3;
+        const bool valid = nn - 2 - g >= l;
         const int mc = valid ? nn - 2 - g : l;
-        const double zc = BG_A(mc, mc);
+        const int mb = mc > 0 ? mc - 1 : 0;
+        const double zc = at(mc, mc), d1 = at(mc + 1, mc + 1), sub = at(mc + 1, mc), sup = at(mc, mc + 1);
+        const double rc = at(mc + 2, mc + 1), below = at(mc, mb), db = at(mb, mb);
         const double rr = x - zc;
         const double ss = y - zc;
-        const double pc = (rr * ss - w) / BG_A(mc + 1, mc) + BG_A(mc, mc + 1);
-        const double qc = BG_A(mc + 1, mc + 1) - zc - rr - ss;
-        const double rc = BG_A(mc + 2, mc + 1);
+        const double pc = ipipe::div_rn(rr * ss - w, sub) + sup;
+        const double qc = d1 - zc - rr - ss;
         const double sc = fabs(pc) + fabs(qc) + fabs(rc);
-        const double vn = (c == 0 ? pc : (c == 1 ? qc : rc)) / sc;
-        const int g0 = lane < 30 ? 3 * g : 0;
+        const double vn = ipipe::div_rn(c == 0 ? pc : (c == 1 ? qc : rc), sc);
+        const int g0 = 4 * g;
         const double pn = __shfl_sync(0xffffffffu, vn, g0);
         const double qn = __shfl_sync(0xffffffffu, vn, g0 + 1);
         const double rn = __shfl_sync(0xffffffffu, vn, g0 + 2);
         bool stop = valid && mc == l;
-        if (valid && mc != l) {
-          const double u = fabs(BG_A(mc, mc - 1)) * (fabs(qn) + fabs(rn));
-          const double v = fabs(pn) * (fabs(BG_A(mc - 1, mc - 1)) + fabs(zc) + fabs(BG_A(mc + 1, mc + 1)));
-          stop = u + v == v;
+        if (nn - 2 > l) {  // the first candidate is not l: its test decides
+          const double u = fabs(below) * (fabs(qn) + fabs(rn));
+          const double v = fabs(pn) * (fabs(db) + fabs(zc) + fabs(d1));
+          if (valid && mc != l) stop = equal_nonneg(u + v, v);
         }
-        const unsigned hit = __ballot_sync(0xffffffffu, stop && c == 0);
-        const int src = __ffs((int)hit) - 1;  // the leader lane of the first group that stops
-        m = nn - 2 - src / 3;
+        const unsigned hit = __ballot_sync(0xffffffffu, stop) & 0x11u;  // the groups' leaders
+        const int src = __ffs((int)hit) - 1;
+        m = nn - 2 - src / 4;
         p = __shfl_sync(0xffffffffu, pn, src);
         q = __shfl_sync(0xffffffffu, qn, src);
         r = __shfl_sync(0xffffffffu, rn, src);
-        z = __shfl_sync(0xffffffffu, zc, src);
       }
-      __syncwarp();
-      {
-        const int i = m + 2 + lane;
-        if (i <= nn) {
-          BG_A(i, i - 2) = 0.0;
-          if (i != m + 2) BG_A(i, i - 3) = 0.0;
-        }
-      }
-      __syncwarp();
+      if (row >= m + 2 && row <= nn && (col == row - 2 || (row != m + 2 && col == row - 3))) av = 0.0;
       for (int k = m; k <= nn - 1; ++k) {
+        const bool three = k != nn - 1;  // the reflection has a third component
+        const int k2 = three ? k + 2 : k + 1;
+        double comp;  // p, q or r by lane
         if (k != m) {
-          p = BG_A(k, k - 1);
-          q = BG_A(k + 1, k - 1);
-          r = 0.0;
-          if (k != nn - 1) r = BG_A(k + 2, k - 1);
+          p = at(k, k - 1);
+          q = at(k + 1, k - 1);
+          r = three ? at(k2, k - 1) : 0.0;
           x = fabs(p) + fabs(q) + fabs(r);
-          if (x != 0.0) {
-            const double v = (lane == 0 ? p : (lane == 1 ? q : r)) / x;
-            p = warp_bcast(v, 0);
-            q = warp_bcast(v, 1);
-            r = warp_bcast(v, 2);
+          comp = col == 0 ? p : (col == 1 ? q : r);
+          if (nonzero(x)) {
+            comp = ipipe::div_rn(comp, x);
+            p = warp_bcast(comp, 0);
+            q = warp_bcast(comp, 1);
+            r = warp_bcast(comp, 2);
           }
+        } else {
+          comp = col == 0 ? p : (col == 1 ? q : r);
         }
+        // the rows' elements of this lane's column, read while the norm and the divisions run
+        const double rk = at(k, col), rk1 = at(k + 1, col), rk2 = at(k2, col);
         double nrm;
         {  // sqrt(p * p + q * q + r * r), evaluated as (p*p + q*q) + r*r
-          const double c = lane == 0 ? p : (lane == 1 ? q : r);
-          const double sq = c * c;
-          nrm = sqrt((warp_bcast(sq, 0) + warp_bcast(sq, 1)) + warp_bcast(sq, 2));
+          const double sq = comp * comp;
+          nrm = ipipe::sqrt_rn((warp_bcast(sq, 0) + warp_bcast(sq, 1)) + warp_bcast(sq, 2));
         }
-        const double s = (p >= 0.0 ? nrm : -nrm);
-        if (s != 0.0) {
-          __syncwarp();
-          if (lane == 0) {
-            if (k == m) {
-              if (l != m) BG_A(k, k - 1) = -BG_A(k, k - 1);
-            } else {
-              BG_A(k, k - 1) = -s * x;
-            }
+        const double s = nonnegative(p) ? nrm : neg(nrm);
+        if (nonzero(s)) {
+          if (k == m) {
+            if (l != m && row == k && col == k - 1) av = neg(av);
+          } else {
+            if (row == k && col == k - 1) av = -s * x;
           }
           p += s;
+          double y1, z1;
           {  // x = p / s, y = q / s, z = r / s, q = q / p, r = r / p
-            const double num = lane == 0 ? p : (lane == 1 || lane == 3 ? q : r);
-            const double v = num / (lane < 3 ? s : p);
+            const int c8 = lane & 7;
+            const double num = c8 == 0 ? p : (c8 == 1 || c8 == 3 ? q : r);
+            const double v = ipipe::div_rn(num, c8 < 3 ? s : p);
             x = warp_bcast(v, 0);
-            y = warp_bcast(v, 1);
-            z = warp_bcast(v, 2);
+            y1 = warp_bcast(v, 1);
+            z1 = warp_bcast(v, 2);
             q = warp_bcast(v, 3);
             r = warp_bcast(v, 4);
           }
-          __syncwarp();
-          // Row and column modifications: lane 4u + c takes column (row) c of the step and, once every lane has
-          // read the old values, applies the u-th of its three independent updates; the updates are selected
-          // without branching, so the three run as one instruction stream (x 1.0 is exact: a - p * 1.0 = a - p).
-          const int c4 = lane & 3, u4 = lane >> 2;
-          {  // row modification, column j = k + c4
-            const int j = k + c4;
-            const bool on = lane < 12 && j <= nn;
-            double pj = 0.0;
-            if (on) {
-              pj = BG_A(k, j) + q * BG_A(k + 1, j);
-              if (k != nn - 1) pj += r * BG_A(k + 2, j);
-            }
-            __syncwarp();
-            if (on && (u4 != 0 || k != nn - 1)) {
-              const int row = k + 2 - u4;
-              const double f = u4 == 0 ? z : (u4 == 1 ? y : x);
-              BG_A(row, j) -= pj * f;
-            }
+          {  // row modification: rows k, k + 1, k + 2 of columns k .. nn
+            double pj = rk + q * rk1;
+            if (three) pj += r * rk2;
+            const double f = row == k ? x : (row == k + 1 ? y1 : z1);
+            if (col >= k && col <= nn && row >= k && row <= k2) av -= pj * f;
           }
-          __syncwarp();
           const int mmin = nn < k + 3 ? nn : k + 3;
-          {  // column modification, row i = l + c4
-            const int i = l + c4;
-            const bool on = lane < 12 && i <= mmin;
-            double pi = 0.0;
-            if (on) {
-              pi = x * BG_A(i, k) + y * BG_A(i, k + 1);
-              if (k != nn - 1) pi += z * BG_A(i, k + 2);
-            }
-            __syncwarp();
-            if (on && (u4 != 0 || k != nn - 1)) {
-              const int col = k + 2 - u4;
-              const double f = u4 == 0 ? r : (u4 == 1 ? q : 1.0);
-              BG_A(i, col) -= pi * f;
-            }
+          {  // column modification: columns k, k + 1, k + 2 of rows l .. mmin (x 1.0 is exact: a - p * 1.0 = a - p)
+            const double ck = at(row, k), ck1 = at(row, k + 1), ck2 = at(row, k2);
+            double pi = x * ck + y1 * ck1;
+            if (three) pi += z1 * ck2;
+            const double f = col == k ? 1.0 : (col == k + 1 ? q : r);
+            if (row >= l && row <= mmin && col >= k && col <= k2) av -= pi * f;
           }
-          __syncwarp();
         }
       }
     }
   }
   return 0;
-#undef BG_A
 }
 #endif
 
-// Eigenvalues of the companion matrix of the monic polynomial c[0] + c[1] t + ... + t^dim. Warp: the whole
-// warp runs hessenberg_eigenvalues_warp on the matrix in sa (its shared memory, dim * dim doubles).
+// Eigenvalues of the companion matrix of the monic polynomial c[0] + c[1] t + ... + t^dim (dim <= 4). Warp: called
+// by a whole converged warp with identical arguments.
 template <bool Warp>
-BG_HD int companion_eigenvalues(const double* c, int dim, double* wr, double* wi, double* sa) {
+BG_HD int companion_eigenvalues(const double* c, int dim, double* wr, double* wi) {
 #ifdef __CUDA_ARCH__
   if constexpr (Warp) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-    for (int e = lane; e < dim * dim; e += 32) {
-      const int i = e / dim, j = e - (e / dim) * dim;
-      sa[e] = (j == dim - 1) ? -c[i] : (j == i - 1 ? 1.0 : 0.0);
+    const int lane = threadIdx.x & 31, i = (lane >> 2) & 3, j = lane & 3;
+    const double ci = i == 0 ? c[0] : (i == 1 ? c[1] : (i == 2 ? c[2] : c[3]));
+    const double av = (i < dim && j == dim - 1) ? -ci : ((i < dim && j == i - 1) ? 1.0 : 0.0);
+    double vr, vi;
+    const int e = hessenberg_eigenvalues_warp(av, dim, vr, vi);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      wr[q] = warp_bcast(vr, q);
+      wi[q] = warp_bcast(vi, q);
     }
-    __syncwarp();
-    return hessenberg_eigenvalues_warp(sa, dim, wr, wi);
+    return e;
   }
 #endif
-  (void)sa;
   double a[16];
   for (int i = 0; i < dim * dim; ++i) a[i] = 0.0;
   for (int i = 1; i < dim; ++i) a[i * dim + (i - 1)] = 1.0;
@@ -475,9 +532,9 @@ BG_HD int companion_eigenvalues(const double* c, int dim, double* wr, double* wi
 }
 
 template <bool Warp = false>
-BG_HD int real_roots_monic(const double* c, int dim, double* roots, int filter, double* sa = nullptr) {
+BG_HD int real_roots_monic(const double* c, int dim, double* roots, int filter) {
   double wr[4], wi[4];
-  if (companion_eigenvalues<Warp>(c, dim, wr, wi, sa) != 0) return 0;
+  if (companion_eigenvalues<Warp>(c, dim, wr, wi) != 0) return 0;
   int count = 0;
   for (int i = 0; i < dim; ++i) {
     if (is_zero(wi[i])) {
@@ -489,15 +546,15 @@ BG_HD int real_roots_monic(const double* c, int dim, double* roots, int filter, 
 }
 
 template <bool Warp = false>
-BG_HD int real_roots_degenerate(double* c, int dim, double* roots, int filter, double* sa = nullptr) {
+BG_HD int real_roots_degenerate(double* c, int dim, double* roots, int filter) {
   while (dim > 0 && is_zero(c[dim])) --dim;
   if (dim == 0) {
     roots[0] = 0.0;
     return (filter == kAllRoots && is_zero(c[0])) ? 1 : 0;
   }
-  const double inv = 1.0 / c[dim];
+  const double inv = ipipe::div_rn(1.0, c[dim]);
   for (int k = 0; k < dim; ++k) c[k] *= inv;
-  return real_roots_monic<Warp>(c, dim, roots, filter, sa);
+  return real_roots_monic<Warp>(c, dim, roots, filter);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -510,24 +567,17 @@ BG_HD void fb_canonical(const double* x, const double* y, double* fb, double* dx
   z2[1] = fma(x[0], x[1], y[0] * y[1]);
   z2[2] = fma(x[0], x[2], y[0] * y[2]);
   const double nz2t = norm2(z2[1], z2[2]);
-  double om1[3], om2[3];
-  om1[0] = om2[0] = 0.5;
+  // the second eigenvector's tangential part; the first's is its opposite
+  const double inv = ipipe::div_rn(1.0, nz2t);
+  double o1 = ipipe::scale2<-1>(z2[1] * inv), o2 = ipipe::scale2<-1>(z2[2] * inv);
   if (is_zero(nz2t)) {
-    om1[1] = -0.5; om1[2] = 0.0;
-    om2[1] = 0.5;  om2[2] = 0.0;
-  } else {
-    const double inv = ipipe::div_rn(1.0, nz2t);
-    const double t1 = z2[1] * inv, t2 = z2[2] * inv;
-    om2[1] = ipipe::scale2<-1>(t1);  om2[2] = ipipe::scale2<-1>(t2);
-    om1[1] = -om2[1]; om1[2] = -om2[2];  // -0.5 t == -(0.5 t) exactly
+    o1 = 0.5;
+    o2 = 0.0;
   }
   const double nz2t2 = ipipe::scale2<1>(nz2t);
-  const double l1 = z2[0] - nz2t2;
-  const double rl1 = ipipe::sqrt_rn(l1 > 0.0 ? l1 : 0.0);
+  const double rl1 = ipipe::sqrt_rn(positive_part(z2[0] - nz2t2));
   const double rl2 = ipipe::sqrt_rn(z2[0] + nz2t2);
-  double z[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) z[k] = fma(rl2, om2[k], rl1 * om1[k]);
+  const double z[3] = {fma(rl2, 0.5, ipipe::scale2<-1>(rl1)), fma(rl2, o1, -(rl1 * o1)), fma(rl2, o2, -(rl1 * o2))};
 #pragma unroll
   for (int k = 0; k < 3; ++k) fb[k] = (x[k] + y[k]) - z[k];
   if (!Jac) return;
@@ -623,7 +673,7 @@ BG_HD void fb_law(bool desaxce, double mu, const double* x, const double* y, dou
 
 // SOCLaw::eval: |fb|^2, |y|^2 when mu < 0
 BG_HD double law_eval(bool desaxce, double mu, const double* x, const double* y) {
-  if (mu < 0) return sq3(y);
+  if (negative(mu)) return sq3(y);
   double fb[3];
   fb_law(desaxce, mu, x, y, fb);
   return sq3(fb);
@@ -633,9 +683,9 @@ BG_HD double law_eval(bool desaxce, double mu, const double* x, const double* y)
 BG_HD void project_cone(double mu, double* x) {
   const double nxt = norm2(x[1], x[2]);
   const double xn = x[0];
-  if (mu < 0) { x[0] = x[1] = x[2] = 0.0; return; }
-  if (nxt <= mu * xn) return;
-  if (mu * nxt <= -xn) { x[0] = x[1] = x[2] = 0.0; return; }
+  if (negative(mu)) { x[0] = x[1] = x[2] = 0.0; return; }
+  if (leq_from_zero(nxt, mu * xn)) return;
+  if (leq_from_zero(mu * nxt, neg(xn))) { x[0] = x[1] = x[2] = 0.0; return; }
   const double den2 = fma(mu, mu, 1.0);
   const double proj = ipipe::div_rn(fma(mu, nxt, xn), den2);
   x[0] = proj;
@@ -680,7 +730,7 @@ struct LocalFB {
     double dy[9];
     fb_mu_jacobian(mu, xs, y, fb, dFdx, dy);
     if (desaxce && !is_zero(s)) {
-      const double c = mu / s;
+      const double c = ipipe::div_rn(mu, s);
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
         const double t = dy[3 * r] * c;
@@ -733,7 +783,7 @@ BG_HD double newton_solve(const LocalFB& f, double tol, double* x) {
     for (int k = 0; k < 3; ++k) dPhi[k] = fma(dF[6 + k], x[2], fma(dF[3 + k], x[1], dF[k] * x[0]));
     SmallLU<3> lu;
     lu.compute(dF);
-    const double mF[3] = {-F[0], -F[1], -F[2]};
+    const double mF[3] = {neg(F[0]), neg(F[1]), neg(F[2])};
     double dx[3];
     lu.solve(mF, dx);
     const double proj = dot3(dx, dPhi);
@@ -747,18 +797,18 @@ BG_HD double newton_solve(const LocalFB& f, double tol, double* x) {
 }
 
 template <bool Warp = false>
-BG_HD bool analytic_coulomb(const double* W, const double* b, double* r, double mu, double* sa = nullptr) {
+BG_HD bool analytic_coulomb(const double* W, const double* b, double* r, double mu) {
   const double wN = W[0];
   if (wN < kEps) return false;
   const double wT0 = W[3], wT1 = W[6];
   const double bN = b[0];
-  const double inv_wN = 1.0 / wN;
+  const double inv_wN = ipipe::div_rn(1.0, wN);
   const double wTwN0 = wT0 * inv_wN, wTwN1 = wT1 * inv_wN;
   const double Wb00 = fma(-wTwN0, wT0, W[4]);
   const double Wb01 = fma(-wTwN0, wT1, W[5]);
   const double Wb10 = fma(-wTwN1, wT0, W[7]);
   const double Wb11 = fma(-wTwN1, wT1, W[8]);
-  const double inv_bN = 1.0 / bN;
+  const double inv_bN = ipipe::div_rn(1.0, bN);
   const double bb0 = b[1] * inv_bN - wTwN0;
   const double bb1 = b[2] * inv_bN - wTwN1;
   const double A = (Wb00 + Wb11) - dot2(wT0, wT1, bb0, bb1);
@@ -766,14 +816,14 @@ BG_HD bool analytic_coulomb(const double* W, const double* b, double* r, double 
   const double B1 = Wb00 * bb1 - Wb01 * bb0;
   const double det = Wb00 * Wb11 - Wb10 * Wb01;
   const double C = det - dot2(wT0, wT1, B0, B1);
-  const double D = (wN * wN) / (mu * mu);
+  const double D = ipipe::div_rn(wN * wN, mu * mu);
   double coeffs[4];
   coeffs[0] = C * C - D * dot2(B0, B1, B0, B1);
   coeffs[1] = 2.0 * (C * A - D * dot2(bb0, bb1, B0, B1));
   coeffs[2] = (2.0 * C + A * A) - D * dot2(bb0, bb1, bb0, bb1);
   coeffs[3] = 2.0 * A;
   double roots[4];
-  const int nRoots = real_roots_monic<Warp>(coeffs, 4, roots, kStrictlyPositiveRoots, sa);
+  const int nRoots = real_roots_monic<Warp>(coeffs, 4, roots, kStrictlyPositiveRoots);
   if (nRoots == 0) return false;
   double alpha = roots[0];
   for (int i = 1; i < nRoots; ++i)
@@ -786,12 +836,12 @@ BG_HD bool analytic_coulomb(const double* W, const double* b, double* r, double 
   lu.solve(rhs, rt);
   r[1] = rt[0];
   r[2] = rt[1];
-  r[0] = norm2(rt[0], rt[1]) / mu;
+  r[0] = ipipe::div_rn(norm2(rt[0], rt[1]), mu);
   return true;
 }
 
 template <bool Warp = false>
-BG_HD bool analytic_soc(const double* W, const double* b, double* r, double mu, double* sa = nullptr) {
+BG_HD bool analytic_soc(const double* W, const double* b, double* r, double mu) {
 #define BG_W(i, j) W[3 * (i) + (j)]
   const double A = ((b[1] * BG_W(1, 2) - b[2] * BG_W(1, 1)) * mu * mu + b[0] * BG_W(0, 2)) - b[2] * BG_W(0, 0);
   const double B = ((b[0] * BG_W(1, 2) + b[1] * BG_W(0, 2)) - 2.0 * b[2] * BG_W(0, 1)) * mu;
@@ -800,12 +850,12 @@ BG_HD bool analytic_soc(const double* W, const double* b, double* r, double mu, 
   const double E = -6.0 * (b[0] * BG_W(1, 2) - b[1] * BG_W(0, 2)) * mu;
   double coeffs[5] = {A + B, C - D, E, C + D, B - A};
   double roots[4];
-  const int nRoots = real_roots_degenerate<Warp>(coeffs, 4, roots, kAllRoots, sa);
+  const int nRoots = real_roots_degenerate<Warp>(coeffs, 4, roots, kAllRoots);
   for (int i = 0; i < nRoots; ++i) {
     const double t = roots[i];
     const double den = 1.0 + t * t;
-    const double CT = (1.0 - t * t) / den;
-    const double ST = (2.0 * t) / den;
+    const double CT = ipipe::div_rn(1.0 - t * t, den);
+    const double ST = ipipe::div_rn(2.0 * t, den);
     const double dir[3] = {1.0, mu * CT, mu * ST};
     const double v0[3] = {mu * BG_W(0, 1) + CT * BG_W(0, 0), mu * BG_W(1, 1) + CT * BG_W(1, 0), mu * BG_W(2, 1) + CT * BG_W(2, 0)};
     const double v1[3] = {mu * BG_W(0, 2) + ST * BG_W(0, 0), mu * BG_W(1, 2) + ST * BG_W(1, 0), mu * BG_W(2, 2) + ST * BG_W(2, 0)};
@@ -814,10 +864,10 @@ BG_HD bool analytic_soc(const double* W, const double* b, double* r, double mu, 
     double rN;
     if (fabs(den0) > fabs(den1)) {
       if (is_zero(den0)) continue;
-      rN = -(CT * b[0] + b[1] * mu) / den0;
+      rN = ipipe::div_rn(-(CT * b[0] + b[1] * mu), den0);
     } else {
       if (is_zero(den1)) continue;
-      rN = -(ST * b[0] + b[2] * mu) / den1;
+      rN = ipipe::div_rn(-(ST * b[0] + b[2] * mu), den1);
     }
     if (rN <= 0) continue;
     r[0] = rN * dir[0];
@@ -834,15 +884,14 @@ BG_HD bool analytic_soc(const double* W, const double* b, double* r, double mu, 
 enum { kPureNewton = 0, kPureEnumerative = 1, kHybrid = 2, kRevHybrid = 3 };
 
 // LocalSOCSolver<3, double, DeSaxce, Strat>::solve (mu < 0: full-pivoting LU solve of A x = -b)
-// Warp: called by a whole converged warp with identical arguments (every lane computes the same values; the
-// companion-matrix eigenvalues use the warp's shared scratch sa, 16 doubles).
+// Warp: called by a whole converged warp with identical arguments (every lane computes the same values).
 template <bool Warp = false>
 BG_HD double local_solve(bool desaxce, int strat, const double* A, const double* b, double* x, double mu, double tol,
-                         double scaling, double* sa = nullptr) {
+                         double scaling) {
   if (mu < 0) {
     SmallLU<3> lu;
     lu.compute(A);
-    const double mb[3] = {-b[0], -b[1], -b[2]};
+    const double mb[3] = {neg(b[0]), neg(b[1]), neg(b[2])};
     lu.solve(mb, x);
     double ax[3];
     matvec3(A, x, ax);
@@ -862,7 +911,7 @@ BG_HD double local_solve(bool desaxce, int strat, const double* A, const double*
       return b[0] * b[0];
     }
     x[1] = x[2] = 0.0;
-    x[0] = (-b[0]) / A[0];
+    x[0] = ipipe::div_rn(neg(b[0]), A[0]);
     return 0.0;
   }
   double res = 0.0;
@@ -874,11 +923,11 @@ BG_HD double local_solve(bool desaxce, int strat, const double* A, const double*
   {
     SmallLU<3> lu;
     lu.compute(A);
-    const double mb[3] = {-b[0], -b[1], -b[2]};
+    const double mb[3] = {neg(b[0]), neg(b[1]), neg(b[2])};
     lu.solve(mb, x);
   }
   if (mu * x[0] >= norm2(x[1], x[2])) return 0.0;
-  const bool ok = desaxce ? analytic_coulomb<Warp>(A, b, x, mu, sa) : analytic_soc<Warp>(A, b, x, mu, sa);
+  const bool ok = desaxce ? analytic_coulomb<Warp>(A, b, x, mu) : analytic_soc<Warp>(A, b, x, mu);
   if (!ok) { x[0] = x0[0]; x[1] = x0[1]; x[2] = x0[2]; }
   if (strat == kRevHybrid) {
     res = newton_solve(fb, tol, x);
@@ -892,17 +941,17 @@ BG_HD double local_solve(bool desaxce, int strat, const double* A, const double*
 
 template <bool Warp = false>
 BG_HD bool law_solve_local(bool desaxce, int strat, const double* A, const double* b, double* x, double mu,
-                           double scaling, double* sa = nullptr) {
-  return kLocalTol > local_solve<Warp>(desaxce, strat, A, b, x, mu, kLocalTol, scaling, sa);
+                           double scaling) {
+  return kLocalTol > local_solve<Warp>(desaxce, strat, A, b, x, mu, kLocalTol, scaling);
 }
 
 BG_HD double nesterov_inertia(double& theta, double q) {
   const double theta_prev = theta;
   const double theta_p2 = theta_prev * theta_prev;
   const double bb = theta_p2 - q;
-  const double delta = sqrt(bb * bb + 4.0 * theta_p2);
-  theta = 0.5 * (delta - bb);
-  return (theta_prev - theta_p2) / (theta_p2 + theta);
+  const double delta = ipipe::sqrt_rn(bb * bb + 4.0 * theta_p2);
+  theta = ipipe::scale2<-1>(delta - bb);
+  return ipipe::div_rn(theta_prev - theta_p2, theta_p2 + theta);
 }
 
 // Smallest eigenvalue of a symmetric 3x3 block by cyclic Jacobi rotations (used for
