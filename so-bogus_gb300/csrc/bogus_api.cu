@@ -155,6 +155,7 @@ struct bogus_gpu_problem {
   DevBuf<long long> slot0;
   DevBuf<int> chunk_order;  // chunks by decreasing segment length (ticket order of the persistent solvers)
   std::vector<int> h_chunk_order;  // the same on the host
+  std::vector<int> h_chunk_seg;    // S of every chunk
   // per-CTA chunk lists of the single-problem kernel for a grid of cta_grid CTAs (0: none built)
   DevBuf<int> cta_ptr, cta_list;
   int cta_grid = 0;
@@ -431,7 +432,7 @@ int ensure_pg_work(bogus_gpu_problem* h, unsigned max_iters) {
   BG_CUDA(h->S0.ensure(n));
   BG_CUDA(h->XB.ensure(n3));
   BG_CUDA(h->Wv.ensure(n3));
-  BG_CUDA(h->csum.ensure(5 * (size_t)C));  // up to 5 reduced quantities (the Conjugated variant)
+  BG_CUDA(h->csum.ensure(8 * (size_t)C));  // up to 5 reduced quantities (the Conjugated variant), twice 4 when flat
   BG_CUDA(h->scal.ensure(8 + 40));         // scalars, then the stripe sums of grid_barrier_combine
   BG_CUDA(h->trace.ensure((size_t)max_iters + 1));
   BG_CUDA(h->pgout.ensure(1));
@@ -479,6 +480,17 @@ struct HyArgs {
   unsigned refresh;
   size_t stride;  // floats between the position buffers' corrections in d
 };
+
+// Grid of the single-problem kernel: one CTA per SM while its 8 warps take no more than a chunk each, then two, then
+// the resident maximum; never more CTAs than chunks.
+int pg_grid(int device, bool fp32, int nchunks) {
+  const int grid = pg_max_grid(device, fp32, true);
+  int sms = 0;
+  if (grid <= 0 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
+  int want = nchunks <= 8 * sms ? sms : (nchunks <= 16 * sms ? 2 * sms : grid);
+  want = std::min(want, nchunks);
+  return std::max(1, std::min(grid, want));
+}
 
 // Runs the persistent solver with r already in X[0]; returns the buffer holding the result. hy: FP64 iterations
 // with FP32 correction products (APGD; no callback: their residuals are those of the corrected products).
@@ -541,15 +553,32 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
   }
   BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 16 * sizeof(unsigned), h->stream));
   BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), h->stream));
-  int grid = pg_max_grid(h->device, false, true);
+  const bool sc = o->variant == BOGUS_GPU_PG_STANDARD || o->variant == BOGUS_GPU_PG_CONJUGATED;
+  int grid = 0, teams = 0, steps = 0;
+  bool resident = false;
+  if (!hy && !sc && !a.lin_momentum) {
+    int sms = 0;
+    BG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    grid = std::min(sms, a.nchunks);
+    teams = (a.nchunks + grid - 1) / grid;
+    for (int b = 0; b < grid; ++b) {  // the lists of ensure_cta_lists
+      int sum = 0;
+      for (int r = 0; r < teams; ++r) {
+        const int k = r * grid + ((r & 1) ? grid - 1 - b : b);
+        if (k < a.nchunks) sum += h->h_chunk_seg[h->h_chunk_order[k]];
+      }
+      steps = std::max(steps, sum);
+    }
+    resident = pg_resident_fits(h->device, teams, steps, h->h_chunk_seg[h->h_chunk_order[0]]);
+  }
+  if (!resident) grid = pg_grid(h->device, false, a.nchunks);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
-  const int want = (a.nchunks + 7) / 8;
-  if (want < grid) grid = want < 1 ? 1 : want;
+  a.flat = !sc && a.nchunks <= kFlatChunks;
   if (int e = ensure_cta_lists(h, grid)) return e;
   a.cta_ptr = h->cta_ptr.p;
   a.cta_list = h->cta_list.p;
   BG_CUDA(cudaEventRecord(h->ev0, h->stream));
-  BG_CUDA(launch_pg_persistent(a, grid, h->stream));
+  BG_CUDA(resident ? launch_pg_resident(a, grid, teams, steps, h->stream) : launch_pg_persistent(a, grid, h->stream));
   BG_CUDA(cudaEventRecord(h->ev1, h->stream));
   PGOut out{};
   int st = 0;
@@ -636,6 +665,7 @@ int ensure_interleaved(bogus_gpu_problem* h) {
   }
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return seg[x] > seg[y]; });
   h->h_chunk_order = order;
+  h->h_chunk_seg = seg;
   h->cta_grid = 0;
   BG_CUDA(h->chunk_order.ensure(C > 0 ? C : 1));
   if (C) BG_CUDA(cudaMemcpyAsync(h->chunk_order.p, order.data(), sizeof(int) * C, cudaMemcpyHostToDevice, h->stream));
@@ -739,10 +769,9 @@ int run_pg_mixed(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* re
   BG_CUDA(launch_convert(n3, h->X.p, h->X32.p, s));
   BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 16 * sizeof(unsigned), s));
   BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), s));
-  int grid = pg_max_grid(h->device, true, true);
+  const int grid = pg_grid(h->device, true, a.nchunks);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
-  const int want = (a.nchunks + 7) / 8;
-  if (want < grid) grid = want < 1 ? 1 : want;
+  a.flat = a.nchunks <= kFlatChunks;
   if (int e = ensure_cta_lists(h, grid)) return e;
   a.cta_ptr = h->cta_ptr.p;
   a.cta_list = h->cta_list.p;
@@ -3828,6 +3857,7 @@ int bogus_gpu_set_wait_limit(int device, double seconds) {
   BG_CUDA(cudaSetDevice(device));
   const unsigned long long ns = (unsigned long long)(seconds * 1e9);
   cudaError_t e = set_wait_limit_pg(ns);
+  if (e == cudaSuccess) e = set_wait_limit_pg_resident(ns);
   if (e == cudaSuccess) e = set_wait_limit_gs(ns);
   if (e == cudaSuccess) e = set_wait_limit_admm(ns);
   if (e == cudaSuccess) e = set_wait_limit_adjoint(ns);

@@ -520,6 +520,99 @@ __device__ __forceinline__ bool mono_barrier_combine(const MonoBarrier& mb, unsi
   return ok;
 }
 
+// ---- flat reducing barrier (problems of a few chunks per SM) ----------------------------------------------
+// Every CTA waits until all have arrived and then combines all chunk sums for itself, in the canonical order: one
+// round trip to L2 after the last arrival in place of the three (stripes, publication, scalars) of
+// mono_barrier_combine. The price is that every CTA repeats the additions (8 stripes x K ceil(C / 256) per SM) and
+// reads all chunk sums, so it pays while they are few (kFlatChunks). A CTA may already write the chunk sums of the
+// next phase while a slower one still reads these: the caller alternates between two buffers, and a CTA that
+// writes a buffer again has passed a barrier that every reader of it arrived at after reading.
+__device__ __forceinline__ void red_add_release_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// One thread, for its whole CTA: arrives at barrier k and returns once every CTA has (false after a wait that ran
+// out). No status word is read on the way out: a CTA whose wait runs out records it, and the others' waits then end
+// too.
+__device__ __forceinline__ bool flat_wait(const MonoBarrier& mb, unsigned k) {
+  red_add_release_u64(mb.mono, 1ull);
+  const unsigned long long target = (unsigned long long)mb.parties * (k + 1ull);
+  unsigned long long t0 = 0;
+  unsigned spins = 0;
+  while (ld_acquire_u64(mb.mono) < target) {
+    if ((++spins & 255u) != 0) continue;
+    if (ld_relaxed_i32(mb.status) != 0) return false;
+    const unsigned long long now = global_timer_ns();
+    if (t0 == 0) t0 = now;
+    else if (now - t0 > wait_limit_ns()) {
+      atomicCAS(mb.status, 0, (int)BOGUS_GPU_TIMEOUT);
+      return false;
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ bool flat_barrier(const MonoBarrier& mb, unsigned k) {
+  bool ok = true;
+  __syncthreads();
+  if (threadIdx.x == 0) ok = flat_wait(mb, k);
+  return __syncthreads_and(ok) != 0;
+}
+
+// The canonical reduction of K <= 4 quantities by one CTA of 8 warps (value q's sums at s + q * stride, count0
+// chunks for q = 0 and count1 for q > 0): warp k takes stripe k of every quantity, its butterflies sharing their
+// first steps (warp_sum2 / warp_sum4: the same tree per quantity); lane q of warp 0 adds quantity q's 8 stripe
+// sums. smem: 32 doubles; the totals in out[0..K) (shared), valid after the call.
+__device__ __forceinline__ void flat_combine(const double* s, size_t stride, int count0, int count1, int K,
+                                             unsigned maxmask, double* smem32, double* out) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double p[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (q >= K) continue;
+    const int C = q == 0 ? count0 : count1;
+    const int per = (C + 7) / 8, b = warp * per, e = min(C, b + per);
+    const double* sq = s + (size_t)q * stride;
+    const bool mx = (maxmask >> q) & 1u;
+    for (int c = b + lane; c < e; c += 128) {
+      double v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = c + 32 * u < e ? ldcg(sq + c + 32 * u) : 0.0;
+      // a chunk sum past the end adds nothing; the first of a lane is placed (0 + v, -0 becoming +0)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c + 32 * u < e) p[q] = mx ? ((v[u] < p[q]) ? p[q] : v[u]) : p[q] + v[u];
+    }
+  }
+  if (maxmask) {
+    for (int q = 0; q < K; ++q) {
+      const double v = ((maxmask >> q) & 1u) ? warp_max_butterfly(p[q]) : warp_sum_butterfly(p[q]);
+      if (lane == 0) smem32[8 * q + warp] = v;
+    }
+  } else if (K > 2) {
+    const double v = warp_sum4_butterfly(p[0], p[1], p[2], p[3]);
+    if ((lane & 7) == 0) smem32[lane + warp] = v;
+  } else if (K == 2) {
+    const double v = warp_sum2_butterfly(p[0], p[1]);
+    if ((lane & 15) == 0) smem32[lane / 2 + warp] = v;
+  } else {
+    const double v = warp_sum_butterfly(p[0]);
+    if (lane == 0) smem32[warp] = v;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < K) {
+    const int q = threadIdx.x;
+    const bool mx = (maxmask >> q) & 1u;
+    double total = smem32[8 * q];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+      const double v = smem32[8 * q + k];
+      total = mx ? ((v < total) ? total : v) : total + v;
+    }
+    out[q] = total;
+  }
+  __syncthreads();
+}
+
 // One warp: wait until reduction `published` - 1 is published (mono[2] >= published). Every lane of the warp
 // must call it; the lanes read the scalars after it returns.
 __device__ __forceinline__ bool mono_await(const MonoBarrier& mb, unsigned long long published) {

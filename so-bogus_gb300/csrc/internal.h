@@ -66,7 +66,8 @@ struct PGArgsT {
   T* S0;
   T* XB;
   T* Wv;          // SPG step w
-  double* csum;   // 4 * nchunks chunk sums
+  double* csum;   // 5 * nchunks chunk sums (4 are enough but for the Conjugated variant); twice 4 * nchunks when flat
+  int flat;       // single-problem kernel with chunk lists: reductions by the flat barrier (few chunks)
   double* scal;   // published scalars
   double* trace;  // residual per iteration (may be null)
   PGOut* out;
@@ -161,10 +162,19 @@ cudaError_t launch_expand_lower(int nnz, const int* src, const double* low, doub
 cudaError_t launch_add(int m, const double* a, const double* b, double* y, cudaStream_t s);
 cudaError_t launch_cadoux_rhs(int n, const double* y, const double* mu, const double* b, double* out, cudaStream_t s);
 
+// Problems of up to this many chunks reduce by the flat barrier. us per SPG iteration (two reductions) on GB300, stripes
+// combined by the last CTAs / flat: 500 contacts 41 / 26, 10 000 46 / 33, 40 000 (1 250 chunks) 65 / 50, the grid rule
+// (pg_grid) included. Every CTA repeats the additions, 8 C / 256 FP64 instructions per quantity and SM: 64 at 2 048
+// chunks, about the round trips saved.
+constexpr int kFlatChunks = 2048;
 // Persistent solvers (kernels_pg.cu)
 cudaError_t launch_pg_persistent(const PGArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_pg_persistent(const PGArgs32& a, int grid, cudaStream_t s);
 int pg_max_grid(int device, bool fp32 = false, bool interleaved = false);
+// Problems that fit the SMs' shared memory (kernels_pg_resident.cu): chunk lists for `ctas` CTAs of up to `teams`
+// chunks, `steps` the largest sum of S (spmv_chunk.cuh) over a CTA's chunks, `longest` the largest S
+bool pg_resident_fits(int device, int teams, int steps, int longest);
+cudaError_t launch_pg_resident(const PGArgs& a, int ctas, int teams, int steps, cudaStream_t s);
 cudaError_t launch_pg_batched(const PGBatchArgs& b, int grid, cudaStream_t s);
 cudaError_t launch_pg_batched(const PGBatchArgs32& b, int grid, cudaStream_t s);
 int pg_batched_grid(int device, bool fp32 = false);
@@ -352,6 +362,7 @@ cudaError_t launch_meche_h(int n, int d, const double* E, const double* HAw, con
 
 // Device-side wait limits (nanoseconds) of the kernel files, set on the current device.
 cudaError_t set_wait_limit_pg(unsigned long long ns);
+cudaError_t set_wait_limit_pg_resident(unsigned long long ns);
 cudaError_t set_wait_limit_gs(unsigned long long ns);
 cudaError_t set_wait_limit_admm(unsigned long long ns);
 cudaError_t set_wait_limit_adjoint(unsigned long long ns);

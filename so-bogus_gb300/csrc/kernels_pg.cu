@@ -171,7 +171,7 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
 
   auto put = [&](int q, int c, double v, bool is_max) {
     v = is_max ? warp_max_butterfly(v) : warp_sum_butterfly(v);
-    if (lane == 0) a.csum[q * C + c] = v;
+    if (lane == 0) ctx.csum()[q * C + c] = v;
   };
   // chunk sums of values 0 and 1 (value 0 the maximum when max0)
   auto put2 = [&](int c, double v0, double v1, bool max0) {
@@ -181,11 +181,11 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
       return;
     }
     const double v = warp_sum2_butterfly(v0, v1);
-    if ((lane & 15) == 0) a.csum[(lane >> 4) * C + c] = v;
+    if ((lane & 15) == 0) ctx.csum()[(lane >> 4) * C + c] = v;
   };
   auto put4 = [&](int c, double v0, double v1, double v2, double v3) {
     const double v = warp_sum4_butterfly(v0, v1, v2, v3);
-    if ((lane & 7) == 0) a.csum[(lane >> 3) * C + c] = v;
+    if ((lane & 7) == 0) ctx.csum()[(lane >> 3) * C + c] = v;
   };
   auto sync = [&]() -> bool { return ctx.sync(); };
   auto sync_reduce = [&](int K, unsigned maxmask) -> bool { return ctx.sync_reduce(K, maxmask); };
@@ -193,7 +193,8 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
   auto sync_reduce_split = [&](int K, unsigned maxmask) -> bool { return ctx.sync_reduce_split(K, maxmask); };
   auto scal = [&](int q) { return ctx.scal(q); };
   // ConstrainedSolverBase::eval: sum / (1 + n), or the maximum with the infinity norm
-  auto residual_of = [&](double reduced) { return a.use_inf ? reduced : reduced / (double)(1 + a.n); };
+  const double n_plus_1 = (double)(1 + a.n);
+  auto residual_of = [&](double reduced) { return a.use_inf ? reduced : ipipe::div_rn(reduced, n_plus_1); };
   unsigned ph[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   unsigned n_refresh = 0;  // HY: refreshes of x_ref
   auto finish = [&](double min_res, unsigned iters, int best_buf, int converged) -> int {
@@ -249,7 +250,7 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
   double alpha = 1.0;
   {
     const double nMx = scal(0);
-    if (nMx > 1.e-16) alpha = dmin(1., scal(1) / nMx);
+    if (nMx > 1.e-16) alpha = dmin(1., ipipe::div_rn(scal(1), nMx));
   }
   if (a.max_iters == 0) {
     return finish(-1.0, 0, 0, 0);
@@ -268,14 +269,14 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
     const T lx[3] = {x[0] * sc, x[1] * sc, x[2] * sc};
     res_i = Ops::law_eval(desaxce, mu, lx, y);
     const T s0 = Ops::cov(desaxce, mu, y);
-    y[0] = y[0] + s0;
+    y[0] = desaxce ? y[0] + s0 : Ops::plus0(y[0]);
     y[1] = Ops::plus0(y[1]);
     y[2] = Ops::plus0(y[2]);
     const T na = T(-alpha_t);
     T xs[3] = {fma(na, y[0], x[0]), fma(na, y[1], x[1]), fma(na, y[2], x[2])};
     Ops::project(mu, xs);
     store3(a.Y, i, y);
-    a.S0[i] = s0;
+    if (desaxce) a.S0[i] = s0;
     store3(B.X(ixs), i, xs);
     store_corr(ixs, i, xs);
     if (spg) {
@@ -284,7 +285,8 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
       const T d[3] = {xs[0] - pv[0], xs[1] - pv[1], xs[2] - pv[2]};
       second_i = Ops::dot3(d, y);
     } else {
-      const T t[3] = {(Ops::half(Mx[0]) + bb[0]) + s0, Ops::plus0(Ops::half(Mx[1]) + bb[1]),
+      const T t0 = Ops::half(Mx[0]) + bb[0];
+      const T t[3] = {desaxce ? t0 + s0 : Ops::plus0(t0), Ops::plus0(Ops::half(Mx[1]) + bb[1]),
                       Ops::plus0(Ops::half(Mx[2]) + bb[2])};
       second_i = Ops::dot3(x, t);
     }
@@ -378,7 +380,7 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
       const double res = residual_of(scal(0)), J = scal(1), s2 = scal(2);
       const double den_c = conj ? scal(3) : 0.0, xp = conj ? scal(4) : 0.0;
       if (a.trace && ctx.writer()) a.trace[it] = res;
-      if (it == 0 || res < min_res) {
+      if (it == 0 || less_from_zero(res, min_res)) {
         min_res = res;
         best_pending = true;
       }
@@ -534,11 +536,11 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
         res = residual_of(scal(0));
         J = scal(1);
         if (a.trace && ctx.writer()) a.trace[it] = res;
-        if (it == 0 || res < min_res) {
+        if (it == 0 || less_from_zero(res, min_res)) {
           min_res = res;
           best_pending = true;
         }
-        converged = res < a.tol;
+        converged = less_from_zero(res, a.tol);
         if (sizeof(T) == 4 && a.stall_iters) {
           stall_run = ((it > 0 && res == prev_res) || exhausted) ? stall_run + 1 : 0;
           prev_res = res;
@@ -578,8 +580,9 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
             load3cg(B.X(ixs), i, xs);
             load3cg(B.X(iprev), i, pv);
             load3cg(a.Y, i, y);
-            const T s0 = ldcg(a.S0 + i);
-            const T t[3] = {(Ops::half(acc[0]) + __ldg(a.b + 3 * i)) + s0, Ops::plus0(Ops::half(acc[1]) + __ldg(a.b + 3 * i + 1)),
+            const T t0 = Ops::half(acc[0]) + __ldg(a.b + 3 * i);
+            const T t[3] = {desaxce ? t0 + ldcg(a.S0 + i) : Ops::plus0(t0),
+                            Ops::plus0(Ops::half(acc[1]) + __ldg(a.b + 3 * i + 1)),
                             Ops::plus0(Ops::half(acc[2]) + __ldg(a.b + 3 * i + 2))};
             v0 = Ops::dot3(xs, t);
             const T d[3] = {xs[0] - x[0], xs[1] - x[1], xs[2] - x[2]};
@@ -611,7 +614,7 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
         if (!sync_reduce(4, 0u)) return -1;
         const double Js = scal(0), decr = scal(1), nrm = scal(2);
         decr2 = scal(3);
-        if (Js < (J + decr) + (.5 / alpha) * nrm) break;
+        if (Js < (J + decr) + ipipe::div_rn(.5, alpha) * nrm) break;
         ++ls;
         alpha *= a.pess;
         if (ls >= a.ls_iters) break;
@@ -635,7 +638,7 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
       if (sizeof(T) == 4) exhausted = ls > 0 && ls >= a.ls_iters;
       ++it;
       const bool more = it < a.max_iters;
-      if (apgd && decr2 < 0) {
+      if (apgd && negative(decr2)) {
         theta = theta_spec;  // nesterov_inertia(theta, 0) (:137), whose value beta_spec already holds
         const int nix = ispec, nprev = ixs;
         ix = nix;
@@ -711,11 +714,11 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
     if (!runA(alpha, false)) return -1;  // y, residual, s, xs = P(x - alpha y), (xs - prev).y
     const double res = residual_of(scal(0)), decr = scal(1);
     if (a.trace && ctx.writer()) a.trace[it] = res;
-    if (it == 0 || res < min_res) {
+    if (it == 0 || less_from_zero(res, min_res)) {
       min_res = res;
       best_pending = true;
     }
-    if (res < a.tol) {
+    if (less_from_zero(res, a.tol)) {
       return finish(min_res, it, best_pending ? ix : 3, 1);
     }
     if (sizeof(T) == 4 && a.stall_iters) {
@@ -723,7 +726,7 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
       prev_res = res;
       if (repeats >= a.stall_iters) return finish(min_res, it, best_pending ? ix : 3, 0);
     }
-    const bool mom = decr < 0.;
+    const bool mom = negative(decr);
     const double beta = mom ? nesterov_inertia(theta, 0.0) : 0.0;
     if (!mom) theta = 1.;
     // D: w and the new x (over the old x); keep the best iterate first
@@ -774,7 +777,7 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
     imx = 1 - imx;
     iprev = ixs;
     ixs = third(ix, iprev);
-    alpha = scal(0) / scal(1);
+    alpha = ipipe::div_rn(scal(0), scal(1));
     alpha = dmin(a_max, dmax(a_min, alpha));
     ++it;
     if (it >= a.max_iters) break;
@@ -797,6 +800,7 @@ template <class T>
 struct GridCtx {
   const PGArgsT<T>& a;
   double* smem8;
+  double* sscal;       // the scalars of the last flat reduction
   ChunkScratchT<T>* cs;
   unsigned* s_cnt;     // 2 shared-memory counters (phase parity) over the CTA's chunk list
   unsigned phase = 0;  // barriers passed (identical in every CTA)
@@ -827,14 +831,22 @@ struct GridCtx {
   }
   unsigned reductions = 0;  // reductions published or pending (identical in every CTA)
   bool pending = false;     // this warp has not yet waited for the last (split) reduction
+  __device__ double* csum() const { return a.csum + (a.flat ? (size_t)(phase & 1u) * 4 * a.nchunks : 0); }
   __device__ MonoBarrier mb() const { return MonoBarrier{a.mono, a.gb.status, gridDim.x + a.phantom_ctas}; }
   __device__ bool sync() {
-    const bool ok = mono_barrier(mb(), phase, [&] { clear_tickets(); });
+    const bool ok = a.flat ? flat_barrier(mb(), phase) : mono_barrier(mb(), phase, [&] { clear_tickets(); });
     reset_cta_counter();
     ++phase;
     return ok;
   }
   __device__ bool reduce(int K, unsigned maxmask, bool split) {
+    if (a.flat) {
+      if (!flat_barrier(mb(), phase)) return false;
+      flat_combine(csum(), (size_t)a.nchunks, a.nchunks, a.nchunks, K, maxmask, smem8, sscal);
+      reset_cta_counter();
+      ++phase;
+      return true;
+    }
     const bool ok = mono_barrier_combine(mb(), phase, reductions, split, a.csum, (size_t)a.nchunks, a.nchunks,
                                          a.nchunks, K, maxmask, a.stripes, a.scal, [&] { clear_tickets(); });
     reset_cta_counter();
@@ -850,7 +862,7 @@ struct GridCtx {
     pending = false;
     return mono_await(mb(), reductions);
   }
-  __device__ double scal(int q) const { return ldcg(a.scal + q); }
+  __device__ double scal(int q) const { return a.flat ? sscal[q] : ldcg(a.scal + q); }
 };
 
 // The solver body; the hybrid instantiation is inlined by force (the compiler's own choice outlines it, with
@@ -863,17 +875,13 @@ __device__ int pg_body(const PGArgsT<T>& a, Ctx& ctx) {
 // Occupancy target: 3 resident CTAs per SM (see pg_max_grid).
 template <class T, bool IL, bool SC = false, bool HY = false>
 __global__ void __launch_bounds__(256, 3) k_pg_persistent(PGArgsT<T> a) {
-  __shared__ double smem8[32];
+  __shared__ double smem8[32], sscal[4];
   __shared__ ChunkScratchT<T> cs[8];
   __shared__ unsigned s_cnt[2];
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0u;
   __syncthreads();
-  GridCtx<T> ctx{a, smem8, cs, s_cnt};
-  if constexpr (HY) {
-    pg_body_inl<T, IL, SC, HY>(a, ctx);
-  } else {
-    pg_body<T, IL, SC, HY>(a, ctx);
-  }
+  GridCtx<T> ctx{a, smem8, sscal, cs, s_cnt};
+  pg_body_inl<T, IL, SC, HY>(a, ctx);
 }
 
 // One problem per CTA (batched solves): phases separated by __syncthreads, scalars reduced by the CTA's
@@ -887,6 +895,7 @@ struct BlockCtx {
   __device__ int first_chunk() const { return threadIdx.x >> 5; }
   __device__ int next_chunk(int c) const { return c + 8; }
   __device__ bool writer() const { return threadIdx.x == 0; }
+  __device__ double* csum() const { return a.csum; }
   __device__ bool sync() {
     __syncthreads();
     return true;
@@ -983,6 +992,7 @@ struct TeamCtx {
   __device__ int first_chunk() { return ticket(); }
   __device__ int next_chunk(int) { return ticket(); }
   __device__ bool writer() const { return rank == 0 && threadIdx.x == 0; }
+  __device__ double* csum() const { return a.csum; }
   __device__ void clear_tickets() {
     if (threadIdx.x == 0) tickets[phase & 1u] = 0u;
   }

@@ -1,0 +1,697 @@
+// Projected-gradient solve (APGD / Descent / SPG, Core/BlockSolvers/ProjectedGradient.impl.hpp:74-155, 288-351) of a
+// problem small enough to stay in the SMs: one cooperative launch of one CTA per SM in which every 32-contact chunk
+// is owned by a team of three warps for the whole solve.
+//
+// What bounds such a problem is latency, not throughput: with a chunk or a few per SM, a warp of k_pg_persistent
+// waits for each block of W it loads (some 15 round trips to L2 per product), runs the nine FMAs of a block one after
+// another (64 cycles each, the latency of GB300's FP64 unit, which one SM's four sub-partitions share at one warp
+// instruction per 19 cycles), and re-reads its contacts' vectors in every phase. Here
+//   - W stays in shared memory: a chunk's interleaved blocks are copied once, so a product's only loads are the
+//     columns (from L1) and the gathers of x, issued two groups of three steps ahead of their FMAs;
+//   - each gathered point is loaded once per team: warp r takes step r of a group and passes it through shared
+//     memory (a gather of 32 scattered contacts holds the load unit for as long as the step's FMAs take);
+//   - the product is split by row component: warp r of the team accumulates component r of every row (3 FMAs per
+//     block in place of 9), and the row-local work by quantity (the law's residual, the step and the objective in the
+//     A phase; the three line-search terms and the momentum point in the C phase);
+//   - the contacts' vectors stay in registers (a small shared array passes them between the team's warps); global
+//     memory carries only the two gathered points, padded to 32 bytes per contact for one 256-bit load each, and
+//     the chunk sums;
+//   - reductions use the flat barrier (every CTA combines the chunk sums itself), and one warp per CTA takes the
+//     line-search and momentum decisions and publishes them in shared memory.
+// Every value goes through the same operations in the same order as in k_pg_persistent (kernels_pg.cu, which has the
+// phases and the reference's line numbers), so the results are identical.
+// us per APGD iteration on GB300 (2.31 products), k_pg_persistent / this kernel: 33 contacts 40 / 17, 500 44 / 18,
+// 2 000 54 / 22, 10 000 57 / 28, 20 000 65 / 35. At 2 000 contacts, of 44 500 cycles: products 20 000 (7 200 of them
+// the chain of FMAs), law and vectors 9 300, barriers 7 000, sums 4 400, decisions 4 000.
+#include "internal.h"
+#include "soc_device.cuh"
+#include "spmv_chunk.cuh"
+
+namespace bogus_gpu {
+
+namespace {
+
+constexpr int kTeamWarps = 3;
+constexpr int kMaxTeams = 5;
+constexpr int kMinWarps = 8;  // a stripe of the reductions each; those past the teams' warps do nothing else
+
+// Shared memory of one team, beside its chunk's block values.
+struct TeamShared {
+  // pieces of the rows, by component (slot: rank of the row among the nonempty + lane), then the product itself
+  double part[kTeamWarps][64];
+  double xs[3][32], y[3][32];   // the last step; the second product of the guess (pieces, then values) before
+  double s0[32];
+  double stage[2][3][3][32];    // the gathered points of two groups of three steps
+  int st[36];                   // row starts of the chunk, relative to its first block
+};
+
+// Scalars of the iteration, written by one warp per CTA after each reduction.
+struct Control {
+  double stripes[32];
+  double alpha, alpha_t, alpha_less, theta, theta_next, beta, J, min_res, half_over_alpha, half_over_less;
+  int go, best;
+  unsigned phases[9];
+};
+
+__device__ __forceinline__ void team_sync(int team) {
+  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(32 * kTeamWarps) : "memory");
+}
+
+// A gathered point: 32 bytes per contact, the fourth value unused.
+__device__ __forceinline__ void load_padded(const double* p, double* x) {
+  double pad;
+  asm volatile("ld.relaxed.gpu.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(pad)
+               : "l"(p));
+}
+__device__ __forceinline__ void store_padded(double* p, const double* x) {
+  __stcg(reinterpret_cast<double2*>(p), make_double2(x[0], x[1]));
+  __stcg(p + 2, x[2]);
+}
+
+template <int V>
+struct Int {
+  static constexpr int value = V;
+};
+
+enum { kAccept = 0, kMomentum = 1, kRetry = 2, kStop = 3 };
+
+// S of chunk c (spmv_chunk.cuh)
+__device__ __forceinline__ int steps_of(const PGArgs& a, int c) {
+  const int nblk = __ldg(a.rowptr + min(32 * c + 32, a.n)) - __ldg(a.rowptr + 32 * c);
+  return nblk > 0 ? (nblk + 31) / 32 : 1;
+}
+
+__global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(PGArgs a, int teams) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int team = warp / kTeamWarps, role = warp - kTeamWarps * team;
+  Control& ctl = *reinterpret_cast<Control*>(smem);
+  const int first = __ldg(a.cta_ptr + blockIdx.x);
+  const bool has = team < teams && first + team < __ldg(a.cta_ptr + blockIdx.x + 1);
+  const int c = has ? __ldg(a.cta_list + first + team) : 0;
+  TeamShared& sh = reinterpret_cast<TeamShared*>(smem + (sizeof(Control) + 15) / 16 * 16)[team < teams ? team : 0];
+  // the CTA's chunks one after another, behind the teams' arrays
+  size_t before = 0;
+  for (int k = 0; k < team && has; ++k) before += (size_t)steps_of(a, __ldg(a.cta_list + first + k));
+  unsigned char* const blocks =
+      smem + (sizeof(Control) + 15) / 16 * 16 + (size_t)teams * sizeof(TeamShared) + before * 32 * 72;
+  const int C = a.nchunks;
+  const int i = 32 * c + lane;
+  const bool on = has && i < a.n;
+  const bool desaxce = a.desaxce != 0, spg = a.variant == 4, apgd = a.variant == 3;
+  const unsigned res_mask = a.use_inf ? 1u : 0u;
+  const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
+  double* const gx = a.MX0;                      // the gathered points: x (or the momentum point) ...
+  double* const gs = a.MX0 + 4 * (size_t)a.n;    // ... and the trial point xs
+  const size_t ip = on ? 4 * (size_t)i : 0;
+
+  // ---- the chunk: blocks and columns to shared memory, this lane's segment and row -------------------------
+  double* const wv = reinterpret_cast<double*>(blocks);
+  const int* col = nullptr;  // this lane's columns: step s at col[32 s]
+  int nblk = 0, S = 0, nv = 0, slot0 = 0, piece0 = 0, pieces = 0;
+  unsigned long long starts = 0;  // bit s: the lane's block s opens a row that its block s - 1 does not belong to
+  if (has) {
+    const int r0 = 32 * c, r1 = min(r0 + 32, a.n);
+    const int B0 = __ldg(a.rowptr + r0);
+    nblk = __ldg(a.rowptr + r1) - B0;
+    S = nblk > 0 ? (nblk + 31) / 32 : 1;
+    if (role == 0) {
+      sh.st[lane] = __ldg(a.rowptr + min(r0 + lane, r1)) - B0;
+      if (lane == 0) sh.st[32] = nblk;
+    }
+    const long long base = __ldg(a.slot0 + c);
+    const int tid = threadIdx.x - 32 * kTeamWarps * team;
+    const double2* sv = reinterpret_cast<const double2*>(a.ival + 9 * base);
+    for (int k = tid; k < S * 32 * 9 / 2; k += 32 * kTeamWarps) reinterpret_cast<double2*>(wv)[k] = __ldcs(sv + k);
+    col = a.icol + base + lane;
+    team_sync(team);
+    const int k0 = lane * S;
+    nv = max(0, min(S, nblk - k0));
+    const int rs = sh.st[lane], re = sh.st[lane + 1];
+    const unsigned filled = __ballot_sync(0xffffffffu, rs < re);
+    auto rank = [&](int t) { return __popc(filled & ((1u << t) - 1u)); };
+    if (nv > 0) {
+      int lo = 0, hi = 31;  // row containing block k0: last t with st[t] <= k0
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (sh.st[mid] <= k0) lo = mid;
+        else hi = mid - 1;
+      }
+      slot0 = rank(lo) + lane;
+      for (int t = lo + 1; t < 32 && sh.st[t] < k0 + nv; ++t)
+        if (sh.st[t] > k0) starts |= 1ull << (sh.st[t] - k0);
+    }
+    if (rs < re) {
+      const int lf = rs / S;
+      piece0 = rank(lane) + lf;
+      pieces = (re - 1) / S - lf + 1;
+    }
+  }
+
+  // group k: steps 3 k .. 3 k + 2, this warp's gather the step 3 k + role (past the end: any contact)
+  auto column = [&](int k) {
+    const int s = min(3 * k + role, S - 1);
+    return lane * S + s < nblk ? __ldg(col + 32 * s) : 32 * c;
+  };
+  const int j0 = has ? column(0) : 0, j1 = has ? column(1) : 0;
+
+  // Component `role` of row `lane` of the chunk's product with the gathered point g (NP = 2: also with g - 1), in
+  // the chunk-segmented order of spmv_chunk.
+  // One step, without divergence: the piece of the row that ends is put away, then three FMAs; a lane past its
+  // segment runs them on the padding and keeps its sum.
+  auto product = [&](const double* __restrict__ g, auto np) -> double2 {
+    constexpr int NP = decltype(np)::value;
+    double* part2 = sh.xs[0] + 64 * role;
+    int slot = slot0;
+    double p = 0.0, q = 0.0;
+    const double* bl = wv + 32 * 3 * role + lane;
+    unsigned long long open = starts;
+    auto step = [&](int s, const double* b, const double* x) {
+      const bool starts_row = open & 1ull;
+      open >>= 1;
+      if (starts_row) sh.part[role][slot] = p;
+      p = starts_row ? 0.0 : p;
+      const bool valid = s < nv;
+      const double pn = fma(b[2], x[2], fma(b[1], x[1], fma(b[0], x[0], p)));
+      p = valid ? pn : p;
+      if (NP == 2) {
+        if (starts_row) part2[slot] = q;
+        q = starts_row ? 0.0 : q;
+        const double qn = fma(b[2], x[2] - 1.0, fma(b[1], x[1] - 1.0, fma(b[0], x[0] - 1.0, q)));
+        q = valid ? qn : q;
+      }
+      slot += starts_row ? 1 : 0;
+    };
+    auto put_stage = [&](int k, const double* x) {
+#pragma unroll
+      for (int e = 0; e < 3; ++e) sh.stage[k & 1][role][e][lane] = x[e];
+    };
+    auto consume = [&](int k) {
+      double b[3][3], x[3][3];  // all loads of the group before its chain of FMAs
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const double* be = bl + 288 * min(3 * k + e, S - 1);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          b[e][r] = be[32 * r];
+          x[e][r] = sh.stage[k & 1][e][r][lane];
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 3; ++e)
+        if (3 * k + e < S) step(3 * k + e, b[e], x[e]);
+      team_sync(team);
+    };
+    // even groups pass through u, odd ones through v (no copies between them: a copy would wait for the load)
+    const int groups = (S + 2) / 3;
+    double u[3], v[3];
+    int ju = column(2), jv = column(3);
+    load_padded(g + 4 * (size_t)j0, u);
+    load_padded(g + 4 * (size_t)j1, v);
+    put_stage(0, u);
+    load_padded(g + 4 * (size_t)ju, u);
+    ju = column(4);
+    team_sync(team);
+    for (int k = 0; k < groups; k += 2) {
+      if (k + 1 < groups) {
+        put_stage(1, v);
+        load_padded(g + 4 * (size_t)jv, v);
+        jv = column(k + 5);
+      }
+      consume(k);
+      if (k + 1 >= groups) break;
+      if (k + 2 < groups) {
+        put_stage(0, u);
+        load_padded(g + 4 * (size_t)ju, u);
+        ju = column(k + 6);
+      }
+      consume(k + 1);
+    }
+    if (nv > 0) {
+      sh.part[role][slot] = p;
+      if (NP == 2) part2[slot] = q;
+    }
+    __syncwarp();
+    double2 acc = make_double2(0.0, 0.0);
+    if (pieces > 0) {
+      acc.x = ipipe::plus_zero(sh.part[role][piece0]);
+      for (int k = 1; k < pieces; ++k) acc.x = acc.x + sh.part[role][piece0 + k];
+      if (NP == 2) {
+        acc.y = ipipe::plus_zero(part2[piece0]);
+        for (int k = 1; k < pieces; ++k) acc.y = acc.y + part2[piece0 + k];
+      }
+    }
+    __syncwarp();
+    sh.part[role][lane] = acc.x;
+    if (NP == 2) part2[lane] = acc.y;
+    team_sync(team);
+    return acc;
+  };
+  // W g for this chunk's contacts, all components to every warp of the team
+  auto team_product = [&](const double* g, double* out) {
+    product(g, Int<1>());
+#pragma unroll
+    for (int k = 0; k < 3; ++k) out[k] = sh.part[k][lane];
+  };
+
+  // ---- barriers ----------------------------------------------------------------------------------------------
+  const MonoBarrier mb{a.mono, a.gb.status, gridDim.x + a.phantom_ctas};
+  unsigned phase = 0;  // barriers passed
+  auto sums = [&]() { return a.csum + (size_t)(phase & 1u) * 4 * C; };
+  auto put = [&](int q, double v) {
+    v = warp_sum_butterfly(v);
+    if (lane == 0) sums()[q * C + c] = v;
+  };
+  // The last warp prepares the next decision (side) while thread 0 waits for the other CTAs.
+  auto arrive_and_wait = [&](auto side) -> bool {
+    bool ok = true;
+    __syncthreads();
+    if (warp == nwarps - 1) side();
+    if (mb.parties > 1u && threadIdx.x == 0) ok = flat_wait(mb, phase);
+    return __syncthreads_and(ok) != 0;
+  };
+  // Barrier, the K reduced quantities, then decide(totals) by warp 0 (the same values in every lane).
+  auto reduce = [&](int K, unsigned maxmask, auto side, auto decide) -> bool {
+    if (!arrive_and_wait(side)) return false;
+    const double* s = sums();
+    const int per = (C + 7) / 8;
+    if (warp < 8) {
+      const int st = warp, b = st * per, e = min(C, b + per);
+      double p[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int k = b + lane; k < e; k += 32) {
+        double v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = q < K ? ldcg(s + q * C + k) : 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q < K) p[q] = (maxmask >> q) & 1u ? ((v[q] < p[q]) ? p[q] : v[q]) : p[q] + v[q];
+      }
+      if (b >= e) {
+        if (lane < K) ctl.stripes[8 * lane + st] = 0.0;
+      } else if (maxmask) {
+        const double v0 = warp_max_butterfly(p[0]), v1 = warp_sum_butterfly(p[1]);  // the residual and one sum
+        if (lane < 2) ctl.stripes[8 * lane + st] = lane ? v1 : v0;
+      } else if (K == 4) {
+        const double v = warp_sum4_butterfly(p[0], p[1], p[2], p[3]);
+        if ((lane & 7) == 0) ctl.stripes[lane + st] = v;
+      } else {
+        const double v = warp_sum2_butterfly(p[0], p[1]);
+        if ((lane & 15) == 0) ctl.stripes[lane / 2 + st] = v;
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const int q = lane < K ? lane : 0;
+      const bool mx = (maxmask >> q) & 1u;
+      double total = ctl.stripes[8 * q];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) {
+        const double v = ctl.stripes[8 * q + k];
+        total = mx ? ((v < total) ? total : v) : total + v;
+      }
+      decide(total);
+    }
+    __syncthreads();
+    ++phase;
+    return true;
+  };
+  auto sync = [&]() -> bool {
+    const bool ok = arrive_and_wait([] {});
+    ++phase;
+    return ok;
+  };
+  auto total_of = [](double total, int q) { return __shfl_sync(0xffffffffu, total, q); };
+
+  // ---- per-contact state, the same in the team's three warps ------------------------------------------------
+  // (x and prev in registers; xs, y and the products in the team's shared memory; b, mu and the scalings are read
+  // where they are used, from L1)
+  double x[3] = {0.0, 0.0, 0.0}, pv[3], Mx[3] = {0.0, 0.0, 0.0};
+  if (on) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) x[k] = a.X0[3 * (size_t)i + k];
+    project_cone(__ldg(a.mu + i), x);  // projectOnConstraints(x) (:90)
+    if (role == 1) store_padded(gx + ip, x);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) pv[k] = x[k];
+  auto load_b = [&](double* b) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) b[k] = __ldg(a.b + 3 * (size_t)i + k);
+  };
+  auto store_best = [&]() {
+    if (on && role == 1)
+      for (int k = 0; k < 3; ++k) a.XB[3 * (size_t)i + k] = x[k];
+  };
+  auto count = [&](int k) {
+    if (threadIdx.x == 0) ++ctl.phases[k];
+  };
+  auto finish = [&](unsigned iters, int converged) {
+    if (!writer) return;
+    a.out->min_res = ctl.min_res;
+    a.out->iters = iters;
+    a.out->best_buf = 3;
+    a.out->converged = converged;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) a.out->phases[k] = ctl.phases[k];
+    a.out->hy_refreshes = 0;
+  };
+  if (threadIdx.x == 0) {
+    ctl.theta = 1.0;
+    ctl.min_res = -1.0;
+    for (int k = 0; k < 9; ++k) ctl.phases[k] = k == 0 ? 1u : 0u;
+  }
+  if (!sync()) return;
+
+  // Mx = W x (:93) and guess_alpha (:21-28)
+  count(1);
+  if (has) {
+    product(gx, Int<2>());
+#pragma unroll
+    for (int k = 0; k < 3; ++k) Mx[k] = sh.part[k][lane];
+    if (role == 0) {
+      const double* second = sh.xs[0] + lane;
+      const double d[3] = {second[0], second[64], second[128]};
+      put(0, on ? sq3(d) : 0.0);
+    } else if (role == 1) {
+      const double d[3] = {x[0] - 1.0, x[1] - 1.0, x[2] - 1.0};
+      put(1, on ? sq3(d) : 0.0);
+    }
+  }
+  if (!reduce(2, 0u, [] {}, [&](double total) {
+        const double nMx = total_of(total, 0), n1 = total_of(total, 1);
+        double alpha = 1.0;
+        if (nMx > 1.e-16) alpha = dmin(1., ipipe::div_rn(n1, nMx));
+        if (lane == 0) {
+          ctl.alpha = alpha;
+          ctl.alpha_t = spg ? alpha : alpha * a.opt;
+        }
+      }))
+    return;
+  if (a.max_iters == 0) {
+    store_best();
+    finish(0, 0);
+    return;
+  }
+
+  unsigned it = 0;
+  const double n_plus_1 = (double)(1 + a.n);
+  // A (:110-125): the residual (warp 0), xs = P(x - alpha_t y) with y += COV(y) (warp 1; SPG: (xs - prev).y), the
+  // objective (warp 2); y, xs and s0 go to the other warps
+  auto phaseA = [&]() {
+    if (!has) return;
+    double v = 0.0;
+    if (on) {
+      const double mu = __ldg(a.mu + i);
+      double b[3];
+      load_b(b);
+      if (role == 0) {
+        const double scal = __ldg(a.scaling + i);
+        const double yr[3] = {Mx[0] + b[0], Mx[1] + b[1], Mx[2] + b[2]};
+        const double lx[3] = {x[0] * scal, x[1] * scal, x[2] * scal};
+        v = law_eval(desaxce, mu, lx, yr);
+      } else if (role == 1) {
+        double yn[3] = {Mx[0] + b[0], Mx[1] + b[1], Mx[2] + b[2]};
+        const double sn = duality_cov(desaxce, mu, yn);
+        yn[0] = desaxce ? yn[0] + sn : ipipe::plus_zero(yn[0]);
+        yn[1] = ipipe::plus_zero(yn[1]);
+        yn[2] = ipipe::plus_zero(yn[2]);
+        const double na = neg(ctl.alpha_t);
+        double p[3] = {fma(na, yn[0], x[0]), fma(na, yn[1], x[1]), fma(na, yn[2], x[2])};
+        project_cone(mu, p);
+        store_padded(gs + ip, p);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          sh.xs[k][lane] = p[k];
+          sh.y[k][lane] = yn[k];
+        }
+        sh.s0[lane] = sn;
+        if (spg) {
+          const double d[3] = {p[0] - pv[0], p[1] - pv[1], p[2] - pv[2]};
+          v = dot3(d, yn);
+        }
+      } else if (!spg) {
+        double first = ipipe::scale2<-1>(Mx[0]) + b[0];
+        if (desaxce) {
+          const double yr[3] = {Mx[0] + b[0], Mx[1] + b[1], Mx[2] + b[2]};
+          first = first + duality_cov(true, mu, yr);
+        } else {
+          first = ipipe::plus_zero(first);
+        }
+        const double t[3] = {first, ipipe::plus_zero(ipipe::scale2<-1>(Mx[1]) + b[1]),
+                             ipipe::plus_zero(ipipe::scale2<-1>(Mx[2]) + b[2])};
+        v = dot3(x, t);
+      }
+    }
+    if (role == 0) {
+      v = a.use_inf ? warp_max_butterfly(v) : warp_sum_butterfly(v);
+      if (lane == 0) sums()[c] = v;
+    } else if (role == (spg ? 1 : 2)) {
+      put(1, v);
+    }
+  };
+  // beside A's barrier: the momentum weight that follows from theta, and 1 / 2 alpha for the line search
+  auto before_top = [&]() {
+    double theta = ctl.theta, beta = 0.0;
+    if (spg || apgd) beta = nesterov_inertia(theta, 0.0);
+    const double hoa = ipipe::div_rn(.5, ctl.alpha_t);
+    if (lane == 0) {
+      ctl.beta = beta;
+      ctl.theta_next = theta;
+      ctl.half_over_alpha = hoa;
+    }
+  };
+  // after A's reduction: the residual, the best iterate, the trace, the objective
+  auto top = [&](double total) {
+    const double reduced = total_of(total, 0), second = total_of(total, 1);
+    const double res = a.use_inf ? reduced : ipipe::div_rn(reduced, n_plus_1);
+    const bool best = it == 0 || less_from_zero(res, ctl.min_res);
+    const bool stop = less_from_zero(res, a.tol);
+    const bool mom = spg ? negative(second) : apgd;
+    __syncwarp();
+    if (lane == 0) {
+      if (a.trace && blockIdx.x == 0) a.trace[it] = res;
+      if (best) ctl.min_res = res;
+      ctl.best = best;
+      ctl.go = stop ? kStop : (mom ? kMomentum : kAccept);
+      ctl.J = second;
+      if (spg) ctl.theta = mom ? ctl.theta_next : 1.0;
+      else ctl.alpha = ctl.alpha_t;
+    }
+  };
+  auto shared3 = [&](const double (*v)[32], double* out) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) out[k] = on ? v[k][lane] : 0.0;
+  };
+
+  count(2);
+  phaseA();
+  if (!spg) {
+    // ---------------------------------------------------------------------------------------- APGD / Descent
+    for (;;) {
+      if (!reduce(2, res_mask, before_top, top)) return;
+      if (ctl.go == kStop) {
+        if (ctl.best) store_best();
+        finish(it, 1);
+        return;
+      }
+      bool pending = ctl.best != 0;
+      unsigned ls = 0;
+      int next;
+      for (;;) {
+        // C (:127-139): Mxs = W xs; Js (warp 0), y.(xs - x) and |xs - x|^2 (warp 1), (xs - prev).y and the momentum
+        // point (warp 2)
+        count(3);
+        if (has) {
+          double xs[3], Ms[3];
+          team_product(gs, Ms);
+          shared3(sh.xs, xs);
+          if (role == 0) {
+            double b[3] = {0.0, 0.0, 0.0};
+            if (on) load_b(b);
+            const double first = ipipe::scale2<-1>(Ms[0]) + b[0];
+            const double t[3] = {desaxce ? first + sh.s0[lane] : ipipe::plus_zero(first),
+                                 ipipe::plus_zero(ipipe::scale2<-1>(Ms[1]) + b[1]),
+                                 ipipe::plus_zero(ipipe::scale2<-1>(Ms[2]) + b[2])};
+            put(0, on ? dot3(xs, t) : 0.0);
+          } else if (role == 1) {
+            double y[3];
+            shared3(sh.y, y);
+            const double d[3] = {xs[0] - x[0], xs[1] - x[1], xs[2] - x[2]};
+            const double v = warp_sum2_butterfly(on ? dot3(y, d) : 0.0, on ? sq3(d) : 0.0);
+            if ((lane & 15) == 0) sums()[(1 + (lane >> 4)) * C + c] = v;
+            if (pending) store_best();
+          } else {
+            double y[3];
+            shared3(sh.y, y);
+            const double bt = ctl.beta;
+            const double d[3] = {xs[0] - pv[0], xs[1] - pv[1], xs[2] - pv[2]};
+            if (apgd && on) {
+              const double xn[3] = {fma(bt, d[0], xs[0]), fma(bt, d[1], xs[1]), fma(bt, d[2], xs[2])};
+              store_padded(gx + ip, xn);
+            }
+            put(3, on ? dot3(d, y) : 0.0);
+          }
+        }
+        pending = false;
+        if (!reduce(4, 0u,
+                    [&] {  // the step that a rejection takes, and its 1 / 2 alpha
+                      const double smaller = ctl.alpha * a.pess;
+                      const double hoa = ipipe::div_rn(.5, smaller);
+                      if (lane == 0) {
+                        ctl.alpha_less = smaller;
+                        ctl.half_over_less = hoa;
+                      }
+                    },
+                    [&](double total) {
+                      const double Js = total_of(total, 0), decr = total_of(total, 1), nrm = total_of(total, 2);
+                      const double decr2 = total_of(total, 3);
+                      const bool accept = Js < (ctl.J + decr) + ctl.half_over_alpha * nrm;
+                      const bool retry = !accept && ls + 1 < a.ls_iters;
+                      const double alpha = accept ? ctl.alpha : ctl.alpha_less;
+                      const double alpha_t = alpha * a.opt;
+                      const bool mom = apgd && negative(decr2);
+                      __syncwarp();
+                      if (lane == 0) {
+                        ctl.alpha = alpha;
+                        ctl.go = retry ? kRetry : (mom ? kMomentum : kAccept);
+                        if (retry) {
+                          ctl.half_over_alpha = ctl.half_over_less;
+                        } else {
+                          ctl.theta = mom ? ctl.theta_next : 1.0;
+                          ctl.alpha_t = alpha_t;
+                        }
+                      }
+                    }))
+          return;
+        next = ctl.go;
+        if (next != kRetry) break;
+        ++ls;
+        // B: retry with a smaller step
+        count(4);
+        if (on && role == 1) {
+          const double na = neg(ctl.alpha);
+          double p[3] = {fma(na, sh.y[0][lane], x[0]), fma(na, sh.y[1][lane], x[1]), fma(na, sh.y[2][lane], x[2])};
+          project_cone(__ldg(a.mu + i), p);
+          store_padded(gs + ip, p);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) sh.xs[k][lane] = p[k];
+        }
+        if (!sync()) return;
+      }
+      ++it;
+      if (it >= a.max_iters) break;
+      if (on && next == kMomentum) load_padded(gx + ip, x);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const double xs = on ? sh.xs[k][lane] : 0.0;
+        if (next != kMomentum) {
+          x[k] = xs;
+          Mx[k] = sh.part[k][lane];
+        }
+        pv[k] = xs;
+      }
+      if (next == kMomentum) {
+        // E + A: Mx = W x (:141), then A of the next iteration
+        count(6);
+        if (has) team_product(gx, Mx);
+      } else {
+        count(2);
+        if (has) team_sync(team);  // phaseA writes the shared xs that the team's warps have just read
+      }
+      phaseA();
+    }
+    finish(it, 0);
+    return;
+  }
+
+  // ---------------------------------------------------------------------------------------------- SPG (:288-351)
+  for (;;) {
+    if (!reduce(2, res_mask, before_top, top)) return;
+    if (ctl.go == kStop) {
+      if (ctl.best) store_best();
+      finish(it, 1);
+      return;
+    }
+    // D: w and the new x
+    count(7);
+    const bool mom = ctl.go == kMomentum;
+    const double bt = ctl.beta;
+    if (ctl.best) store_best();
+    double xs[3], Ms[3] = {0.0, 0.0, 0.0};
+    shared3(sh.xs, xs);
+    double w[3] = {0.0, 0.0, 0.0};
+    if (on && role == 1) {
+      double xn[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (mom) {
+          w[k] = fma(bt, xs[k] - pv[k], xs[k]) - x[k];
+          xn[k] = x[k] + w[k];
+        } else {
+          w[k] = xs[k] - x[k];
+          xn[k] = xs[k];
+        }
+      }
+      store_padded(gx + ip, xn);
+    }
+    if (!sync()) return;
+    // E: Mx_new = W x; z = -Mx_old + Mx_new; w.z (warp 1), |z|^2 (warp 0)
+    count(8);
+    if (on) load_padded(gx + ip, x);
+    if (has) {
+      team_product(gx, Ms);
+      const double z[3] = {-Mx[0] + Ms[0], -Mx[1] + Ms[1], -Mx[2] + Ms[2]};
+      if (role == 0) put(1, on ? sq3(z) : 0.0);
+      else if (role == 1) put(0, on ? dot3(w, z) : 0.0);
+    }
+    if (!reduce(2, 0u, [] {}, [&](double total) {
+          double alpha = ipipe::div_rn(total_of(total, 0), total_of(total, 1));
+          alpha = dmin(1.e6, dmax(1.e-6, alpha));
+          if (lane == 0) ctl.alpha_t = alpha;
+        }))
+      return;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      Mx[k] = Ms[k];
+      pv[k] = xs[k];
+    }
+    ++it;
+    if (it >= a.max_iters) break;
+    count(2);
+    phaseA();
+  }
+  finish(it, 0);
+}
+
+// teams per CTA, and the largest sum of S over a CTA's chunks
+size_t resident_smem(int teams, int steps) {
+  return (sizeof(Control) + 15) / 16 * 16 + (size_t)teams * sizeof(TeamShared) + (size_t)steps * 32 * 72;
+}
+
+}  // namespace
+
+// Whether the resident kernel takes a problem whose CTAs own up to `teams` chunks with up to `steps` steps (S) in sum:
+// a team per chunk, every chunk's block values (72 bytes each) in shared memory, a lane's row starts in 64 bits.
+bool pg_resident_fits(int device, int teams, int steps, int longest) {
+  int limit = 0;
+  if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return false;
+  return teams >= 1 && teams <= kMaxTeams && longest <= 64 && resident_smem(teams, steps) <= (size_t)limit;
+}
+
+cudaError_t launch_pg_resident(const PGArgs& a, int ctas, int teams, int steps, cudaStream_t s) {
+  const size_t bytes = resident_smem(teams, steps);
+  const void* fn = (const void*)k_pg_resident;
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) return e;
+  PGArgs copy = a;
+  int t = teams;
+  const int warps = kTeamWarps * teams > kMinWarps ? kTeamWarps * teams : kMinWarps;
+  void* args[] = {&copy, &t};
+  return cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(32 * warps), args, bytes, s);
+}
+
+// Sets this file's copy of the device-side wait limit on the current device.
+BOGUS_GPU_WAIT_LIMIT_SETTER(set_wait_limit_pg_resident)
+
+}  // namespace bogus_gpu
