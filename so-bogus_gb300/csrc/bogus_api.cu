@@ -89,7 +89,8 @@ struct GSCache {
   DevBuf<unsigned char> skip, processed;
   DevBuf<unsigned long long> tile_max;
   DevBuf<double> ndx_ref;
-  DevBuf<unsigned> flow, done;  // dataflow sweep: position counter and tag, per-contact visit tags
+  // dataflow sweep: position counter and tag; tagged positions (assembled) or per-contact visit tags (matrix-free)
+  DevBuf<unsigned> flow, rec, done;
   DevBuf<int> pdep;             // matrix-free sweep: previous contact on each slot's body
   int flow_grid = 0;
   double auto_reg = -1.0;
@@ -111,7 +112,7 @@ struct GSCache {
     rowptr.release(); col.release(); val.release(); local.release(); reg.release(); scaling.release();
     b.release(); mu.release(); x.release(); nx2.release(); ndx2.release(); y.release(); chunk.release();
     scalar.release(); xbest.release(); skip.release(); processed.release(); tile_max.release(); ndx_ref.release();
-    flow.release(); done.release(); pdep.release();
+    flow.release(); rec.release(); done.release(); pdep.release();
     valid = false;
   }
 };
@@ -919,7 +920,7 @@ int prepare_gs(bogus_gpu_problem* h, double auto_reg, int use_coloring) {
   BG_CUDA(g.chunk.ensure((n + 31) / 32 + 1));
   BG_CUDA(g.scalar.ensure(2));
   BG_CUDA(g.flow.ensure(2));
-  BG_CUDA(g.done.ensure(n > 0 ? n : 1));
+  BG_CUDA(g.rec.ensure(8 * (size_t)(n > 0 ? n : 1)));
   BG_CUDA(h->status.ensure(1));
   g.flow_grid = gs_flow_grid(h->device);
   if (g.flow_grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "occupancy query failed (Gauss-Seidel sweep)");
@@ -927,7 +928,6 @@ int prepare_gs(bogus_gpu_problem* h, double auto_reg, int use_coloring) {
   {
     const unsigned f0[2] = {0u, 1u};
     BG_CUDA(cudaMemcpyAsync(g.flow.p, f0, sizeof(f0), cudaMemcpyHostToDevice, s));
-    BG_CUDA(cudaMemsetAsync(g.done.p, 0, sizeof(unsigned) * (n > 0 ? n : 1), s));
   }
   BG_CUDA(cudaMemcpyAsync(g.rowptr.p, pf.rowptr.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s));
   if (nnz) {
@@ -1386,7 +1386,7 @@ GSArgs gs_args(bogus_gpu_problem* h, const bogus_gpu_gs_options* o) {
   a.desaxce = o->static_problem ? 0 : 1;
   a.strat = o->local_strategy;
   a.flow = g.flow.p;
-  a.done = g.done.p;
+  a.rec = g.rec.p;
   a.status = h->status.p;
   return a;
 }
@@ -1460,6 +1460,8 @@ int run_gs_core(bogus_gpu_problem* h, const bogus_gpu_gs_options* o, double* res
   unsigned it;
   int parity = 0;
   bool converged = false;
+  BG_CUDA(launch_gs_records(a, s));
+  h->last_launches += 1;
   for (it = 1; it <= o->max_iters; ++it) {
     if (int e = launch_sweep(h, h->gs, a, parity, abs_skip_tol, o->skip_tol, abs_skip_iters, key, false)) return e;
     parity ^= 1;

@@ -137,11 +137,9 @@ BG_HD float rsqrt_approx(float x) {
 #endif
 }
 
-// v 2^(150 - f) as an integer, for a float v whose exponent field is f, f + 1 or f + 2
-BG_HD uint32_t fixed_of(float v, uint32_t f) {
-  const uint32_t u = fbits(v);
-  return ((u & 0x7FFFFFu) | 0x800000u) << ((u >> 23) - f);
-}
+// v 2^(151 - f) for a float v in [2^(f - 127), 2^(f - 126)], from the line through its bit patterns there; for a v
+// slightly below, the line's value (as far below again: a worse starting point by one bit, not an error)
+BG_HD uint32_t fixed_of(float v, uint32_t f) { return 2u * fbits(v) - ((f - 1u) << 24); }
 BG_HD uint64_t mul_wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
 BG_HD uint32_t lo32(uint64_t v) { return (uint32_t)v; }
 BG_HD uint32_t hi32(uint64_t v) { return (uint32_t)(v >> 32); }
@@ -153,8 +151,10 @@ BG_HD uint64_t mulhi_est(uint64_t a, uint64_t b) {
 }
 // (s r) >> 32 for a signed s, |s| < 2^62, and r < 2^26
 BG_HD int64_t mul_shift32(int64_t s, uint32_t r) {
-  return (int64_t)(int32_t)(s >> 32) * (int64_t)r + (int64_t)hi32(mul_wide((uint32_t)s, r));
+  return (int64_t)(int32_t)(s >> 32) * (int32_t)r + (int64_t)hi32(mul_wide((uint32_t)s, r));
 }
+// v + 1, or v when rem < 0
+BG_HD uint64_t round_up(uint64_t v, uint64_t rem) { return (v + 1) + (uint64_t)(int64_t)((int32_t)hi32(rem) >> 31); }
 
 // Correctly rounded a / b when b is normal and a is zero, or a and the quotient are normal; `ok` false otherwise
 // (the returned value is then meaningless).
@@ -169,7 +169,7 @@ BG_HD double div_core(uint64_t ua, uint64_t ub, bool& ok) {
   const bool zero = (ua << 1) == 0;
   ok = (eb - 1u < 2046u) && (zero || ((ea - 1u < 2046u) && (e >= 1) && (e <= 2045)));
   // r0 ~ 1 / b for b = B / 2^53 in [1/2, 1) from the leading 24 bits, as R0 / 2^24 (r0 from just below 1 to 2)
-  const uint32_t R0 = fixed_of(rcp_approx(bitsf(0x3F000000u | (uint32_t)((B >> 29) & 0x7FFFFFu))), 126u);
+  const uint32_t R0 = fixed_of(rcp_approx(bitsf(0x3F000000u | (uint32_t)((B >> 29) & 0x7FFFFFu))), 127u);
   // eps = 1 - b r0, exact at 2^-77: the product's bits from 2^77 up are those of 1
   const int64_t E = -(int64_t)(B * R0);
   const int32_t Eh = (int32_t)(E >> 32);                // eps 2^45
@@ -179,8 +179,8 @@ BG_HD double div_core(uint64_t ua, uint64_t ub, bool& ok) {
   const uint64_t R = ((uint64_t)R0 << 38) + (uint64_t)(mul_shift32(E + (e2 >> 13) + (e3 >> 1), R0) >> 7);
   // the rounded quotient or one less: q = A r 2^7 carries 8 bits below the last place, within 8 units
   const uint64_t m = (mulhi_est(A << 9, R) + (128 - 8)) >> 8;
-  const int64_t rem = (int64_t)((A << 53) - (2 * m + 1) * B);  // sign of A / B - (m + 1/2); never a tie
-  const uint64_t mant = m + (rem > 0 ? 1 : 0);                 // in [2^52, 2^53)
+  // the sign of A / B - (m + 1/2), which is never zero
+  const uint64_t mant = round_up(m, (A << 53) - (2 * m + 1) * B);  // in [2^52, 2^53)
   return from_bits(zero ? sign : (sign | ((uint64_t)(uint32_t)(e - 1) << 52)) + mant);
 }
 
@@ -193,7 +193,7 @@ BG_HD double sqrt_core(uint64_t ux, bool& ok) {
   const uint64_t M = ((ux & kMant) | kHidden) << (odd ? 1 : 0);  // m = M / 2^52 in [1, 4)
   // y0 ~ 1 / sqrt(m) from the leading 24 bits, as Y0 / 2^25 (y0 from just below 1/2 to 1)
   const uint32_t Y0 = fixed_of(
-      rsqrt_approx(bitsf((odd ? 0x40000000u : 0x3F800000u) | (uint32_t)((ux >> 29) & 0x7FFFFFu))), 125u);
+      rsqrt_approx(bitsf((odd ? 0x40000000u : 0x3F800000u) | (uint32_t)((ux >> 29) & 0x7FFFFFu))), 126u);
   // eps = 1 - m y0^2 at 2^-70 (the product's last 32 bits dropped)
   const uint64_t Z = mul_wide(Y0, Y0);
   const uint64_t P = hi32(mul_wide(lo32(M), lo32(Z))) + mul_wide(lo32(M), hi32(Z)) + mul_wide(hi32(M), lo32(Z)) +
@@ -207,8 +207,8 @@ BG_HD double sqrt_core(uint64_t ux, bool& ok) {
   const uint64_t Y = ((uint64_t)Y0 << 37) + (uint64_t)mul_shift32(S, Y0);
   // the rounded root or one less: M y 2^7 carries 7 bits below the last place, within 4 units
   const uint64_t m = (mulhi_est(M << 9, Y) + (64 - 4)) >> 7;
-  const int64_t rem = (int64_t)((M << 52) - m * (m + 1));  // positive when sqrt(M 2^52) > m + 1/2; never a tie
-  const uint64_t mant = m + (rem > 0 ? 1 : 0);
+  // sqrt(M 2^52) > m + 1/2 when M 2^52 >= m (m + 1) + 1 (an integer, and never m (m + 1) + 1/4)
+  const uint64_t mant = round_up(m, (M << 52) - m * (m + 1) - 1);
   return from_bits(zero ? ux : ((uint64_t)((ex + 1021u - (odd ? 1u : 0u)) >> 1) << 52) + mant);
 }
 

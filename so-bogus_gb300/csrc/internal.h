@@ -210,9 +210,11 @@ struct GSArgs {
   const int* cb;
   double* Mx;
   int d;
-  // dataflow sweep: flow[0] = next sweep position to hand out, flow[1] = the sweep's tag; done[i] = tag once
-  // contact i has been visited in this sweep; status records a wait that ran out
+  // dataflow sweep: flow[0] = next sweep position to hand out, flow[1] = the sweep's tag; rec: the positions with
+  // the tag of the sweep that set them, 8 words per contact (assembled sweep); done[i] = tag once contact i has been
+  // visited (matrix-free sweep); status records a wait that ran out
   unsigned* flow;
+  unsigned* rec;
   unsigned* done;
   int* status;
   const int* pdep;  // matrix-free sweep: per contact slot, the previous contact on that body (-1: none)
@@ -220,6 +222,7 @@ struct GSArgs {
 constexpr int kGSTile = 1024;
 constexpr int kGSFlowWarps = 4;  // warps per CTA of the dataflow sweep
 cudaError_t launch_gs_flow(const GSArgs& a, int grid, int parity, cudaStream_t s);
+cudaError_t launch_gs_records(const GSArgs& a, cudaStream_t s);  // before the first sweep from a new a.x
 int gs_flow_grid(int device);
 cudaError_t launch_gs_skip(const GSArgs& a, int parity, double abs_skip_tol, double skip_tol, int abs_skip_iters,
                            cudaStream_t s);

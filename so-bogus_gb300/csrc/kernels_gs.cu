@@ -22,12 +22,13 @@ namespace bogus_gpu {
 __device__ __forceinline__ unsigned long long dbits(double v) { return (unsigned long long)__double_as_longlong(v); }
 
 // Dataflow sweep: one launch visits every contact. Each warp takes the next contact in level order from a
-// counter and waits only for the earlier neighbours of its contact (flags set when they are visited): a
+// counter and waits only for the earlier neighbours of its contact (their records carry the sweep's tag once they
+// are visited): a
 // contact starts as soon as its own earlier neighbours are done, not when the slowest contact of the previous
 // level is (a launch per level would wait for it; the sweep is latency bound, the local solves being long
 // dependent FP64 chains). Level order rather than sweep order keeps the contacts in flight mostly independent
-// (consecutive contacts of the sweep often share a body). An earlier neighbour has been visited (its flag was
-// set after its x was written), a later neighbour has not (it waits for this contact's flag), so every contact
+// (consecutive contacts of the sweep often share a body). An earlier neighbour has been visited (its record carries
+// the tag), a later neighbour has not (it waits for this contact's record), so every contact
 // sees the values of the sequential sweep. A warp waits only for contacts of lower levels, handed out before its own and so already taken by
 // running warps: the sweep always progresses. Every wait is bounded (wait_limit_ns()); a wait that runs
 // out records BOGUS_GPU_TIMEOUT and the warp stops.
@@ -48,16 +49,68 @@ __device__ __forceinline__ bool gs_wait_done(const unsigned* f, unsigned tag, co
   }
 }
 
-// The whole warp works on its contact: lanes stage the row's blocks (before waiting, they do not change) and the
-// neighbours' x (after); lanes 0-2 accumulate one component of the split row each (the three chains of the
-// scalar loop); every lane then runs the same local solve, whose eigenvalue step is shared across the lanes
-// (local_solve<true>), and lane 0 writes the result.
-__global__ void __launch_bounds__(32 * kGSFlowWarps) k_gs_flow(GSArgs a, int parity) {
+// The positions of a sweep travel as records: two 16-byte words per contact, (x0, low half of x2, tag) and (x1, high
+// half of x2, tag), each written and read by one 128-bit access. A record that carries the sweep's tag is the
+// contact's new position, so a waiting warp polls the values themselves: no flag, no fence before it, and no second
+// round trip for x after it.
+struct XRecord {
+  unsigned __int128 a, b;
+};
+__device__ __forceinline__ XRecord load_record(const unsigned* rec, int j) {
+  XRecord r;
+  const unsigned* p = rec + 8 * (size_t)j;
+  asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(r.a) : "l"(p));
+  asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(r.b) : "l"(p + 4));
+  return r;
+}
+__device__ __forceinline__ bool record_has(const XRecord& r, unsigned tag) {
+  return (unsigned)(r.a >> 96) == tag && (unsigned)(r.b >> 96) == tag;
+}
+__device__ __forceinline__ void unpack_record(const XRecord& r, double* x) {
+  x[0] = __longlong_as_double((long long)(unsigned long long)r.a);
+  x[1] = __longlong_as_double((long long)(unsigned long long)r.b);
+  const unsigned lo = (unsigned)(r.a >> 64), hi = (unsigned)(r.b >> 64);
+  x[2] = __longlong_as_double((long long)(((unsigned long long)hi << 32) | lo));
+}
+__device__ __forceinline__ void store_record(unsigned* rec, int j, const double* x, unsigned tag) {
+  const unsigned long long z = dbits(x[2]);
+  const unsigned __int128 t = (unsigned __int128)tag << 96;
+  const unsigned __int128 a = t | ((unsigned __int128)(unsigned)z << 64) | dbits(x[0]);
+  const unsigned __int128 b = t | ((unsigned __int128)(z >> 32) << 64) | dbits(x[1]);
+  unsigned* p = rec + 8 * (size_t)j;
+  asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(a) : "memory");
+  asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p + 4), "q"(b) : "memory");
+}
+
+// Records of the positions before the first sweep: they carry the tag before its own.
+__global__ void k_gs_records(GSArgs a) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  const double x[3] = {a.x[3 * i], a.x[3 * i + 1], a.x[3 * i + 2]};
+  store_record(a.rec, i, x, a.flow[1] - 1u);
+}
+
+cudaError_t launch_gs_records(const GSArgs& a, cudaStream_t s) {
+  if (a.n <= 0) return cudaSuccess;
+  k_gs_records<<<(a.n + 127) / 128, 128, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+// The whole warp works on its contact. What needs no neighbour is done before the wait: lanes stage the row's blocks,
+// every lane factorises the diagonal block (LocalPrep). Then lane q polls neighbour q's record while lanes 0-2
+// accumulate one component of the split row each (the three chains of the scalar loop), in the row's order, as far as
+// the neighbours are in: the last one to finish is followed only by the rest of the row. Every lane then runs the same
+// local solve, whose eigenvalue step is shared across the lanes (local_solve<true>), and lane 0 writes the result.
+//
+// Bound by the latency of the sweep's dependency chains, above all of the companion-matrix QR. Sweep of 50 000 contacts
+// in colored order / 501 in their own order, GB300: with flags, x read after them and the row and the factorisation
+// after x, GS_BEFORE; GS_AFTER with records.
+__global__ void __launch_bounds__(32 * kGSFlowWarps, 2) k_gs_flow(GSArgs a, int parity) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   __shared__ double sB[kGSFlowWarps][32][12];
-  __shared__ int sJ[kGSFlowWarps][32];
   const unsigned tag = ld_acquire_u32(a.flow + 1);
   const int ntiles = (a.n + kGSTile - 1) / kGSTile;
+  const bool desaxce = a.desaxce != 0;
   for (;;) {
     unsigned t = 0;
     if (lane == 0) t = atomicAdd(a.flow, 1u);
@@ -65,61 +118,91 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_gs_flow(GSArgs a, int par
     if (t >= (unsigned)a.n) return;
     const int i = a.order[t];
     const unsigned char sk = a.skip[i];
+    double lx[3];
+    unpack_record(load_record(a.rec, i), lx);
     __syncwarp();  // every lane has read the counter before lane 0 changes it: the branch below is warp-uniform
     if (sk) {
       if (lane == 0) {
         a.skip[i] = (unsigned char)(sk - 1);
         a.processed[i] = 0;
-        st_release_u32(a.done + i, tag);
+        store_record(a.rec, i, lx, tag);
       }
       continue;
     }
-    double lx[3] = {ldcg(a.x + 3 * i), ldcg(a.x + 3 * i + 1), ldcg(a.x + 3 * i + 2)};
-    const double reg = a.reg[i];
-    const int rc = lane < 3 ? lane : 0;  // the component lanes 0-2 accumulate
-    double lbr = a.b[3 * i + rc] - reg * lx[rc];
-    const int k0 = a.rowptr[i], k1 = a.rowptr[i + 1];
-    bool ok_wait = true;
-    for (int base = k0; base < k1; base += 32) {
-      const int k = base + lane;
-      int j = i;
-      if (k < k1) {
-        j = a.col[k];
-        sJ[w][lane] = j;
-        const double* B = a.val + 9 * (size_t)k;
-#pragma unroll
-        for (int e = 0; e < 9; ++e) sB[w][lane][e] = B[e];
-        if (j < i && !gs_wait_done(a.done + j, tag, a.status)) ok_wait = false;
-        sB[w][lane][9] = ldcg(a.x + 3 * j);
-        sB[w][lane][10] = ldcg(a.x + 3 * j + 1);
-        sB[w][lane][11] = ldcg(a.x + 3 * j + 2);
-      }
-      if (!__all_sync(0xffffffffu, ok_wait)) return;
-      if (lane < 3) {
-        const int cnt = min(32, k1 - base);
-        double s = lbr;
-        for (int q = 0; q < cnt; ++q) {
-          if (sJ[w][q] == i) continue;
-          const double* B = sB[w][q];
-          s = fma(B[3 * rc + 0], B[9], s);
-          s = fma(B[3 * rc + 1], B[10], s);
-          s = fma(B[3 * rc + 2], B[11], s);
-        }
-        lbr = s;
-      }
-      __syncwarp();
-    }
-    const double lb[3] = {__shfl_sync(0xffffffffu, lbr, 0), __shfl_sync(0xffffffffu, lbr, 1),
-                          __shfl_sync(0xffffffffu, lbr, 2)};
     double A[9];
 #pragma unroll
     for (int e = 0; e < 9; ++e) A[e] = a.local[9 * (size_t)i + e];
-    double ldx[3] = {-lx[0], -lx[1], -lx[2]};
-    const double sc = a.scaling[i];
-    const bool ok = law_solve_local<true>(a.desaxce != 0, a.strat, A, lb, lx, a.mu[i], sc);
-    if (lane == 0) {
+    const double mu = a.mu[i], sc = a.scaling[i];
+    const int rc = lane < 3 ? lane : 0;  // the component lanes 0-2 accumulate
+    double s = a.b[3 * i + rc] - a.reg[i] * lx[rc];
+    const int k0 = a.rowptr[i], k1 = a.rowptr[i + 1];
+    LocalPrep pre;
+    for (int base = k0; base < k1 || base == k0; base += 32) {
+      const int cnt = min(32, k1 - base);
+      int j = i;
+      if (lane < cnt) {
+        const int k = base + lane;
+        j = a.col[k];
+        const double* B = a.val + 9 * (size_t)k;
 #pragma unroll
-      for (int k = 0; k < 3; ++k) ldx[k] = ldx[k] + lx[k];
+        for (int e = 0; e < 9; ++e) sB[w][lane][e] = B[e];
+      }
+      const unsigned own = __ballot_sync(0xffffffffu, lane < cnt && j == i);
+      if (base == k0) pre.compute(A, mu, desaxce);
+      // an earlier neighbour's record must carry this sweep's tag; a later neighbour's cannot change before this
+      // contact is done; the contact's own block is left out
+      const bool earlier = j < i;
+      bool ready = j == i;
+      int done = 0;
+      unsigned long long t0 = 0;
+      unsigned idle = 0;
+      for (;;) {
+        XRecord r;
+        if (!ready) r = load_record(a.rec, j);
+        // (the loads run beside the chain over the neighbours that are in)
+        const unsigned in = __ballot_sync(0xffffffffu, ready);
+        const int upto = min(cnt, in == 0xffffffffu ? 32 : __ffs((int)~in) - 1);
+        __syncwarp();
+        const bool idled = upto <= done;
+        if (lane < 3) {
+          for (int q = done; q < upto; ++q) {
+            if ((own >> q) & 1u) continue;
+            const double* B = sB[w][q];
+            s = fma(B[3 * rc + 0], B[9], s);
+            s = fma(B[3 * rc + 1], B[10], s);
+            s = fma(B[3 * rc + 2], B[11], s);
+          }
+        }
+        done = upto;
+        if (done >= cnt) break;
+        if (!ready && (!earlier || record_has(r, tag))) {
+          unpack_record(r, &sB[w][lane][9]);
+          ready = true;
+        }
+        if (idled && ++idle > 1) {
+          __nanosleep(40);
+          if ((idle & 63u) == 0) {
+            bool stop = ld_relaxed_i32(a.status) != 0;
+            const unsigned long long now = global_timer_ns();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > wait_limit_ns()) {
+              if (lane == 0) atomicCAS(a.status, 0, (int)BOGUS_GPU_TIMEOUT);
+              stop = true;
+            }
+            if (__any_sync(0xffffffffu, stop)) return;
+          }
+        }
+      }
+      __syncwarp();
+    }
+    const double lb[3] = {__shfl_sync(0xffffffffu, s, 0), __shfl_sync(0xffffffffu, s, 1),
+                          __shfl_sync(0xffffffffu, s, 2)};
+    const double x0[3] = {lx[0], lx[1], lx[2]};
+    const bool ok = law_solve_local<true>(desaxce, a.strat, A, pre, lb, lx, mu, sc);
+    if (lane == 0) {
+      double ldx[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) ldx[k] = -x0[k] + lx[k];
       if (!ok) {
         ldx[0] *= .5;
         ldx[1] *= .5;
@@ -127,7 +210,8 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_gs_flow(GSArgs a, int par
       }
       double xn[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) xn[k] = ldcg(a.x + 3 * i + k) + ldx[k];
+      for (int k = 0; k < 3; ++k) xn[k] = x0[k] + ldx[k];
+      store_record(a.rec, i, xn, tag);
 #pragma unroll
       for (int k = 0; k < 3; ++k) a.x[3 * i + k] = xn[k];
       const double s2 = sc * sc;
@@ -137,8 +221,6 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_gs_flow(GSArgs a, int par
       a.ndx2[i] = ndx2;
       a.processed[i] = 1;
       if (ndx2 > 0.0) atomicMax(a.tile_max + parity * ntiles + i / kGSTile, dbits(ndx2));
-      __threadfence();
-      st_release_u32(a.done + i, tag);
     }
     __syncwarp();
   }
@@ -248,6 +330,12 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_pgs_flow(GSArgs a, int pa
     t = __shfl_sync(0xffffffffu, t, 0);
     if (t >= (unsigned)a.n) return;
     const int i = a.order[t];
+    double A[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) A[e] = a.local[9 * (size_t)i + e];
+    const double mu = a.mu[i], sc = a.scaling[i];
+    LocalPrep pre;  // before the wait: it needs no neighbour
+    pre.compute(A, mu, a.desaxce != 0);
     bool ok_wait = true;
     if (lane < 2) {
       const int j = a.pdep[2 * i + lane];
@@ -265,9 +353,6 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_pgs_flow(GSArgs a, int pa
       continue;
     }
     double lx[3] = {ldcg(a.x + 3 * i), ldcg(a.x + 3 * i + 1), ldcg(a.x + 3 * i + 2)};
-    double A[9];
-#pragma unroll
-    for (int e = 0; e < 9; ++e) A[e] = a.local[9 * (size_t)i + e];
     const int rc = lane < 3 ? lane : 0;
     double lbr = a.b[3 * i + rc] - dot3(&A[3 * rc], lx);
     for (int sl = 0; sl < 2; ++sl) {
@@ -282,8 +367,7 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps) k_pgs_flow(GSArgs a, int pa
     const double lb[3] = {__shfl_sync(0xffffffffu, lbr, 0), __shfl_sync(0xffffffffu, lbr, 1),
                           __shfl_sync(0xffffffffu, lbr, 2)};
     double ldx[3] = {-lx[0], -lx[1], -lx[2]};
-    const double sc = a.scaling[i];
-    const bool ok = law_solve_local<true>(a.desaxce != 0, a.strat, A, lb, lx, a.mu[i], sc);
+    const bool ok = law_solve_local<true>(a.desaxce != 0, a.strat, A, pre, lb, lx, mu, sc);
 #pragma unroll
     for (int k = 0; k < 3; ++k) ldx[k] = ldx[k] + lx[k];
     if (!ok) {

@@ -796,27 +796,45 @@ BG_HD double newton_solve(const LocalFB& f, double tol, double* x) {
   return Phi_best;
 }
 
+// The part of a local problem that does not depend on b: the factorised matrix and, for the Coulomb law's closed form,
+// the Schur complement of its normal row. A Gauss-Seidel sweep forms it while the contact waits for its neighbours.
+struct LocalPrep {
+  SmallLU<3> lu;
+  double wTwN0, wTwN1, Wb00, Wb01, Wb10, Wb11, det, D;
+
+  BG_HD void compute(const double* W, double mu, bool coulomb) {
+    lu.compute(W);
+    if (!coulomb || negative(mu) || is_zero(mu) || W[0] < kEps) {
+      wTwN0 = wTwN1 = Wb00 = Wb01 = Wb10 = Wb11 = det = D = 0.0;
+      return;
+    }
+    const double wN = W[0], wT0 = W[3], wT1 = W[6];
+    const double inv_wN = ipipe::div_rn(1.0, wN);
+    wTwN0 = wT0 * inv_wN;
+    wTwN1 = wT1 * inv_wN;
+    Wb00 = fma(-wTwN0, wT0, W[4]);
+    Wb01 = fma(-wTwN0, wT1, W[5]);
+    Wb10 = fma(-wTwN1, wT0, W[7]);
+    Wb11 = fma(-wTwN1, wT1, W[8]);
+    det = Wb00 * Wb11 - Wb10 * Wb01;
+    D = ipipe::div_rn(wN * wN, mu * mu);
+  }
+};
+
 template <bool Warp = false>
-BG_HD bool analytic_coulomb(const double* W, const double* b, double* r, double mu) {
-  const double wN = W[0];
-  if (wN < kEps) return false;
+BG_HD bool analytic_coulomb(const double* W, const LocalPrep& pre, const double* b, double* r, double mu) {
+  if (W[0] < kEps) return false;
   const double wT0 = W[3], wT1 = W[6];
+  const double wTwN0 = pre.wTwN0, wTwN1 = pre.wTwN1, Wb00 = pre.Wb00, Wb01 = pre.Wb01, Wb10 = pre.Wb10, Wb11 = pre.Wb11;
   const double bN = b[0];
-  const double inv_wN = ipipe::div_rn(1.0, wN);
-  const double wTwN0 = wT0 * inv_wN, wTwN1 = wT1 * inv_wN;
-  const double Wb00 = fma(-wTwN0, wT0, W[4]);
-  const double Wb01 = fma(-wTwN0, wT1, W[5]);
-  const double Wb10 = fma(-wTwN1, wT0, W[7]);
-  const double Wb11 = fma(-wTwN1, wT1, W[8]);
   const double inv_bN = ipipe::div_rn(1.0, bN);
   const double bb0 = b[1] * inv_bN - wTwN0;
   const double bb1 = b[2] * inv_bN - wTwN1;
   const double A = (Wb00 + Wb11) - dot2(wT0, wT1, bb0, bb1);
   const double B0 = Wb11 * bb0 - Wb10 * bb1;
   const double B1 = Wb00 * bb1 - Wb01 * bb0;
-  const double det = Wb00 * Wb11 - Wb10 * Wb01;
-  const double C = det - dot2(wT0, wT1, B0, B1);
-  const double D = ipipe::div_rn(wN * wN, mu * mu);
+  const double C = pre.det - dot2(wT0, wT1, B0, B1);
+  const double D = pre.D;
   double coeffs[4];
   coeffs[0] = C * C - D * dot2(B0, B1, B0, B1);
   coeffs[1] = 2.0 * (C * A - D * dot2(bb0, bb1, B0, B1));
@@ -886,13 +904,11 @@ enum { kPureNewton = 0, kPureEnumerative = 1, kHybrid = 2, kRevHybrid = 3 };
 // LocalSOCSolver<3, double, DeSaxce, Strat>::solve (mu < 0: full-pivoting LU solve of A x = -b)
 // Warp: called by a whole converged warp with identical arguments (every lane computes the same values).
 template <bool Warp = false>
-BG_HD double local_solve(bool desaxce, int strat, const double* A, const double* b, double* x, double mu, double tol,
-                         double scaling) {
-  if (mu < 0) {
-    SmallLU<3> lu;
-    lu.compute(A);
+BG_HD double local_solve(bool desaxce, int strat, const double* A, const LocalPrep& pre, const double* b, double* x,
+                         double mu, double tol, double scaling) {
+  if (negative(mu)) {
     const double mb[3] = {neg(b[0]), neg(b[1]), neg(b[2])};
-    lu.solve(mb, x);
+    pre.lu.solve(mb, x);
     double ax[3];
     matvec3(A, x, ax);
     const double res[3] = {ax[0] + b[0], ax[1] + b[1], ax[2] + b[2]};
@@ -921,13 +937,11 @@ BG_HD double local_solve(bool desaxce, int strat, const double* A, const double*
   }
   const double x0[3] = {x[0], x[1], x[2]};
   {
-    SmallLU<3> lu;
-    lu.compute(A);
     const double mb[3] = {neg(b[0]), neg(b[1]), neg(b[2])};
-    lu.solve(mb, x);
+    pre.lu.solve(mb, x);
   }
   if (mu * x[0] >= norm2(x[1], x[2])) return 0.0;
-  const bool ok = desaxce ? analytic_coulomb<Warp>(A, b, x, mu) : analytic_soc<Warp>(A, b, x, mu);
+  const bool ok = desaxce ? analytic_coulomb<Warp>(A, pre, b, x, mu) : analytic_soc<Warp>(A, b, x, mu);
   if (!ok) { x[0] = x0[0]; x[1] = x0[1]; x[2] = x0[2]; }
   if (strat == kRevHybrid) {
     res = newton_solve(fb, tol, x);
@@ -939,10 +953,21 @@ BG_HD double local_solve(bool desaxce, int strat, const double* A, const double*
   return res;
 }
 
+BG_HD double local_solve(bool desaxce, int strat, const double* A, const double* b, double* x, double mu, double tol,
+                         double scaling) {
+  LocalPrep pre;
+  pre.compute(A, mu, desaxce);
+  return local_solve<false>(desaxce, strat, A, pre, b, x, mu, tol, scaling);
+}
+
 template <bool Warp = false>
+BG_HD bool law_solve_local(bool desaxce, int strat, const double* A, const LocalPrep& pre, const double* b, double* x,
+                           double mu, double scaling) {
+  return kLocalTol > local_solve<Warp>(desaxce, strat, A, pre, b, x, mu, kLocalTol, scaling);
+}
 BG_HD bool law_solve_local(bool desaxce, int strat, const double* A, const double* b, double* x, double mu,
                            double scaling) {
-  return kLocalTol > local_solve<Warp>(desaxce, strat, A, b, x, mu, kLocalTol, scaling);
+  return kLocalTol > local_solve(desaxce, strat, A, b, x, mu, kLocalTol, scaling);
 }
 
 BG_HD double nesterov_inertia(double& theta, double q) {
