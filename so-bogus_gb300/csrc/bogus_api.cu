@@ -423,6 +423,38 @@ int check_finite(const double* v, size_t m, const char* what) {
   return BOGUS_GPU_OK;
 }
 
+// Grid of a persistent kernel with 8 warps per CTA (max: its resident CTAs): one CTA per SM while its warps take no more
+// than a chunk each, then two, then the maximum; never more CTAs than chunks.
+int spread_grid(int device, int max, int nchunks) {
+  int sms = 0;
+  if (max <= 0 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
+  int want = nchunks <= 8 * sms ? sms : (nchunks <= 16 * sms ? 2 * sms : max);
+  want = std::min(want, nchunks);
+  return std::max(1, std::min(max, want));
+}
+
+// Workspace of the phased kernels (ADMM, DualAMA, adjoint): barrier words and two buffers of `sums` chunk sums.
+int ensure_phases(bogus_gpu_problem* h, size_t sums) {
+  BG_CUDA(h->csum.ensure(2 * (sums > 0 ? sums : 1)));
+  BG_CUDA(h->scal.ensure(8 + 32));  // scalars, then the stripe sums of grid_barrier_combine
+  BG_CUDA(h->barrier.ensure(16));   // [0, 1] barrier, [2] tickets, [4] combine count, [8, 9] the monotonic counter
+  BG_CUDA(h->status.ensure(1));
+  return BOGUS_GPU_OK;
+}
+PhaseState phase_state(const bogus_gpu_problem* h, size_t sums, int chunks) {
+  PhaseState p{};
+  p.mono = reinterpret_cast<unsigned long long*>(h->barrier.p + 8);
+  p.ticket = h->barrier.p + 2;
+  p.combine_count = h->barrier.p + 4;
+  p.csum = h->csum.p;
+  p.half = sums;
+  p.stripes = h->scal.p + 8;
+  p.scal = h->scal.p;
+  p.gb = GridBarrier{h->barrier.p, h->barrier.p + 1, h->status.p, 0};
+  p.flat = chunks <= kFlatChunks;
+  return p;
+}
+
 int ensure_pg_work(bogus_gpu_problem* h, unsigned max_iters) {
   const int n = h->W.n;
   const size_t n3 = 3 * (size_t)n;
@@ -482,15 +514,8 @@ struct HyArgs {
   size_t stride;  // floats between the position buffers' corrections in d
 };
 
-// Grid of the single-problem kernel: one CTA per SM while its 8 warps take no more than a chunk each, then two, then
-// the resident maximum; never more CTAs than chunks.
 int pg_grid(int device, bool fp32, int nchunks) {
-  const int grid = pg_max_grid(device, fp32, true);
-  int sms = 0;
-  if (grid <= 0 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-  int want = nchunks <= 8 * sms ? sms : (nchunks <= 16 * sms ? 2 * sms : grid);
-  want = std::min(want, nchunks);
-  return std::max(1, std::min(grid, want));
+  return spread_grid(device, pg_max_grid(device, fp32, true), nchunks);
 }
 
 // Runs the persistent solver with r already in X[0]; returns the buffer holding the result. hy: FP64 iterations
@@ -2418,10 +2443,7 @@ int run_adjoint(bogus_gpu_problem* h, const bogus_gpu_adjoint_options* o, double
   BG_CUDA(h->adj_dmu.ensure(n > 0 ? n : 1));
   BG_CUDA(h->adj_out.ensure(1));
   const int C = (n + 31) / 32;
-  BG_CUDA(h->csum.ensure(4 * (size_t)(C > 0 ? C : 1)));
-  BG_CUDA(h->scal.ensure(8 + 32));  // scalars, then the stripe sums of grid_barrier_combine
-  BG_CUDA(h->barrier.ensure(8));
-  BG_CUDA(h->status.ensure(1));
+  if (int e = ensure_phases(h, 2 * (size_t)C)) return e;
   if (int e = ensure_interleaved(h)) return e;
   AdjArgs a{};
   a.n = n;
@@ -2449,13 +2471,8 @@ int run_adjoint(bogus_gpu_problem* h, const bogus_gpu_adjoint_options* o, double
   a.Q = h->adj_Q.p;
   a.S = h->adj_S.p;
   a.dmu = h->adj_dmu.p;
-  a.csum = h->csum.p;
-  a.scal = h->scal.p;
   a.out = h->adj_out.p;
-  a.gb = GridBarrier{h->barrier.p, h->barrier.p + 1, h->status.p};
-  a.tickets = h->barrier.p + 2;
-  a.combine_count = h->barrier.p + 4;
-  a.stripes = h->scal.p + 8;
+  a.ps = phase_state(h, 2 * (size_t)C, C);
   a.tol = o->tol;
   a.max_iters = o->max_iters;
   if (o->coulomb) {
@@ -2466,12 +2483,10 @@ int run_adjoint(bogus_gpu_problem* h, const bogus_gpu_adjoint_options* o, double
     a.Sh = h->adj_Sh.p;
     a.Tv = h->adj_Tv.p;
   }
-  BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 8 * sizeof(unsigned), s));
+  BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 16 * sizeof(unsigned), s));
   BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), s));
-  int grid = adjoint_max_grid(h->device);
+  const int grid = spread_grid(h->device, adjoint_max_grid(h->device), C);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
-  const int want = (C + 7) / 8;
-  if (want < grid) grid = want < 1 ? 1 : want;
   BG_CUDA(cudaEventRecord(h->ev0, s));
   BG_CUDA(o->coulomb ? launch_adjoint_coulomb(a, grid, s) : launch_adjoint(a, grid, s));
   BG_CUDA(cudaEventRecord(h->ev1, s));
@@ -2744,12 +2759,9 @@ int bogus_gpu_solve_admm(bogus_gpu_problem* h, const bogus_gpu_admm_options* o, 
   if (f) BG_CUDA(h->a_f.ensure(m));
   if (prox) BG_CUDA(h->a_prox.ensure(m * d));
   const int C = (n + 31) / 32;
-  BG_CUDA(h->csum.ensure(2 * (size_t)(C > 0 ? C : 1)));
-  BG_CUDA(h->scal.ensure(8 + 32));  // scalars, then the stripe sums of grid_barrier_combine
+  if (int e = ensure_phases(h, 2 * (size_t)C)) return e;
   BG_CUDA(h->trace.ensure((size_t)o->max_iters + 1));
   BG_CUDA(h->admm_out.ensure(1));
-  BG_CUDA(h->barrier.ensure(8));
-  BG_CUDA(h->status.ensure(1));
   if (n > 0) {
     BG_CUDA(cudaMemcpyAsync(h->a_w.p, w, sizeof(double) * n3, cudaMemcpyHostToDevice, s));
     if (h->frames_valid) BG_CUDA(launch_frame(n, h->frames.p, h->a_w.p, h->a_w.p, true, s));
@@ -2781,14 +2793,9 @@ int bogus_gpu_solve_admm(bogus_gpu_problem* h, const bogus_gpu_admm_options* o, 
   a.yprev = h->a_yprev.p;
   a.r_spare[0] = h->a_rs1.p;
   a.r_spare[1] = h->a_rs2.p;
-  a.csum = h->csum.p;
-  a.scal = h->scal.p;
   a.trace = h->trace.p;
   a.out = h->admm_out.p;
-  a.gb = GridBarrier{h->barrier.p, h->barrier.p + 1, h->status.p};
-  a.tickets = h->barrier.p + 2;
-  a.combine_count = h->barrier.p + 4;
-  a.stripes = h->scal.p + 8;
+  a.ps = phase_state(h, 2 * (size_t)C, C);
   a.lambda = lambda;
   a.gamma = o->step_size;
   a.tol = o->tol;
@@ -2796,13 +2803,10 @@ int bogus_gpu_solve_admm(bogus_gpu_problem* h, const bogus_gpu_admm_options* o, 
   a.accelerated = o->variant == BOGUS_GPU_ADMM_ACCELERATED;
   a.use_inf = o->use_infinity_norm ? 1 : 0;
   a.scaling = h->a_sc.p;
-  BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 8 * sizeof(unsigned), s));
+  BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 16 * sizeof(unsigned), s));
   BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), s));
-  int grid = admm_max_grid(h->device, d);
+  const int grid = spread_grid(h->device, admm_max_grid(h->device, d), ((n > nb ? n : nb) + 31) / 32);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
-  const int units = ((n > nb ? n : nb) + 31) / 32;
-  const int want = (units + 7) / 8;
-  if (want < grid) grid = want < 1 ? 1 : want;
   BG_CUDA(cudaEventRecord(h->ev0, s));
   BG_CUDA(launch_admm(a, grid, s));
   BG_CUDA(cudaEventRecord(h->ev1, s));
@@ -2889,12 +2893,9 @@ int bogus_gpu_solve_dual_ama(bogus_gpu_problem* h, const bogus_gpu_dual_ama_opti
   BG_CUDA(h->a_mu.ensure(n > 0 ? n : 1));
   const int C = (n + 31) / 32, CB = (nb + 31) / 32;
   const int CC = C > CB ? C : CB;
-  BG_CUDA(h->csum.ensure(3 * (size_t)(CC > 0 ? CC : 1)));
-  BG_CUDA(h->scal.ensure(8 + 32));  // scalars, then the stripe sums of grid_barrier_combine
+  if (int e = ensure_phases(h, 3 * (size_t)CC)) return e;
   BG_CUDA(h->trace.ensure((size_t)o->max_iters + 1));
   BG_CUDA(h->dama_out.ensure(1));
-  BG_CUDA(h->barrier.ensure(8));
-  BG_CUDA(h->status.ensure(1));
   if (n > 0) {
     BG_CUDA(cudaMemcpyAsync(h->a_w.p, w, sizeof(double) * n3, cudaMemcpyHostToDevice, s));
     if (h->frames_valid) BG_CUDA(launch_frame(n, h->frames.p, h->a_w.p, h->a_w.p, true, s));
@@ -2933,14 +2934,9 @@ int bogus_gpu_solve_dual_ama(bogus_gpu_problem* h, const bogus_gpu_dual_ama_opti
   a.yp_spare = h->dm_yp2.p;
   a.r_best = h->dm_rb.p;
   a.v_best = h->dm_vb.p;
-  a.csum = h->csum.p;
-  a.scal = h->scal.p;
   a.trace = h->trace.p;
   a.out = h->dama_out.p;
-  a.gb = GridBarrier{h->barrier.p, h->barrier.p + 1, h->status.p};
-  a.tickets = h->barrier.p + 2;
-  a.combine_count = h->barrier.p + 4;
-  a.stripes = h->scal.p + 8;
+  a.ps = phase_state(h, 3 * (size_t)CC, CC);
   a.tol = o->tol;
   a.gamma = o->fp_step_size;
   a.lambda0 = o->proj_step_size;
@@ -2952,12 +2948,10 @@ int bogus_gpu_solve_dual_ama(bogus_gpu_problem* h, const bogus_gpu_dual_ama_opti
   a.accelerated = o->variant == BOGUS_GPU_ADMM_ACCELERATED;
   a.use_inf = o->use_infinity_norm ? 1 : 0;
   a.desaxce = static_problem ? 0 : 1;
-  BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 8 * sizeof(unsigned), s));
+  BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 16 * sizeof(unsigned), s));
   BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), s));
-  int grid = dama_max_grid(h->device, d);
+  const int grid = spread_grid(h->device, dama_max_grid(h->device, d), CC);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
-  const int want = (CC + 7) / 8;
-  if (want < grid) grid = want < 1 ? 1 : want;
   BG_CUDA(cudaEventRecord(h->ev0, s));
   BG_CUDA(launch_dama(a, grid, s));
   BG_CUDA(cudaEventRecord(h->ev1, s));

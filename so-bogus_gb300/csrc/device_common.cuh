@@ -385,24 +385,6 @@ __device__ __forceinline__ bool grid_barrier_combine(const GridBarrier& gb, unsi
   return ok;
 }
 
-// Dynamic work split: warps take 32-contact (or 32-body) chunks from a ticket counter, one per phase parity,
-// cleared by the last CTA of the barrier that ends the phase (every draw of the phase is done by then), so SMs
-// whose sub-partitions finish early take more chunks. Chunk sums are stored by chunk index, so the reduction
-// order does not depend on which warp handled a chunk.
-struct Tickets {
-  unsigned* t;         // 2 counters, zero at launch
-  unsigned phase = 0;  // barriers passed (identical in every CTA)
-  __device__ int next() {
-    int c = 0;
-    if ((threadIdx.x & 31) == 0) c = (int)atomicAdd(t + (phase & 1u), 1u);
-    return __shfl_sync(0xffffffffu, c, 0);
-  }
-  // run by every thread of the barrier's last CTA
-  __device__ void clear() {
-    if (threadIdx.x == 0) t[phase & 1u] = 0u;
-  }
-};
-
 // ---- grid barrier on monotonic counters (single-problem persistent solvers) ------------------------------
 // mono[0] counts CTA arrivals, mono[1] finished stripe combinations, mono[2] published reductions; all start
 // at zero at launch and only grow. Barrier k of a launch is complete when mono[0] reaches parties (k + 1),
@@ -520,6 +502,12 @@ __device__ __forceinline__ bool mono_barrier_combine(const MonoBarrier& mb, unsi
   return ok;
 }
 
+// Problems of up to this many chunks reduce by the flat barrier. us per SPG iteration (two reductions) on GB300, stripes
+// combined by the last CTAs / flat: 500 contacts 41 / 26, 10 000 46 / 33, 40 000 (1 250 chunks) 65 / 50, the grid rule
+// (pg_grid) included. Every CTA repeats the additions, 8 C / 256 FP64 instructions per quantity and SM: 64 at 2 048
+// chunks, about the round trips saved.
+constexpr int kFlatChunks = 2048;
+
 // ---- flat reducing barrier (problems of a few chunks per SM) ----------------------------------------------
 // Every CTA waits until all have arrived and then combines all chunk sums for itself, in the canonical order: one
 // round trip to L2 after the last arrival in place of the three (stripes, publication, scalars) of
@@ -612,6 +600,69 @@ __device__ __forceinline__ void flat_combine(const double* s, size_t stride, int
   }
   __syncthreads();
 }
+
+// Phases of a persistent kernel (ADMM, DualAMA, the adjoint): units of work (32-contact or 32-body chunks) handed to
+// the warps, barriers, reductions. A phase opens with begin(units); a warp takes units from next() until it returns
+// one past the end.
+// - Work: while every unit gets a warp of its own, unit u goes to CTA u % G, so a small problem spreads over the SMs
+//   before a CTA gets a second unit, and nothing is drawn; beyond that, units come from a ticket counter. The counter
+//   is never reset: a phase's draws are its units and one failing draw per warp, so every CTA knows where the next
+//   phase starts.
+// - Reductions: the flat barrier up to kFlatChunks chunks (two buffers of chunk sums, sums(), alternating by phase),
+//   else the stripes of grid_barrier_combine. Both add in the canonical order.
+struct PhaseState {
+  unsigned long long* mono;
+  unsigned* ticket;         // zero at launch
+  unsigned* combine_count;  // grid_barrier_combine's counter; zero at launch
+  double* csum;             // two buffers of `half` doubles when flat, one otherwise
+  size_t half;
+  double* stripes;
+  double* scal;
+  GridBarrier gb;
+  int flat;
+};
+struct Phases {
+  const PhaseState& s;
+  double* smem32;
+  double* out;  // 4 shared scalars
+  unsigned phase = 0, base = 0, units = 0;
+  int turn = 0;
+  __device__ void begin(int n) {
+    units = (unsigned)n;
+    turn = 0;
+  }
+  __device__ bool one_each() const { return units <= gridDim.x * (blockDim.x >> 5); }
+  __device__ int next() {
+    if (one_each()) return turn++ == 0 ? (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x) : (int)units;
+    unsigned c = 0;
+    if ((threadIdx.x & 31) == 0) c = atomicAdd(s.ticket, 1u) - base;
+    return (int)__shfl_sync(0xffffffffu, c, 0);
+  }
+  __device__ void close() {
+    if (!one_each()) base += units + gridDim.x * (blockDim.x >> 5);
+    ++phase;
+  }
+  __device__ double* sums() const { return s.csum + (s.flat ? (size_t)(phase & 1u) * s.half : 0); }
+  __device__ MonoBarrier mb() const { return MonoBarrier{s.mono, s.gb.status, gridDim.x}; }
+  __device__ bool sync() {
+    const bool ok = s.flat ? flat_barrier(mb(), phase) : grid_barrier(s.gb, [] {});
+    close();
+    return ok;
+  }
+  // K <= 4 quantities, quantity q's chunk sums at sums() + q * stride: count0 chunks for q = 0, count1 for the others
+  __device__ bool reduce(int K, size_t stride, int count0, int count1, unsigned maxmask) {
+    if (s.flat) {
+      if (!flat_barrier(mb(), phase)) return false;
+      flat_combine(sums(), stride, count0, count1, K, maxmask, smem32, out);
+    } else if (!grid_barrier_combine(s.gb, s.combine_count, s.csum, stride, count0, count1, K, maxmask, s.stripes,
+                                     s.scal, [] {})) {
+      return false;
+    }
+    close();
+    return true;
+  }
+  __device__ double scal(int q) const { return s.flat ? out[q] : ldcg(s.scal + q); }
+};
 
 // One warp: wait until reduction `published` - 1 is published (mono[2] >= published). Every lane of the warp
 // must call it; the lanes read the scalars after it returns.

@@ -162,11 +162,6 @@ cudaError_t launch_expand_lower(int nnz, const int* src, const double* low, doub
 cudaError_t launch_add(int m, const double* a, const double* b, double* y, cudaStream_t s);
 cudaError_t launch_cadoux_rhs(int n, const double* y, const double* mu, const double* b, double* out, cudaStream_t s);
 
-// Problems of up to this many chunks reduce by the flat barrier. us per SPG iteration (two reductions) on GB300, stripes
-// combined by the last CTAs / flat: 500 contacts 41 / 26, 10 000 46 / 33, 40 000 (1 250 chunks) 65 / 50, the grid rule
-// (pg_grid) included. Every CTA repeats the additions, 8 C / 256 FP64 instructions per quantity and SM: 64 at 2 048
-// chunks, about the round trips saved.
-constexpr int kFlatChunks = 2048;
 // Persistent solvers (kernels_pg.cu)
 cudaError_t launch_pg_persistent(const PGArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_pg_persistent(const PGArgs32& a, int grid, cudaStream_t s);
@@ -260,14 +255,9 @@ struct ADMMArgs {
   double* inv_mu;      // n (written)
   double *x, *r, *ut, *z, *zacc, *yprev;
   double* r_spare[2];  // 3 n each: the two candidate updates of r (r, r_spare[0], r_spare[1] rotate)
-  double* csum;        // 2 x nchunks
-  double* scal;        // published scalars
-  unsigned* combine_count;  // grid_barrier_combine's counter; zero at launch
-  unsigned* tickets;        // 2 chunk-ticket counters (one per phase parity); zero at launch
-  double* stripes;          // 8 stripe sums per reduced quantity
+  PhaseState ps;       // chunk sums: 2 x nchunks
   double* trace;       // max_iters entries, or null
   ADMMOut* out;
-  GridBarrier gb;
   double lambda, gamma, tol;
   unsigned max_iters;
   int accelerated, use_inf;
@@ -296,14 +286,9 @@ struct DamaArgs {
   const double* scaling;  // n
   double *v, *r, *rs, *x, *HrBp, *ut, *g, *y_prev, *r_best, *v_best;
   double *v_spare, *yp_spare;  // nbodies x d each: the line search's candidate v and y_prev
-  double* csum;           // 3 x max(contact chunks, body chunks)
-  double* scal;
-  unsigned* combine_count;  // grid_barrier_combine's counter; zero at launch
-  unsigned* tickets;        // 2 chunk-ticket counters (one per phase parity); zero at launch
-  double* stripes;          // 8 stripe sums per reduced quantity
+  PhaseState ps;          // chunk sums: 3 x max(contact chunks, body chunks)
   double* trace;          // max_iters
   DamaOut* out;
-  GridBarrier gb;
   double tol, gamma, lambda0, opt, pess, m_true;
   unsigned max_iters, ls_iters;
   int accelerated, use_inf, desaxce;
@@ -334,13 +319,8 @@ struct AdjArgs {
   double *P, *R, *Z, *Dir, *Y, *Q;  // conjugate-gradient vectors (3 per contact)
   double* S;           // out: dL/db
   double* dmu;         // out: dL/dmu
-  double* csum;
-  double* scal;
-  unsigned* combine_count;  // grid_barrier_combine's counter; zero at launch
-  unsigned* tickets;        // 2 chunk-ticket counters (one per phase parity); zero at launch
-  double* stripes;          // 8 stripe sums per reduced quantity
+  PhaseState ps;  // chunk sums: 2 x nchunks
   AdjOut* out;
-  GridBarrier gb;
   double tol;
   unsigned max_iters;
   // Coulomb law (De Saxce change of variable, bi-conjugate gradients stabilised): per contact (|u_T|, tau) with

@@ -20,7 +20,7 @@
 //   dL/db = s = -V M p,   lam_hat (masked) = v_k^T (g + W s),   lam_hat (unmasked) = p_k / (alpha theta_k),
 //   dL/dmu_i = K_i^T V_i lam_hat_i with K = dP/dmu(x).
 // A persistent cooperative kernel runs the setup, the CG iterations and the final pass; reductions use the
-// canonical order of the solver kernels, waits are bounded (grid_barrier).
+// canonical order of the solver kernels, waits are bounded (Phases).
 #include "internal.h"
 #include "soc_device.cuh"
 #include "spmv_chunk.cuh"
@@ -138,36 +138,17 @@ __device__ __forceinline__ void basis_apply_t(const double* V, const double* D, 
   }
 }
 
-// Warps take chunks from ticket counters (Tickets: dynamic balance; the chunk sums stay in chunk order).
-struct AdjCtx {
-  const AdjArgs& a;
-  double* smem8;
-  Tickets tk{a.tickets};
-  __device__ int next() { return tk.next(); }
-  __device__ bool sync() {
-    const bool ok = grid_barrier(a.gb, [&] { tk.clear(); });
-    ++tk.phase;
-    return ok;
-  }
-  __device__ bool sync_reduce(int K) {
-    const bool ok = grid_barrier_combine(a.gb, a.combine_count, a.csum, (size_t)a.nchunks, a.nchunks, a.nchunks, K,
-                                         0u, a.stripes, a.scal, [&] { tk.clear(); });
-    ++tk.phase;
-    return ok;
-  }
-};
-
 __global__ void __launch_bounds__(256) k_adjoint(AdjArgs a) {
-  __shared__ double smem8[8];
+  __shared__ double smem32[32], out[4];
   __shared__ ChunkScratch cs[8];
-  AdjCtx ctx{a, smem8};
+  Phases ctx{a.ps, smem32, out};
   ChunkScratch& sh = cs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int C = a.nchunks;
   const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
   auto put = [&](int q, int c, double v) {
     v = warp_sum_butterfly(v);
-    if (lane == 0) a.csum[q * C + c] = v;
+    if (lane == 0) ctx.sums()[q * C + c] = v;
   };
   auto product = [&](int c, const double* src, double* acc) {
     spmv_chunk<1>(a.rowptr, InterleavedBlocks<double>{a.icol, a.ival, a.slot0}, a.n, c, sh,
@@ -176,6 +157,7 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjArgs a) {
 
   // setup: x = r - alpha (W r + b), the basis, the preconditioner, rhs c = m o V^T g; p = 0, res = c,
   // z = Pinv c, dir = z, Y = V (m o dir)
+  ctx.begin(C);
   for (int c = ctx.next(); c < C; c = ctx.next()) {
     const int i = 32 * c + lane;
     double acc[3] = {0.0, 0.0, 0.0};
@@ -211,15 +193,16 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjArgs a) {
     put(0, c, rr);
     put(1, c, rz);
   }
-  if (!ctx.sync_reduce(2)) return;
-  const double rr0 = ldcg(a.scal);
+  if (!ctx.reduce(2, (size_t)C, C, C, 0u)) return;
+  const double rr0 = ctx.scal(0);
   double rr = rr0;
-  double rz = ldcg(a.scal + 1);
+  double rz = ctx.scal(1);
   unsigned it = 0;
   const double stop = a.tol * a.tol * rr0;
   for (; it < a.max_iters; ++it) {
     if (!(rr > stop)) break;
     // q = D o dir + m o V^T W Y, dir . q
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       double acc[3] = {0.0, 0.0, 0.0};
@@ -237,10 +220,11 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjArgs a) {
       }
       put(0, c, dq);
     }
-    if (!ctx.sync_reduce(1)) return;
-    const double dq = ldcg(a.scal);
+    if (!ctx.reduce(1, (size_t)C, C, C, 0u)) return;
+    const double dq = ctx.scal(0);
     if (!(dq > 0.0)) break;  // S is positive definite on the unmasked components; guards exact convergence
     const double step = rz / dq;
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       double v = 0.0, w = 0.0;
@@ -265,11 +249,12 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjArgs a) {
       put(0, c, v);
       put(1, c, w);
     }
-    if (!ctx.sync_reduce(2)) return;
-    rr = ldcg(a.scal);
-    const double rz_new = ldcg(a.scal + 1);
+    if (!ctx.reduce(2, (size_t)C, C, C, 0u)) return;
+    rr = ctx.scal(0);
+    const double rz_new = ctx.scal(1);
     const double beta = rz_new / rz;
     rz = rz_new;
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       if (i < a.n) {
@@ -287,6 +272,7 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjArgs a) {
     if (!ctx.sync()) return;
   }
   // s = dL/db = -V (m o p)
+  ctx.begin(C);
   for (int c = ctx.next(); c < C; c = ctx.next()) {
     const int i = 32 * c + lane;
     if (i < a.n) {
@@ -301,6 +287,7 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjArgs a) {
   }
   if (!ctx.sync()) return;
   // lam_hat and dL/dmu = K^T V lam_hat
+  ctx.begin(C);
   for (int c = ctx.next(); c < C; c = ctx.next()) {
     const int i = 32 * c + lane;
     double acc[3] = {0.0, 0.0, 0.0};
@@ -401,16 +388,16 @@ __device__ void precond_block_coulomb(const double* V, const double* D, const do
 }
 
 __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
-  __shared__ double smem8[8];
+  __shared__ double smem32[32], out[4];
   __shared__ ChunkScratch cs[8];
-  AdjCtx ctx{a, smem8};
+  Phases ctx{a.ps, smem32, out};
   ChunkScratch& sh = cs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int C = a.nchunks;
   const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
   auto put = [&](int q, int c, double v) {
     v = warp_sum_butterfly(v);
-    if (lane == 0) a.csum[q * C + c] = v;
+    if (lane == 0) ctx.sums()[q * C + c] = v;
   };
   auto product = [&](int c, const double* src, double* acc) {
     spmv_chunk<1>(a.rowptr, InterleavedBlocks<double>{a.icol, a.ival, a.slot0}, a.n, c, sh,
@@ -430,6 +417,7 @@ __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
   };
   // setup: u = W r + b, s(u), x = r - alpha (u + s(u)), the basis, tau, the preconditioner; rhs c = m o V^T g;
   // p = 0, residual = shadow = c, direction = v = 0
+  ctx.begin(C);
   for (int c = ctx.next(); c < C; c = ctx.next()) {
     const int i = 32 * c + lane;
     double acc[3] = {0.0, 0.0, 0.0};
@@ -472,8 +460,8 @@ __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
     }
     put(0, c, rr);
   }
-  if (!ctx.sync_reduce(1)) return;
-  const double rr0 = ldcg(a.scal);
+  if (!ctx.reduce(1, (size_t)C, C, C, 0u)) return;
+  const double rr0 = ctx.scal(0);
   double rr = rr0, rho_old = 1.0, alpha = 1.0, omega = 1.0, rho = rr0;
   unsigned it = 0;
   const double stop = a.tol * a.tol * rr0;
@@ -481,6 +469,7 @@ __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
     if (!(rr > stop)) break;
     const double beta = (rho / rho_old) * (alpha / omega);
     // direction = r + beta (direction - omega v); ph = Pinv direction; Y = T^T V (m o ph)
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       if (i < a.n) {
@@ -500,6 +489,7 @@ __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
     }
     if (!ctx.sync()) return;
     // v = A ph; shadow . v
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       double acc[3] = {0.0, 0.0, 0.0};
@@ -515,11 +505,12 @@ __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
       }
       put(0, c, hv);
     }
-    if (!ctx.sync_reduce(1)) return;
-    const double hv = ldcg(a.scal);
+    if (!ctx.reduce(1, (size_t)C, C, C, 0u)) return;
+    const double hv = ctx.scal(0);
     if (!(hv != 0.0)) break;  // breakdown (or exact convergence)
     alpha = rho / hv;
     // s = r - alpha v; sh = Pinv s; Y = T^T V (m o sh)
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       if (i < a.n) {
@@ -538,6 +529,7 @@ __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
     }
     if (!ctx.sync()) return;
     // t = A sh; t . s, t . t
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       double acc[3] = {0.0, 0.0, 0.0};
@@ -555,10 +547,11 @@ __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
       put(0, c, ts);
       put(1, c, tt);
     }
-    if (!ctx.sync_reduce(2)) return;
-    const double ts = ldcg(a.scal), tt = ldcg(a.scal + 1);
+    if (!ctx.reduce(2, (size_t)C, C, C, 0u)) return;
+    const double ts = ctx.scal(0), tt = ctx.scal(1);
     omega = tt > 0.0 ? ts / tt : 0.0;
     // p += alpha ph + omega sh; r = s - omega t; shadow . r, r . r
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       double hr = 0.0, r2 = 0.0;
@@ -582,16 +575,17 @@ __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
       put(0, c, hr);
       put(1, c, r2);
     }
-    if (!ctx.sync_reduce(2)) return;
+    if (!ctx.reduce(2, (size_t)C, C, C, 0u)) return;
     rho_old = rho;
-    rho = ldcg(a.scal);
-    rr = ldcg(a.scal + 1);
+    rho = ctx.scal(0);
+    rr = ctx.scal(1);
     if (!(omega != 0.0)) {
       ++it;
       break;
     }
   }
   // s = dL/db = -T^T V (m o p)
+  ctx.begin(C);
   for (int c = ctx.next(); c < C; c = ctx.next()) {
     const int i = 32 * c + lane;
     if (i < a.n) {
@@ -605,6 +599,7 @@ __global__ void __launch_bounds__(256) k_adjoint_coulomb(AdjArgs a) {
   }
   if (!ctx.sync()) return;
   // lam_hat and dL/dmu = K^T V lam_hat - |u_T| (V m o p)_N
+  ctx.begin(C);
   for (int c = ctx.next(); c < C; c = ctx.next()) {
     const int i = 32 * c + lane;
     double acc[3] = {0.0, 0.0, 0.0};

@@ -20,7 +20,7 @@
 // Body b's H^T accumulation runs over its contacts in increasing contact index, rows 0..2, one FMA chain
 // per dof; contact rows accumulate w, then the slots in body order, dofs 0..d-1; the prox product is an FMA
 // chain over the dofs. Sums use the canonical order (32-contact butterflies, 8 stripes), so the GPU's
-// iterates and residuals equal the CPU oracle's bit for bit. Waits are bounded (grid_barrier).
+// iterates and residuals equal the CPU oracle's bit for bit. Waits are bounded (Phases).
 #include "internal.h"
 #include "soc_device.cuh"
 
@@ -29,25 +29,6 @@ namespace bogus_gpu {
 namespace {
 
 constexpr int kMaxDof = 12;
-
-struct AdmmCtx {
-  const ADMMArgs& a;
-  double* smem8;
-  int nchunks;
-  Tickets tk{a.tickets};
-  __device__ int next() { return tk.next(); }
-  __device__ bool sync() {
-    const bool ok = grid_barrier(a.gb, [&] { tk.clear(); });
-    ++tk.phase;
-    return ok;
-  }
-  __device__ bool sync_reduce2(unsigned maxmask) {
-    const bool ok = grid_barrier_combine(a.gb, a.combine_count, a.csum, (size_t)nchunks, nchunks, nchunks, 2, maxmask,
-                                         a.stripes, a.scal, [&] { tk.clear(); });
-    ++tk.phase;
-    return ok;
-  }
-};
 
 // D > 0: d fixed at compile time (registers); D == 0: runtime d <= kMaxDof.
 template <int D>
@@ -94,12 +75,12 @@ __device__ __forceinline__ void store3(double* p, int i, const double* v) {
 }
 
 template <int D>
-__device__ void admm_body(const ADMMArgs& a, AdmmCtx& ctx) {
+__device__ void admm_body(const ADMMArgs& a, Phases& ctx) {
   constexpr int DM = D > 0 ? D : kMaxDof;
   constexpr bool kPair = D > 0 && D % 2 == 0;
   const int d = dofs<D>(a);
   const int lane = threadIdx.x & 31;
-  const int C = ctx.nchunks;
+  const int C = (a.n + 31) / 32;
   const int CB = (a.nbodies + 31) / 32;
   const double gamma = a.gamma;
   const double inv_gamma = 1. / gamma;
@@ -108,11 +89,12 @@ __device__ void admm_body(const ADMMArgs& a, AdmmCtx& ctx) {
   const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
   auto put = [&](int q, int c, double v, bool is_max) {
     v = is_max ? warp_max_butterfly(v) : warp_sum_butterfly(v);
-    if (lane == 0) a.csum[q * C + c] = v;
+    if (lane == 0) ctx.sums()[q * C + c] = v;
   };
 
   // Setup (:64-77): ut = w + H x, z = P(ut - r / gamma), y_prev = -r / gamma, zacc = z_prev = z (the last two
   // derived: plain = true)
+  ctx.begin(C);
   for (int c = ctx.next(); c < C; c = ctx.next()) {
     const int i = 32 * c + lane;
     if (i < a.n) {
@@ -143,6 +125,7 @@ __device__ void admm_body(const ADMMArgs& a, AdmmCtx& ctx) {
       constexpr int H2 = kPair ? D / 2 : 1;
       const int half = lane & 1;
       const int CB2 = (a.nbodies + 15) / 16;
+      ctx.begin(CB2);
       for (int c = ctx.next(); c < CB2; c = ctx.next()) {
         const int slot = 16 * c + (lane >> 1);
         const bool on = slot < a.nbodies;
@@ -213,6 +196,7 @@ __device__ void admm_body(const ADMMArgs& a, AdmmCtx& ctx) {
         }
       }
     } else {
+      ctx.begin(CB);
       for (int c = ctx.next(); c < CB; c = ctx.next()) {
         const int slot = 32 * c + lane;
         if (slot < a.nbodies) {
@@ -305,6 +289,7 @@ __device__ void admm_body(const ADMMArgs& a, AdmmCtx& ctx) {
     const int ia = (cur + 1) % 3, ip = a.accelerated ? (cur + 2) % 3 : (cur + 1) % 3;
     double* r_acc = rb[ia];
     double* r_plain = rb[ip];
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       double ev = 0.0, gap = 0.0;
@@ -348,10 +333,11 @@ __device__ void admm_body(const ADMMArgs& a, AdmmCtx& ctx) {
       put(0, c, ev, a.use_inf != 0);
       put(1, c, gap, a.use_inf != 0);
     }
-    if (!ctx.sync_reduce2(a.use_inf ? 3u : 0u)) return;
+    if (!ctx.reduce(2, (size_t)C, C, C, a.use_inf ? 3u : 0u)) return;
     {
-      const double e0 = ldcg(a.scal), g0 = ldcg(a.scal + 1);
-      res = a.use_inf ? e0 + g0 : e0 / (double)(1 + a.n) + g0 / (double)(1 + 3 * (size_t)a.n);
+      const double e0 = ctx.scal(0), g0 = ctx.scal(1);
+      res = a.use_inf ? e0 + g0
+                      : ipipe::div_rn(e0, (double)(1 + a.n)) + ipipe::div_rn(g0, (double)(1 + 3 * (size_t)a.n));
     }
     if (a.trace && writer) a.trace[it] = res;
     if (res < a.tol) break;
@@ -369,6 +355,7 @@ __device__ void admm_body(const ADMMArgs& a, AdmmCtx& ctx) {
   }
   // the final r in the caller's buffer (nothing reads the spare buffers after the last barrier)
   if (cur != 0) {
+    ctx.begin(C);
     for (int c = ctx.next(); c < C; c = ctx.next()) {
       const int i = 32 * c + lane;
       if (i < a.n) {
@@ -387,8 +374,8 @@ __device__ void admm_body(const ADMMArgs& a, AdmmCtx& ctx) {
 
 template <int D>
 __global__ void __launch_bounds__(256) k_admm_persistent(ADMMArgs a) {
-  __shared__ double smem8[8];
-  AdmmCtx ctx{a, smem8, (a.n + 31) / 32};
+  __shared__ double smem32[32], out[4];
+  Phases ctx{a.ps, smem32, out};
   admm_body<D>(a, ctx);
 }
 
@@ -410,7 +397,7 @@ __global__ void __launch_bounds__(256) k_admm_persistent(ADMMArgs a) {
 // body's contacts in increasing order, rows inner; H z and H v as the ADMM kernel's products; dof norms each body's
 // dofs left to right, then the canonical sum over bodies.
 template <int D>
-__device__ void dama_body(const DamaArgs& a, double* smem8) {
+__device__ void dama_body(const DamaArgs& a, Phases& ctx) {
   constexpr int DM = D > 0 ? D : kMaxDof;
   const int d = D > 0 ? D : a.d;
   const int lane = threadIdx.x & 31;
@@ -420,21 +407,13 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
   const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
   auto put = [&](int q, int c, double v, bool is_max) {
     v = is_max ? warp_max_butterfly(v) : warp_sum_butterfly(v);
-    if (lane == 0) a.csum[q * CC + c] = v;
+    if (lane == 0) ctx.sums()[q * CC + c] = v;
   };
-  Tickets tk{a.tickets};
-  auto next = [&]() { return tk.next(); };
-  auto sync = [&]() {
-    const bool ok = grid_barrier(a.gb, [&] { tk.clear(); });
-    ++tk.phase;
-    return ok;
-  };
+  auto next = [&]() { return ctx.next(); };
+  auto sync = [&]() { return ctx.sync(); };
   // value 0 over count0 chunks, values 1.. over count1 chunks
   auto sync_reduce = [&](int K, int count0, int count1, unsigned maxmask) {
-    const bool ok = grid_barrier_combine(a.gb, a.combine_count, a.csum, (size_t)CC, count0, count1, K, maxmask,
-                                         a.stripes, a.scal, [&] { tk.clear(); });
-    ++tk.phase;
-    return ok;
+    return ctx.reduce(K, (size_t)CC, count0, count1, maxmask);
   };
   // H^T src for body b (d values): per dof, contacts in increasing order, rows inner
   auto body_HT = [&](int b, const double* src, double* out) {
@@ -496,6 +475,7 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
   double* vn = a.v_spare;
   double* ypn = a.yp_spare;
   // H^T r once
+  ctx.begin(CB);
   for (int c = next(); c < CB; c = next()) {
     const int b = 32 * c + lane;
     if (b < a.nbodies) {
@@ -512,6 +492,7 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
   int stopped = 0;
   for (; it < a.max_iters; ++it) {
     // Q1: tickets [0, CB) take body chunks, [CB, CB + C) contact chunks
+    ctx.begin(CB + C);
     for (int t = next(); t < CB + C; t = next()) {
       if (t >= CB) {
         const int c = t - CB;
@@ -553,10 +534,10 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
     }
     if (!sync_reduce(3, C, CB, inf ? 3u : 0u)) return;
     {
-      const double e0 = ldcg(a.scal), z0 = ldcg(a.scal + 1);
-      res = (inf ? e0 : e0 / (double)(1 + a.n)) + (inf ? z0 : z0 / (1.0 + a.m_true));
+      const double e0 = ctx.scal(0), z0 = ctx.scal(1);
+      res = (inf ? e0 : ipipe::div_rn(e0, (double)(1 + a.n))) + (inf ? z0 : ipipe::div_rn(z0, 1.0 + a.m_true));
     }
-    const double h0 = ldcg(a.scal + 2);
+    const double h0 = ctx.scal(2);
     if (a.trace && writer) a.trace[it] = res;
     const bool best = res < min_res || it == 0;
     if (best) min_res = res;
@@ -575,6 +556,7 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
     if (!done && a.ls_iters != 0) lambda *= a.opt;
     double* q3_out = a.ls_iters == 0 ? r : rs;
     const int q2_end = C + (best ? CB : 0);
+    ctx.begin(q2_end);
     for (int t = next(); t < q2_end; t = next()) {
       if (t >= C) {
         const int b = 32 * (t - C) + lane;
@@ -635,6 +617,7 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
         if (ls > 0) {
           ++trials;
           // Q3: r_s = P(r - lambda g) for a later trial
+          ctx.begin(C);
           for (int c = next(); c < C; c = next()) {
             const int i = 32 * c + lane;
             if (i < a.n) {
@@ -647,6 +630,7 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
           if (!sync()) return;
         }
         // Q4
+        ctx.begin(CB);
         for (int c = next(); c < CB; c = next()) {
           const int b = 32 * c + lane;
           double ph = 0.0;
@@ -674,7 +658,7 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
           put(0, c, ph, false);
         }
         if (!sync_reduce(1, CB, CB, 0u)) return;
-        const double hh = ldcg(a.scal);
+        const double hh = ctx.scal(0);
         if (hh < h0) break;
         lambda *= a.pess;
       }
@@ -692,6 +676,7 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
     }
     // Q5 (no line search): z = H^T r - x, y = v + gamma z, v = y + beta (y - y_prev)
     if (a.ls_iters == 0) {
+      ctx.begin(CB);
       for (int c = next(); c < CB; c = next()) {
         const int b = 32 * c + lane;
         if (b < a.nbodies) {
@@ -723,8 +708,9 @@ __device__ void dama_body(const DamaArgs& a, double* smem8) {
 
 template <int D>
 __global__ void __launch_bounds__(256) k_dama_persistent(DamaArgs a) {
-  __shared__ double smem8[8];
-  dama_body<D>(a, smem8);
+  __shared__ double smem32[32], out[4];
+  Phases ctx{a.ps, smem32, out};
+  dama_body<D>(a, ctx);
 }
 
 }  // namespace
