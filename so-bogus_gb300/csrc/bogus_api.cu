@@ -152,7 +152,8 @@ struct bogus_gpu_problem {
   // projected-gradient work
   DevBuf<double> X, MX, Y, S0, XB, Wv, csum, scal, trace;
   // interleaved copy of W (coalesced chunk layout read by the single-problem solvers), valid while W is unchanged
-  bool il_valid = false;
+  bool il_valid = false;      // the interleaved copy
+  bool chunks_valid = false;  // h_chunk_order, h_chunk_seg
   DevBuf<long long> slot0;
   DevBuf<int> chunk_order;  // chunks by decreasing segment length (ticket order of the persistent solvers)
   std::vector<int> h_chunk_order;  // the same on the host
@@ -221,6 +222,11 @@ struct bogus_gpu_problem {
   std::vector<int> h_contact_ptr, h_problem_nnz;
   DevBuf<int> contact_ptr, chunk_ptr, queue, col_local, next;
   DevBuf<PGOut> batch_out;
+  // resident form of the batched solve (plan_resident_batch): job lists per CTA, barrier counters; rb_ctas 0: not used
+  DevBuf<int> rb_ptr;
+  DevBuf<ResidentJob> rb_jobs;
+  DevBuf<unsigned long long> rb_mono;
+  int rb_ctas = 0, rb_teams = 0, rb_steps = 0;
   DevBuf<unsigned> team_cnt;  // team schedule of the batched solve: counters, jobs, published scalars
   DevBuf<int> team_job;
   DevBuf<double> team_scal;
@@ -295,6 +301,7 @@ int upload_full(bogus_gpu_problem* h, const HostBSR& f, const double* b, const d
   h->fp32_valid = false;
   h->fp32p_valid = false;
   h->il_valid = false;
+  h->chunks_valid = false;
   h->adj_valid = false;
   return BOGUS_GPU_OK;
 }
@@ -382,6 +389,7 @@ int set_dual_lower(bogus_gpu_problem* h, int n, const int* rowptr, const int* co
   h->fp32_valid = false;
   h->fp32p_valid = false;
   h->il_valid = false;
+  h->chunks_valid = false;
   h->adj_valid = false;
   return BOGUS_GPU_OK;
 }
@@ -474,6 +482,7 @@ int ensure_pg_work(bogus_gpu_problem* h, unsigned max_iters) {
   return BOGUS_GPU_OK;
 }
 
+int ensure_chunks(bogus_gpu_problem* h);
 int ensure_interleaved(bogus_gpu_problem* h);
 int ensure_cta_lists(bogus_gpu_problem* h, int G);
 int ensure_incidence(bogus_gpu_problem* h);
@@ -524,17 +533,13 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
            const HyArgs* hy = nullptr) {
   const int n = h->W.n;
   const size_t n3 = 3 * (size_t)n;
-  if (int e = ensure_interleaved(h)) return e;
+  if (int e = ensure_chunks(h)) return e;
   PGArgs a{};
   a.n = n;
   a.nchunks = (n + 31) / 32;
   a.rowptr = h->W.rowptr;
   a.col = h->W.col;
   a.val = h->W.val;
-  a.icol = h->icol.p;
-  a.ival = h->ival.p;
-  a.slot0 = h->slot0.p;
-  a.chunk_order = h->chunk_order.p;
   a.b = h->b.p;
   a.mu = h->mu.p;
   a.scaling = h->scaling.p;
@@ -595,9 +600,16 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
       }
       steps = std::max(steps, sum);
     }
-    resident = pg_resident_fits(h->device, teams, steps, h->h_chunk_seg[h->h_chunk_order[0]]);
+    resident = pg_resident_fits(h->device, teams, steps, h->h_chunk_seg[h->h_chunk_order[0]], n);
   }
-  if (!resident) grid = pg_grid(h->device, false, a.nchunks);
+  if (!resident) {
+    if (int e = ensure_interleaved(h)) return e;
+    a.icol = h->icol.p;
+    a.ival = h->ival.p;
+    a.slot0 = h->slot0.p;
+    a.chunk_order = h->chunk_order.p;
+    grid = pg_grid(h->device, false, a.nchunks);
+  }
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
   a.flat = !sc && a.nchunks <= kFlatChunks;
   if (int e = ensure_cta_lists(h, grid)) return e;
@@ -673,26 +685,36 @@ int ensure_cta_lists(bogus_gpu_problem* h, int G) {
   return BOGUS_GPU_OK;
 }
 
-int ensure_interleaved(bogus_gpu_problem* h) {
-  if (h->il_valid) return BOGUS_GPU_OK;
+// S of every chunk and the chunks by decreasing S, on the host.
+int ensure_chunks(bogus_gpu_problem* h) {
+  if (h->chunks_valid) return BOGUS_GPU_OK;
   const int n = h->W.n;
   const int C = (n + 31) / 32;
   std::vector<int> rp(n + 1);
-  BG_CUDA(cudaMemcpy(rp.data(), h->W.rowptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
-  std::vector<long long> s0(C + 1, 0);
-  std::vector<int> seg(C), order(C);
+  BG_CUDA(cudaMemcpyAsync(rp.data(), h->W.rowptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, h->stream));
+  BG_CUDA(cudaStreamSynchronize(h->stream));
+  h->h_chunk_seg.resize(C);
+  h->h_chunk_order.resize(C);
   for (int c = 0; c < C; ++c) {
-    const int r1 = std::min(32 * c + 32, n);
-    const int T = rp[r1] - rp[32 * c];
-    const long long S = T > 0 ? (T + 31) / 32 : 1;
-    s0[c + 1] = s0[c] + 32 * S;
-    seg[c] = (int)S;
-    order[c] = c;
+    const int T = rp[std::min(32 * c + 32, n)] - rp[32 * c];
+    h->h_chunk_seg[c] = T > 0 ? (T + 31) / 32 : 1;
+    h->h_chunk_order[c] = c;
   }
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return seg[x] > seg[y]; });
-  h->h_chunk_order = order;
-  h->h_chunk_seg = seg;
+  const std::vector<int>& seg = h->h_chunk_seg;
+  std::stable_sort(h->h_chunk_order.begin(), h->h_chunk_order.end(), [&](int x, int y) { return seg[x] > seg[y]; });
   h->cta_grid = 0;
+  h->chunks_valid = true;
+  return BOGUS_GPU_OK;
+}
+
+int ensure_interleaved(bogus_gpu_problem* h) {
+  if (h->il_valid) return BOGUS_GPU_OK;
+  if (int e = ensure_chunks(h)) return e;
+  const int n = h->W.n;
+  const int C = (n + 31) / 32;
+  std::vector<long long> s0(C + 1, 0);
+  for (int c = 0; c < C; ++c) s0[c + 1] = s0[c] + 32 * (long long)h->h_chunk_seg[c];
+  const std::vector<int>& order = h->h_chunk_order;
   BG_CUDA(h->chunk_order.ensure(C > 0 ? C : 1));
   if (C) BG_CUDA(cudaMemcpyAsync(h->chunk_order.p, order.data(), sizeof(int) * C, cudaMemcpyHostToDevice, h->stream));
   const size_t slots = (size_t)s0[C];
@@ -1147,6 +1169,9 @@ int bogus_gpu_destroy(bogus_gpu_problem* h) {
   h->col_local.release();
   h->next.release();
   h->batch_out.release();
+  h->rb_ptr.release();
+  h->rb_jobs.release();
+  h->rb_mono.release();
   h->cb.release();
   h->pgout.release();
   h->barrier.release();
@@ -1261,6 +1286,7 @@ int bogus_gpu_set_dual_device(bogus_gpu_problem* h, int n, int nnzb, const int* 
   h->fp32_valid = false;
   h->fp32p_valid = false;
   h->il_valid = false;
+  h->chunks_valid = false;
   h->adj_valid = false;
   return BOGUS_GPU_OK;
 }
@@ -2713,6 +2739,7 @@ int bogus_gpu_add_compliance(bogus_gpu_problem* h, const double* c) {
   h->fp32_valid = false;
   h->fp32p_valid = false;
   h->il_valid = false;
+  h->chunks_valid = false;
   h->adj_valid = false;
   return BOGUS_GPU_OK;
 }
@@ -3139,9 +3166,105 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
   h->fp32_valid = false;
   h->fp32p_valid = false;
   h->il_valid = false;
+  h->chunks_valid = false;
   h->adj_valid = false;
   return BOGUS_GPU_OK;
 }
+
+}  // extern "C"
+
+namespace {
+
+// Plan of the resident form of the batched solve (kernels_pg_resident.cu): each problem on as many CTAs as its chunks
+// need at up to m each, the problems in decreasing size, each given the CTAs that are free first; m is the one of 1 ..
+// kMaxTeams that ends first by estimate. The plan is kept where it ends before the rule's shape by estimate. For one
+// iteration on GB300 (us), a CTA with m chunks takes 10 + 4.6 m and 5 more when the problem spans CTAs; with one CTA per
+// problem (8 warps, W streamed, two CTAs per SM) a problem takes 24 and 2.8 per chunk up to 8 chunks, 7 beyond, in a
+// team 35 and 16 per chunk of a warp, and all problems together no less than 5.2 per chunk and SM. So batches whose
+// largest problems would outlast the others (up to a few hundred problems) are resident, thousands of problems or a
+// few dozen that fill the GPU each are not.
+// ms for 100 iterations, the rule's shape / resident: 24 problems of 16 to 64 contacts 3.3 / 2.3, 64 of 16 to 256
+// 4.6 / 2.7, 256 of 16 to 1 024 24.0 / 10.8, 400 of 16 to 1 024 26.1 / 14.3.
+BatchShape rule_shape(const bogus_gpu_problem* h, bool fp32);
+int plan_resident_batch(bogus_gpu_problem* h, const std::vector<int>& rp, const std::vector<int>& queue) {
+  h->rb_ctas = 0;
+  const int np = h->nproblems;
+  int sms = 0;
+  BG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+  if (np == 0 || sms <= 0) return BOGUS_GPU_OK;
+  const BatchShape rule = rule_shape(h, false);
+  double chunks = 0.0, largest = 0.0, total = 0.0;
+  for (int p = 0; p < np; ++p) {
+    const int C = (h->h_contact_ptr[p + 1] - h->h_contact_ptr[p] + 31) / 32;
+    const double alone = rule.schedule == 0 ? 24.0 + (C <= 8 ? 2.8 : 7.0) * C
+                                            : 35.0 + 16.0 * ((C + 8 * rule.team_size - 1) / (8 * rule.team_size));
+    chunks += C;
+    largest = std::max(largest, alone);
+    total += alone;
+  }
+  double best = std::max(largest, 5.2 * chunks / sms);  // the rule's shape
+  if (rule.schedule == 0) best = std::max(best, 1.3 * total / (2 * sms));
+  std::vector<std::vector<ResidentJob>> kept;
+  for (int teams = 1; teams <= pg_resident_max_teams(); ++teams) {
+    std::vector<double> busy(sms, 0.0);
+    std::vector<std::vector<ResidentJob>> jobs(sms);
+    std::vector<int> by(sms);
+    int steps = 1, longest = 1, most = 0, used = 1;
+    bool fits = true;
+    for (int p : queue) {
+      const int c0 = h->h_contact_ptr[p], n = h->h_contact_ptr[p + 1] - c0, C = (n + 31) / 32;
+      const int g = std::max(1, (C + teams - 1) / teams);
+      if (g > sms) {
+        fits = false;
+        break;
+      }
+      most = std::max(most, n);
+      std::vector<int> sum(g, 0);
+      for (int c = 0; c < C; ++c) {
+        const int T = rp[c0 + std::min(32 * c + 32, n)] - rp[c0 + 32 * c], S = T > 0 ? (T + 31) / 32 : 1;
+        longest = std::max(longest, S);
+        steps = std::max(steps, sum[c % g] += S);
+      }
+      const int m = (C + g - 1) / g;
+      used = std::max(used, m);
+      // the g CTAs that are free first (ties by index)
+      for (int b = 0; b < sms; ++b) by[b] = b;
+      std::partial_sort(by.begin(), by.begin() + g, by.end(),
+                        [&](int x, int y) { return busy[x] < busy[y] || (busy[x] == busy[y] && x < y); });
+      const double end = busy[by[g - 1]] + 10.0 + 4.6 * m + (g > 1 ? 5.0 : 0.0);
+      for (int r = 0; r < g; ++r) {
+        jobs[by[r]].push_back(ResidentJob{p, r, g});
+        busy[by[r]] = end;
+      }
+    }
+    if (!fits || !pg_resident_fits(h->device, used, steps, longest, most)) continue;
+    const double end = *std::max_element(busy.begin(), busy.end());
+    if (end >= best) continue;
+    best = end;
+    kept.swap(jobs);
+    h->rb_teams = used;
+    h->rb_steps = steps;
+  }
+  if (kept.empty()) return BOGUS_GPU_OK;
+  std::vector<int> ptr(1, 0);
+  std::vector<ResidentJob> flat;
+  for (int b = 0; b < sms; ++b) {
+    flat.insert(flat.end(), kept[b].begin(), kept[b].end());
+    ptr.push_back((int)flat.size());
+  }
+  BG_CUDA(h->rb_ptr.ensure(ptr.size()));
+  BG_CUDA(h->rb_jobs.ensure(flat.size()));
+  BG_CUDA(h->rb_mono.ensure(np));
+  BG_CUDA(cudaMemcpyAsync(h->rb_ptr.p, ptr.data(), sizeof(int) * ptr.size(), cudaMemcpyHostToDevice, h->stream));
+  BG_CUDA(cudaMemcpyAsync(h->rb_jobs.p, flat.data(), sizeof(ResidentJob) * flat.size(), cudaMemcpyHostToDevice, h->stream));
+  BG_CUDA(cudaStreamSynchronize(h->stream));
+  h->rb_ctas = sms;
+  return BOGUS_GPU_OK;
+}
+
+}  // namespace
+
+extern "C" {
 
 int bogus_gpu_set_batch(bogus_gpu_problem* h, int nproblems, const int* cptr) {
   if (int e = check_handle(h)) return e;
@@ -3189,6 +3312,7 @@ int bogus_gpu_set_batch(bogus_gpu_problem* h, int nproblems, const int* cptr) {
   BG_CUDA(cudaStreamSynchronize(s));
   h->nproblems = nproblems;
   h->h_contact_ptr.assign(cptr, cptr + nproblems + 1);
+  if (int e = plan_resident_batch(h, rp, queue)) return e;
   h->h_problem_nnz = nnz;
   h->tuned_shape[0] = h->tuned_shape[1] = BatchShape{};
   h->tune_ms.clear();
@@ -3483,7 +3607,20 @@ int run_pg_batch(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* re
   }
   BatchShape sh;
   if (int e = choose_shape(h, ba, false, sizeof(double) * 3 * (size_t)h->W.n, h->X.p, &sh)) return e;
-  if (int e = launch_shape(h, sh, &ba, nullptr, true)) return e;
+  // the rule's shape may be taken over by the resident form (the caller's and the tuner's are kept)
+  if (h->rb_ctas && !hy && !ba.base.lin_momentum && h->forced_shape.schedule < 0 && !h->batch_tuning) {
+    BG_CUDA(h->status.ensure(1));
+    BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), h->stream));
+    BG_CUDA(cudaMemsetAsync(h->rb_mono.p, 0, sizeof(unsigned long long) * np, h->stream));
+    ba.base.gb.status = h->status.p;
+    BG_CUDA(cudaEventRecord(h->ev0, h->stream));
+    BG_CUDA(launch_pg_resident_batch(ba, h->rb_ptr.p, h->rb_jobs.p, h->rb_mono.p, h->rb_ctas, h->rb_teams, h->rb_steps,
+                                     h->stream));
+    BG_CUDA(cudaEventRecord(h->ev1, h->stream));
+    h->last_shape = sh;
+  } else if (int e = launch_shape(h, sh, &ba, nullptr, true)) {
+    return e;
+  }
   std::vector<PGOut> out(np);
   if (np) BG_CUDA(cudaMemcpyAsync(out.data(), h->batch_out.p, sizeof(PGOut) * np, cudaMemcpyDeviceToHost, h->stream));
   BG_CUDA(cudaStreamSynchronize(h->stream));
@@ -3511,7 +3648,7 @@ int batch_checks(bogus_gpu_problem* h, const bogus_gpu_pg_options* o) {
   BG_CUDA(h->Wv.ensure(3 * (size_t)n));
   size_t tot_chunks = 0;
   for (int p = 0; p < h->nproblems; ++p) tot_chunks += (h->h_contact_ptr[p + 1] - h->h_contact_ptr[p] + 31) / 32;
-  BG_CUDA(h->csum.ensure(4 * tot_chunks + 4));
+  BG_CUDA(h->csum.ensure(8 * tot_chunks + 8));  // two buffers of 4 in the resident form
   return BOGUS_GPU_OK;
 }
 

@@ -166,10 +166,18 @@ cudaError_t launch_cadoux_rhs(int n, const double* y, const double* mu, const do
 cudaError_t launch_pg_persistent(const PGArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_pg_persistent(const PGArgs32& a, int grid, cudaStream_t s);
 int pg_max_grid(int device, bool fp32 = false, bool interleaved = false);
-// Problems that fit the SMs' shared memory (kernels_pg_resident.cu): chunk lists for `ctas` CTAs of up to `teams`
-// chunks, `steps` the largest sum of S (spmv_chunk.cuh) over a CTA's chunks, `longest` the largest S
-bool pg_resident_fits(int device, int teams, int steps, int longest);
+// Problems that fit the SMs' shared memory (kernels_pg_resident.cu): `ctas` CTAs of up to `teams` chunks, `steps` the
+// largest sum of S (spmv_chunk.cuh) over a CTA's chunks, `longest` the largest S
+bool pg_resident_fits(int device, int teams, int steps, int longest, int n);
+int pg_resident_max_teams();
 cudaError_t launch_pg_resident(const PGArgs& a, int ctas, int teams, int steps, cudaStream_t s);
+// A CTA's part in one problem of a batch: the chunks rank, rank + ctas, ...
+struct ResidentJob {
+  int problem, rank, ctas;
+};
+// CTA b works through jobs[job_ptr[b] .. job_ptr[b + 1]); mono: one barrier counter per problem, zero at launch
+cudaError_t launch_pg_resident_batch(const PGBatchArgs& b, const int* job_ptr, const ResidentJob* jobs,
+                                     unsigned long long* mono, int ctas, int teams, int steps, cudaStream_t s);
 cudaError_t launch_pg_batched(const PGBatchArgs& b, int grid, cudaStream_t s);
 cudaError_t launch_pg_batched(const PGBatchArgs32& b, int grid, cudaStream_t s);
 int pg_batched_grid(int device, bool fp32 = false);

@@ -25,24 +25,15 @@
 // the chain of FMAs), law and vectors 9 300, barriers 7 000, sums 4 400, decisions 4 000.
 #include "internal.h"
 #include "soc_device.cuh"
-#include "spmv_chunk.cuh"
+#include "resident.cuh"
 
 namespace bogus_gpu {
 
 namespace {
 
-constexpr int kTeamWarps = 3;
-constexpr int kMaxTeams = 5;
-constexpr int kMinWarps = 8;  // a stripe of the reductions each; those past the teams' warps do nothing else
-
-// Shared memory of one team, beside its chunk's block values.
 struct TeamShared {
-  // pieces of the rows, by component (slot: rank of the row among the nonempty + lane), then the product itself
-  double part[kTeamWarps][64];
-  double xs[3][32], y[3][32];   // the last step; the second product of the guess (pieces, then values) before
-  double s0[32];
-  double stage[2][3][3][32];    // the gathered points of two groups of three steps
-  int st[36];                   // row starts of the chunk, relative to its first block
+  TeamCore core;
+  double xs[3][32], y[3][32];  // the last step; the second product of the guess (pieces, then values) before
 };
 
 // Scalars of the iteration, written by one warp per CTA after each reduction.
@@ -53,210 +44,54 @@ struct Control {
   unsigned phases[9];
 };
 
-__device__ __forceinline__ void team_sync(int team) {
-  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(32 * kTeamWarps) : "memory");
-}
-
-// A gathered point: 32 bytes per contact, the fourth value unused.
-__device__ __forceinline__ void load_padded(const double* p, double* x) {
-  double pad;
-  asm volatile("ld.relaxed.gpu.global.v4.f64 {%0, %1, %2, %3}, [%4];"
-               : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(pad)
-               : "l"(p));
-}
-__device__ __forceinline__ void store_padded(double* p, const double* x) {
-  __stcg(reinterpret_cast<double2*>(p), make_double2(x[0], x[1]));
-  __stcg(p + 2, x[2]);
-}
-
-template <int V>
-struct Int {
-  static constexpr int value = V;
-};
-
 enum { kAccept = 0, kMomentum = 1, kRetry = 2, kStop = 3 };
 
-// S of chunk c (spmv_chunk.cuh)
-__device__ __forceinline__ int steps_of(const PGArgs& a, int c) {
-  const int nblk = __ldg(a.rowptr + min(32 * c + 32, a.n)) - __ldg(a.rowptr + 32 * c);
-  return nblk > 0 ? (nblk + 31) / 32 : 1;
-}
+// The CTA's part in a solve: rank among the CTAs (parties) that share the problem, and its chunks, one per team.
+struct Place {
+  int rank;
+  unsigned parties;
+  int first, stride, count;  // chunks list[first + k stride] (list null: the index itself), k < count
+  const int* list;
+  __device__ int chunk(int k) const {
+    const int j = first + k * stride;
+    return list ? __ldg(list + j) : j;
+  }
+};
 
-__global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(PGArgs a, int teams) {
-  extern __shared__ __align__(16) unsigned char smem[];
+__device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const Place& place, unsigned char* smem) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int team = warp / kTeamWarps, role = warp - kTeamWarps * team;
   Control& ctl = *reinterpret_cast<Control*>(smem);
-  const int first = __ldg(a.cta_ptr + blockIdx.x);
-  const bool has = team < teams && first + team < __ldg(a.cta_ptr + blockIdx.x + 1);
-  const int c = has ? __ldg(a.cta_list + first + team) : 0;
+  const bool has = team < place.count;
+  const int c = has ? place.chunk(team) : 0;
   TeamShared& sh = reinterpret_cast<TeamShared*>(smem + (sizeof(Control) + 15) / 16 * 16)[team < teams ? team : 0];
-  // the CTA's chunks one after another, behind the teams' arrays
-  size_t before = 0;
-  for (int k = 0; k < team && has; ++k) before += (size_t)steps_of(a, __ldg(a.cta_list + first + k));
-  unsigned char* const blocks =
-      smem + (sizeof(Control) + 15) / 16 * 16 + (size_t)teams * sizeof(TeamShared) + before * 32 * 72;
   const int C = a.nchunks;
   const int i = 32 * c + lane;
   const bool on = has && i < a.n;
   const bool desaxce = a.desaxce != 0, spg = a.variant == 4, apgd = a.variant == 3;
   const unsigned res_mask = a.use_inf ? 1u : 0u;
-  const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
+  const bool writer = place.rank == 0 && threadIdx.x == 0;
   double* const gx = a.MX0;                      // the gathered points: x (or the momentum point) ...
   double* const gs = a.MX0 + 4 * (size_t)a.n;    // ... and the trial point xs
   const size_t ip = on ? 4 * (size_t)i : 0;
 
-  // ---- the chunk: blocks and columns to shared memory, this lane's segment and row -------------------------
-  double* const wv = reinterpret_cast<double*>(blocks);
-  const int* col = nullptr;  // this lane's columns: step s at col[32 s]
-  int nblk = 0, S = 0, nv = 0, slot0 = 0, piece0 = 0, pieces = 0;
-  unsigned long long starts = 0;  // bit s: the lane's block s opens a row that its block s - 1 does not belong to
+  ResidentChunk chunk{sh.core, lane, role, team};
   if (has) {
-    const int r0 = 32 * c, r1 = min(r0 + 32, a.n);
-    const int B0 = __ldg(a.rowptr + r0);
-    nblk = __ldg(a.rowptr + r1) - B0;
-    S = nblk > 0 ? (nblk + 31) / 32 : 1;
-    if (role == 0) {
-      sh.st[lane] = __ldg(a.rowptr + min(r0 + lane, r1)) - B0;
-      if (lane == 0) sh.st[32] = nblk;
-    }
-    const long long base = __ldg(a.slot0 + c);
-    const int tid = threadIdx.x - 32 * kTeamWarps * team;
-    const double2* sv = reinterpret_cast<const double2*>(a.ival + 9 * base);
-    for (int k = tid; k < S * 32 * 9 / 2; k += 32 * kTeamWarps) reinterpret_cast<double2*>(wv)[k] = __ldcs(sv + k);
-    col = a.icol + base + lane;
-    team_sync(team);
-    const int k0 = lane * S;
-    nv = max(0, min(S, nblk - k0));
-    const int rs = sh.st[lane], re = sh.st[lane + 1];
-    const unsigned filled = __ballot_sync(0xffffffffu, rs < re);
-    auto rank = [&](int t) { return __popc(filled & ((1u << t) - 1u)); };
-    if (nv > 0) {
-      int lo = 0, hi = 31;  // row containing block k0: last t with st[t] <= k0
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (sh.st[mid] <= k0) lo = mid;
-        else hi = mid - 1;
-      }
-      slot0 = rank(lo) + lane;
-      for (int t = lo + 1; t < 32 && sh.st[t] < k0 + nv; ++t)
-        if (sh.st[t] > k0) starts |= 1ull << (sh.st[t] - k0);
-    }
-    if (rs < re) {
-      const int lf = rs / S;
-      piece0 = rank(lane) + lf;
-      pieces = (re - 1) / S - lf + 1;
-    }
+    size_t before = 0;  // the CTA's chunks one after another, behind the teams' arrays
+    for (int k = 0; k < team; ++k) before += (size_t)steps_of(a.rowptr, a.n, place.chunk(k));
+    chunk.load(a.rowptr, a.col, a.val, a.n, c,
+               smem + (sizeof(Control) + 15) / 16 * 16 + (size_t)teams * sizeof(TeamShared) + before * kStepBytes);
   }
-
-  // group k: steps 3 k .. 3 k + 2, this warp's gather the step 3 k + role (past the end: any contact)
-  auto column = [&](int k) {
-    const int s = min(3 * k + role, S - 1);
-    return lane * S + s < nblk ? __ldg(col + 32 * s) : 32 * c;
-  };
-  const int j0 = has ? column(0) : 0, j1 = has ? column(1) : 0;
-
-  // Component `role` of row `lane` of the chunk's product with the gathered point g (NP = 2: also with g - 1), in
-  // the chunk-segmented order of spmv_chunk.
-  // One step, without divergence: the piece of the row that ends is put away, then three FMAs; a lane past its
-  // segment runs them on the padding and keeps its sum.
-  auto product = [&](const double* __restrict__ g, auto np) -> double2 {
-    constexpr int NP = decltype(np)::value;
-    double* part2 = sh.xs[0] + 64 * role;
-    int slot = slot0;
-    double p = 0.0, q = 0.0;
-    const double* bl = wv + 32 * 3 * role + lane;
-    unsigned long long open = starts;
-    auto step = [&](int s, const double* b, const double* x) {
-      const bool starts_row = open & 1ull;
-      open >>= 1;
-      if (starts_row) sh.part[role][slot] = p;
-      p = starts_row ? 0.0 : p;
-      const bool valid = s < nv;
-      const double pn = fma(b[2], x[2], fma(b[1], x[1], fma(b[0], x[0], p)));
-      p = valid ? pn : p;
-      if (NP == 2) {
-        if (starts_row) part2[slot] = q;
-        q = starts_row ? 0.0 : q;
-        const double qn = fma(b[2], x[2] - 1.0, fma(b[1], x[1] - 1.0, fma(b[0], x[0] - 1.0, q)));
-        q = valid ? qn : q;
-      }
-      slot += starts_row ? 1 : 0;
-    };
-    auto put_stage = [&](int k, const double* x) {
-#pragma unroll
-      for (int e = 0; e < 3; ++e) sh.stage[k & 1][role][e][lane] = x[e];
-    };
-    auto consume = [&](int k) {
-      double b[3][3], x[3][3];  // all loads of the group before its chain of FMAs
-#pragma unroll
-      for (int e = 0; e < 3; ++e) {
-        const double* be = bl + 288 * min(3 * k + e, S - 1);
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          b[e][r] = be[32 * r];
-          x[e][r] = sh.stage[k & 1][e][r][lane];
-        }
-      }
-#pragma unroll
-      for (int e = 0; e < 3; ++e)
-        if (3 * k + e < S) step(3 * k + e, b[e], x[e]);
-      team_sync(team);
-    };
-    // even groups pass through u, odd ones through v (no copies between them: a copy would wait for the load)
-    const int groups = (S + 2) / 3;
-    double u[3], v[3];
-    int ju = column(2), jv = column(3);
-    load_padded(g + 4 * (size_t)j0, u);
-    load_padded(g + 4 * (size_t)j1, v);
-    put_stage(0, u);
-    load_padded(g + 4 * (size_t)ju, u);
-    ju = column(4);
-    team_sync(team);
-    for (int k = 0; k < groups; k += 2) {
-      if (k + 1 < groups) {
-        put_stage(1, v);
-        load_padded(g + 4 * (size_t)jv, v);
-        jv = column(k + 5);
-      }
-      consume(k);
-      if (k + 1 >= groups) break;
-      if (k + 2 < groups) {
-        put_stage(0, u);
-        load_padded(g + 4 * (size_t)ju, u);
-        ju = column(k + 6);
-      }
-      consume(k + 1);
-    }
-    if (nv > 0) {
-      sh.part[role][slot] = p;
-      if (NP == 2) part2[slot] = q;
-    }
-    __syncwarp();
-    double2 acc = make_double2(0.0, 0.0);
-    if (pieces > 0) {
-      acc.x = ipipe::plus_zero(sh.part[role][piece0]);
-      for (int k = 1; k < pieces; ++k) acc.x = acc.x + sh.part[role][piece0 + k];
-      if (NP == 2) {
-        acc.y = ipipe::plus_zero(part2[piece0]);
-        for (int k = 1; k < pieces; ++k) acc.y = acc.y + part2[piece0 + k];
-      }
-    }
-    __syncwarp();
-    sh.part[role][lane] = acc.x;
-    if (NP == 2) part2[lane] = acc.y;
-    team_sync(team);
-    return acc;
-  };
+  const double (*const part)[64] = sh.core.part;
   // W g for this chunk's contacts, all components to every warp of the team
   auto team_product = [&](const double* g, double* out) {
-    product(g, Int<1>());
+    chunk.product<1>(g);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) out[k] = sh.part[k][lane];
+    for (int k = 0; k < 3; ++k) out[k] = part[k][lane];
   };
 
   // ---- barriers ----------------------------------------------------------------------------------------------
-  const MonoBarrier mb{a.mono, a.gb.status, gridDim.x + a.phantom_ctas};
+  const MonoBarrier mb{a.mono, a.gb.status, place.parties + a.phantom_ctas};
   unsigned phase = 0;  // barriers passed
   auto sums = [&]() { return a.csum + (size_t)(phase & 1u) * 4 * C; };
   auto put = [&](int q, double v) {
@@ -327,6 +162,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
   // (x and prev in registers; xs, y and the products in the team's shared memory; b, mu and the scalings are read
   // where they are used, from L1)
   double x[3] = {0.0, 0.0, 0.0}, pv[3], Mx[3] = {0.0, 0.0, 0.0};
+  double s0 = 0.0;  // COV(y)_N of the last A (warp 0)
   if (on) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) x[k] = a.X0[3 * (size_t)i + k];
@@ -366,9 +202,9 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
   // Mx = W x (:93) and guess_alpha (:21-28)
   count(1);
   if (has) {
-    product(gx, Int<2>());
+    chunk.product<2>(gx, sh.xs[0]);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) Mx[k] = sh.part[k][lane];
+    for (int k = 0; k < 3; ++k) Mx[k] = part[k][lane];
     if (role == 0) {
       const double* second = sh.xs[0] + lane;
       const double d[3] = {second[0], second[64], second[128]};
@@ -410,6 +246,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
         const double yr[3] = {Mx[0] + b[0], Mx[1] + b[1], Mx[2] + b[2]};
         const double lx[3] = {x[0] * scal, x[1] * scal, x[2] * scal};
         v = law_eval(desaxce, mu, lx, yr);
+        s0 = duality_cov(desaxce, mu, yr);
       } else if (role == 1) {
         double yn[3] = {Mx[0] + b[0], Mx[1] + b[1], Mx[2] + b[2]};
         const double sn = duality_cov(desaxce, mu, yn);
@@ -425,7 +262,6 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
           sh.xs[k][lane] = p[k];
           sh.y[k][lane] = yn[k];
         }
-        sh.s0[lane] = sn;
         if (spg) {
           const double d[3] = {p[0] - pv[0], p[1] - pv[1], p[2] - pv[2]};
           v = dot3(d, yn);
@@ -470,7 +306,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
     const bool mom = spg ? negative(second) : apgd;
     __syncwarp();
     if (lane == 0) {
-      if (a.trace && blockIdx.x == 0) a.trace[it] = res;
+      if (a.trace && place.rank == 0) a.trace[it] = res;
       if (best) ctl.min_res = res;
       ctl.best = best;
       ctl.go = stop ? kStop : (mom ? kMomentum : kAccept);
@@ -510,7 +346,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
             double b[3] = {0.0, 0.0, 0.0};
             if (on) load_b(b);
             const double first = ipipe::scale2<-1>(Ms[0]) + b[0];
-            const double t[3] = {desaxce ? first + sh.s0[lane] : ipipe::plus_zero(first),
+            const double t[3] = {desaxce ? first + s0 : ipipe::plus_zero(first),
                                  ipipe::plus_zero(ipipe::scale2<-1>(Ms[1]) + b[1]),
                                  ipipe::plus_zero(ipipe::scale2<-1>(Ms[2]) + b[2])};
             put(0, on ? dot3(xs, t) : 0.0);
@@ -587,7 +423,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
         const double xs = on ? sh.xs[k][lane] : 0.0;
         if (next != kMomentum) {
           x[k] = xs;
-          Mx[k] = sh.part[k][lane];
+          Mx[k] = part[k][lane];
         }
         pv[k] = xs;
       }
@@ -664,31 +500,91 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
   finish(it, 0);
 }
 
+// One problem on the whole grid.
+__global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(PGArgs a, int teams) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int first = __ldg(a.cta_ptr + blockIdx.x);
+  const Place place{(int)blockIdx.x, gridDim.x, first, 1, __ldg(a.cta_ptr + blockIdx.x + 1) - first, a.cta_list};
+  resident_solve(a, teams, place, smem);
+}
+
+// A batch: every CTA works through its own list of jobs, a job being its part in one problem (the chunks rank,
+// rank + ctas, ...). The lists hold the problems in one global order, so a CTA waits in a problem's barriers only for
+// CTAs that are at this problem or at earlier ones.
+__global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1)
+    k_pg_resident_batch(PGBatchArgs ba, const int* job_ptr, const ResidentJob* jobs, unsigned long long* mono, int teams) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ PGArgs a;
+  for (int j = __ldg(job_ptr + blockIdx.x); j < __ldg(job_ptr + blockIdx.x + 1); ++j) {
+    const ResidentJob job = jobs[j];
+    const size_t c0 = ba.contact_ptr[job.problem];
+    const int n = (int)(ba.contact_ptr[job.problem + 1] - c0);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      a = ba.base;
+      a.n = n;
+      a.nchunks = (n + 31) / 32;
+      a.rowptr = ba.base.rowptr + c0;
+      a.b = ba.base.b + 3 * c0;
+      a.mu = ba.base.mu + c0;
+      a.scaling = ba.base.scaling + c0;
+      a.X0 = ba.base.X0 + 3 * c0;
+      a.MX0 = ba.base.MX0 + 8 * c0;  // two gathered points, padded
+      a.XB = ba.base.XB + 3 * c0;
+      a.csum = ba.base.csum + 8 * (size_t)ba.chunk_ptr[job.problem];
+      a.trace = nullptr;
+      a.out = ba.base.out + job.problem;
+      a.mono = mono + job.problem;
+    }
+    __syncthreads();
+    const int mine = a.nchunks > job.rank ? (a.nchunks - job.rank + job.ctas - 1) / job.ctas : 0;
+    const Place place{job.rank, (unsigned)job.ctas, job.rank, job.ctas, mine, nullptr};
+    resident_solve(a, teams, place, smem);
+    // the best iterate over the initial one, by the lanes that stored it
+    const int warp = threadIdx.x >> 5, i = 32 * (job.rank + (warp / kTeamWarps) * job.ctas) + (threadIdx.x & 31);
+    if (warp / kTeamWarps < mine && warp % kTeamWarps == 1 && i < n)
+      for (int k = 0; k < 3; ++k) ba.r[3 * (c0 + i) + k] = a.XB[3 * i + k];
+  }
+}
+
 // teams per CTA, and the largest sum of S over a CTA's chunks
 size_t resident_smem(int teams, int steps) {
-  return (sizeof(Control) + 15) / 16 * 16 + (size_t)teams * sizeof(TeamShared) + (size_t)steps * 32 * 72;
+  return (sizeof(Control) + 15) / 16 * 16 + (size_t)teams * sizeof(TeamShared) + (size_t)steps * kStepBytes;
 }
 
 }  // namespace
 
-// Whether the resident kernel takes a problem whose CTAs own up to `teams` chunks with up to `steps` steps (S) in sum:
-// a team per chunk, every chunk's block values (72 bytes each) in shared memory, a lane's row starts in 64 bits.
-bool pg_resident_fits(int device, int teams, int steps, int longest) {
+// Whether the resident kernel takes CTAs with up to `teams` chunks of up to `steps` steps (S) in sum and `longest` each:
+// a team per chunk, every chunk's blocks in shared memory, a lane's row starts in 64 bits, columns in 16.
+bool pg_resident_fits(int device, int teams, int steps, int longest, int n) {
   int limit = 0;
   if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return false;
-  return teams >= 1 && teams <= kMaxTeams && longest <= 64 && resident_smem(teams, steps) <= (size_t)limit;
+  return teams >= 1 && teams <= kMaxTeams && longest <= 64 && n <= 65536 && resident_smem(teams, steps) + 1024 <= (size_t)limit;
 }
 
-cudaError_t launch_pg_resident(const PGArgs& a, int ctas, int teams, int steps, cudaStream_t s) {
+int pg_resident_max_teams() { return kMaxTeams; }
+
+namespace {
+cudaError_t launch_resident(const void* fn, void** args, int ctas, int teams, int steps, cudaStream_t s) {
   const size_t bytes = resident_smem(teams, steps);
-  const void* fn = (const void*)k_pg_resident;
   const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e != cudaSuccess) return e;
-  PGArgs copy = a;
-  int t = teams;
   const int warps = kTeamWarps * teams > kMinWarps ? kTeamWarps * teams : kMinWarps;
-  void* args[] = {&copy, &t};
   return cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(32 * warps), args, bytes, s);
+}
+}  // namespace
+
+cudaError_t launch_pg_resident(const PGArgs& a, int ctas, int teams, int steps, cudaStream_t s) {
+  PGArgs copy = a;
+  void* args[] = {&copy, &teams};
+  return launch_resident((const void*)k_pg_resident, args, ctas, teams, steps, s);
+}
+
+cudaError_t launch_pg_resident_batch(const PGBatchArgs& b, const int* job_ptr, const ResidentJob* jobs,
+                                     unsigned long long* mono, int ctas, int teams, int steps, cudaStream_t s) {
+  PGBatchArgs copy = b;
+  void* args[] = {&copy, &job_ptr, &jobs, &mono, &teams};
+  return launch_resident((const void*)k_pg_resident_batch, args, ctas, teams, steps, s);
 }
 
 // Sets this file's copy of the device-side wait limit on the current device.

@@ -1,0 +1,205 @@
+// A 32-contact chunk of W owned by a team of three warps of one SM for the whole of a kernel: its blocks in shared
+// memory, and the product with a gathered point in the canonical chunk-segmented order (spmv_chunk.cuh).
+//
+// Warp r of the team accumulates component r of every row (3 FMAs per block in place of 9: the FP64 unit's latency is
+// 64 cycles whatever the lanes), and gathers every third point for all three (a gather of 32 scattered contacts holds
+// the load unit for as long as a step's FMAs take). Points are 32 bytes per contact, one 256-bit load each, issued two
+// groups of three steps ahead of their FMAs. A product of a 2 000-contact chunk (20 steps) takes 8 600 cycles on
+// GB300: 4 000 in the chain of FMAs, 2 600 from the first column to the first FMA and from the last to the exchanged
+// result, the rest in shared-memory loads and the team's barriers.
+#pragma once
+
+#include "device_common.cuh"
+#include "fp64_int.cuh"
+
+namespace bogus_gpu {
+
+constexpr int kTeamWarps = 3;
+constexpr int kMaxTeams = 5;
+constexpr int kMinWarps = 8;  // a stripe of the reductions each; those past the teams' warps do nothing else
+
+// Shared memory of one team, beside its chunk's blocks.
+struct TeamCore {
+  // pieces of the rows, by component (slot: rank of the row among the nonempty + lane), then the product itself
+  double part[kTeamWarps][64];
+  double stage[2][3][3][32];  // the gathered points of two groups of three steps
+  int st[36];                 // row starts of the chunk, relative to its first block
+};
+constexpr int kStepBytes = 32 * (72 + 2);  // block values and 16-bit columns of a step
+
+__device__ __forceinline__ void team_sync(int team) {
+  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(32 * kTeamWarps) : "memory");
+}
+
+// A gathered point: 32 bytes per contact, the fourth value unused.
+__device__ __forceinline__ void load_padded(const double* p, double* x) {
+  double pad;
+  asm volatile("ld.relaxed.gpu.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(pad)
+               : "l"(p));
+}
+__device__ __forceinline__ void store_padded(double* p, const double* x) {
+  __stcg(reinterpret_cast<double2*>(p), make_double2(x[0], x[1]));
+  __stcg(p + 2, x[2]);
+}
+
+// S of chunk c (spmv_chunk.cuh)
+__device__ __forceinline__ int steps_of(const int* rowptr, int n, int c) {
+  const int nblk = __ldg(rowptr + min(32 * c + 32, n)) - __ldg(rowptr + 32 * c);
+  return nblk > 0 ? (nblk + 31) / 32 : 1;
+}
+
+struct ResidentChunk {
+  TeamCore& sh;
+  const int lane, role, team;
+  double* wv = nullptr;          // value e of step s: wv[32 (9 s + e) + lane]
+  unsigned short* wc = nullptr;  // column of step s: wc[32 s + lane]
+  int S = 0, nv = 0, slot0 = 0, piece0 = 0, pieces = 0;
+  unsigned long long starts = 0;  // bit s: the lane's block s opens a row that its block s - 1 does not belong to
+
+  // Copies the blocks of chunk c of a BSR matrix of n <= 65536 rows (at most 64 steps) to `blocks` and finds this lane's
+  // segment and row.
+  __device__ void load(const int* rowptr, const int* col, const double* val, int n, int c, unsigned char* blocks) {
+    const int r0 = 32 * c, r1 = min(r0 + 32, n);
+    const int B0 = __ldg(rowptr + r0);
+    const int nblk = __ldg(rowptr + r1) - B0;
+    S = nblk > 0 ? (nblk + 31) / 32 : 1;
+    wv = reinterpret_cast<double*>(blocks);
+    wc = reinterpret_cast<unsigned short*>(wv + (size_t)S * 32 * 9);
+    if (role == 0) {
+      sh.st[lane] = __ldg(rowptr + min(r0 + lane, r1)) - B0;
+      if (lane == 0) sh.st[32] = nblk;
+    }
+    const int tid = 32 * role + lane;
+    // block k is met by lane k / S at step k % S; the padding past the last block gets a valid column (its lane
+    // drops the result)
+    for (int k = tid; k < nblk * 9; k += 32 * kTeamWarps) {
+      const int b = k / 9, e = k - 9 * b, l = b / S;
+      wv[32 * (9 * (b - l * S) + e) + l] = __ldcs(val + 9 * (size_t)B0 + k);
+    }
+    for (int k = nblk * 9 + tid; k < S * 32 * 9; k += 32 * kTeamWarps) {
+      const int b = k / 9, e = k - 9 * b, l = b / S;
+      wv[32 * (9 * (b - l * S) + e) + l] = 0.0;
+    }
+    for (int k = tid; k < S * 32; k += 32 * kTeamWarps) {
+      const int l = k / S;
+      wc[32 * (k - l * S) + l] = (unsigned short)(k < nblk ? __ldcs(col + B0 + k) : r0);
+    }
+    team_sync(team);
+    const int k0 = lane * S;
+    nv = max(0, min(S, nblk - k0));
+    const int rs = sh.st[lane], re = sh.st[lane + 1];
+    const unsigned filled = __ballot_sync(0xffffffffu, rs < re);
+    auto rank = [&](int t) { return __popc(filled & ((1u << t) - 1u)); };
+    if (nv > 0) {
+      int lo = 0, hi = 31;  // row containing block k0: last t with st[t] <= k0
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (sh.st[mid] <= k0) lo = mid;
+        else hi = mid - 1;
+      }
+      slot0 = rank(lo) + lane;
+      for (int t = lo + 1; t < 32 && sh.st[t] < k0 + nv; ++t)
+        if (sh.st[t] > k0) starts |= 1ull << (sh.st[t] - k0);
+    }
+    if (rs < re) {
+      const int lf = rs / S;
+      piece0 = rank(lane) + lf;
+      pieces = (re - 1) / S - lf + 1;
+    }
+  }
+
+  // group k: steps 3 k .. 3 k + 2, this warp's gather the step 3 k + role (past the end: any contact)
+  __device__ __forceinline__ const double* point(const double* g, int k) const {
+    return g + 4 * (size_t)wc[32 * min(3 * k + role, S - 1) + lane];
+  }
+  __device__ __forceinline__ void put_stage(int k, const double* x) {
+#pragma unroll
+    for (int e = 0; e < 3; ++e) sh.stage[k & 1][role][e][lane] = x[e];
+  }
+
+  // The chunk's product with the gathered point g: component r of row `lane` in sh.part[r][lane] for every warp of the
+  // team. NP = 2: also the product with g - 1, in part2 (3 x 64 doubles). A lane past its segment runs the FMAs on
+  // the padding and keeps its sum, so a step has no divergence.
+  template <int NP>
+  __device__ __forceinline__ void product(const double* __restrict__ g, double* part2_all = nullptr) {
+    double* part2 = part2_all + 64 * role;
+    int slot = slot0;
+    double p = 0.0, q = 0.0;
+    const double* bl = wv + 32 * 3 * role + lane;
+    unsigned long long open = starts;
+    auto step = [&](int s, const double* b, const double* x) {
+      const bool starts_row = open & 1ull;
+      open >>= 1;
+      if (starts_row) sh.part[role][slot] = p;
+      p = starts_row ? 0.0 : p;
+      const bool valid = s < nv;
+      const double pn = fma(b[2], x[2], fma(b[1], x[1], fma(b[0], x[0], p)));
+      p = valid ? pn : p;
+      if (NP == 2) {
+        if (starts_row) part2[slot] = q;
+        q = starts_row ? 0.0 : q;
+        const double qn = fma(b[2], x[2] - 1.0, fma(b[1], x[1] - 1.0, fma(b[0], x[0] - 1.0, q)));
+        q = valid ? qn : q;
+      }
+      slot += starts_row ? 1 : 0;
+    };
+    auto consume = [&](int k) {
+      double b[3][3], x[3][3];  // all loads of the group before its chain of FMAs
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const double* be = bl + 288 * min(3 * k + e, S - 1);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          b[e][r] = be[32 * r];
+          x[e][r] = sh.stage[k & 1][e][r][lane];
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 3; ++e)
+        if (3 * k + e < S) step(3 * k + e, b[e], x[e]);
+      team_sync(team);
+    };
+    // even groups pass through u, odd ones through v (no copies between them: a copy would wait for the load)
+    const int groups = (S + 2) / 3;
+    double u[3], v[3];
+    load_padded(point(g, 0), u);
+    load_padded(point(g, 1), v);
+    put_stage(0, u);
+    load_padded(point(g, 2), u);
+    team_sync(team);
+    for (int k = 0; k < groups; k += 2) {
+      if (k + 1 < groups) {
+        put_stage(1, v);
+        load_padded(point(g, k + 3), v);
+      }
+      consume(k);
+      if (k + 1 >= groups) break;
+      if (k + 2 < groups) {
+        put_stage(0, u);
+        load_padded(point(g, k + 4), u);
+      }
+      consume(k + 1);
+    }
+    if (nv > 0) {
+      sh.part[role][slot] = p;
+      if (NP == 2) part2[slot] = q;
+    }
+    __syncwarp();
+    double a = 0.0, a2 = 0.0;
+    if (pieces > 0) {
+      a = ipipe::plus_zero(sh.part[role][piece0]);
+      for (int k = 1; k < pieces; ++k) a = a + sh.part[role][piece0 + k];
+      if (NP == 2) {
+        a2 = ipipe::plus_zero(part2[piece0]);
+        for (int k = 1; k < pieces; ++k) a2 = a2 + part2[piece0 + k];
+      }
+    }
+    __syncwarp();
+    sh.part[role][lane] = a;
+    if (NP == 2) part2[lane] = a2;
+    team_sync(team);
+  }
+};
+
+}  // namespace bogus_gpu

@@ -53,3 +53,36 @@ def test_teams(oracle, n):
     D, O = _pair(oracle, n, n // 3, 7)
     for variant, coulomb in ((3, False), (4, True)):
         _compare(D, O, n, variant, coulomb, False, 15, np.zeros(3 * n))
+
+
+@pytest.mark.parametrize("sizes", [[1, 31, 32, 33, 160, 161, 1], [16] * 40 + [700, 340, 5, 64], [0, 50, 0, 200]])
+def test_batch(oracle, sizes):
+    """Batches whose problems span one and several CTAs, several problems per CTA, and empty problems: each problem as the
+    oracle solves it alone."""
+    import bogus_gpu
+    from bogus_gpu import generator
+
+    parts = [generator.random_pairs(max(2, n // 3), n, seed=90 + k) if n else None for k, n in enumerate(sizes)]
+    off = np.concatenate([[0], np.cumsum([d.nbodies if d else 0 for d in parts])])
+    live = [(d, o) for d, o in zip(parts, off) if d]
+    cat = lambda f: np.concatenate([f(d, o) for d, o in live])  # noqa: E731
+    D = bogus_gpu.DualFrictionProblem()
+    D.computeFrom(bogus_gpu.PrimalFrictionProblem(
+        cat(lambda d, o: d.minv), cat(lambda d, o: d.objA + o), cat(lambda d, o: np.where(d.objB >= 0, d.objB + o, -1)),
+        cat(lambda d, o: d.HA), cat(lambda d, o: d.HB), cat(lambda d, o: d.b), cat(lambda d, o: d.mu)))
+    ptr = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    D.setBatch(ptr)
+    for variant, static in ((3, True), (4, False), (1, True)):
+        pg = bogus_gpu.ProjectedGradient()
+        pg.setDefaultVariant(variant)
+        pg.setMaxIters(60)
+        pg.setTol(1e-8)
+        r = np.zeros(3 * ptr[-1])
+        res, its = D.solveBatchWith(pg, r, staticProblem=static)
+        for p, d in enumerate(parts):
+            if d is None:
+                continue
+            rp, cl, vl = oracle.PrimalProblem(d.minv, d.objA, d.objB, d.HA, d.HB).assemble()
+            ro, xo, io = oracle.DualProblem(rp, cl, vl, d.b, d.mu).solve_pg(
+                np.zeros(3 * d.n), variant=variant, coulomb=not static, tol=1e-8, max_iters=60)
+            assert res[p] == ro and its[p] == io and np.array_equal(r[3 * ptr[p]:3 * ptr[p + 1]], xo), (p, variant)
