@@ -24,15 +24,15 @@
 namespace bogus_gpu {
 
 // assembly kernels (kernels_assembly.cu)
-struct AssemblyPlan {
-  int n = 0, nbodies = 0, ndof = 0;
-  int nlow = 0;  // lower blocks to compute
-};
 cudaError_t launch_assembly_T(int n, int ndof, const double* minv, const int* cb, const double* H, double* T,
                               cudaStream_t s);
-cudaError_t launch_assembly_W(int nlow, int ndof, const int* li, const int* lj, const int* pair_off,
-                              const int* pair_ti, const int* pair_tj, const double* H, const double* T,
-                              const int* pos_ij, const int* pos_ji, double* val, cudaStream_t s);
+cudaError_t launch_assembly_slots(int n, int d, const int* cb, const int* objA, const double* HA, const double* HB,
+                                  double* H, cudaStream_t s);
+cudaError_t launch_lower_count(int n, const int* cb, const int* bptr, const int* bent, int* count, cudaStream_t s);
+cudaError_t launch_lower_fill(int n, const int* cb, const int* bptr, const int* bent, const int* rowptr, int* row,
+                              int* col, cudaStream_t s);
+cudaError_t launch_assembly_W(int nlow, int ndof, const int* row, const int* col, const int* cb, const double* H,
+                              const double* T, double* val, cudaStream_t s);
 cudaError_t launch_assembly_b(int n, int nbodies, int ndof, const double* minv, const double* f, const int* cb,
                               const double* H, const double* w, double* mf, double* b, cudaStream_t s);
 
@@ -149,6 +149,9 @@ struct bogus_gpu_problem {
   DevBuf<double> low_val[2];
   DevBuf<int> full_src, pat_upper, pat_cursor, pat_check;
   std::vector<double> host_b, host_mu;
+  DevBuf<int> asm_row;      // assembly: the row of every lower block
+  std::vector<int> h_bptr;  // the bodies' contact lists (bptr, bent) on the host
+  bool lists_valid = false;
   // projected-gradient work
   DevBuf<double> X, MX, Y, S0, XB, Wv, csum, scal, trace;
   // interleaved copy of W (coalesced chunk layout read by the single-problem solvers), valid while W is unchanged
@@ -1149,6 +1152,7 @@ int bogus_gpu_destroy(bogus_gpu_problem* h) {
   for (auto* b : {&h->a_prox, &h->a_f, &h->a_w, &h->a_mu, &h->a_invmu, &h->a_x, &h->a_r, &h->a_ut, &h->a_z, &h->a_zacc,
                   &h->a_rs1, &h->a_rs2, &h->a_yprev})
     b->release();
+  h->asm_row.release();
   h->bptr.release();
   h->bent.release();
   h->border.release();
@@ -2137,6 +2141,7 @@ int bogus_gpu_meche_from_primal(bogus_gpu_problem* h, unsigned nobj, const unsig
   h->h_cb = std::move(cbh);
   h->pgs.valid = false;
   h->h_objA = std::move(oA);
+  h->lists_valid = false;
   h->admm_incidence_valid = false;
   h->meche_ndof.assign(ndof, ndof + nobj);
   h->body_dofs.assign(ndof, ndof + nobj);
@@ -2312,35 +2317,29 @@ int bogus_gpu_set_primal(bogus_gpu_problem* h, int nbodies, int ndof, const doub
   if (int e = check_finite(HA, (size_t)ncontacts * 3 * ndof, "HA")) return e;
   if (int e = check_finite(HB, (size_t)ncontacts * 3 * ndof, "HB")) return e;
   std::vector<int> cbh(2 * (size_t)ncontacts);
-  std::vector<double> Hh(2 * (size_t)ncontacts * 3 * ndof, 0.0);
-  const size_t hs = 3 * (size_t)ndof;
   for (int i = 0; i < ncontacts; ++i) {
     const int a = objA[i], b = objB[i];
     if (a < 0 || a >= nbodies || b < -1 || b >= nbodies) return fail(BOGUS_GPU_BAD_INPUT, "body index out of range");
     // slots ordered by body index; a repeated body counts once (slot A)
-    int s0 = a, s1 = -1;
-    const double* h0 = HA + i * hs;
-    const double* h1 = nullptr;
-    if (b >= 0 && b != a) {
-      if (b < a) {
-        s0 = b; s1 = a; h0 = HB + i * hs; h1 = HA + i * hs;
-      } else {
-        s1 = b; h1 = HB + i * hs;
-      }
-    }
-    cbh[2 * (size_t)i] = s0;
-    cbh[2 * (size_t)i + 1] = s1;
-    std::copy(h0, h0 + hs, &Hh[(2 * (size_t)i) * hs]);
-    if (h1) std::copy(h1, h1 + hs, &Hh[(2 * (size_t)i + 1) * hs]);
+    const bool two = b >= 0 && b != a;
+    cbh[2 * (size_t)i] = two && b < a ? b : a;
+    cbh[2 * (size_t)i + 1] = two ? (b < a ? a : b) : -1;
   }
   if (int e = set_device(h)) return e;
+  const size_t nh = 3 * (size_t)ndof * ncontacts;
   BG_CUDA(h->minv.ensure((size_t)nbodies * ndof * ndof));
-  BG_CUDA(h->H.ensure(Hh.size()));
+  BG_CUDA(h->H.ensure(2 * nh));
   BG_CUDA(h->cb.ensure(cbh.size()));
   BG_CUDA(cudaMemcpyAsync(h->minv.p, minv, sizeof(double) * nbodies * ndof * ndof, cudaMemcpyHostToDevice, h->stream));
   if (ncontacts) {
-    BG_CUDA(cudaMemcpyAsync(h->H.p, Hh.data(), sizeof(double) * Hh.size(), cudaMemcpyHostToDevice, h->stream));
+    // the caller's blocks as they are, arranged into slots on the device (T, of the same size, is free until W's assembly)
+    BG_CUDA(h->T.ensure(2 * nh));
+    BG_CUDA(h->asm_row.ensure(ncontacts));
+    BG_CUDA(cudaMemcpyAsync(h->T.p, HA, sizeof(double) * nh, cudaMemcpyHostToDevice, h->stream));
+    BG_CUDA(cudaMemcpyAsync(h->T.p + nh, HB, sizeof(double) * nh, cudaMemcpyHostToDevice, h->stream));
     BG_CUDA(cudaMemcpyAsync(h->cb.p, cbh.data(), sizeof(int) * cbh.size(), cudaMemcpyHostToDevice, h->stream));
+    BG_CUDA(cudaMemcpyAsync(h->asm_row.p, objA, sizeof(int) * ncontacts, cudaMemcpyHostToDevice, h->stream));
+    BG_CUDA(launch_assembly_slots(ncontacts, ndof, h->cb.p, h->asm_row.p, h->T.p, h->T.p + nh, h->H.p, h->stream));
   }
   BG_CUDA(cudaStreamSynchronize(h->stream));
   h->nbodies = nbodies;
@@ -2349,6 +2348,7 @@ int bogus_gpu_set_primal(bogus_gpu_problem* h, int nbodies, int ndof, const doub
   h->h_cb = std::move(cbh);
   h->pgs.valid = false;
   h->h_objA.assign(objA, objA + ncontacts);
+  h->lists_valid = false;
   h->admm_incidence_valid = false;
   h->body_dofs.assign(nbodies, ndof);
   h->frames_valid = false;
@@ -2391,11 +2391,13 @@ namespace {
 
 // Body -> (contact, slot) incidences in increasing contact order (ADMM's H^T products, the adjoint's
 // primal gradients), built once per primal problem.
-int ensure_incidence(bogus_gpu_problem* h) {
-  if (h->admm_incidence_valid) return BOGUS_GPU_OK;
+int ensure_body_lists(bogus_gpu_problem* h) {
+  if (h->lists_valid) return BOGUS_GPU_OK;
   const int n = h->ncontacts, nb = h->nbodies;
   cudaStream_t s = h->stream;
-  std::vector<int> bp(nb + 1, 0), be;
+  std::vector<int>& bp = h->h_bptr;
+  std::vector<int> be;
+  bp.assign(nb + 1, 0);
   for (int i = 0; i < n; ++i)
     for (int t = 0; t < 2; ++t)
       if (h->h_cb[2 * (size_t)i + t] >= 0) ++bp[h->h_cb[2 * (size_t)i + t] + 1];
@@ -2411,6 +2413,18 @@ int ensure_incidence(bogus_gpu_problem* h) {
   BG_CUDA(h->bent.ensure(be.size()));
   BG_CUDA(cudaMemcpyAsync(h->bptr.p, bp.data(), sizeof(int) * (nb + 1), cudaMemcpyHostToDevice, s));
   BG_CUDA(cudaMemcpyAsync(h->bent.p, be.data(), sizeof(int) * be.size(), cudaMemcpyHostToDevice, s));
+  BG_CUDA(cudaStreamSynchronize(s));
+  h->lists_valid = true;
+  return BOGUS_GPU_OK;
+}
+
+// The lists, the order in which ADMM's body phase takes the bodies, and the error function's scalings.
+int ensure_incidence(bogus_gpu_problem* h) {
+  if (h->admm_incidence_valid) return BOGUS_GPU_OK;
+  if (int e = ensure_body_lists(h)) return e;
+  const int n = h->ncontacts, nb = h->nbodies;
+  cudaStream_t s = h->stream;
+  const std::vector<int>& bp = h->h_bptr;
   // bodies by decreasing contact count, stable: a warp's 32 bodies then loop over about as many contacts
   // each, so the lanes of the H^T r loop stay busy (a body's own arithmetic does not depend on the order)
   {
@@ -3033,108 +3047,57 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
   if (int e = check_finite(mu, n, "mu")) return e;
   if (f)
     if (int e = check_finite(f, (size_t)nb * d, "f")) return e;
-  // symbolic part: lower blocks (i, j <= i) of contacts sharing a body, shared (slot_i, slot_j) pairs
-  std::vector<std::vector<int>> by_body(nb);
-  for (int i = 0; i < n; ++i)
-    for (int t = 0; t < 2; ++t)
-      if (h->h_cb[2 * (size_t)i + t] >= 0) by_body[h->h_cb[2 * (size_t)i + t]].push_back(i);
-  HostBSR low;
-  low.n = n;
-  low.rowptr.assign(n + 1, 0);
-  std::vector<int> li, lj, pair_off(1, 0), pair_ti, pair_tj, cols;
-  for (int i = 0; i < n; ++i) {
-    cols.clear();
-    for (int t = 0; t < 2; ++t) {
-      const int k = h->h_cb[2 * (size_t)i + t];
-      if (k < 0) continue;
-      for (int j : by_body[k])
-        if (j <= i) cols.push_back(j);
-    }
-    std::sort(cols.begin(), cols.end());
-    cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
-    for (int j : cols) {
-      li.push_back(i);
-      lj.push_back(j);
-      for (int ti = 0; ti < 2; ++ti)
-        for (int tj = 0; tj < 2; ++tj) {
-          const int bi = h->h_cb[2 * (size_t)i + ti], bj = h->h_cb[2 * (size_t)j + tj];
-          if (bi >= 0 && bi == bj) {
-            pair_ti.push_back(ti);
-            pair_tj.push_back(tj);
-          }
-        }
-      pair_off.push_back((int)pair_ti.size());
-      low.col.push_back(j);
-    }
-    low.rowptr[i + 1] = (int)low.col.size();
-  }
-  const int nlow = (int)li.size();
-  // full-structure positions of every lower block and of its transpose
-  HostBSR fullpat;
-  fullpat.n = n;
-  {
-    std::vector<int> cnt(n + 1, 0);
-    for (int k = 0; k < nlow; ++k) {
-      ++cnt[li[k] + 1];
-      if (lj[k] != li[k]) ++cnt[lj[k] + 1];
-    }
-    fullpat.rowptr.assign(n + 1, 0);
-    for (int i = 0; i < n; ++i) fullpat.rowptr[i + 1] = fullpat.rowptr[i] + cnt[i + 1];
-  }
-  std::vector<int> pos_ij(nlow), pos_ji(nlow, -1);
-  fullpat.col.assign(fullpat.rowptr[n], 0);
-  {
-    std::vector<int> pos(fullpat.rowptr.begin(), fullpat.rowptr.end() - 1);
-    for (int k = 0; k < nlow; ++k) {  // lower blocks come row by row, columns increasing
-      pos_ij[k] = pos[li[k]]++;
-      fullpat.col[pos_ij[k]] = lj[k];
-      if (lj[k] != li[k]) {
-        pos_ji[k] = pos[lj[k]]++;
-        fullpat.col[pos_ji[k]] = li[k];
-      }
-    }
-  }
-  const int nnz = fullpat.rowptr[n];
-  DevBuf<int> d_li, d_lj, d_off, d_ti, d_tj, d_pij, d_pji;
-  BG_CUDA(d_li.ensure(nlow)); BG_CUDA(d_lj.ensure(nlow)); BG_CUDA(d_off.ensure(nlow + 1));
-  BG_CUDA(d_ti.ensure(pair_ti.size())); BG_CUDA(d_tj.ensure(pair_tj.size()));
-  BG_CUDA(d_pij.ensure(nlow)); BG_CUDA(d_pji.ensure(nlow));
+  if (int e = ensure_body_lists(h)) return e;
   cudaStream_t s = h->stream;
   auto up = [&](void* dst, const void* src, size_t bytes) {
     return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess;
   };
-  BG_CUDA(up(d_li.p, li.data(), sizeof(int) * nlow));
-  BG_CUDA(up(d_lj.p, lj.data(), sizeof(int) * nlow));
-  BG_CUDA(up(d_off.p, pair_off.data(), sizeof(int) * (nlow + 1)));
-  BG_CUDA(up(d_ti.p, pair_ti.data(), sizeof(int) * pair_ti.size()));
-  BG_CUDA(up(d_tj.p, pair_tj.data(), sizeof(int) * pair_tj.size()));
-  BG_CUDA(up(d_pij.p, pos_ij.data(), sizeof(int) * nlow));
-  BG_CUDA(up(d_pji.p, pos_ji.data(), sizeof(int) * nlow));
-  BG_CUDA(h->rowptr.ensure(n + 1));
-  BG_CUDA(h->col.ensure(nnz));
-  BG_CUDA(h->val.ensure(9 * (size_t)nnz));
+  // the pattern of the lower triangle (the staging set of the lower-triangle buffers, as in set_dual_lower)
+  const int nx = 1 - h->low_cur;
+  BG_CUDA(h->low_rowptr[nx].ensure(n + 1));
+  BG_CUDA(h->pat_upper.ensure(n > 0 ? n : 1));
+  BG_CUDA(h->pat_cursor.ensure(n > 0 ? n : 1));
   BG_CUDA(h->diag.ensure(n));
   BG_CUDA(h->b.ensure(3 * (size_t)n));
   BG_CUDA(h->mu.ensure(n));
   BG_CUDA(h->scaling.ensure(n));
+  BG_CUDA(h->rowptr.ensure(n + 1));
   BG_CUDA(h->T.ensure(2 * (size_t)n * d * 3));
   BG_CUDA(h->mf.ensure((size_t)nb * d));
-  BG_CUDA(up(h->rowptr.p, fullpat.rowptr.data(), sizeof(int) * (n + 1)));
-  BG_CUDA(up(h->col.p, fullpat.col.data(), sizeof(int) * nnz));
+  BG_CUDA(h->vx.ensure(3 * (size_t)n));
   BG_CUDA(up(h->mu.p, mu, sizeof(double) * n));
-  DevBuf<double> d_w, d_f;
-  BG_CUDA(d_w.ensure(3 * (size_t)n));
-  BG_CUDA(up(d_w.p, w, sizeof(double) * 3 * n));
-  if (h->frames_valid) BG_CUDA(launch_frame(n, h->frames.p, d_w.p, d_w.p, true, s));
+  BG_CUDA(up(h->vx.p, w, sizeof(double) * 3 * n));
+  if (h->frames_valid) BG_CUDA(launch_frame(n, h->frames.p, h->vx.p, h->vx.p, true, s));
   if (f) {
-    BG_CUDA(d_f.ensure((size_t)nb * d));
-    BG_CUDA(up(d_f.p, f, sizeof(double) * nb * d));
+    BG_CUDA(h->a_f.ensure((size_t)nb * d));
+    BG_CUDA(up(h->a_f.p, f, sizeof(double) * nb * d));
+  }
+  if (n == 0) {
+    BG_CUDA(cudaMemsetAsync(h->low_rowptr[nx].p, 0, sizeof(int), s));
+    BG_CUDA(cudaMemsetAsync(h->rowptr.p, 0, sizeof(int), s));
   }
   BG_CUDA(cudaEventRecord(h->ev0, s));
+  BG_CUDA(launch_lower_count(n, h->cb.p, h->bptr.p, h->bent.p, h->pat_upper.p, s));
+  BG_CUDA(launch_prefix_sum(n, h->pat_upper.p, h->pat_cursor.p, h->low_rowptr[nx].p, s));
+  int nlow = 0;
+  BG_CUDA(cudaMemcpyAsync(&nlow, h->low_rowptr[nx].p + n, sizeof(int), cudaMemcpyDeviceToHost, s));
   BG_CUDA(launch_assembly_T(n, d, h->minv.p, h->cb.p, h->H.p, h->T.p, s));
-  BG_CUDA(launch_assembly_W(nlow, d, d_li.p, d_lj.p, d_off.p, d_ti.p, d_tj.p, h->H.p, h->T.p, d_pij.p, d_pji.p,
-                            h->val.p, s));
-  BG_CUDA(launch_assembly_b(n, nb, d, h->minv.p, f ? d_f.p : nullptr, h->cb.p, h->H.p, d_w.p, h->mf.p, h->b.p, s));
+  BG_CUDA(launch_assembly_b(n, nb, d, h->minv.p, f ? h->a_f.p : nullptr, h->cb.p, h->H.p, h->vx.p, h->mf.p, h->b.p, s));
+  h->host_b.resize(3 * (size_t)n);
+  if (n) BG_CUDA(cudaMemcpyAsync(h->host_b.data(), h->b.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s));
+  BG_CUDA(cudaStreamSynchronize(s));
+  const int nnz = 2 * nlow - n;  // every row has its diagonal block
+  BG_CUDA(h->low_col[nx].ensure(nlow > 0 ? nlow : 1));
+  BG_CUDA(h->low_val[nx].ensure(9 * (size_t)(nlow > 0 ? nlow : 1)));
+  BG_CUDA(h->asm_row.ensure(nlow > 0 ? nlow : 1));
+  BG_CUDA(h->full_src.ensure(nnz > 0 ? nnz : 1));
+  BG_CUDA(h->col.ensure(nnz));
+  BG_CUDA(h->val.ensure(9 * (size_t)nnz));
+  BG_CUDA(launch_lower_fill(n, h->cb.p, h->bptr.p, h->bent.p, h->low_rowptr[nx].p, h->asm_row.p, h->low_col[nx].p, s));
+  BG_CUDA(launch_assembly_W(nlow, d, h->asm_row.p, h->low_col[nx].p, h->cb.p, h->H.p, h->T.p, h->low_val[nx].p, s));
+  BG_CUDA(launch_full_pattern(n, h->low_rowptr[nx].p, h->low_col[nx].p, h->pat_upper.p, h->pat_cursor.p, h->rowptr.p,
+                              h->col.p, h->full_src.p, s));
+  BG_CUDA(launch_expand_lower(nnz, h->full_src.p, h->low_val[nx].p, h->val.p, s));
   BG_CUDA(cudaEventRecord(h->ev1, s));
   h->W.n = n;
   h->W.nnzb = nnz;
@@ -3143,23 +3106,16 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
   h->W.val = h->val.p;
   h->W.diag = h->diag.p;
   BG_CUDA(launch_diag_and_scaling(h->W, h->scaling.p, s));
-  // host copies for the Gauss-Seidel coloring / permutation
-  low.val.resize(9 * (size_t)nlow);
-  std::vector<double> fullval(9 * (size_t)nnz);
-  if (nnz) BG_CUDA(cudaMemcpyAsync(fullval.data(), h->val.p, sizeof(double) * 9 * (size_t)nnz, cudaMemcpyDeviceToHost, s));
-  h->host_b.resize(3 * (size_t)n);
-  if (n) BG_CUDA(cudaMemcpyAsync(h->host_b.data(), h->b.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s));
   BG_CUDA(cudaStreamSynchronize(s));
   BG_CUDA(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
-  h->last_launches = 3;
-  for (int k = 0; k < nlow; ++k) std::copy(&fullval[9 * (size_t)pos_ij[k]], &fullval[9 * (size_t)pos_ij[k]] + 9, &low.val[9 * (size_t)k]);
-  h->host_lower = std::move(low);
-  h->host_lower_valid = true;
-  h->low_pending = false;
+  h->last_launches = 15;
+  // the host copy of the lower triangle is downloaded when first needed (ensure_host_lower)
+  h->low_cur = nx;
+  h->host_lower_valid = false;
+  h->low_pending = true;
+  h->host_lower.n = n;
   h->permuted = false;
   h->host_mu.assign(mu, mu + n);
-  d_li.release(); d_lj.release(); d_off.release(); d_ti.release(); d_tj.release(); d_pij.release(); d_pji.release();
-  d_w.release(); d_f.release();
   h->has_dual = true;
   h->gs.valid = false;
   h->nproblems = 0;

@@ -158,6 +158,7 @@ cudaError_t launch_check_lower(int n, const int* rowptr, const int* col, int* ou
 cudaError_t launch_check_full(int n, int nnzb, const int* rowptr, const int* col, int* out, cudaStream_t s);
 cudaError_t launch_full_pattern(int n, const int* rowptr, const int* col, int* upper, int* cursor, int* frowptr,
                                 int* fcol, int* src, cudaStream_t s);
+cudaError_t launch_prefix_sum(int n, const int* count, int* tiles, int* rowptr, cudaStream_t s);
 cudaError_t launch_expand_lower(int nnz, const int* src, const double* low, double* full, cudaStream_t s);
 cudaError_t launch_add(int m, const double* a, const double* b, double* y, cudaStream_t s);
 cudaError_t launch_cadoux_rhs(int n, const double* y, const double* mu, const double* b, double* out, cudaStream_t s);

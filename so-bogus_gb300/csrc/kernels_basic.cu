@@ -205,9 +205,9 @@ __global__ void k_count_upper(int n, const int* __restrict__ rowptr, const int* 
 
 // frowptr = exclusive prefix sum of the full row lengths (lower length + upper[i]), in three coalesced passes:
 // the sum of each tile of 1024 rows, an exclusive scan of the tile sums (one CTA), then each tile's scan plus
-// its offset. frowptr[n] receives the total.
+// its offset. frowptr[n] receives the total. A null rowptr counts as zero lengths.
 __device__ __forceinline__ int full_row_length(int i, int n, const int* __restrict__ rowptr, const int* __restrict__ upper) {
-  return i < n ? (__ldg(rowptr + i + 1) - __ldg(rowptr + i)) + __ldg(upper + i) : 0;
+  return i < n ? (rowptr ? __ldg(rowptr + i + 1) - __ldg(rowptr + i) : 0) + __ldg(upper + i) : 0;
 }
 // inclusive scan of v over the 1024 threads of the CTA; warp totals in ws[32]
 __device__ __forceinline__ int cta_inclusive_scan(int v, int* ws) {
@@ -332,6 +332,16 @@ cudaError_t launch_full_pattern(int n, const int* rowptr, const int* col, int* u
   if ((e = cudaMemsetAsync(cursor, 0, sizeof(int) * n, s)) != cudaSuccess) return e;
   k_place_lower<<<g, 256, 0, s>>>(n, rowptr, col, frowptr, fcol, src, cursor);
   k_sort_upper<<<g, 256, 0, s>>>(n, rowptr, frowptr, fcol, src);
+  return cudaGetLastError();
+}
+
+// rowptr = exclusive prefix sum of n counts (n + 1 entries); tiles: ceil(n / 1024) integers of scratch
+cudaError_t launch_prefix_sum(int n, const int* count, int* tiles, int* rowptr, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  const int ntiles = (n + 1023) / 1024;
+  k_rowlen_tiles<<<ntiles, 1024, 0, s>>>(n, nullptr, count, tiles);
+  k_scan_tiles<<<1, 1024, 0, s>>>(ntiles, tiles);
+  k_rowptr_tiles<<<ntiles, 1024, 0, s>>>(n, nullptr, count, tiles, rowptr);
   return cudaGetLastError();
 }
 
