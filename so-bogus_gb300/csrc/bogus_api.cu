@@ -216,6 +216,7 @@ struct bogus_gpu_problem {
   std::vector<unsigned> meche_ndof;
   // adjoint: per-contact basis, CG vectors, the last solution r and s = dL/db (device and host copies)
   DevBuf<double> adj_V, adj_Pc, adj_D, adj_K, adj_P, adj_R, adj_Z, adj_Dir, adj_Y, adj_Q, adj_S, adj_dmu, adj_r, adj_g;
+  DevBuf<double> adj_G;  // the resident kernel's gathered point, padded to 4 per contact
   DevBuf<double> adj_Tc, adj_Rh, adj_Ph, adj_Sv, adj_Sh, adj_Tv;  // Coulomb law: |u_T| and tau, BiCGSTAB vectors
   DevBuf<AdjOut> adj_out;
   bool adj_valid = false;
@@ -516,6 +517,30 @@ PGTraffic pg_traffic(const PGOut& out, int n, long long nnzb, int variant, doubl
   return t;
 }
 
+// What the resident kernels need of a problem's chunks dealt to one CTA per SM by ensure_cta_lists (ensure_chunks first).
+struct ResidentSize {
+  int ctas = 0, teams = 0, steps = 0, longest = 0;
+};
+int resident_size(const bogus_gpu_problem* h, ResidentSize* r) {
+  const int C = (int)h->h_chunk_order.size();
+  int sms = 0;
+  BG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+  *r = ResidentSize{};
+  if (C == 0) return BOGUS_GPU_OK;
+  r->ctas = std::min(sms, C);
+  r->teams = (C + r->ctas - 1) / r->ctas;
+  r->longest = h->h_chunk_seg[h->h_chunk_order[0]];
+  for (int b = 0; b < r->ctas; ++b) {
+    int sum = 0;
+    for (int t = 0; t < r->teams; ++t) {
+      const int k = t * r->ctas + ((t & 1) ? r->ctas - 1 - b : b);
+      if (k < C) sum += h->h_chunk_seg[h->h_chunk_order[k]];
+    }
+    r->steps = std::max(r->steps, sum);
+  }
+  return BOGUS_GPU_OK;
+}
+
 // FP32 correction products of an FP64 refinement (k_pg_persistent<double, true, false, true>).
 struct HyArgs {
   const float* ival;
@@ -588,22 +613,13 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
   BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 16 * sizeof(unsigned), h->stream));
   BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), h->stream));
   const bool sc = o->variant == BOGUS_GPU_PG_STANDARD || o->variant == BOGUS_GPU_PG_CONJUGATED;
-  int grid = 0, teams = 0, steps = 0;
+  int grid = 0;
+  ResidentSize rs;
   bool resident = false;
   if (!hy && !sc && !a.lin_momentum) {
-    int sms = 0;
-    BG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    grid = std::min(sms, a.nchunks);
-    teams = (a.nchunks + grid - 1) / grid;
-    for (int b = 0; b < grid; ++b) {  // the lists of ensure_cta_lists
-      int sum = 0;
-      for (int r = 0; r < teams; ++r) {
-        const int k = r * grid + ((r & 1) ? grid - 1 - b : b);
-        if (k < a.nchunks) sum += h->h_chunk_seg[h->h_chunk_order[k]];
-      }
-      steps = std::max(steps, sum);
-    }
-    resident = pg_resident_fits(h->device, teams, steps, h->h_chunk_seg[h->h_chunk_order[0]], n);
+    if (int e = resident_size(h, &rs)) return e;
+    grid = rs.ctas;
+    resident = pg_resident_fits(h->device, rs.teams, rs.steps, rs.longest, n);
   }
   if (!resident) {
     if (int e = ensure_interleaved(h)) return e;
@@ -619,7 +635,7 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
   a.cta_ptr = h->cta_ptr.p;
   a.cta_list = h->cta_list.p;
   BG_CUDA(cudaEventRecord(h->ev0, h->stream));
-  BG_CUDA(resident ? launch_pg_resident(a, grid, teams, steps, h->stream) : launch_pg_persistent(a, grid, h->stream));
+  BG_CUDA(resident ? launch_pg_resident(a, grid, rs.teams, rs.steps, h->stream) : launch_pg_persistent(a, grid, h->stream));
   BG_CUDA(cudaEventRecord(h->ev1, h->stream));
   PGOut out{};
   int st = 0;
@@ -1164,6 +1180,7 @@ int bogus_gpu_destroy(bogus_gpu_problem* h) {
                   &h->adj_Ph, &h->adj_Sv, &h->adj_Sh, &h->adj_Tv})
     b->release();
   h->adj_out.release();
+  h->adj_G.release();
   h->rowptr.release();
   h->col.release();
   h->diag.release();
@@ -2483,16 +2500,29 @@ int run_adjoint(bogus_gpu_problem* h, const bogus_gpu_adjoint_options* o, double
   BG_CUDA(h->adj_dmu.ensure(n > 0 ? n : 1));
   BG_CUDA(h->adj_out.ensure(1));
   const int C = (n + 31) / 32;
-  if (int e = ensure_phases(h, 2 * (size_t)C)) return e;
-  if (int e = ensure_interleaved(h)) return e;
+  if (int e = ensure_phases(h, 4 * (size_t)C)) return e;
+  if (int e = ensure_chunks(h)) return e;
+  ResidentSize rs;
+  if (int e = resident_size(h, &rs)) return e;
+  const bool resident = !o->coulomb && adjoint_resident_fits(h->device, rs.teams, rs.steps, rs.longest, n);
   AdjArgs a{};
   a.n = n;
   a.nchunks = C;
   a.rowptr = h->W.rowptr;
-  a.icol = h->icol.p;
-  a.ival = h->ival.p;
-  a.slot0 = h->slot0.p;
   a.val = h->W.val;
+  a.col = h->W.col;
+  if (resident) {
+    if (int e = ensure_cta_lists(h, rs.ctas)) return e;
+    BG_CUDA(h->adj_G.ensure(4 * (size_t)n));
+    a.cta_ptr = h->cta_ptr.p;
+    a.cta_list = h->cta_list.p;
+    a.G = h->adj_G.p;
+  } else {
+    if (int e = ensure_interleaved(h)) return e;
+    a.icol = h->icol.p;
+    a.ival = h->ival.p;
+    a.slot0 = h->slot0.p;
+  }
   a.b = h->b.p;
   a.mu = h->mu.p;
   a.scaling = h->scaling.p;
@@ -2525,10 +2555,11 @@ int run_adjoint(bogus_gpu_problem* h, const bogus_gpu_adjoint_options* o, double
   }
   BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 16 * sizeof(unsigned), s));
   BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), s));
-  const int grid = spread_grid(h->device, adjoint_max_grid(h->device), C);
+  const int grid = resident ? rs.ctas : spread_grid(h->device, adjoint_max_grid(h->device), C);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
   BG_CUDA(cudaEventRecord(h->ev0, s));
-  BG_CUDA(o->coulomb ? launch_adjoint_coulomb(a, grid, s) : launch_adjoint(a, grid, s));
+  BG_CUDA(resident ? launch_adjoint_resident(a, grid, rs.teams, rs.steps, s)
+                   : (o->coulomb ? launch_adjoint_coulomb(a, grid, s) : launch_adjoint(a, grid, s)));
   BG_CUDA(cudaEventRecord(h->ev1, s));
   AdjOut out{};
   int st = 0;

@@ -316,7 +316,11 @@ struct AdjArgs {
   const int* icol;     // W, both triangles, interleaved (InterleavedBlocks)
   const double* ival;
   const long long* slot0;
-  const double* val;   // W, plain BSR (diagonal blocks)
+  const double* val;   // W, plain BSR (diagonal blocks; all of it in the resident kernel)
+  const int* col;
+  const int* cta_ptr;  // the resident kernel's chunk lists (as PGArgsT)
+  const int* cta_list;
+  double* G;           // the resident kernel's gathered point, 4 per contact
   const double* b;
   const double* mu;
   const double* scaling;  // per-contact fixed-point step 1 / scaling_i
@@ -340,6 +344,8 @@ struct AdjArgs {
 cudaError_t launch_adjoint(const AdjArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_adjoint_coulomb(const AdjArgs& a, int grid, cudaStream_t s);
 int adjoint_max_grid(int device);
+bool adjoint_resident_fits(int device, int teams, int steps, int longest, int n);
+cudaError_t launch_adjoint_resident(const AdjArgs& a, int ctas, int teams, int steps, cudaStream_t s);
 // Helpers of the primal gradients and of the compliance term (kernels_grad.cu)
 cudaError_t launch_body_transpose(int nbodies, int d, const int* bptr, const int* bent, const double* H,
                                   const double* minv, const double* vec, const double* f, double* out,

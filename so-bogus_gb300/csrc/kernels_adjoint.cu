@@ -22,6 +22,7 @@
 // A persistent cooperative kernel runs the setup, the CG iterations and the final pass; reductions use the
 // canonical order of the solver kernels, waits are bounded (Phases).
 #include "internal.h"
+#include "resident.cuh"
 #include "soc_device.cuh"
 #include "spmv_chunk.cuh"
 
@@ -314,6 +315,208 @@ __global__ void __launch_bounds__(256) k_adjoint(AdjArgs a) {
     a.out->iters = it;
     a.out->rel_res = rr0 > 0.0 ? sqrt(rr / rr0) : 0.0;
   }
+}
+
+// k_adjoint for problems that fit the SMs' shared memory (resident.cuh): a team of three warps per chunk, warp r with
+// component r of every CG vector, the rows and columns of the basis and the preconditioner that it needs in registers;
+// the team exchanges the other components through shared memory, and global memory carries only the gathered point and
+// the chunk sums. The operations and their order are k_adjoint's, so the results are identical.
+// Adjoint of 4 x 2 500 contacts on GB300: 4.35 ms with k_adjoint, 2.39 ms here.
+struct AdjTeam {
+  TeamCore core;
+  double ex[3][32];
+};
+struct AdjControl {
+  double stripes[32];
+  double rr, rz, step, beta;
+  int stop;
+};
+
+__global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_adjoint_resident(AdjArgs a, int teams) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int team = warp / kTeamWarps, role = warp - kTeamWarps * team;
+  AdjControl& ctl = *reinterpret_cast<AdjControl*>(smem);
+  const int first = __ldg(a.cta_ptr + blockIdx.x);
+  const bool has = team < teams && first + team < __ldg(a.cta_ptr + blockIdx.x + 1);
+  const int c = has ? __ldg(a.cta_list + first + team) : 0;
+  AdjTeam& sh = reinterpret_cast<AdjTeam*>(smem + (sizeof(AdjControl) + 15) / 16 * 16)[team < teams ? team : 0];
+  const int C = a.nchunks, i = 32 * c + lane;
+  const bool on = has && i < a.n;
+  ResidentChunk chunk{sh.core, lane, role, team};
+  if (has) {
+    size_t before = 0;
+    for (int k = 0; k < team; ++k) before += (size_t)steps_of(a.rowptr, a.n, __ldg(a.cta_list + first + k));
+    chunk.load(a.rowptr, a.col, a.val, a.n, c,
+               smem + (sizeof(AdjControl) + 15) / 16 * 16 + (size_t)teams * sizeof(AdjTeam) + before * kStepBytes);
+  }
+  ResidentReduce red{MonoBarrier{a.ps.mono, a.ps.gb.status, gridDim.x}, a.ps.csum, C, ctl.stripes, lane, warp, nwarps};
+  // every component of v (this warp's) for the lane's contact
+  auto exchange = [&](double v, double* out) {
+    sh.ex[role][lane] = v;
+    team_sync(team);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) out[k] = sh.ex[k][lane];
+    team_sync(team);
+  };
+
+  // setup (k_adjoint): the gathered point is r
+  if (on) a.G[4 * (size_t)i + role] = __ldg(a.r + 3 * (size_t)i + role);
+  if (!red.sync()) return;
+  double Vr[3] = {0.0, 0.0, 0.0}, Vc[3] = {0.0, 0.0, 0.0}, Pr[3] = {0.0, 0.0, 0.0};  // row and column of V, row of Pinv
+  double Dk = -1.0, p = 0.0, res = 0.0, d = 0.0, q = 0.0, z = 0.0;
+  // y_role = (V (m o v))_role, v this warp's component
+  auto basis = [&](double v) -> double {
+    double m[3];
+    exchange(Dk < 0.0 ? 0.0 : v, m);
+    return Vr[0] * m[0] + Vr[1] * m[1] + Vr[2] * m[2];
+  };
+  if (has) {
+    chunk.product<1>(a.G);
+    double rr = 0.0, rz = 0.0, cr = 0.0;
+    if (on) {
+      double x[3], V[9], D[3], K[3], g[3], cv[3], Wii[9], Pinv[9], zv[3];
+      const double al = 1.0 / __ldg(a.scaling + i);
+      for (int k = 0; k < 3; ++k)
+        x[k] = __ldg(a.r + 3 * (size_t)i + k) - al * (sh.core.part[k][lane] + __ldg(a.b + 3 * i + k));
+      projection_basis(__ldg(a.mu + i), x, al, V, D, K);
+      const int dk = __ldg(a.diag + i);
+      for (int k = 0; k < 9; ++k) Wii[k] = dk >= 0 ? __ldg(a.val + 9 * (size_t)dk + k) : 0.0;
+      precond_block(V, D, Wii, Pinv);
+      if (role == 0) {  // for the last pass
+        for (int k = 0; k < 9; ++k) a.V[9 * (size_t)i + k] = V[k];
+        st3(a.D, i, D);
+        st3(a.K, i, K);
+      }
+      ld3(a.g, i, g);
+      basis_apply_t(V, D, g, cv);
+      mat3_apply(Pinv, cv, zv);
+      rr = cv[0] * cv[0] + cv[1] * cv[1] + cv[2] * cv[2];
+      rz = cv[0] * zv[0] + cv[1] * zv[1] + cv[2] * zv[2];
+      double y[3];
+      basis_apply(V, D, zv, y);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        if (role == k) {
+          for (int e = 0; e < 3; ++e) {
+            Vr[e] = V[3 * k + e];
+            Vc[e] = V[3 * e + k];
+            Pr[e] = Pinv[3 * k + e];
+          }
+          Dk = D[k];
+          res = cv[k];
+          d = zv[k];
+          cr = y[k];
+        }
+    }
+    team_sync(team);  // the product has been read: the gathered point may go
+    if (role == 0) red.put(0, c, rr);
+    else if (role == 1) red.put(1, c, rz);
+    z = cr;  // Y of the first iteration, written once every CTA has read r
+  }
+  if (!red.reduce(2, 0u, [] {}, [&](double total) {
+        const double v = total_of(total, 0), w = total_of(total, 1);
+        if (lane == 0) {
+          ctl.rr = v;
+          ctl.rz = w;
+        }
+      }))
+    return;
+  if (on) a.G[4 * (size_t)i + role] = z;
+  if (!red.sync()) return;
+  const double rr0 = ctl.rr;
+  const double stop = a.tol * a.tol * rr0;
+  unsigned it = 0;
+  for (; it < a.max_iters; ++it) {
+    if (!(ctl.rr > stop)) break;
+    // q = D o dir + m o V^T W Y, dir . q
+    if (has) {
+      chunk.product<1>(a.G);
+      const double a0 = sh.core.part[0][lane], a1 = sh.core.part[1][lane], a2 = sh.core.part[2][lane];
+      const double t = Vc[0] * a0 + Vc[1] * a1 + Vc[2] * a2;
+      q = Dk < 0.0 ? 0.0 : Dk * d + t;
+      double m[3];
+      exchange(d * q, m);
+      if (role == 0) red.put(0, c, on ? m[0] + m[1] + m[2] : 0.0);
+    }
+    if (!red.reduce(1, 0u, [] {}, [&](double total) {
+          const double dq = total_of(total, 0);
+          const double step = ipipe::div_rn(ctl.rz, dq);
+          if (lane == 0) {
+            ctl.step = step;
+            ctl.stop = !(dq > 0.0);  // S is positive definite on the unmasked components; guards exact convergence
+          }
+        }))
+      return;
+    if (ctl.stop) break;
+    const double step = ctl.step;
+    if (has) {
+      p = fma(step, d, p);
+      res = fma(-step, q, res);
+      double r3[3], m[3];
+      exchange(res, r3);
+      z = Pr[0] * r3[0] + Pr[1] * r3[1] + Pr[2] * r3[2];
+      exchange(res * z, m);
+      if (role == 0) red.put(0, c, on ? r3[0] * r3[0] + r3[1] * r3[1] + r3[2] * r3[2] : 0.0);
+      else if (role == 1) red.put(1, c, on ? m[0] + m[1] + m[2] : 0.0);
+    }
+    if (!red.reduce(2, 0u, [] {}, [&](double total) {
+          const double rr = total_of(total, 0), rz = total_of(total, 1);
+          const double beta = ipipe::div_rn(rz, ctl.rz);
+          __syncwarp();
+          if (lane == 0) {
+            ctl.rr = rr;
+            ctl.rz = rz;
+            ctl.beta = beta;
+          }
+        }))
+      return;
+    if (has) {
+      d = fma(ctl.beta, d, z);
+      const double y = basis(d);
+      if (on) a.G[4 * (size_t)i + role] = y;
+    }
+    if (!red.sync()) return;
+  }
+  // s = dL/db = -V (m o p)
+  if (has) {
+    const double s = -basis(p);
+    if (on) {
+      a.S[3 * (size_t)i + role] = s;
+      a.G[4 * (size_t)i + role] = s;
+    }
+  }
+  if (!red.sync()) return;
+  // lam_hat and dL/dmu = K^T V lam_hat
+  if (has) {
+    chunk.product<1>(a.G);
+    double pv[3];
+    exchange(p, pv);
+    if (on && role == 0) {
+      double V[9], D[3], g[3], K[3], e[3], lh[3];
+      for (int k = 0; k < 9; ++k) V[k] = a.V[9 * (size_t)i + k];
+      ld3(a.D, i, D);
+      ld3(a.g, i, g);
+      ld3(a.K, i, K);
+      const double al = 1.0 / __ldg(a.scaling + i);
+      for (int k = 0; k < 3; ++k) e[k] = g[k] + sh.core.part[k][lane];
+      for (int k = 0; k < 3; ++k) {
+        if (D[k] < 0.0) lh[k] = V[k] * e[0] + V[3 + k] * e[1] + V[6 + k] * e[2];
+        else lh[k] = pv[k] * (1.0 + al * D[k]) / al;  // p / (alpha theta), theta = 1 / (1 + alpha D)
+      }
+      double dm = 0.0;
+      for (int r2 = 0; r2 < 3; ++r2) dm += K[r2] * (V[3 * r2] * lh[0] + V[3 * r2 + 1] * lh[1] + V[3 * r2 + 2] * lh[2]);
+      a.dmu[i] = dm;
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.out->iters = it;
+    a.out->rel_res = rr0 > 0.0 ? sqrt(ctl.rr / rr0) : 0.0;
+  }
+}
+
+size_t adjoint_resident_smem(int teams, int steps) {
+  return (sizeof(AdjControl) + 15) / 16 * 16 + (size_t)teams * sizeof(AdjTeam) + (size_t)steps * kStepBytes;
 }
 
 // ---- Coulomb law ----------------------------------------------------------------------------------------
@@ -640,6 +843,24 @@ cudaError_t launch_adjoint_coulomb(const AdjArgs& a, int grid, cudaStream_t s) {
   AdjArgs copy = a;
   void* args[] = {&copy};
   return cudaLaunchCooperativeKernel((const void*)k_adjoint_coulomb, dim3(grid), dim3(256), args, 0, s);
+}
+
+bool adjoint_resident_fits(int device, int teams, int steps, int longest, int n) {
+  int limit = 0;
+  if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return false;
+  return teams >= 1 && teams <= kMaxTeams && longest <= 64 && n <= 65536 &&
+         adjoint_resident_smem(teams, steps) + 1024 <= (size_t)limit;
+}
+
+cudaError_t launch_adjoint_resident(const AdjArgs& a, int ctas, int teams, int steps, cudaStream_t s) {
+  const size_t bytes = adjoint_resident_smem(teams, steps);
+  const void* fn = (const void*)k_adjoint_resident;
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) return e;
+  AdjArgs copy = a;
+  void* args[] = {&copy, &teams};
+  const int warps = kTeamWarps * teams > kMinWarps ? kTeamWarps * teams : kMinWarps;
+  return cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(32 * warps), args, bytes, s);
 }
 
 int adjoint_max_grid(int device) {

@@ -91,72 +91,11 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
   };
 
   // ---- barriers ----------------------------------------------------------------------------------------------
-  const MonoBarrier mb{a.mono, a.gb.status, place.parties + a.phantom_ctas};
-  unsigned phase = 0;  // barriers passed
-  auto sums = [&]() { return a.csum + (size_t)(phase & 1u) * 4 * C; };
-  auto put = [&](int q, double v) {
-    v = warp_sum_butterfly(v);
-    if (lane == 0) sums()[q * C + c] = v;
-  };
-  // The last warp prepares the next decision (side) while thread 0 waits for the other CTAs.
-  auto arrive_and_wait = [&](auto side) -> bool {
-    bool ok = true;
-    __syncthreads();
-    if (warp == nwarps - 1) side();
-    if (mb.parties > 1u && threadIdx.x == 0) ok = flat_wait(mb, phase);
-    return __syncthreads_and(ok) != 0;
-  };
-  // Barrier, the K reduced quantities, then decide(totals) by warp 0 (the same values in every lane).
-  auto reduce = [&](int K, unsigned maxmask, auto side, auto decide) -> bool {
-    if (!arrive_and_wait(side)) return false;
-    const double* s = sums();
-    const int per = (C + 7) / 8;
-    if (warp < 8) {
-      const int st = warp, b = st * per, e = min(C, b + per);
-      double p[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int k = b + lane; k < e; k += 32) {
-        double v[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = q < K ? ldcg(s + q * C + k) : 0.0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (q < K) p[q] = (maxmask >> q) & 1u ? ((v[q] < p[q]) ? p[q] : v[q]) : p[q] + v[q];
-      }
-      if (b >= e) {
-        if (lane < K) ctl.stripes[8 * lane + st] = 0.0;
-      } else if (maxmask) {
-        const double v0 = warp_max_butterfly(p[0]), v1 = warp_sum_butterfly(p[1]);  // the residual and one sum
-        if (lane < 2) ctl.stripes[8 * lane + st] = lane ? v1 : v0;
-      } else if (K == 4) {
-        const double v = warp_sum4_butterfly(p[0], p[1], p[2], p[3]);
-        if ((lane & 7) == 0) ctl.stripes[lane + st] = v;
-      } else {
-        const double v = warp_sum2_butterfly(p[0], p[1]);
-        if ((lane & 15) == 0) ctl.stripes[lane / 2 + st] = v;
-      }
-    }
-    __syncthreads();
-    if (warp == 0) {
-      const int q = lane < K ? lane : 0;
-      const bool mx = (maxmask >> q) & 1u;
-      double total = ctl.stripes[8 * q];
-#pragma unroll
-      for (int k = 1; k < 8; ++k) {
-        const double v = ctl.stripes[8 * q + k];
-        total = mx ? ((v < total) ? total : v) : total + v;
-      }
-      decide(total);
-    }
-    __syncthreads();
-    ++phase;
-    return true;
-  };
-  auto sync = [&]() -> bool {
-    const bool ok = arrive_and_wait([] {});
-    ++phase;
-    return ok;
-  };
-  auto total_of = [](double total, int q) { return __shfl_sync(0xffffffffu, total, q); };
+  ResidentReduce red{MonoBarrier{a.mono, a.gb.status, place.parties + a.phantom_ctas}, a.csum, C, ctl.stripes, lane, warp, nwarps};
+  auto sums = [&]() { return red.sums(); };
+  auto put = [&](int q, double v) { red.put(q, c, v); };
+  auto reduce = [&](int K, unsigned maxmask, auto side, auto decide) { return red.reduce(K, maxmask, side, decide); };
+  auto sync = [&]() { return red.sync(); };
 
   // ---- per-contact state, the same in the team's three warps ------------------------------------------------
   // (x and prev in registers; xs, y and the products in the team's shared memory; b, mu and the scalings are read

@@ -202,4 +202,83 @@ struct ResidentChunk {
   }
 };
 
+// Barriers and reductions of kernels whose CTAs own chunks: the flat barrier, one stripe per warp, the totals and the
+// decision by warp 0. Every thread of the CTA calls; chunk sums alternate between two buffers of 4 C.
+struct ResidentReduce {
+  const MonoBarrier mb;
+  double* csum;
+  const int C;
+  double* stripes;  // 32 shared doubles
+  const int lane, warp, nwarps;
+  unsigned phase = 0;  // barriers passed
+  __device__ double* sums() const { return csum + (size_t)(phase & 1u) * 4 * C; }
+  // sum of v over the warp as chunk c's value of quantity q
+  __device__ void put(int q, int c, double v) {
+    v = warp_sum_butterfly(v);
+    if (lane == 0) sums()[q * C + c] = v;
+  }
+  // The last warp prepares the next decision (side) while thread 0 waits for the other CTAs.
+  template <class Side>
+  __device__ bool arrive_and_wait(Side&& side) {
+    bool ok = true;
+    __syncthreads();
+    if (warp == nwarps - 1) side();
+    if (mb.parties > 1u && threadIdx.x == 0) ok = flat_wait(mb, phase);
+    return __syncthreads_and(ok) != 0;
+  }
+  __device__ bool sync() {
+    const bool ok = arrive_and_wait([] {});
+    ++phase;
+    return ok;
+  }
+  // Barrier, K <= 4 quantities (value 0 a maximum where maxmask; K == 2 then), then decide(total) by warp 0, lane q < K
+  // holding quantity q's total (read the others with total_of).
+  template <class Side, class Decide>
+  __device__ bool reduce(int K, unsigned maxmask, Side&& side, Decide&& decide) {
+    if (!arrive_and_wait(side)) return false;
+    const double* s = sums();
+    const int per = (C + 7) / 8;
+    if (warp < 8) {
+      const int st = warp, b = st * per, e = min(C, b + per);
+      double p[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int k = b + lane; k < e; k += 32) {
+        double v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = q < K ? ldcg(s + q * C + k) : 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q < K) p[q] = (maxmask >> q) & 1u ? ((v[q] < p[q]) ? p[q] : v[q]) : p[q] + v[q];
+      }
+      if (b >= e) {
+        if (lane < K) stripes[8 * lane + st] = 0.0;
+      } else if (maxmask) {
+        const double v0 = warp_max_butterfly(p[0]), v1 = warp_sum_butterfly(p[1]);
+        if (lane < 2) stripes[8 * lane + st] = lane ? v1 : v0;
+      } else if (K > 2) {
+        const double v = warp_sum4_butterfly(p[0], p[1], p[2], p[3]);
+        if ((lane & 7) == 0) stripes[lane + st] = v;
+      } else {
+        const double v = warp_sum2_butterfly(p[0], p[1]);
+        if ((lane & 15) == 0) stripes[lane / 2 + st] = v;
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const int q = lane < K ? lane : 0;
+      const bool mx = (maxmask >> q) & 1u;
+      double total = stripes[8 * q];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) {
+        const double v = stripes[8 * q + k];
+        total = mx ? ((v < total) ? total : v) : total + v;
+      }
+      decide(total);
+    }
+    __syncthreads();
+    ++phase;
+    return true;
+  }
+};
+__device__ __forceinline__ double total_of(double total, int q) { return __shfl_sync(0xffffffffu, total, q); }
+
 }  // namespace bogus_gpu

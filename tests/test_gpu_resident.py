@@ -86,3 +86,30 @@ def test_batch(oracle, sizes):
             ro, xo, io = oracle.DualProblem(rp, cl, vl, d.b, d.mu).solve_pg(
                 np.zeros(3 * d.n), variant=variant, coulomb=not static, tol=1e-8, max_iters=60)
             assert res[p] == ro and its[p] == io and np.array_equal(r[3 * ptr[p]:3 * ptr[p + 1]], xo), (p, variant)
+
+
+@pytest.mark.parametrize("n,nbodies", [(1, 2), (33, 30), (161, 120)])
+def test_adjoint(oracle, n, nbodies):
+    """The adjoint's resident kernel (a partial chunk, one past a chunk, several CTAs) against the dense gradients, within
+    the adjoint tests' 1e-8 of the largest entry (conjugate gradients stop at 1e-13)."""
+    import adjoint
+    import bogus_gpu
+
+    D, _ = _pair(oracle, n, nbodies, 60 + n)
+    D.add_compliance(0.05)
+    rp, cl, vl = D.W_lower()
+    b, mu = np.empty(3 * n), np.empty(n)
+    assert bogus_gpu.lib().bogus_gpu_get_dual_rhs(D.handle, b.ctypes.data, mu.ctypes.data) == 0
+    _, r, _ = oracle.DualProblem(rp, cl, vl.reshape(-1), b, mu).solve_gs(np.zeros(3 * n), coulomb=False, tol=1e-32,
+                                                                         max_iters=3000, coloring=False)
+    W = np.zeros((3 * n, 3 * n))
+    for i in range(n):
+        for k in range(rp[i], rp[i + 1]):
+            j = cl[k]
+            W[3 * i:3 * i + 3, 3 * j:3 * j + 3] = vl[k]
+            W[3 * j:3 * j + 3, 3 * i:3 * i + 3] = vl[k].T
+    g = np.random.default_rng(n).standard_normal(3 * n)
+    s_o, dmu_o, _ = adjoint.implicit_gradient(W, b, mu, r, g)
+    s, dmu = D.adjoint(r, g, tol=1e-13)
+    assert np.abs(s - s_o).max() <= 1e-8 * max(np.abs(s_o).max(), 1e-300)
+    assert np.abs(dmu - dmu_o).max() <= 1e-8 * max(1.0, np.abs(dmu_o).max())
