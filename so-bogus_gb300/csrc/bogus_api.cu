@@ -173,6 +173,7 @@ struct bogus_gpu_problem {
   // FP32 correction products of the FP64 refinement: v - x_ref for 4 position buffers, x_ref, W x_ref
   DevBuf<float> hy_d;
   DevBuf<double> hy_xref, hy_wxref;
+  DevBuf<double> hy_scratch;  // k_pg_resident32: per-warp scratch of its FP64 products
   bool fp32p_valid = false;
   DevBuf<PGOut> pgout;
   DevBuf<unsigned> barrier;
@@ -549,6 +550,7 @@ struct HyArgs {
   double* wxref;
   unsigned refresh;
   size_t stride;  // floats between the position buffers' corrections in d
+  bool resident = false;  // k_pg_resident32 (corrections 4 floats per contact)
 };
 
 int pg_grid(int device, bool fp32, int nchunks) {
@@ -621,7 +623,7 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
     grid = rs.ctas;
     resident = pg_resident_fits(h->device, rs.teams, rs.steps, rs.longest, n);
   }
-  if (!resident) {
+  if (!resident) {  // or k_pg_resident32, which reads the FP64 copy at its refreshes
     if (int e = ensure_interleaved(h)) return e;
     a.icol = h->icol.p;
     a.ival = h->ival.p;
@@ -629,13 +631,21 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
     a.chunk_order = h->chunk_order.p;
     grid = pg_grid(h->device, false, a.nchunks);
   }
+  if (hy && hy->resident) {
+    if (int e = resident_size(h, &rs)) return e;
+    grid = rs.ctas;
+    BG_CUDA(h->hy_scratch.ensure(pg_resident32_scratch(rs.ctas, rs.teams) / sizeof(double) + 1));
+  }
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
   a.flat = !sc && a.nchunks <= kFlatChunks;
   if (int e = ensure_cta_lists(h, grid)) return e;
   a.cta_ptr = h->cta_ptr.p;
   a.cta_list = h->cta_list.p;
   BG_CUDA(cudaEventRecord(h->ev0, h->stream));
-  BG_CUDA(resident ? launch_pg_resident(a, grid, rs.teams, rs.steps, h->stream) : launch_pg_persistent(a, grid, h->stream));
+  BG_CUDA(resident ? launch_pg_resident(a, grid, rs.teams, rs.steps, h->stream)
+          : hy && hy->resident
+              ? launch_pg_resident32(a, grid, rs.teams, rs.steps, h->hy_scratch.p, h->stream)
+              : launch_pg_persistent(a, grid, h->stream));
   BG_CUDA(cudaEventRecord(h->ev1, h->stream));
   PGOut out{};
   int st = 0;
@@ -753,12 +763,13 @@ int ensure_fp32(bogus_gpu_problem* h) {
   const int n = h->W.n;
   const size_t n3 = 3 * (size_t)n;
   cudaStream_t s = h->stream;
-  BG_CUDA(h->X32.ensure(3 * n3));
+  const size_t n4 = 4 * (size_t)n;  // positions: 3 or 4 floats per contact
+  BG_CUDA(h->X32.ensure(3 * n4));
   BG_CUDA(h->MX32.ensure(4 * n3));
   BG_CUDA(h->Y32.ensure(n3));
   BG_CUDA(h->S032.ensure(n));
-  BG_CUDA(h->XB32.ensure(n3));
-  BG_CUDA(h->Wv32.ensure(n3));
+  BG_CUDA(h->XB32.ensure(n4));
+  BG_CUDA(h->Wv32.ensure(n4));
   if (int e = ensure_interleaved(h)) return e;
   if (h->fp32_valid) return BOGUS_GPU_OK;
   BG_CUDA(h->val32.ensure(h->ival.n));
@@ -796,6 +807,10 @@ int run_pg_mixed(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* re
   if (int e = ensure_fp32(h)) return e;
   if (int e = ensure_pg_work(h, o->max_iters > o->refine_max_iters ? o->max_iters : o->refine_max_iters)) return e;
   cudaStream_t s = h->stream;
+  ResidentSize rs;
+  if (int e = resident_size(h, &rs)) return e;
+  const bool resident = pg_resident32_fits(h->device, rs.teams, rs.steps, rs.longest, n);
+  const size_t nx = resident ? 4 * (size_t)n : n3;
   PGArgs32 a{};
   a.n = n;
   a.nchunks = (n + 31) / 32;
@@ -810,8 +825,8 @@ int run_pg_mixed(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* re
   a.mu = h->mu32.p;
   a.scaling = h->sc32.p;
   a.X0 = h->X32.p;
-  a.X1 = h->X32.p + n3;
-  a.X2 = h->X32.p + 2 * n3;
+  a.X1 = h->X32.p + nx;
+  a.X2 = h->X32.p + 2 * nx;
   a.MX0 = h->MX32.p;
   a.MX1 = h->MX32.p + n3;
   a.MX2 = h->MX32.p + 2 * n3;
@@ -833,17 +848,17 @@ int run_pg_mixed(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* re
   // the line search retry more often (measured slower, with a worse starting point for the FP64 part)
   a.lin_momentum = 0;
   a.stall_iters = o->fp32_stall_iters;
-  BG_CUDA(launch_convert(n3, h->X.p, h->X32.p, s));
+  BG_CUDA(resident ? launch_pad_positions(n, h->X.p, h->X32.p, s) : launch_convert(n3, h->X.p, h->X32.p, s));
   BG_CUDA(cudaMemsetAsync(h->barrier.p, 0, 16 * sizeof(unsigned), s));
   BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), s));
-  const int grid = pg_grid(h->device, true, a.nchunks);
+  const int grid = resident ? rs.ctas : pg_grid(h->device, true, a.nchunks);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
   a.flat = a.nchunks <= kFlatChunks;
   if (int e = ensure_cta_lists(h, grid)) return e;
   a.cta_ptr = h->cta_ptr.p;
   a.cta_list = h->cta_list.p;
   BG_CUDA(cudaEventRecord(h->ev0, s));
-  BG_CUDA(launch_pg_persistent(a, grid, s));
+  BG_CUDA(resident ? launch_pg_resident32(a, grid, rs.teams, rs.steps, s) : launch_pg_persistent(a, grid, s));
   BG_CUDA(cudaEventRecord(h->ev1, s));
   PGOut out{};
   int st = 0;
@@ -854,8 +869,8 @@ int run_pg_mixed(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* re
   BG_CUDA(cudaEventElapsedTime(&ms32, h->ev0, h->ev1));
   if (st != 0) return fail(st, "device-side wait timed out in the FP32 projected-gradient kernel");
   const float* b32 =
-      out.best_buf == 3 ? h->XB32.p : (out.best_buf == 4 ? h->Wv32.p : h->X32.p + (size_t)out.best_buf * n3);
-  BG_CUDA(launch_convert(n3, b32, h->X.p, s));
+      out.best_buf == 3 ? h->XB32.p : (out.best_buf == 4 ? h->Wv32.p : h->X32.p + (size_t)out.best_buf * nx);
+  BG_CUDA(resident ? launch_unpad_positions(n, b32, h->X.p, s) : launch_convert(n3, b32, h->X.p, s));
   const unsigned it32 = out.iters;
   const PGTraffic t32 = pg_traffic(out, n, h->W.nnzb, o->variant, 4.0, lin_momentum(o) != 0);
   bogus_gpu_pg_options o64 = *o;
@@ -865,10 +880,10 @@ int run_pg_mixed(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* re
   float msh = 0.f;
   bogus_gpu_solve_stats sth{};
   if (o->fp32_products_refresh) {
-    BG_CUDA(h->hy_d.ensure(4 * n3));
+    BG_CUDA(h->hy_d.ensure(4 * nx));
     BG_CUDA(h->hy_xref.ensure(n3));
     BG_CUDA(h->hy_wxref.ensure(n3));
-    const HyArgs hy{h->val32.p, h->hy_d.p, h->hy_xref.p, h->hy_wxref.p, o->fp32_products_refresh, n3};
+    const HyArgs hy{h->val32.p, h->hy_d.p, h->hy_xref.p, h->hy_wxref.p, o->fp32_products_refresh, nx, resident};
     double resh = 0.0;
     const double* besth = nullptr;
     const int hst = run_pg(h, &o64, &resh, &ith, &besth, &hy);
@@ -3978,6 +3993,7 @@ int bogus_gpu_set_wait_limit(int device, double seconds) {
   const unsigned long long ns = (unsigned long long)(seconds * 1e9);
   cudaError_t e = set_wait_limit_pg(ns);
   if (e == cudaSuccess) e = set_wait_limit_pg_resident(ns);
+  if (e == cudaSuccess) e = set_wait_limit_pg_resident32(ns);
   if (e == cudaSuccess) e = set_wait_limit_gs(ns);
   if (e == cudaSuccess) e = set_wait_limit_admm(ns);
   if (e == cudaSuccess) e = set_wait_limit_adjoint(ns);

@@ -546,7 +546,7 @@ __device__ __forceinline__ bool flat_barrier(const MonoBarrier& mb, unsigned k) 
   return __syncthreads_and(ok) != 0;
 }
 
-// The canonical reduction of K <= 4 quantities by one CTA of 8 warps (value q's sums at s + q * stride, count0
+// The canonical reduction of K <= 4 quantities by one CTA of 8 or more warps (value q's sums at s + q * stride, count0
 // chunks for q = 0 and count1 for q > 0): warp k takes stripe k of every quantity, its butterflies sharing their
 // first steps (warp_sum2 / warp_sum4: the same tree per quantity); lane q of warp 0 adds quantity q's 8 stripe
 // sums. smem: 32 doubles; the totals in out[0..K) (shared), valid after the call.
@@ -556,7 +556,7 @@ __device__ __forceinline__ void flat_combine(const double* s, size_t stride, int
   double p[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    if (q >= K) continue;
+    if (q >= K || warp >= 8) continue;
     const int C = q == 0 ? count0 : count1;
     const int per = (C + 7) / 8, b = warp * per, e = min(C, b + per);
     const double* sq = s + (size_t)q * stride;
@@ -571,7 +571,8 @@ __device__ __forceinline__ void flat_combine(const double* s, size_t stride, int
         if (c + 32 * u < e) p[q] = mx ? ((v[u] < p[q]) ? p[q] : v[u]) : p[q] + v[u];
     }
   }
-  if (maxmask) {
+  if (warp >= 8) {
+  } else if (maxmask) {
     for (int q = 0; q < K; ++q) {
       const double v = ((maxmask >> q) & 1u) ? warp_max_butterfly(p[q]) : warp_sum_butterfly(p[q]);
       if (lane == 0) smem32[8 * q + warp] = v;

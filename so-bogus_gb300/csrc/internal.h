@@ -172,6 +172,16 @@ int pg_max_grid(int device, bool fp32 = false, bool interleaved = false);
 bool pg_resident_fits(int device, int teams, int steps, int longest, int n);
 int pg_resident_max_teams();
 cudaError_t launch_pg_resident(const PGArgs& a, int ctas, int teams, int steps, cudaStream_t s);
+// FP32-refined solves whose FP32 copy of W fits (kernels_pg_resident32.cu): `ctas` CTAs of up to `chunks` chunks, `steps` the
+// largest sum of their S, `longest` the largest S. Positions (FP32) or corrections (FP64 iterations with FP32 correction
+// products, hy_ival the interleaved FP32 copy) 4 floats per contact; scratch: pg_resident32_scratch bytes.
+bool pg_resident32_fits(int device, int chunks, int steps, int longest, int n);
+size_t pg_resident32_scratch(int ctas, int chunks);
+cudaError_t launch_pg_resident32(const PGArgs32& a, int ctas, int chunks, int steps, cudaStream_t s);
+cudaError_t launch_pg_resident32(const PGArgs& a, int ctas, int chunks, int steps, void* scratch, cudaStream_t s);
+// FP64 positions (3 per contact) to and from 4 floats per contact.
+cudaError_t launch_pad_positions(int n, const double* src, float* dst, cudaStream_t s);
+cudaError_t launch_unpad_positions(int n, const float* src, double* dst, cudaStream_t s);
 // A CTA's part in one problem of a batch: the chunks rank, rank + ctas, ...
 struct ResidentJob {
   int problem, rank, ctas;
@@ -361,6 +371,7 @@ cudaError_t launch_meche_h(int n, int d, const double* E, const double* HAw, con
 // Device-side wait limits (nanoseconds) of the kernel files, set on the current device.
 cudaError_t set_wait_limit_pg(unsigned long long ns);
 cudaError_t set_wait_limit_pg_resident(unsigned long long ns);
+cudaError_t set_wait_limit_pg_resident32(unsigned long long ns);
 cudaError_t set_wait_limit_gs(unsigned long long ns);
 cudaError_t set_wait_limit_admm(unsigned long long ns);
 cudaError_t set_wait_limit_adjoint(unsigned long long ns);

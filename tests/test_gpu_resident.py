@@ -113,3 +113,50 @@ def test_adjoint(oracle, n, nbodies):
     s, dmu = D.adjoint(r, g, tol=1e-13)
     assert np.abs(s - s_o).max() <= 1e-8 * max(np.abs(s_o).max(), 1e-300)
     assert np.abs(dmu - dmu_o).max() <= 1e-8 * max(1.0, np.abs(dmu_o).max())
+
+
+@pytest.mark.parametrize("n,nbodies", [(1, 2), (33, 30), (70, 4), (64, 24), (32 * SM + 1, 1600), (8 * 32 * SM + 1, 13000),
+                                       (49999, 16000), (52000, 10000)])
+def test_refined(oracle, n, nbodies):
+    """The FP32-refined solve (kernels_pg_resident32.cu; the last two sizes around the shared-memory limit): FP32 part,
+    iterations with FP32 correction products and the FP64 check as the oracle's restatements of the three, one after the
+    other."""
+    import bogus_gpu
+
+    D, O = _pair(oracle, n, nbodies, 50 + n)
+    first, budget, refresh = (60, 40, 7) if n < 1000 else (12, 10, 4)
+    for static in (True, False):
+        pg = bogus_gpu.ProjectedGradient()
+        pg.setTol(1e-12)
+        pg.setMaxIters(first)
+        pg.setMixedPrecision(True, budget)
+        pg.setFp32CorrectionProducts(refresh)
+        r = np.zeros(3 * n)
+        res = D.solveWith(pg, r, staticProblem=static)
+        st = D.solve_stats()
+        _, x, k = O.solve_pg_fp32(np.zeros(3 * n), coulomb=not static, tol=1e-12, max_iters=first, stall_iters=4)
+        assert k == st["iterations"] - st["refine_iterations"]
+        _, x, ith = O.solve_pg(x, variant=3, coulomb=not static, tol=1e-12, max_iters=budget, hy_refresh=refresh)
+        assert ith == st["fp32_product_iterations"]
+        res_o, x, it = O.solve_pg(x, variant=3, coulomb=not static, tol=1e-12, max_iters=max(1, budget - ith))
+        assert it == st["refine_iterations"] - ith and res == res_o and np.array_equal(r, x)
+
+
+@pytest.mark.parametrize("variant", [1, 4])  # Descent, SPG
+def test_refined_variants(oracle, variant):
+    """The FP32 part of the other variants against the same solve as a batch of one (k_pg_batch, the plain arrays)."""
+    import bogus_gpu
+
+    n = 777
+    D, _ = _pair(oracle, n, 300, 3)
+    pg = bogus_gpu.ProjectedGradient()
+    pg.setDefaultVariant(variant)
+    pg.setTol(1e-11)
+    pg.setMaxIters(80)
+    pg.setMixedPrecision(True, 20)
+    a, b = np.zeros(3 * n), np.zeros(3 * n)
+    res = D.solveWith(pg, a, staticProblem=True)
+    its = D.last_iterations
+    D.setBatch(np.array([0, n], dtype=np.int32))
+    rb, ib = D.solveBatchWith(pg, b, staticProblem=True)
+    assert rb[0] == res and ib[0] == its and np.array_equal(a, b)
