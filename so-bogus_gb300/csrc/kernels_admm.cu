@@ -396,9 +396,15 @@ __global__ void __launch_bounds__(256) k_admm_persistent(ADMMArgs a) {
 // Orders: M v chains over the dofs from 0 and is added to f (subtracted from H^T r - f); H^T r per dof over the
 // body's contacts in increasing order, rows inner; H z and H v as the ADMM kernel's products; dof norms each body's
 // dofs left to right, then the canonical sum over bodies.
+//
+// Bodies (compile-time d, 32 d <= 256): a CTA takes a chunk of 32 bodies, thread D b + q the chain of dof q of body b, so
+// a warp's loads of H cover whole rows of a few bodies and its loop ends with the longest of those. A lane per body
+// ran all d chains itself, one FP64 instruction per 64 cycles and as many steps as the busiest of 32 bodies, on one
+// warp of an SM: AMA_FIG.
 template <int D>
-__device__ void dama_body(const DamaArgs& a, Phases& ctx) {
+__device__ void dama_body(const DamaArgs& a, Phases& ctx, double* shared) {
   constexpr int DM = D > 0 ? D : kMaxDof;
+  constexpr bool kSpread = D > 0 && 32 * D <= 256;
   const int d = D > 0 ? D : a.d;
   const int lane = threadIdx.x & 31;
   const int C = (a.n + 31) / 32, CB = (a.nbodies + 31) / 32;
@@ -434,6 +440,35 @@ __device__ void dama_body(const DamaArgs& a, Phases& ctx) {
           out[q] = s;
         }
     }
+  };
+  // kSpread: (H^T src) of dof q of body b, one thread; the incidence indices two steps ahead, H and src one
+  auto dof_HT = [&](int b, int q, const double* src) {
+    const int e0 = __ldg(a.bptr + b), e1 = __ldg(a.bptr + b + 1);
+    int ent1 = e0 < e1 ? __ldg(a.bent + e0) : 0, ent2 = e0 + 1 < e1 ? __ldg(a.bent + e0 + 1) : 0;
+    double hn[3] = {0.0, 0.0, 0.0}, rn[3] = {0.0, 0.0, 0.0};
+    auto load = [&](int ent) {
+      const double* Hb = a.H + (size_t)ent * 3 * D + q;
+#pragma unroll
+      for (int rr = 0; rr < 3; ++rr) hn[rr] = __ldg(Hb + rr * D);
+      load3(src, ent >> 1, rn);
+    };
+    if (e0 < e1) load(ent1);
+    double s = 0.0;
+    for (int e = e0; e < e1; ++e) {
+      const double hc[3] = {hn[0], hn[1], hn[2]}, rc[3] = {rn[0], rn[1], rn[2]};
+      ent1 = ent2;
+      ent2 = e + 2 < e1 ? __ldg(a.bent + e + 2) : 0;
+      if (e + 1 < e1) load(ent1);
+#pragma unroll
+      for (int rr = 0; rr < 3; ++rr) s = fma(hc[rr], rc[rr], s);
+    }
+    return s;
+  };
+  // kSpread: the chunks of 32 bodies, a CTA each: f(chunk, body or -1, dof)
+  auto body_chunks = [&](auto&& f) {
+    ctx.begin(0);
+    const int lb = threadIdx.x / DM, q = threadIdx.x % DM;
+    for (int c = blockIdx.x; c < CB; c += gridDim.x) f(c, lb < 32 && 32 * c + lb < a.nbodies ? 32 * c + lb : -1, q);
   };
   // (M_b src)_a: fma chain over the dofs from 0
   auto body_M = [&](int b, const double* src, int row) {
@@ -475,15 +510,21 @@ __device__ void dama_body(const DamaArgs& a, Phases& ctx) {
   double* vn = a.v_spare;
   double* ypn = a.yp_spare;
   // H^T r once
-  ctx.begin(CB);
-  for (int c = next(); c < CB; c = next()) {
-    const int b = 32 * c + lane;
-    if (b < a.nbodies) {
-      double h[DM];
-      body_HT(b, r, h);
+  if constexpr (kSpread) {
+    body_chunks([&](int, int b, int q) {
+      if (b >= 0) a.HrBp[(size_t)b * D + q] = dof_HT(b, q, r);
+    });
+  } else {
+    ctx.begin(CB);
+    for (int c = next(); c < CB; c = next()) {
+      const int b = 32 * c + lane;
+      if (b < a.nbodies) {
+        double h[DM];
+        body_HT(b, r, h);
 #pragma unroll
-      for (int q = 0; q < DM; ++q)
-        if (q < d) a.HrBp[(size_t)b * d + q] = h[q];
+        for (int q = 0; q < DM; ++q)
+          if (q < d) a.HrBp[(size_t)b * d + q] = h[q];
+      }
     }
   }
   if (!sync()) return;
@@ -630,32 +671,72 @@ __device__ void dama_body(const DamaArgs& a, Phases& ctx) {
           if (!sync()) return;
         }
         // Q4
-        ctx.begin(CB);
-        for (int c = next(); c < CB; c = next()) {
-          const int b = 32 * c + lane;
-          double ph = 0.0;
-          if (b < a.nbodies) {
-            double hr[DM], y[DM];
-            body_HT(b, rs, hr);
+        if constexpr (kSpread) {
+          double* sy = shared;            // y by thread
+          double* sg = shared + 32 * DM;  // the dofs' squares
+          body_chunks([&](int c, int b, int q) {
+            const size_t o = (size_t)b * D + q;
+            double hr = 0.0, fq = 0.0, Mq[DM];
+            if (b >= 0) {
+              fq = __ldg(a.f + o);
 #pragma unroll
-            for (int q = 0; q < DM; ++q)
-              if (q < d) {
-                a.HrBp[(size_t)b * d + q] = hr[q];
-                const double zq = hr[q] - ldcg(a.x + (size_t)b * d + q);
-                const double yk = ldcg(vc + (size_t)b * d + q) + a.gamma * zq;
-                y[q] = yk + beta * (yk - ldcg(ypc + (size_t)b * d + q));
-                // the velocity update of this trial (Q5's values, should the trial be the last)
-                vn[(size_t)b * d + q] = y[q];
-                ypn[(size_t)b * d + q] = yk;
-              }
+              for (int m = 0; m < DM; ++m) Mq[m] = __ldg(a.M + o * D + m);
+              const double xq = ldcg(a.x + o), vq = ldcg(vc + o), yp = ldcg(ypc + o);
+              hr = dof_HT(b, q, rs);
+              a.HrBp[o] = hr;
+              const double yk = vq + a.gamma * (hr - xq);
+              const double y = yk + beta * (yk - yp);
+              // the velocity update of this trial (Q5's values, should the trial be the last)
+              vn[o] = y;
+              ypn[o] = yk;
+              sy[threadIdx.x] = y;
+            }
+            __syncthreads();
+            if (b >= 0) {
+              const double* yb = sy + threadIdx.x - q;
+              double t = 0.0;
 #pragma unroll
-            for (int q = 0; q < DM; ++q)
-              if (q < d) {
-                const double gq = (hr[q] - __ldg(a.f + (size_t)b * d + q)) - body_M(b, y, q);
-                ph = ph + gq * gq;
-              }
+              for (int m = 0; m < DM; ++m) t = fma(Mq[m], yb[m], t);
+              const double gq = (hr - fq) - t;
+              sg[threadIdx.x] = gq * gq;
+            }
+            __syncthreads();
+            if (threadIdx.x < 32) {  // (the next chunk's squares are written after its first barrier)
+              double ph = 0.0;
+              if (32 * c + lane < a.nbodies)
+#pragma unroll
+                for (int m = 0; m < DM; ++m) ph = ph + sg[DM * lane + m];
+              put(0, c, ph, false);
+            }
+          });
+        } else {
+          ctx.begin(CB);
+          for (int c = next(); c < CB; c = next()) {
+            const int b = 32 * c + lane;
+            double ph = 0.0;
+            if (b < a.nbodies) {
+              double hr[DM], y[DM];
+              body_HT(b, rs, hr);
+#pragma unroll
+              for (int q = 0; q < DM; ++q)
+                if (q < d) {
+                  a.HrBp[(size_t)b * d + q] = hr[q];
+                  const double zq = hr[q] - ldcg(a.x + (size_t)b * d + q);
+                  const double yk = ldcg(vc + (size_t)b * d + q) + a.gamma * zq;
+                  y[q] = yk + beta * (yk - ldcg(ypc + (size_t)b * d + q));
+                  // the velocity update of this trial (Q5's values, should the trial be the last)
+                  vn[(size_t)b * d + q] = y[q];
+                  ypn[(size_t)b * d + q] = yk;
+                }
+#pragma unroll
+              for (int q = 0; q < DM; ++q)
+                if (q < d) {
+                  const double gq = (hr[q] - __ldg(a.f + (size_t)b * d + q)) - body_M(b, y, q);
+                  ph = ph + gq * gq;
+                }
+            }
+            put(0, c, ph, false);
           }
-          put(0, c, ph, false);
         }
         if (!sync_reduce(1, CB, CB, 0u)) return;
         const double hh = ctx.scal(0);
@@ -675,7 +756,18 @@ __device__ void dama_body(const DamaArgs& a, Phases& ctx) {
       ypn = t;
     }
     // Q5 (no line search): z = H^T r - x, y = v + gamma z, v = y + beta (y - y_prev)
-    if (a.ls_iters == 0) {
+    if (kSpread && a.ls_iters == 0) {
+      body_chunks([&](int, int b, int q) {
+        if (b < 0) return;
+        const size_t o = (size_t)b * D + q;
+        const double xq = ldcg(a.x + o), vq = ldcg(vc + o), yp = ldcg(ypc + o);
+        const double hr = dof_HT(b, q, r);
+        a.HrBp[o] = hr;
+        const double yk = vq + a.gamma * (hr - xq);
+        vc[o] = yk + beta * (yk - yp);
+        ypc[o] = yk;
+      });
+    } else if (a.ls_iters == 0) {
       ctx.begin(CB);
       for (int c = next(); c < CB; c = next()) {
         const int b = 32 * c + lane;
@@ -709,8 +801,9 @@ __device__ void dama_body(const DamaArgs& a, Phases& ctx) {
 template <int D>
 __global__ void __launch_bounds__(256) k_dama_persistent(DamaArgs a) {
   __shared__ double smem32[32], out[4];
+  __shared__ double shared[D > 0 ? 64 * D : 1];
   Phases ctx{a.ps, smem32, out};
-  dama_body<D>(a, ctx);
+  dama_body<D>(a, ctx, shared);
 }
 
 }  // namespace
