@@ -436,6 +436,12 @@ int check_finite(const double* v, size_t m, const char* what) {
   return BOGUS_GPU_OK;
 }
 
+// At most a chunk per warp of one CTA per SM (8 warps).
+bool few_chunks(int device, int nchunks) {
+  int sms = 0;
+  return cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && nchunks <= 8 * sms;
+}
+
 // Grid of a persistent kernel with 8 warps per CTA (max: its resident CTAs): one CTA per SM while its warps take no more
 // than a chunk each, then two, then the maximum; never more CTAs than chunks.
 int spread_grid(int device, int max, int nchunks) {
@@ -2895,7 +2901,7 @@ int bogus_gpu_solve_admm(bogus_gpu_problem* h, const bogus_gpu_admm_options* o, 
   const int grid = spread_grid(h->device, admm_max_grid(h->device, d), ((n > nb ? n : nb) + 31) / 32);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
   BG_CUDA(cudaEventRecord(h->ev0, s));
-  BG_CUDA(launch_admm(a, grid, s));
+  BG_CUDA(launch_admm(a, grid, few_chunks(h->device, ((n > nb ? n : nb) + 31) / 32), s));
   BG_CUDA(cudaEventRecord(h->ev1, s));
   ADMMOut out{};
   int st = 0;
@@ -3040,7 +3046,7 @@ int bogus_gpu_solve_dual_ama(bogus_gpu_problem* h, const bogus_gpu_dual_ama_opti
   const int grid = spread_grid(h->device, dama_max_grid(h->device, d), CC);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
   BG_CUDA(cudaEventRecord(h->ev0, s));
-  BG_CUDA(launch_dama(a, grid, s));
+  BG_CUDA(launch_dama(a, grid, few_chunks(h->device, CC), s));
   BG_CUDA(cudaEventRecord(h->ev1, s));
   DamaOut out{};
   int st = 0;

@@ -282,7 +282,8 @@ struct ADMMArgs {
   int accelerated, use_inf;
   const double* scaling;  // n: the error function's scalings (1 unless H is square at the block level)
 };
-cudaError_t launch_admm(const ADMMArgs& a, int grid, cudaStream_t s);
+// few: at most one 32-contact or 32-body chunk per warp of one CTA per SM (grid at most the SMs)
+cudaError_t launch_admm(const ADMMArgs& a, int grid, bool few, cudaStream_t s);
 int admm_max_grid(int device, int d);
 
 // DualAMA (kernels_admm.cu): Core/BlockSolvers/ADMM.impl.hpp:128-303 with A = M, B = 0, trivial preconditioner.
@@ -312,7 +313,7 @@ struct DamaArgs {
   unsigned max_iters, ls_iters;
   int accelerated, use_inf, desaxce;
 };
-cudaError_t launch_dama(const DamaArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_dama(const DamaArgs& a, int grid, bool few, cudaStream_t s);
 int dama_max_grid(int device, int d);
 
 // Adjoint of the SOC solve (kernels_adjoint.cu).

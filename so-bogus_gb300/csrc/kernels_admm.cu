@@ -74,10 +74,57 @@ __device__ __forceinline__ void store3(double* p, int i, const double* v) {
   p[3 * i + 2] = v[2];
 }
 
-template <int D>
+// The chain of dof q of H^T r over one body's incidences [e0, e1), from s: contacts in increasing order, rows inner. H
+// and r are loaded kAhead incidences ahead of the accumulation and the incidence indices as far ahead of those: with
+// loads one step ahead a step took the 1500 cycles of its loads, with four 64 per FMA and little else.
+// adjust(contact, r) changes the r read.
+template <int D, class Adjust>
+__device__ __forceinline__ double dof_chain(const int* __restrict__ bent, const double* __restrict__ H, const double* r,
+                                            int e0, int e1, int q, double s, Adjust&& adjust) {
+  constexpr int kAhead = 4;
+  int ent[kAhead], now[kAhead];
+  double h[kAhead][3], x[kAhead][3];
+  auto load = [&](int d) {
+    const double* Hb = H + (size_t)now[d] * 3 * D + q;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) h[d][k] = __ldg(Hb + k * D);
+    load3(r, now[d] >> 1, x[d]);
+  };
+#pragma unroll
+  for (int d = 0; d < kAhead; ++d) now[d] = e0 + d < e1 ? __ldg(bent + e0 + d) : 0;
+#pragma unroll
+  for (int d = 0; d < kAhead; ++d) ent[d] = e0 + kAhead + d < e1 ? __ldg(bent + e0 + kAhead + d) : 0;
+#pragma unroll
+  for (int d = 0; d < kAhead; ++d)
+    if (e0 + d < e1) load(d);
+  for (int e = e0; e < e1; e += kAhead) {
+#pragma unroll
+    for (int d = 0; d < kAhead; ++d) {
+      const int i = now[d] >> 1;
+      const double hc[3] = {h[d][0], h[d][1], h[d][2]};
+      double xc[3] = {x[d][0], x[d][1], x[d][2]};
+      now[d] = ent[d];
+      if (e + d + kAhead < e1) load(d);
+      ent[d] = e + d + 2 * kAhead < e1 ? __ldg(bent + e + d + 2 * kAhead) : 0;
+      if (e + d < e1) {
+        adjust(i, xc);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s = fma(hc[k], xc[k], s);
+      }
+    }
+  }
+  return s;
+}
+
+// Few: problems of up to a 32-contact chunk per warp of one CTA per SM, which are bound by latency: the loads of a body's
+// chain run four incidences ahead (156 registers). The larger ones are bound by throughput and keep the registers of two
+// CTAs per SM. 100 iterations on GB300, ms without / with Few: 300 contacts 2.54 / 1.88, 9999 2.69 / 2.11, 30 000 3.14 /
+// 2.95; 60 000 4.73 / 5.17 and 150 000 9.45 / 10.8 (the line lies at 38 912, where a warp would get a second chunk).
+// P2 takes most of what is left (18 700 of an iteration's 56 000 cycles at 30 000 contacts, its FP64 instructions' own
+// time); each barrier takes 2800, the reduction 3400.
+template <int D, bool Few>
 __device__ void admm_body(const ADMMArgs& a, Phases& ctx) {
   constexpr int DM = D > 0 ? D : kMaxDof;
-  constexpr bool kPair = D > 0 && D % 2 == 0;
   const int d = dofs<D>(a);
   const int lane = threadIdx.x & 31;
   const int C = (a.n + 31) / 32;
@@ -119,10 +166,44 @@ __device__ void admm_body(const ADMMArgs& a, Phases& ctx) {
   for (it = 0; it < a.max_iters; ++it) {
     const double* rc = rb[cur];
     // P1: x = prox(prox_arg) per body (lane order a.border: bodies of similar contact counts share a warp).
-    // Even compile-time d: a lane pair per body, each lane the FMA chains of half the dofs (16 bodies per warp,
-    // twice the chunks to spread over the warps), the halves exchanged exactly for the prox product.
-    if (kPair) {
-      constexpr int H2 = kPair ? D / 2 : 1;
+    // Few bodies, compile-time d: 32 / d bodies per warp, lane d k + q the chain of dof q of the k-th (its loads of H cover whole
+    // rows); the lanes of a body exchange their dofs exactly for the prox product. Units are dealt in turn (the order
+    // is by decreasing contact count, so that is even), without draws.
+    if constexpr (Few && D > 0) {
+      constexpr int NB = 32 / DM;
+      const int k = lane / DM, q = lane % DM;
+      const int units = (a.nbodies + NB - 1) / NB;
+      ctx.begin(0);
+      for (int c = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; c < units; c += gridDim.x * (blockDim.x >> 5)) {
+        const int slot = NB * c + k;
+        const bool on = k < NB && slot < a.nbodies;
+        const int b = on ? (a.border ? __ldg(a.border + slot) : slot) : 0;
+        const size_t o = (size_t)b * D + q;
+        double P[DM];
+#pragma unroll
+        for (int m = 0; m < DM; ++m) P[m] = on ? __ldg(a.prox + o * D + m) : 0.0;
+        const double fq = on && a.f ? __ldg(a.f + o) : 0.0;
+        double acc = on && with_lambda ? il * ldcg(a.x + o) : 0.0;
+        acc = dof_chain<DM>(a.bent, a.H, rc, on ? __ldg(a.bptr + b) : 0, on ? __ldg(a.bptr + b + 1) : 0, q, acc,
+                            [&](int i, double* rv) {
+                              if (!with_lambda) return;
+                              double za[3], ut[3];
+                              load3(plain ? a.z : a.zacc, i, za);
+                              load3(a.ut, i, ut);
+                              for (int m = 0; m < 3; ++m) rv[m] = fma(gamma, za[m] - ut[m], rv[m]);
+                            });
+        // QuadraticProxOp::eval: res = prox (rhs - f)
+        if (on && a.f) acc = acc - fq;
+        __syncwarp();
+        double sum = 0.0;
+#pragma unroll
+        for (int m = 0; m < DM; ++m) sum = fma(P[m], __shfl_sync(0xffffffffu, acc, lane - q + m), sum);
+        if (on) a.x[o] = sum;
+      }
+    } else if constexpr (D > 0 && D % 2 == 0) {
+      // Even compile-time d: a lane pair per body, each lane the FMA chains of half the dofs (16 bodies per warp,
+      // twice the chunks to spread over the warps), the halves exchanged exactly for the prox product.
+      constexpr int H2 = D / 2;
       const int half = lane & 1;
       const int CB2 = (a.nbodies + 15) / 16;
       ctx.begin(CB2);
@@ -176,7 +257,7 @@ __device__ void admm_body(const ADMMArgs& a, Phases& ctx) {
 #pragma unroll
           for (int k = 0; k < H2; ++k) acc[k] = acc[k] - __ldg(a.f + (size_t)b * D + q0 + k);
         }
-        double full[kPair ? D : 1];
+        double full[D];
 #pragma unroll
         for (int k = 0; k < H2; ++k) {
           const double other = __shfl_xor_sync(0xffffffffu, acc[k], 1);
@@ -202,44 +283,15 @@ __device__ void admm_body(const ADMMArgs& a, Phases& ctx) {
         if (slot < a.nbodies) {
           const int b = a.border ? __ldg(a.border + slot) : slot;
           double acc[DM];
-          const double* xb = a.x + (size_t)b * d;
-  #pragma unroll
+          double* xb = a.x + (size_t)b * d;
+#pragma unroll
           for (int q = 0; q < DM; ++q)
             if (q < d) acc[q] = with_lambda ? il * ldcg(xb + q) : 0.0;
           const int e0 = __ldg(a.bptr + b), e1 = __ldg(a.bptr + b + 1);
-          // Loads run ahead of the accumulation (its order is unchanged): the incidence indices two steps
-          // ahead and, for a compile-time d, the H rows and r of the next incidence, so that no step waits on
-          // the dependent index -> H / r load chain.
-          constexpr bool kPre = D > 0;
-          int ent1 = e0 < e1 ? __ldg(a.bent + e0) : 0;
-          int ent2 = e0 + 1 < e1 ? __ldg(a.bent + e0 + 1) : 0;
-          double Hn[kPre ? 3 * DM : 1], rn[3] = {0.0, 0.0, 0.0};
-          if (kPre && e0 < e1) {
-            const double* Hb = a.H + (size_t)ent1 * 3 * DM;
-  #pragma unroll
-            for (int k = 0; k < (kPre ? 3 * DM : 1); ++k) Hn[k] = __ldg(Hb + k);
-            load3(rc, ent1 >> 1, rn);
-          }
           for (int e = e0; e < e1; ++e) {
-            const int ent = ent1;
-            ent1 = ent2;
-            ent2 = e + 2 < e1 ? __ldg(a.bent + e + 2) : 0;
-            const int i = ent >> 1;
-            double Hc[kPre ? 3 * DM : 1];
+            const int ent = __ldg(a.bent + e), i = ent >> 1;
             double rv[3];
-            if (kPre) {
-  #pragma unroll
-              for (int k = 0; k < (kPre ? 3 * DM : 1); ++k) Hc[k] = Hn[k];
-              rv[0] = rn[0]; rv[1] = rn[1]; rv[2] = rn[2];
-              if (e + 1 < e1) {
-                const double* Hb = a.H + (size_t)ent1 * 3 * DM;
-  #pragma unroll
-                for (int k = 0; k < (kPre ? 3 * DM : 1); ++k) Hn[k] = __ldg(Hb + k);
-                load3(rc, ent1 >> 1, rn);
-              }
-            } else {
-              load3(rc, i, rv);
-            }
+            load3(rc, i, rv);
             if (with_lambda) {
               double za[3], ut[3];
               load3(plain ? a.z : a.zacc, i, za);
@@ -247,37 +299,32 @@ __device__ void admm_body(const ADMMArgs& a, Phases& ctx) {
               for (int k = 0; k < 3; ++k) rv[k] = fma(gamma, za[k] - ut[k], rv[k]);
             }
             const double* Hb = a.H + (size_t)ent * 3 * d;
-  #pragma unroll
+#pragma unroll
             for (int q = 0; q < DM; ++q) {
               if (q < d) {
                 double s = acc[q];
-                for (int rr = 0; rr < 3; ++rr) s = fma(kPre ? Hc[rr * DM + q] : __ldg(Hb + rr * d + q), rv[rr], s);
+                for (int rr = 0; rr < 3; ++rr) s = fma(__ldg(Hb + rr * d + q), rv[rr], s);
                 acc[q] = s;
               }
             }
           }
           // QuadraticProxOp::eval: res = prox (rhs - f)
           if (a.f) {
-  #pragma unroll
+#pragma unroll
             for (int q = 0; q < DM; ++q)
               if (q < d) acc[q] = acc[q] - __ldg(a.f + (size_t)b * d + q);
           }
           const double* P = a.prox + (size_t)b * d * d;
-          double xn[DM];
-  #pragma unroll
+#pragma unroll
           for (int m = 0; m < DM; ++m) {
             if (m < d) {
               double s = 0.0;
-  #pragma unroll
+#pragma unroll
               for (int q = 0; q < DM; ++q)
                 if (q < d) s = fma(__ldg(P + m * d + q), acc[q], s);
-              xn[m] = s;
+              xb[m] = s;
             }
           }
-          double* xw = a.x + (size_t)b * d;
-  #pragma unroll
-          for (int m = 0; m < DM; ++m)
-            if (m < d) xw[m] = xn[m];
         }
       }
     }
@@ -372,11 +419,11 @@ __device__ void admm_body(const ADMMArgs& a, Phases& ctx) {
   }
 }
 
-template <int D>
+template <int D, bool Few>
 __global__ void __launch_bounds__(256) k_admm_persistent(ADMMArgs a) {
   __shared__ double smem32[32], out[4];
   Phases ctx{a.ps, smem32, out};
-  admm_body<D>(a, ctx);
+  admm_body<D, Few>(a, ctx);
 }
 
 
@@ -397,14 +444,15 @@ __global__ void __launch_bounds__(256) k_admm_persistent(ADMMArgs a) {
 // body's contacts in increasing order, rows inner; H z and H v as the ADMM kernel's products; dof norms each body's
 // dofs left to right, then the canonical sum over bodies.
 //
-// Bodies (compile-time d, 32 d <= 256): a CTA takes a chunk of 32 bodies, thread D b + q the chain of dof q of body b, so
+// Bodies (Few, compile-time d, 32 d <= 256): a CTA takes a chunk of 32 bodies, thread D b + q the chain of dof q of body b, so
 // a warp's loads of H cover whole rows of a few bodies and its loop ends with the longest of those. A lane per body
 // ran all d chains itself, one FP64 instruction per 64 cycles and as many steps as the busiest of 32 bodies, on one
-// warp of an SM: AMA_FIG.
-template <int D>
+// warp of an SM. 100 iterations on GB300, ms, lane per body / this: 300 contacts 4.46 / 2.81, 9999 5.54 / 3.34, 30 000
+// 6.22 / 4.63, 60 000 8.57 / 8.53, 150 000 15.4 / 17.6 (larger problems keep the lane per body).
+template <int D, bool Few>
 __device__ void dama_body(const DamaArgs& a, Phases& ctx, double* shared) {
   constexpr int DM = D > 0 ? D : kMaxDof;
-  constexpr bool kSpread = D > 0 && 32 * D <= 256;
+  constexpr bool kSpread = Few && D > 0 && 32 * D <= 256;
   const int d = D > 0 ? D : a.d;
   const int lane = threadIdx.x & 31;
   const int C = (a.n + 31) / 32, CB = (a.nbodies + 31) / 32;
@@ -441,28 +489,9 @@ __device__ void dama_body(const DamaArgs& a, Phases& ctx, double* shared) {
         }
     }
   };
-  // kSpread: (H^T src) of dof q of body b, one thread; the incidence indices two steps ahead, H and src one
+  // kSpread: (H^T src) of dof q of body b, one thread
   auto dof_HT = [&](int b, int q, const double* src) {
-    const int e0 = __ldg(a.bptr + b), e1 = __ldg(a.bptr + b + 1);
-    int ent1 = e0 < e1 ? __ldg(a.bent + e0) : 0, ent2 = e0 + 1 < e1 ? __ldg(a.bent + e0 + 1) : 0;
-    double hn[3] = {0.0, 0.0, 0.0}, rn[3] = {0.0, 0.0, 0.0};
-    auto load = [&](int ent) {
-      const double* Hb = a.H + (size_t)ent * 3 * D + q;
-#pragma unroll
-      for (int rr = 0; rr < 3; ++rr) hn[rr] = __ldg(Hb + rr * D);
-      load3(src, ent >> 1, rn);
-    };
-    if (e0 < e1) load(ent1);
-    double s = 0.0;
-    for (int e = e0; e < e1; ++e) {
-      const double hc[3] = {hn[0], hn[1], hn[2]}, rc[3] = {rn[0], rn[1], rn[2]};
-      ent1 = ent2;
-      ent2 = e + 2 < e1 ? __ldg(a.bent + e + 2) : 0;
-      if (e + 1 < e1) load(ent1);
-#pragma unroll
-      for (int rr = 0; rr < 3; ++rr) s = fma(hc[rr], rc[rr], s);
-    }
-    return s;
+    return dof_chain<DM>(a.bent, a.H, src, __ldg(a.bptr + b), __ldg(a.bptr + b + 1), q, 0.0, [](int, double*) {});
   };
   // kSpread: the chunks of 32 bodies, a CTA each: f(chunk, body or -1, dof)
   auto body_chunks = [&](auto&& f) {
@@ -798,28 +827,30 @@ __device__ void dama_body(const DamaArgs& a, Phases& ctx, double* shared) {
   }
 }
 
-template <int D>
+template <int D, bool Few>
 __global__ void __launch_bounds__(256) k_dama_persistent(DamaArgs a) {
   __shared__ double smem32[32], out[4];
-  __shared__ double shared[D > 0 ? 64 * D : 1];
+  __shared__ double shared[Few ? 64 * D : 1];
   Phases ctx{a.ps, smem32, out};
-  dama_body<D>(a, ctx, shared);
+  dama_body<D, Few>(a, ctx, shared);
 }
 
 }  // namespace
 
-cudaError_t launch_admm(const ADMMArgs& a, int grid, cudaStream_t s) {
+cudaError_t launch_admm(const ADMMArgs& a, int grid, bool few, cudaStream_t s) {
   ADMMArgs copy = a;
   void* args[] = {&copy};
-  const void* fn = a.d == 6 ? (const void*)k_admm_persistent<6> : (const void*)k_admm_persistent<0>;
+  const void* fn = a.d != 6 ? (const void*)k_admm_persistent<0, false>
+                   : few ? (const void*)k_admm_persistent<6, true>
+                         : (const void*)k_admm_persistent<6, false>;
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(256), args, 0, s);
 }
 
 int admm_max_grid(int device, int d) {
   int sms = 0, per = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-  const cudaError_t e = d == 6 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_admm_persistent<6>, 256, 0)
-                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_admm_persistent<0>, 256, 0);
+  const cudaError_t e = d == 6 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_admm_persistent<6, false>, 256, 0)
+                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_admm_persistent<0, false>, 256, 0);
   if (e != cudaSuccess) return 0;
   if (per > 2) per = 2;
   return per * sms;
@@ -829,18 +860,20 @@ int admm_max_grid(int device, int d) {
 
 namespace bogus_gpu {
 
-cudaError_t launch_dama(const DamaArgs& a, int grid, cudaStream_t s) {
+cudaError_t launch_dama(const DamaArgs& a, int grid, bool few, cudaStream_t s) {
   DamaArgs copy = a;
   void* args[] = {&copy};
-  const void* fn = a.d == 6 ? (const void*)k_dama_persistent<6> : (const void*)k_dama_persistent<0>;
+  const void* fn = a.d != 6 ? (const void*)k_dama_persistent<0, false>
+                   : few ? (const void*)k_dama_persistent<6, true>
+                         : (const void*)k_dama_persistent<6, false>;
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(256), args, 0, s);
 }
 
 int dama_max_grid(int device, int d) {
   int sms = 0, per = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-  const cudaError_t e = d == 6 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dama_persistent<6>, 256, 0)
-                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dama_persistent<0>, 256, 0);
+  const cudaError_t e = d == 6 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dama_persistent<6, false>, 256, 0)
+                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dama_persistent<0, false>, 256, 0);
   if (e != cudaSuccess) return 0;
   if (per > 2) per = 2;
   return per * sms;
