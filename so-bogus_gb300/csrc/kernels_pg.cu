@@ -107,16 +107,19 @@ __device__ int pg_body(const PGArgsT<T>& a, Ctx& ctx) {
   return pg_body_inl<T, IL, SC, HY>(a, ctx);
 }
 
-// Occupancy target: 3 resident CTAs per SM (see pg_max_grid).
-template <class T, bool IL, bool SC = false, bool HY = false>
-__global__ void __launch_bounds__(256, 3) k_pg_persistent(PGArgsT<T> a) {
+// Occupancy target: 3 resident CTAs per SM (see pg_max_grid). FEW (FP64, at most 2 CTAs per SM launched, a chunk or less
+// per warp): the registers of the third CTA hold the next two blocks and points instead, since a warp's own latency
+// counts there. us per APGD iteration on GB300 without / with: 26 000 contacts 69.7 / 58.7, 38 000 80.4 / 70.6, 50 000
+// 85.7 / 78.0, 77 000 98.2 / 92.3.
+template <class T, bool IL, bool SC = false, bool HY = false, bool FEW = false>
+__global__ void __launch_bounds__(256, FEW ? 2 : 3) k_pg_persistent(PGArgsT<T> a) {
   __shared__ double smem8[32], sscal[4];
   __shared__ ChunkScratchT<T> cs[8];
   __shared__ unsigned s_cnt[2];
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0u;
   __syncthreads();
   GridCtx<T> ctx{a, smem8, sscal, cs, s_cnt};
-  pg_body_inl<T, IL, SC, HY>(a, ctx);
+  pg_body_inl<T, IL, SC, HY, false, FEW>(a, ctx);
 }
 
 // One problem per CTA (batched solves): phases separated by __syncthreads, scalars reduced by the CTA's
@@ -412,10 +415,16 @@ cudaError_t launch_pg_persistent(const PGArgs& a, int grid, cudaStream_t s) {
   if ((sc || hy) && !a.slot0) return cudaErrorInvalidValue;  // they run on the interleaved copy only
   if (hy && (a.variant != 3 || a.lin_momentum || !a.hy_ival || !a.hy_d || !a.hy_xref || !a.hy_wxref))
     return cudaErrorInvalidValue;
+  int device = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return e;
+  const bool few = a.slot0 && grid <= 2 * sms;
   const void* fn = sc ? (const void*)k_pg_persistent<double, true, true>
                       : (hy ? (const void*)k_pg_persistent<double, true, false, true>
-                            : (a.slot0 ? (const void*)k_pg_persistent<double, true>
-                                       : (const void*)k_pg_persistent<double, false>));
+                            : few ? (const void*)k_pg_persistent<double, true, false, false, true>
+                                  : (a.slot0 ? (const void*)k_pg_persistent<double, true>
+                                             : (const void*)k_pg_persistent<double, false>));
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(256), args, 0, s);
 }
 

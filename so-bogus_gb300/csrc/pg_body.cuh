@@ -138,9 +138,10 @@ struct BlocksOf<T, true> {
 // register allocation of the APGD / Descent / SPG kernels).
 // HY: APGD with FP32 correction products (FP64 iterates, law and reductions; its own instantiation as well):
 // W v = W x_ref + W32 (v - x_ref)_32, x_ref and W x_ref refreshed in FP64 every hy_refresh iterations.
+// AHEAD: FP64 products with their loads two blocks ahead (spmv_chunk).
 // RES: the FP32 copy of W lives in shared memory, each warp owning one chunk (ctx.chunk32, kernels_pg_resident32.cu); the
 // FP32 points that its products gather (the positions of the FP32 solve, the corrections of HY) are 4 floats apart.
-template <class T, bool IL, bool SC = false, bool HY = false, bool RES = false, class Ctx>
+template <class T, bool IL, bool SC = false, bool HY = false, bool RES = false, bool AHEAD = false, class Ctx>
 __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
   constexpr int ST = RES && sizeof(T) == 4 ? 4 : 3;
   using Ops = SocOps<T>;
@@ -153,7 +154,7 @@ __device__ __forceinline__ int pg_body_inl(const PGArgsT<T>& a, Ctx& ctx) {
       ctx.chunk32.template product<1>(xsrc, acc, acc);
       return;
     }
-    spmv_chunk<1, true>(a.rowptr, blocks, a.n, c, sh, [&](int j, T* x) { load3cg(xsrc, j, x); }, acc);
+    spmv_chunk<1, true, AHEAD>(a.rowptr, blocks, a.n, c, sh, [&](int j, T* x) { load3cg(xsrc, j, x); }, acc);
   };
   const int lane = threadIdx.x & 31;
   // HY: the FP32 correction v - x_ref of position buffer k (0, 1, 2 or 4), written beside every position that a

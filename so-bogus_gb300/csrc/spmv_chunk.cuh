@@ -67,7 +67,7 @@ __device__ __forceinline__ float zero_plus(float v) { return 0.f + v; }
 // Every lane of the warp must call it (warp-uniform c). acc (and acc2) hold init on entry, the result on
 // exit, for row 32c + lane (lanes past n get unspecified values). ZeroInit: every init is +0, so the first
 // piece of a row is placed rather than added (the same value).
-template <int NP, bool ZeroInit = false, class T, class Src, class Gather>
+template <int NP, bool ZeroInit = false, bool Ahead = false, class T, class Src, class Gather>
 __device__ __forceinline__ void spmv_chunk(const int* __restrict__ rowptr, Src src, int n, int c,
                                            ChunkScratchT<T>& sh, Gather&& gather, T* acc, T* acc2 = nullptr) {
   const int lane = threadIdx.x & 31;
@@ -102,8 +102,9 @@ __device__ __forceinline__ void spmv_chunk(const int* __restrict__ rowptr, Src s
   // The next block's column index and gathered x are loaded one block ahead, so the dependent col -> x load
   // chain of block k + 1 overlaps the accumulation of block k (the arithmetic order is unchanged).
   // FP32: the block values and gathered x are loaded two blocks ahead (the FP32 solve is bound by load
-  // latency); FP64: x one block ahead (the FP64 solve is bound by its FMA pipe; registers set occupancy)
-  constexpr bool kAhead = sizeof(T) == 4;
+  // latency), FP64 too where few warps share an SM (Ahead); else FP64: x one block ahead (the FP64 solve is bound by its
+  // FMA pipe; registers set occupancy)
+  constexpr bool kAhead = Ahead || sizeof(T) == 4;
   T xn[3] = {T(0), T(0), T(0)}, xm[3] = {T(0), T(0), T(0)};
   T bn[9], bm[9];
   if (k0 < e) gather(src.column(k0, 0), xn);

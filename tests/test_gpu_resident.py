@@ -55,6 +55,14 @@ def test_teams(oracle, n):
         _compare(D, O, n, variant, coulomb, False, 15, np.zeros(3 * n))
 
 
+@pytest.mark.parametrize("n", [16 * 32 * SM, 16 * 32 * SM + 1])
+def test_general(oracle, n):
+    """The general kernel on both sides of the line between its two register budgets (kernels_pg.cu)."""
+    D, O = _pair(oracle, n, n // 4, 11)
+    for variant, coulomb in ((3, False), (4, True), (1, False)):
+        _compare(D, O, n, variant, coulomb, False, 6, np.zeros(3 * n))
+
+
 @pytest.mark.parametrize("sizes", [[1, 31, 32, 33, 160, 161, 1], [16] * 40 + [700, 340, 5, 64], [0, 50, 0, 200]])
 def test_batch(oracle, sizes):
     """Batches whose problems span one and several CTAs, several problems per CTA, and empty problems: each problem as the
