@@ -623,11 +623,12 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
   const bool sc = o->variant == BOGUS_GPU_PG_STANDARD || o->variant == BOGUS_GPU_PG_CONJUGATED;
   int grid = 0;
   ResidentSize rs;
-  bool resident = false;
+  bool resident = false, cluster = false;
   if (!hy && !sc && !a.lin_momentum) {
     if (int e = resident_size(h, &rs)) return e;
     grid = rs.ctas;
     resident = pg_resident_fits(h->device, rs.teams, rs.steps, rs.longest, n);
+    cluster = resident && !a.phantom_ctas && pg_resident_cluster_fits(h->device, a.nchunks, rs.longest);
   }
   if (!resident) {  // or k_pg_resident32, which reads the FP64 copy at its refreshes
     if (int e = ensure_interleaved(h)) return e;
@@ -648,7 +649,8 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
   a.cta_ptr = h->cta_ptr.p;
   a.cta_list = h->cta_list.p;
   BG_CUDA(cudaEventRecord(h->ev0, h->stream));
-  BG_CUDA(resident ? launch_pg_resident(a, grid, rs.teams, rs.steps, h->stream)
+  BG_CUDA(cluster    ? launch_pg_resident_cluster(a, rs.longest, h->stream)
+          : resident ? launch_pg_resident(a, grid, rs.teams, rs.steps, h->stream)
           : hy && hy->resident
               ? launch_pg_resident32(a, grid, rs.teams, rs.steps, h->hy_scratch.p, h->stream)
               : launch_pg_persistent(a, grid, h->stream));

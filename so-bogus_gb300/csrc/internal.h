@@ -171,6 +171,9 @@ int pg_max_grid(int device, bool fp32 = false, bool interleaved = false);
 // largest sum of S (spmv_chunk.cuh) over a CTA's chunks, `longest` the largest S
 bool pg_resident_fits(int device, int teams, int steps, int longest, int n);
 int pg_resident_max_teams();
+// Problems of a few chunks, on one cluster of a CTA each; not for tests with phantom CTAs.
+bool pg_resident_cluster_fits(int device, int chunks, int longest);
+cudaError_t launch_pg_resident_cluster(const PGArgs& a, int longest, cudaStream_t s);
 cudaError_t launch_pg_resident(const PGArgs& a, int ctas, int teams, int steps, cudaStream_t s);
 // FP32-refined solves whose FP32 copy of W fits (kernels_pg_resident32.cu): `ctas` CTAs of up to `chunks` chunks, `steps` the
 // largest sum of their S, `longest` the largest S. Positions (FP32) or corrections (FP64 iterations with FP32 correction

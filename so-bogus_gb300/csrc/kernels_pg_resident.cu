@@ -58,41 +58,159 @@ struct Place {
   }
 };
 
+// Stores into the shared memory of every CTA of the cluster (the address is this CTA's own).
+__device__ __forceinline__ void store_cluster(const double* p, int rank, double v) {
+  asm volatile("{ .reg .b32 r; mapa.shared::cluster.u32 r, %0, %1; st.shared::cluster.f64 [r], %2; }" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(p)),
+               "r"(rank), "d"(v)
+               : "memory");
+}
+__device__ __forceinline__ void store_cluster3(const double* p, int rank, const double* x) {
+  asm volatile(
+      "{ .reg .b32 r; mapa.shared::cluster.u32 r, %0, %1; st.shared::cluster.v2.f64 [r], {%2, %3}; "
+      "st.shared::cluster.f64 [r+16], %4; }" ::"r"((unsigned)__cvta_generic_to_shared(p)),
+      "r"(rank), "d"(x[0]), "d"(x[1]), "d"(x[2])
+      : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// ResidentReduce for a cluster: the hardware's barrier in place of the counter in global memory, and the chunk sums
+// written to every CTA's shared memory. At most 16 CTAs and kClusterChunks chunks (two per stripe), so warp 0 reduces
+// alone: lane 8 q + k forms stripe k of quantity q.
+constexpr int kClusterChunks = 16;
+struct ClusterReduce {
+  double* csum;  // 2 x 4 x C doubles of this CTA's shared memory
+  const int C;
+  double* stripes;
+  const int lane, warp, nwarps, parties;
+  unsigned phase = 0;
+  __device__ double* sums() const { return csum + (size_t)(phase & 1u) * 4 * C; }
+  // v: quantity q of chunk c, in every lane
+  __device__ void put_total(int q, int c, double v) {
+    if (lane < parties) store_cluster(sums() + q * C + c, lane, v);
+  }
+  // quantity q in lanes 0-15, q + 1 in the others
+  __device__ void put_totals(int q, int c, double v) {
+    if ((lane & 15) < parties) store_cluster(sums() + (q + (lane >> 4)) * C + c, lane & 15, v);
+  }
+  __device__ void put(int q, int c, double v) { put_total(q, c, warp_sum_butterfly(v)); }
+  template <class Side>
+  __device__ void arrive_and_wait(Side&& side) {
+    __syncwarp();
+    cluster_arrive();
+    if (warp == nwarps - 1) side();
+    __syncwarp();
+    cluster_wait();
+  }
+  __device__ bool sync() {
+    arrive_and_wait([] {});
+    ++phase;
+    return true;
+  }
+  template <class Side, class Decide>
+  __device__ bool reduce(int K, unsigned maxmask, Side&& side, Decide&& decide) {
+    arrive_and_wait(side);
+    if (warp == 0) {
+      // stripe k: chunks [k per, (k + 1) per); what a warp's butterfly over the two and zeros gives
+      const double* s = sums();
+      const int q = lane >> 3, k = lane & 7, per = (C + 7) / 8, b = k * per, e = min(C, b + per);
+      const bool mx = (maxmask >> q) & 1u;
+      double v = 0.0;
+      if (q < K && b < e) {
+        const double v0 = s[q * C + b], v1 = b + 1 < e ? s[q * C + b + 1] : 0.0;
+        if (mx) {
+          const double m0 = v0 < 0.0 ? 0.0 : v0, m1 = v1 < 0.0 ? 0.0 : v1;
+          v = m0 < m1 ? m1 : m0;
+        } else {
+          v = (0.0 + v0) + (0.0 + v1);
+        }
+      }
+      stripes[lane] = v;
+      __syncwarp();
+      const int t = lane < K ? lane : 0;
+      const bool tmx = (maxmask >> t) & 1u;
+      double total = stripes[8 * t];
+#pragma unroll
+      for (int j = 1; j < 8; ++j) {
+        const double w = stripes[8 * t + j];
+        total = tmx ? ((w < total) ? total : w) : total + w;
+      }
+      decide(total);
+    }
+    __syncthreads();
+    ++phase;
+    return true;
+  }
+};
+
+// The CTA's shared memory: the scalars, the teams' arrays, (cluster) the two gathered points of all contacts and the
+// chunk sums, the chunks' blocks.
+__host__ __device__ inline size_t teams_offset() { return (sizeof(Control) + 15) / 16 * 16; }
+__host__ __device__ inline size_t points_offset(int teams) { return teams_offset() + (size_t)teams * sizeof(TeamShared); }
+__host__ __device__ inline size_t cluster_bytes(int chunks) { return (size_t)chunks * (2 * 32 * 4 + 2 * 4) * sizeof(double); }
+
+// CL: the CTAs of the problem are one cluster.
+template <bool CL>
 __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const Place& place, unsigned char* smem) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int team = warp / kTeamWarps, role = warp - kTeamWarps * team;
   Control& ctl = *reinterpret_cast<Control*>(smem);
   const bool has = team < place.count;
   const int c = has ? place.chunk(team) : 0;
-  TeamShared& sh = reinterpret_cast<TeamShared*>(smem + (sizeof(Control) + 15) / 16 * 16)[team < teams ? team : 0];
+  TeamShared& sh = reinterpret_cast<TeamShared*>(smem + teams_offset())[team < teams ? team : 0];
   const int C = a.nchunks;
   const int i = 32 * c + lane;
   const bool on = has && i < a.n;
   const bool desaxce = a.desaxce != 0, spg = a.variant == 4, apgd = a.variant == 3;
   const unsigned res_mask = a.use_inf ? 1u : 0u;
   const bool writer = place.rank == 0 && threadIdx.x == 0;
-  double* const gx = a.MX0;                      // the gathered points: x (or the momentum point) ...
-  double* const gs = a.MX0 + 4 * (size_t)a.n;    // ... and the trial point xs
+  // the gathered points: x (or the momentum point) and the trial point xs
+  double* const gx = CL ? reinterpret_cast<double*>(smem + points_offset(teams)) : a.MX0;
+  double* const gs = gx + 4 * (size_t)(CL ? 32 * C : a.n);
+  auto put_point = [&](double* g, const double* v) {
+    if constexpr (CL) {
+#pragma unroll 4
+      for (int r = 0; r < (int)place.parties; ++r) store_cluster3(g, r, v);
+    } else {
+      store_padded(g, v);
+    }
+  };
   const size_t ip = on ? 4 * (size_t)i : 0;
+
+  auto own_point = [&](const double* g, double* v) {
+    if constexpr (CL) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[k] = g[k];
+    } else {
+      load_padded(g, v);
+    }
+  };
 
   ResidentChunk chunk{sh.core, lane, role, team};
   if (has) {
     size_t before = 0;  // the CTA's chunks one after another, behind the teams' arrays
     for (int k = 0; k < team; ++k) before += (size_t)steps_of(a.rowptr, a.n, place.chunk(k));
     chunk.load(a.rowptr, a.col, a.val, a.n, c,
-               smem + (sizeof(Control) + 15) / 16 * 16 + (size_t)teams * sizeof(TeamShared) + before * kStepBytes);
+               smem + points_offset(teams) + (CL ? cluster_bytes(C) : 0) + before * kStepBytes);
   }
   const double (*const part)[64] = sh.core.part;
   // W g for this chunk's contacts, all components to every warp of the team
   auto team_product = [&](const double* g, double* out) {
-    chunk.product<1>(g);
+    if constexpr (CL) chunk.product_local<1>(g);
+    else chunk.product<1>(g);
 #pragma unroll
     for (int k = 0; k < 3; ++k) out[k] = part[k][lane];
   };
 
   // ---- barriers ----------------------------------------------------------------------------------------------
-  ResidentReduce red{MonoBarrier{a.mono, a.gb.status, place.parties + a.phantom_ctas}, a.csum, C, ctl.stripes, lane, warp, nwarps};
-  auto sums = [&]() { return red.sums(); };
+  auto red = [&] {
+    if constexpr (CL)
+      return ClusterReduce{gs + 4 * (size_t)32 * C, C, ctl.stripes, lane, warp, nwarps, (int)place.parties};
+    else
+      return ResidentReduce{MonoBarrier{a.mono, a.gb.status, place.parties + a.phantom_ctas}, a.csum, C, ctl.stripes, lane, warp,
+                            nwarps};
+  }();
   auto put = [&](int q, double v) { red.put(q, c, v); };
   auto reduce = [&](int K, unsigned maxmask, auto side, auto decide) { return red.reduce(K, maxmask, side, decide); };
   auto sync = [&]() { return red.sync(); };
@@ -106,7 +224,7 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
 #pragma unroll
     for (int k = 0; k < 3; ++k) x[k] = a.X0[3 * (size_t)i + k];
     project_cone(__ldg(a.mu + i), x);  // projectOnConstraints(x) (:90)
-    if (role == 1) store_padded(gx + ip, x);
+    if (role == 1) put_point(gx + ip, x);
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) pv[k] = x[k];
@@ -141,7 +259,8 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
   // Mx = W x (:93) and guess_alpha (:21-28)
   count(1);
   if (has) {
-    chunk.product<2>(gx, sh.xs[0]);
+    if constexpr (CL) chunk.product_local<2>(gx, sh.xs[0]);
+    else chunk.product<2>(gx, sh.xs[0]);
 #pragma unroll
     for (int k = 0; k < 3; ++k) Mx[k] = part[k][lane];
     if (role == 0) {
@@ -195,7 +314,7 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
         const double na = neg(ctl.alpha_t);
         double p[3] = {fma(na, yn[0], x[0]), fma(na, yn[1], x[1]), fma(na, yn[2], x[2])};
         project_cone(mu, p);
-        store_padded(gs + ip, p);
+        put_point(gs + ip, p);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           sh.xs[k][lane] = p[k];
@@ -220,7 +339,7 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
     }
     if (role == 0) {
       v = a.use_inf ? warp_max_butterfly(v) : warp_sum_butterfly(v);
-      if (lane == 0) sums()[c] = v;
+      red.put_total(0, c, v);
     } else if (role == (spg ? 1 : 2)) {
       put(1, v);
     }
@@ -294,7 +413,7 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
             shared3(sh.y, y);
             const double d[3] = {xs[0] - x[0], xs[1] - x[1], xs[2] - x[2]};
             const double v = warp_sum2_butterfly(on ? dot3(y, d) : 0.0, on ? sq3(d) : 0.0);
-            if ((lane & 15) == 0) sums()[(1 + (lane >> 4)) * C + c] = v;
+            red.put_totals(1, c, v);
             if (pending) store_best();
           } else {
             double y[3];
@@ -303,7 +422,7 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
             const double d[3] = {xs[0] - pv[0], xs[1] - pv[1], xs[2] - pv[2]};
             if (apgd && on) {
               const double xn[3] = {fma(bt, d[0], xs[0]), fma(bt, d[1], xs[1]), fma(bt, d[2], xs[2])};
-              store_padded(gx + ip, xn);
+              put_point(gx + ip, xn);
             }
             put(3, on ? dot3(d, y) : 0.0);
           }
@@ -348,7 +467,7 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
           const double na = neg(ctl.alpha);
           double p[3] = {fma(na, sh.y[0][lane], x[0]), fma(na, sh.y[1][lane], x[1]), fma(na, sh.y[2][lane], x[2])};
           project_cone(__ldg(a.mu + i), p);
-          store_padded(gs + ip, p);
+          put_point(gs + ip, p);
 #pragma unroll
           for (int k = 0; k < 3; ++k) sh.xs[k][lane] = p[k];
         }
@@ -356,7 +475,7 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
       }
       ++it;
       if (it >= a.max_iters) break;
-      if (on && next == kMomentum) load_padded(gx + ip, x);
+      if (on && next == kMomentum) own_point(gx + ip, x);
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         const double xs = on ? sh.xs[k][lane] : 0.0;
@@ -408,12 +527,12 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
           xn[k] = xs[k];
         }
       }
-      store_padded(gx + ip, xn);
+      put_point(gx + ip, xn);
     }
     if (!sync()) return;
     // E: Mx_new = W x; z = -Mx_old + Mx_new; w.z (warp 1), |z|^2 (warp 0)
     count(8);
-    if (on) load_padded(gx + ip, x);
+    if (on) own_point(gx + ip, x);
     if (has) {
       team_product(gx, Ms);
       const double z[3] = {-Mx[0] + Ms[0], -Mx[1] + Ms[1], -Mx[2] + Ms[2]};
@@ -444,7 +563,26 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
   extern __shared__ __align__(16) unsigned char smem[];
   const int first = __ldg(a.cta_ptr + blockIdx.x);
   const Place place{(int)blockIdx.x, gridDim.x, first, 1, __ldg(a.cta_ptr + blockIdx.x + 1) - first, a.cta_list};
-  resident_solve(a, teams, place, smem);
+  resident_solve<false>(a, teams, place, smem);
+}
+
+// One problem of at most kClusterChunks chunks on one cluster, a CTA per chunk. With so few chunks the trips through L2
+// count most: an arrival at the counter and the poll that sees it (1.35 us a barrier), the chunk sums read back, the
+// gathered points. Here the hardware's cluster barrier separates the phases, every CTA holds all points and chunk sums
+// in its own shared memory (a chunk's team writes them into each CTA's), and a product gathers from there.
+// us per iteration on GB300, k_pg_resident / this kernel, APGD and SPG: 33 contacts 16.6 / 12.6 and 12.2 / 9.9, 200 17.9 /
+// 13.0 and 13.4 / 10.5, 500 18.3 / 14.4 and 13.5 / 11.3. With two or three chunks per CTA, to go beyond 16, the SM's one
+// FP64 unit costs more than the barriers do: 1000 contacts 20.1 / 21.7, 1500 20.3 / 26.7.
+__global__ void __launch_bounds__(32 * kMinWarps, 1) k_pg_resident_cluster(PGArgs a, int teams) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int rank = (int)blockIdx.x, ctas = (int)gridDim.x;
+  const Place place{rank, gridDim.x, rank, ctas, (a.nchunks - rank + ctas - 1) / ctas, nullptr};
+  cluster_arrive();  // every CTA's shared memory is there before the first store into it
+  cluster_wait();
+  resident_solve<true>(a, teams, place, smem);
+  __syncwarp();
+  cluster_arrive();  // and stays until the last
+  cluster_wait();
 }
 
 // A batch: every CTA works through its own list of jobs, a job being its part in one problem (the chunks rank,
@@ -478,7 +616,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1)
     __syncthreads();
     const int mine = a.nchunks > job.rank ? (a.nchunks - job.rank + job.ctas - 1) / job.ctas : 0;
     const Place place{job.rank, (unsigned)job.ctas, job.rank, job.ctas, mine, nullptr};
-    resident_solve(a, teams, place, smem);
+    resident_solve<false>(a, teams, place, smem);
     // the best iterate over the initial one, by the lanes that stored it
     const int warp = threadIdx.x >> 5, i = 32 * (job.rank + (warp / kTeamWarps) * job.ctas) + (threadIdx.x & 31);
     if (warp / kTeamWarps < mine && warp % kTeamWarps == 1 && i < n)
@@ -488,7 +626,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1)
 
 // teams per CTA, and the largest sum of S over a CTA's chunks
 size_t resident_smem(int teams, int steps) {
-  return (sizeof(Control) + 15) / 16 * 16 + (size_t)teams * sizeof(TeamShared) + (size_t)steps * kStepBytes;
+  return points_offset(teams) + (size_t)steps * kStepBytes;
 }
 
 }  // namespace
@@ -511,12 +649,54 @@ cudaError_t launch_resident(const void* fn, void** args, int ctas, int teams, in
   const int warps = kTeamWarps * teams > kMinWarps ? kTeamWarps * teams : kMinWarps;
   return cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(32 * warps), args, bytes, s);
 }
+cudaLaunchConfig_t cluster_config(int ctas, size_t bytes, cudaStream_t s, cudaLaunchAttribute* at) {
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)ctas;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(32 * kMinWarps);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
 }  // namespace
 
 cudaError_t launch_pg_resident(const PGArgs& a, int ctas, int teams, int steps, cudaStream_t s) {
   PGArgs copy = a;
   void* args[] = {&copy, &teams};
   return launch_resident((const void*)k_pg_resident, args, ctas, teams, steps, s);
+}
+
+// One CTA per chunk, a cluster of up to 16 (more than the portable 8).
+bool pg_resident_cluster_fits(int device, int chunks, int longest) {
+  int limit = 0;
+  if (chunks < 1 || chunks > kClusterChunks || longest > 64) return false;
+  if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return false;
+  const size_t bytes = resident_smem(1, longest) + cluster_bytes(chunks);
+  if (bytes + 1024 > (size_t)limit) return false;
+  const void* fn = (const void*)k_pg_resident_cluster;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, limit - 1024) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  cudaLaunchAttribute at{};
+  cudaLaunchConfig_t cfg = cluster_config(chunks, bytes, nullptr, &at);
+  int active = 0;
+  if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return active >= 1;
+}
+
+cudaError_t launch_pg_resident_cluster(const PGArgs& a, int longest, cudaStream_t s) {
+  cudaLaunchAttribute at{};
+  cudaLaunchConfig_t cfg = cluster_config(a.nchunks, resident_smem(1, longest) + cluster_bytes(a.nchunks), s, &at);
+  return cudaLaunchKernelEx(&cfg, k_pg_resident_cluster, a, 1);
 }
 
 cudaError_t launch_pg_resident_batch(const PGBatchArgs& b, const int* job_ptr, const ResidentJob* jobs,

@@ -181,6 +181,73 @@ struct ResidentChunk {
       }
       consume(k + 1);
     }
+    exchange<NP>(slot, p, q, part2);
+  }
+
+  // The same product with points in the CTA's own shared memory: every warp reads all of them itself, the next group of
+  // three steps while the FMAs of one run, so the team meets only at the end. No warp of the team may still read the
+  // previous product.
+  template <int NP>
+  __device__ __forceinline__ void product_local(const double* g, double* part2_all = nullptr) {
+    double* part2 = part2_all + 64 * role;
+    int slot = slot0;
+    double p = 0.0, q = 0.0;
+    const double* bl = wv + 32 * 3 * role + lane;
+    unsigned long long open = starts;
+    struct Group {
+      double b[3][3], x[3][3];
+    };
+    auto load = [&](int k, Group& t) {
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const int s = min(3 * k + e, S - 1);
+        const double* pt = g + 4 * (size_t)wc[32 * s + lane];
+        const double2 xy = *reinterpret_cast<const double2*>(pt);
+        t.x[e][0] = xy.x;
+        t.x[e][1] = xy.y;
+        t.x[e][2] = pt[2];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) t.b[e][r] = bl[288 * s + 32 * r];
+      }
+    };
+    auto consume = [&](int k, const Group& t) {
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const int s = 3 * k + e;
+        if (s >= S) break;
+        const bool starts_row = open & 1ull;
+        open >>= 1;
+        if (starts_row) sh.part[role][slot] = p;
+        p = starts_row ? 0.0 : p;
+        const bool valid = s < nv;
+        const double pn = fma(t.b[e][2], t.x[e][2], fma(t.b[e][1], t.x[e][1], fma(t.b[e][0], t.x[e][0], p)));
+        p = valid ? pn : p;
+        if (NP == 2) {
+          if (starts_row) part2[slot] = q;
+          q = starts_row ? 0.0 : q;
+          const double qn =
+              fma(t.b[e][2], t.x[e][2] - 1.0, fma(t.b[e][1], t.x[e][1] - 1.0, fma(t.b[e][0], t.x[e][0] - 1.0, q)));
+          q = valid ? qn : q;
+        }
+        slot += starts_row ? 1 : 0;
+      }
+    };
+    const int groups = (S + 2) / 3;
+    Group u, v;
+    load(0, u);
+    for (int k = 0; k < groups; k += 2) {
+      if (k + 1 < groups) load(k + 1, v);
+      consume(k, u);
+      if (k + 1 >= groups) break;
+      if (k + 2 < groups) load(k + 2, u);
+      consume(k + 1, v);
+    }
+    exchange<NP>(slot, p, q, part2);
+  }
+
+  // The last pieces, the rows' sums, and the result to every warp of the team.
+  template <int NP>
+  __device__ __forceinline__ void exchange(int slot, double p, double q, double* part2) {
     if (nv > 0) {
       sh.part[role][slot] = p;
       if (NP == 2) part2[slot] = q;
@@ -212,11 +279,16 @@ struct ResidentReduce {
   const int lane, warp, nwarps;
   unsigned phase = 0;  // barriers passed
   __device__ double* sums() const { return csum + (size_t)(phase & 1u) * 4 * C; }
-  // sum of v over the warp as chunk c's value of quantity q
-  __device__ void put(int q, int c, double v) {
-    v = warp_sum_butterfly(v);
+  // v: quantity q of chunk c, in every lane
+  __device__ void put_total(int q, int c, double v) {
     if (lane == 0) sums()[q * C + c] = v;
   }
+  // quantity q in lanes 0-15, q + 1 in the others
+  __device__ void put_totals(int q, int c, double v) {
+    if ((lane & 15) == 0) sums()[(q + (lane >> 4)) * C + c] = v;
+  }
+  // sum of v over the warp as chunk c's value of quantity q
+  __device__ void put(int q, int c, double v) { put_total(q, c, warp_sum_butterfly(v)); }
   // The last warp prepares the next decision (side) while thread 0 waits for the other CTAs.
   template <class Side>
   __device__ bool arrive_and_wait(Side&& side) {

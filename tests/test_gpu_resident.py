@@ -55,6 +55,14 @@ def test_teams(oracle, n):
         _compare(D, O, n, variant, coulomb, False, 15, np.zeros(3 * n))
 
 
+@pytest.mark.parametrize("n,nbodies", [(31, 12), (33, 11), (255, 90), (256, 300), (257, 90), (481, 160), (512, 200), (513, 200)])
+def test_cluster(oracle, n, nbodies):
+    """Problems of one cluster: one CTA, one and two chunks per stripe of the sums, the last size and the first past it."""
+    D, O = _pair(oracle, n, nbodies, 70 + n)
+    for variant, coulomb, inf_norm in ((3, False, True), (3, True, False), (4, False, False), (4, True, True), (1, False, False)):
+        _compare(D, O, n, variant, coulomb, inf_norm, 60, np.zeros(3 * n))
+
+
 @pytest.mark.parametrize("n", [16 * 32 * SM, 16 * 32 * SM + 1])
 def test_general(oracle, n):
     """The general kernel on both sides of the line between its two register budgets (kernels_pg.cu)."""
