@@ -319,6 +319,10 @@ BG_HD int hessenberg_eigenvalues(double* a, int n, double* wr, double* wi) {
 // Bound by the latency of that chain (one contact's solve on the critical path of the sweep). Divisions and square
 // roots, half of it on the FP64 unit, run on the integer pipe; the sign, zero and equality tests are integer
 // comparisons; elements are exchanged by shuffles (no shared memory and its barriers).
+// An FP64 instruction takes its 64 cycles of the unit whether or not another waits for it, so products of one step that
+// need not be apart share an instruction across lanes (the row modification's two by half of the warp, the column
+// modification's three by column), and the one that nothing waits for follows the division: 501 contacts, 100 sweeps
+// 47.0 -> 45.8 ms; 50 000 colored, 25 sweeps 69.9 -> 68.6.
 __device__ __forceinline__ double warp_bcast(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 __device__ __forceinline__ bool nonnegative(double v) { return ipipe::to_bits(v) <= kSign; }  // v >= 0 (not NaN)
 // a == b for a, b >= 0 (or NaN, which equals nothing)
@@ -466,11 +470,7 @@ __device__ inline int hessenberg_eigenvalues_warp(double av, int n, double& wr, 
         }
         const double s = nonnegative(p) ? nrm : neg(nrm);
         if (nonzero(s)) {
-          if (k == m) {
-            if (l != m && row == k && col == k - 1) av = neg(av);
-          } else {
-            if (row == k && col == k - 1) av = -s * x;
-          }
+          const double scale = x;
           p += s;
           double y1, z1;
           {  // x = p / s, y = q / s, z = r / s, q = q / p, r = r / p
@@ -483,17 +483,27 @@ __device__ inline int hessenberg_eigenvalues_warp(double av, int n, double& wr, 
             q = warp_bcast(v, 3);
             r = warp_bcast(v, 4);
           }
-          {  // row modification: rows k, k + 1, k + 2 of columns k .. nn
-            double pj = rk + q * rk1;
-            if (three) pj += r * rk2;
+          // column k - 1 (no later step of this loop reads it)
+          if (row == k && col == k - 1) {
+            if (k != m) av = neg(s) * scale;
+            else if (l != m) av = neg(av);
+          }
+          {  // row modification: rows k, k + 1, k + 2 of columns k .. nn; the two products on a half of the warp each
+            const bool upper = lane >= 16;
+            const double pr = (upper ? r : q) * (upper ? rk2 : rk1);
+            const double po = __shfl_xor_sync(0xffffffffu, pr, 16);
+            double pj = rk + (upper ? po : pr);
+            if (three) pj += upper ? pr : po;
             const double f = row == k ? x : (row == k + 1 ? y1 : z1);
             if (col >= k && col <= nn && row >= k && row <= k2) av -= pj * f;
           }
           const int mmin = nn < k + 3 ? nn : k + 3;
           {  // column modification: columns k, k + 1, k + 2 of rows l .. mmin (x 1.0 is exact: a - p * 1.0 = a - p)
-            const double ck = at(row, k), ck1 = at(row, k + 1), ck2 = at(row, k2);
-            double pi = x * ck + y1 * ck1;
-            if (three) pi += z1 * ck2;
+            // each element's product by its own lane, gathered by the row
+            const double pc = (col == k ? x : (col == k + 1 ? y1 : z1)) * av;
+            double pi = __shfl_sync(0xffffffffu, pc, 4 * row + k) + __shfl_sync(0xffffffffu, pc, 4 * row + k + 1);
+            const double p2 = __shfl_sync(0xffffffffu, pc, 4 * row + k2);
+            if (three) pi += p2;
             const double f = col == k ? 1.0 : (col == k + 1 ? q : r);
             if (row >= l && row <= mmin && col >= k && col <= k2) av -= pi * f;
           }
