@@ -150,7 +150,7 @@ struct bogus_gpu_problem {
   DevBuf<int> full_src, pat_upper, pat_cursor, pat_check;
   std::vector<double> host_b, host_mu;
   DevBuf<int> asm_row;      // assembly: the row of every lower block
-  std::vector<int> h_bptr;  // the bodies' contact lists (bptr, bent) on the host
+  std::vector<int> h_bptr, h_bent;  // the bodies' contact lists (bptr, bent) on the host
   bool lists_valid = false;
   // projected-gradient work
   DevBuf<double> X, MX, Y, S0, XB, Wv, csum, scal, trace;
@@ -2436,7 +2436,7 @@ int ensure_body_lists(bogus_gpu_problem* h) {
   const int n = h->ncontacts, nb = h->nbodies;
   cudaStream_t s = h->stream;
   std::vector<int>& bp = h->h_bptr;
-  std::vector<int> be;
+  std::vector<int>& be = h->h_bent;  // (kept: the upload may still read it)
   bp.assign(nb + 1, 0);
   for (int i = 0; i < n; ++i)
     for (int t = 0; t < 2; ++t)
@@ -2453,7 +2453,6 @@ int ensure_body_lists(bogus_gpu_problem* h) {
   BG_CUDA(h->bent.ensure(be.size()));
   BG_CUDA(cudaMemcpyAsync(h->bptr.p, bp.data(), sizeof(int) * (nb + 1), cudaMemcpyHostToDevice, s));
   BG_CUDA(cudaMemcpyAsync(h->bent.p, be.data(), sizeof(int) * be.size(), cudaMemcpyHostToDevice, s));
-  BG_CUDA(cudaStreamSynchronize(s));
   h->lists_valid = true;
   return BOGUS_GPU_OK;
 }

@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(1024) k_rowptr_tiles(int n, const int* __restr
   __shared__ int ws[32];
   const int i = blockIdx.x * 1024 + threadIdx.x;
   const int v = full_row_length(i, n, rowptr, upper);
-  const int inc = cta_inclusive_scan(v, ws) + tile_off[blockIdx.x];
+  const int inc = cta_inclusive_scan(v, ws) + (tile_off ? tile_off[blockIdx.x] : 0);
   if (i < n) frowptr[i] = inc - v;
   if (i == n - 1) frowptr[n] = inc;
 }
@@ -317,6 +317,16 @@ cudaError_t launch_check_full(int n, int nnzb, const int* rowptr, const int* col
   return cudaGetLastError();
 }
 
+// frowptr from the row lengths (full_row_length); a single tile has no other's sum to add
+static void launch_tiles(int n, const int* rowptr, const int* upper, int* tiles, int* frowptr, cudaStream_t s) {
+  const int ntiles = (n + 1023) / 1024;
+  if (ntiles > 1) {
+    k_rowlen_tiles<<<ntiles, 1024, 0, s>>>(n, rowptr, upper, tiles);
+    k_scan_tiles<<<1, 1024, 0, s>>>(ntiles, tiles);
+  }
+  k_rowptr_tiles<<<ntiles, 1024, 0, s>>>(n, rowptr, upper, ntiles > 1 ? tiles : nullptr, frowptr);
+}
+
 cudaError_t launch_full_pattern(int n, const int* rowptr, const int* col, int* upper, int* cursor, int* frowptr,
                                 int* fcol, int* src, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
@@ -325,10 +335,7 @@ cudaError_t launch_full_pattern(int n, const int* rowptr, const int* col, int* u
   const int g = (n + 255) / 256;
   k_count_upper<<<g, 256, 0, s>>>(n, rowptr, col, upper);
   // the tile sums use `cursor` (n ints; ceil(n / 1024) <= n), zeroed afterwards for k_place_lower
-  const int ntiles = (n + 1023) / 1024;
-  k_rowlen_tiles<<<ntiles, 1024, 0, s>>>(n, rowptr, upper, cursor);
-  k_scan_tiles<<<1, 1024, 0, s>>>(ntiles, cursor);
-  k_rowptr_tiles<<<ntiles, 1024, 0, s>>>(n, rowptr, upper, cursor, frowptr);
+  launch_tiles(n, rowptr, upper, cursor, frowptr, s);
   if ((e = cudaMemsetAsync(cursor, 0, sizeof(int) * n, s)) != cudaSuccess) return e;
   k_place_lower<<<g, 256, 0, s>>>(n, rowptr, col, frowptr, fcol, src, cursor);
   k_sort_upper<<<g, 256, 0, s>>>(n, rowptr, frowptr, fcol, src);
@@ -338,10 +345,7 @@ cudaError_t launch_full_pattern(int n, const int* rowptr, const int* col, int* u
 // rowptr = exclusive prefix sum of n counts (n + 1 entries); tiles: ceil(n / 1024) integers of scratch
 cudaError_t launch_prefix_sum(int n, const int* count, int* tiles, int* rowptr, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  const int ntiles = (n + 1023) / 1024;
-  k_rowlen_tiles<<<ntiles, 1024, 0, s>>>(n, nullptr, count, tiles);
-  k_scan_tiles<<<1, 1024, 0, s>>>(ntiles, tiles);
-  k_rowptr_tiles<<<ntiles, 1024, 0, s>>>(n, nullptr, count, tiles, rowptr);
+  launch_tiles(n, nullptr, count, tiles, rowptr, s);
   return cudaGetLastError();
 }
 
