@@ -554,21 +554,30 @@ __device__ __forceinline__ void flat_combine(const double* s, size_t stride, int
                                              unsigned maxmask, double* smem32, double* out) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double p[4] = {0.0, 0.0, 0.0, 0.0};
+  if (warp < 8) {
+    const int per0 = (count0 + 7) / 8, per1 = (count1 + 7) / 8;
+    const int b0 = warp * per0, b1 = warp * per1, e0 = min(count0, b0 + per0), e1 = min(count1, b1 + per1);
+    // the loads of all quantities before the sums: one trip to L2 per 128 chunks of a stripe, not one per quantity (200 FP32
+    // and 100 correction iterations at 50 000 contacts 10.80 -> 10.46 ms, APGD at 38 000 70.6 -> 65.9 us per iteration)
+    for (int o = lane; o < max(per0, per1); o += 128) {
+      double v[4][4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    if (q >= K || warp >= 8) continue;
-    const int C = q == 0 ? count0 : count1;
-    const int per = (C + 7) / 8, b = warp * per, e = min(C, b + per);
-    const double* sq = s + (size_t)q * stride;
-    const bool mx = (maxmask >> q) & 1u;
-    for (int c = b + lane; c < e; c += 128) {
-      double v[4];
+      for (int q = 0; q < 4; ++q)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = c + 32 * u < e ? ldcg(sq + c + 32 * u) : 0.0;
+        for (int u = 0; u < 4; ++u) {
+          const int c = (q == 0 ? b0 : b1) + o + 32 * u;
+          v[q][u] = q < K && c < (q == 0 ? e0 : e1) ? ldcg(s + (size_t)q * stride + c) : 0.0;
+        }
       // a chunk sum past the end adds nothing; the first of a lane is placed (0 + v, -0 becoming +0)
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (c + 32 * u < e) p[q] = mx ? ((v[u] < p[q]) ? p[q] : v[u]) : p[q] + v[u];
+      for (int q = 0; q < 4; ++q) {
+        const bool mx = (maxmask >> q) & 1u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = (q == 0 ? b0 : b1) + o + 32 * u;
+          if (q < K && c < (q == 0 ? e0 : e1)) p[q] = mx ? ((v[q][u] < p[q]) ? p[q] : v[q][u]) : p[q] + v[q][u];
+        }
+      }
     }
   }
   if (warp >= 8) {

@@ -109,8 +109,8 @@ __device__ int pg_body(const PGArgsT<T>& a, Ctx& ctx) {
 
 // Occupancy target: 3 resident CTAs per SM (see pg_max_grid). FEW (FP64, at most 2 CTAs per SM launched, a chunk or less
 // per warp): the registers of the third CTA hold the next two blocks and points instead, since a warp's own latency
-// counts there. us per APGD iteration on GB300 without / with: 26 000 contacts 69.7 / 58.7, 38 000 80.4 / 70.6, 50 000
-// 85.7 / 78.0, 77 000 98.2 / 92.3.
+// counts there. us per APGD iteration on GB300 without / with (before the reductions' loads came together, which took
+// 38 000 to 65.9): 26 000 contacts 69.7 / 58.7, 38 000 80.4 / 70.6, 50 000 85.7 / 78.0, 77 000 98.2 / 92.3.
 template <class T, bool IL, bool SC = false, bool HY = false, bool FEW = false>
 __global__ void __launch_bounds__(256, FEW ? 2 : 3) k_pg_persistent(PGArgsT<T> a) {
   __shared__ double smem8[32], sscal[4];
