@@ -44,10 +44,10 @@ BG_HD bool negative(double v) {                             // v < 0.0
   const uint64_t u = ipipe::to_bits(v);
   return u > kSign && u <= (kSign | kInfBits);
 }
-// a <= t and a < t for a >= 0 (or NaN) and any t
+// a <= t and a < t for a >= 0, -0 (a product with mu = -0) or NaN, and any t
 BG_HD bool leq_from_zero(double a, double t) {
   const uint64_t ut = ipipe::to_bits(ipipe::plus_zero(t));  // a negative t has a larger bit pattern than infinity
-  return ut <= kInfBits && ipipe::to_bits(a) <= ut;
+  return ut <= kInfBits && abs_bits(a) <= ut;
 }
 BG_HD bool less_from_zero(double a, double t) {
   const uint64_t ut = ipipe::to_bits(t);
