@@ -167,6 +167,21 @@ cudaError_t launch_cadoux_rhs(int n, const double* y, const double* mu, const do
 cudaError_t launch_pg_persistent(const PGArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_pg_persistent(const PGArgs32& a, int grid, cudaStream_t s);
 int pg_max_grid(int device, bool fp32 = false, bool interleaved = false);
+// Shared memory that a launch of the kernels below may take of a CTA's: the device's largest less what their static arrays
+// and the system need. 0 after a failed query.
+inline size_t resident_shared_limit(int device) {
+  int limit = 0;
+  if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return 0;
+  return limit > 1024 ? (size_t)limit - 1024 : 0;
+}
+// Lets fn take that much on the current device. The attribute belongs to the function, not to a launch: with each launch
+// setting its own size, a host thread with a smaller problem made another's launch fail. One value for all.
+inline cudaError_t allow_resident_shared(const void* fn) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)resident_shared_limit(device));
+}
 // Problems that fit the SMs' shared memory (kernels_pg_resident.cu): `ctas` CTAs of up to `teams` chunks, `steps` the
 // largest sum of S (spmv_chunk.cuh) over a CTA's chunks, `longest` the largest S
 bool pg_resident_fits(int device, int teams, int steps, int longest, int n);

@@ -846,16 +846,14 @@ cudaError_t launch_adjoint_coulomb(const AdjArgs& a, int grid, cudaStream_t s) {
 }
 
 bool adjoint_resident_fits(int device, int teams, int steps, int longest, int n) {
-  int limit = 0;
-  if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return false;
   return teams >= 1 && teams <= kMaxTeams && longest <= 64 && n <= 65536 &&
-         adjoint_resident_smem(teams, steps) + 1024 <= (size_t)limit;
+         adjoint_resident_smem(teams, steps) <= resident_shared_limit(device);
 }
 
 cudaError_t launch_adjoint_resident(const AdjArgs& a, int ctas, int teams, int steps, cudaStream_t s) {
   const size_t bytes = adjoint_resident_smem(teams, steps);
   const void* fn = (const void*)k_adjoint_resident;
-  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const cudaError_t e = allow_resident_shared(fn);
   if (e != cudaSuccess) return e;
   AdjArgs copy = a;
   void* args[] = {&copy, &teams};

@@ -549,9 +549,8 @@ size_t resident_smem(int teams, int steps) {
 // Whether the resident kernel takes CTAs with up to `teams` chunks of up to `steps` steps (S) in sum and `longest` each:
 // a team per chunk, every chunk's blocks in shared memory, a lane's row starts in 64 bits, columns in 16.
 bool pg_resident_fits(int device, int teams, int steps, int longest, int n) {
-  int limit = 0;
-  if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return false;
-  return teams >= 1 && teams <= kMaxTeams && longest <= 64 && n <= 65536 && resident_smem(teams, steps) + 1024 <= (size_t)limit;
+  return teams >= 1 && teams <= kMaxTeams && longest <= 64 && n <= 65536 &&
+         resident_smem(teams, steps) <= resident_shared_limit(device);
 }
 
 int pg_resident_max_teams() { return kMaxTeams; }
@@ -559,7 +558,7 @@ int pg_resident_max_teams() { return kMaxTeams; }
 namespace {
 cudaError_t launch_resident(const void* fn, void** args, int ctas, int teams, int steps, cudaStream_t s) {
   const size_t bytes = resident_smem(teams, steps);
-  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const cudaError_t e = allow_resident_shared(fn);
   if (e != cudaSuccess) return e;
   const int warps = kTeamWarps * teams > kMinWarps ? kTeamWarps * teams : kMinWarps;
   return cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(32 * warps), args, bytes, s);
@@ -587,14 +586,12 @@ cudaError_t launch_pg_resident(const PGArgs& a, int ctas, int teams, int steps, 
 
 // One CTA per chunk, a cluster of up to 16 (more than the portable 8).
 bool pg_resident_cluster_fits(int device, int chunks, int longest) {
-  int limit = 0;
   if (chunks < 1 || chunks > kClusterChunks || longest > 64) return false;
-  if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return false;
   const size_t bytes = resident_smem(1, longest) + cluster_bytes(chunks);
-  if (bytes + 1024 > (size_t)limit) return false;
+  if (bytes > resident_shared_limit(device)) return false;
   const void* fn = (const void*)k_pg_resident_cluster;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, limit - 1024) != cudaSuccess) {
+      allow_resident_shared(fn) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

@@ -205,7 +205,7 @@ template <class T, bool HY>
 cudaError_t launch32(const PGArgsT<T>& a, int ctas, int chunks, int steps, ChunkScratchT<T>* scratch, cudaStream_t s) {
   const size_t bytes = resident32_smem(chunks, steps);
   const void* fn = (const void*)k_pg_resident32<T, HY>;
-  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const cudaError_t e = allow_resident_shared(fn);
   if (e != cudaSuccess) return e;
   PGArgsT<T> copy = a;
   void* args[] = {&copy, &scratch};
@@ -229,10 +229,8 @@ __global__ void k_unpad_positions(int n, const float4* __restrict__ src, double*
 }  // namespace
 
 bool pg_resident32_fits(int device, int chunks, int steps, int longest, int n) {
-  int limit = 0;
-  if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return false;
   return chunks >= 1 && chunks <= kMaxWarps && longest <= 64 && n <= 65536 &&
-         resident32_smem(chunks, steps) + 1024 <= (size_t)limit;
+         resident32_smem(chunks, steps) <= resident_shared_limit(device);
 }
 
 size_t pg_resident32_scratch(int ctas, int chunks) { return sizeof(ChunkScratch) * (size_t)ctas * warps_of(chunks); }
