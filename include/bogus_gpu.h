@@ -412,14 +412,15 @@ int bogus_gpu_get_stream(const bogus_gpu_problem* h, void** stream);
 /* Limit of every device-side wait of the library's kernels on `device` (grid barriers of the persistent
  * solvers, the Gauss-Seidel sweep's flag waits), in seconds within [1e-6, 3600]; default 4. A wait that runs
  * out makes the kernel record BOGUS_GPU_TIMEOUT and return, and the call reports TIMEOUT; the CUDA context
- * stays usable. The setting holds for every handle and the allocation-free entry point on that device until
+ * stays usable. In a batched solve a CTA that waits for others to finish earlier problems waits as long as those make
+ * progress. The setting holds for every handle and the allocation-free entry point on that device until
  * changed; set it while no solve runs there. The caller's current device is left as it was. No counterpart
  * in the reference (its solvers run on the host). */
 int bogus_gpu_set_wait_limit(int device, double seconds);
 
 /* Test of the timeout path (no counterpart in the reference). While `on` is non-zero, the single-problem
- * projected-gradient solves of this handle (bogus_gpu_solve_pg / _pg_device, FP64) launch their kernel with
- * barriers that wait for one CTA more than the launch holds: the first barrier can never complete, its
+ * projected-gradient solves of this handle (bogus_gpu_solve_pg / _pg_device, FP64) and those of its batched solves
+ * that keep W in shared memory launch their kernel with barriers that wait for one CTA more than the launch holds: the first barrier can never complete, its
  * bounded wait runs out after the wait limit, and the solve returns BOGUS_GPU_TIMEOUT without touching r.
  * Turn it off to solve normally again on the same handle. */
 int bogus_gpu_test_wait_timeout(bogus_gpu_problem* h, int on);

@@ -3263,7 +3263,7 @@ int plan_resident_batch(bogus_gpu_problem* h, const std::vector<int>& rp, const 
   }
   BG_CUDA(h->rb_ptr.ensure(ptr.size()));
   BG_CUDA(h->rb_jobs.ensure(flat.size()));
-  BG_CUDA(h->rb_mono.ensure(np));
+  BG_CUDA(h->rb_mono.ensure((size_t)np + 1));
   BG_CUDA(cudaMemcpyAsync(h->rb_ptr.p, ptr.data(), sizeof(int) * ptr.size(), cudaMemcpyHostToDevice, h->stream));
   BG_CUDA(cudaMemcpyAsync(h->rb_jobs.p, flat.data(), sizeof(ResidentJob) * flat.size(), cudaMemcpyHostToDevice, h->stream));
   BG_CUDA(cudaStreamSynchronize(h->stream));
@@ -3620,8 +3620,9 @@ int run_pg_batch(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* re
   if (h->rb_ctas && !hy && !ba.base.lin_momentum && h->forced_shape.schedule < 0 && !h->batch_tuning) {
     BG_CUDA(h->status.ensure(1));
     BG_CUDA(cudaMemsetAsync(h->status.p, 0, sizeof(int), h->stream));
-    BG_CUDA(cudaMemsetAsync(h->rb_mono.p, 0, sizeof(unsigned long long) * np, h->stream));
+    BG_CUDA(cudaMemsetAsync(h->rb_mono.p, 0, sizeof(unsigned long long) * ((size_t)np + 1), h->stream));
     ba.base.gb.status = h->status.p;
+    ba.base.phantom_ctas = h->test_wait_timeout ? 1u : 0u;
     BG_CUDA(cudaEventRecord(h->ev0, h->stream));
     BG_CUDA(launch_pg_resident_batch(ba, h->rb_ptr.p, h->rb_jobs.p, h->rb_mono.p, h->rb_ctas, h->rb_teams, h->rb_steps,
                                      h->stream));

@@ -28,6 +28,14 @@ __device__ __forceinline__ int ld_relaxed_i32(const int* p) {
   asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_add_relaxed_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -521,18 +529,22 @@ __device__ __forceinline__ void red_add_release_u64(unsigned long long* p, unsig
 
 // One thread, for its whole CTA: arrives at barrier k and returns once every CTA has (false after a wait that ran
 // out). No status word is read on the way out: a CTA whose wait runs out records it, and the others' waits then end
-// too.
-__device__ __forceinline__ bool flat_wait(const MonoBarrier& mb, unsigned k) {
+// too. progress: a counter that CTAs advance as they work; while it moves, the limit starts anew.
+__device__ __forceinline__ bool flat_wait(const MonoBarrier& mb, unsigned k,
+                                          const unsigned long long* progress = nullptr) {
   red_add_release_u64(mb.mono, 1ull);
   const unsigned long long target = (unsigned long long)mb.parties * (k + 1ull);
-  unsigned long long t0 = 0;
+  unsigned long long t0 = 0, seen = 0;
   unsigned spins = 0;
   while (ld_acquire_u64(mb.mono) < target) {
     if ((++spins & 255u) != 0) continue;
     if (ld_relaxed_i32(mb.status) != 0) return false;
     const unsigned long long now = global_timer_ns();
-    if (t0 == 0) t0 = now;
-    else if (now - t0 > wait_limit_ns()) {
+    const unsigned long long moved = progress ? ld_relaxed_u64(progress) : 0;
+    if (t0 == 0 || moved != seen) {
+      t0 = now;
+      seen = moved;
+    } else if (now - t0 > wait_limit_ns()) {
       atomicCAS(mb.status, 0, (int)BOGUS_GPU_TIMEOUT);
       return false;
     }

@@ -204,7 +204,8 @@ cudaError_t launch_unpad_positions(int n, const float* src, double* dst, cudaStr
 struct ResidentJob {
   int problem, rank, ctas;
 };
-// CTA b works through jobs[job_ptr[b] .. job_ptr[b + 1]); mono: one barrier counter per problem, zero at launch
+// CTA b works through jobs[job_ptr[b] .. job_ptr[b + 1]); mono: one barrier counter per problem and one of all barriers,
+// zero at launch
 cudaError_t launch_pg_resident_batch(const PGBatchArgs& b, const int* job_ptr, const ResidentJob* jobs,
                                      unsigned long long* mono, int ctas, int teams, int steps, cudaStream_t s);
 cudaError_t launch_pg_batched(const PGBatchArgs& b, int grid, cudaStream_t s);

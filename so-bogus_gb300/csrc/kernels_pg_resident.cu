@@ -53,6 +53,7 @@ struct Place {
   unsigned parties;
   int first, stride, count;  // chunks list[first + k stride] (list null: the index itself), k < count
   const int* list;
+  unsigned long long* progress;  // ResidentReduce::progress
   __device__ int chunk(int k) const {
     const int j = first + k * stride;
     return list ? __ldg(list + j) : j;
@@ -124,7 +125,7 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
       return ClusterReduce{gs + 4 * (size_t)32 * C, C, ctl.stripes, lane, warp, nwarps, (int)place.parties};
     else
       return ResidentReduce{MonoBarrier{a.mono, a.gb.status, place.parties + a.phantom_ctas}, a.csum, C, ctl.stripes, lane, warp,
-                            nwarps};
+                            nwarps, place.progress};
   }();
   auto put = [&](int q, double v) { red.put(q, c, v); };
   auto reduce = [&](int K, unsigned maxmask, auto side, auto decide) { return red.reduce(K, maxmask, side, decide); };
@@ -477,7 +478,7 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
 __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(PGArgs a, int teams) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int first = __ldg(a.cta_ptr + blockIdx.x);
-  const Place place{(int)blockIdx.x, gridDim.x, first, 1, __ldg(a.cta_ptr + blockIdx.x + 1) - first, a.cta_list};
+  const Place place{(int)blockIdx.x, gridDim.x, first, 1, __ldg(a.cta_ptr + blockIdx.x + 1) - first, a.cta_list, nullptr};
   resident_solve<false>(a, teams, place, smem);
 }
 
@@ -491,7 +492,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1) k_pg_resident(
 __global__ void __launch_bounds__(32 * kMinWarps, 1) k_pg_resident_cluster(PGArgs a, int teams) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int rank = (int)blockIdx.x, ctas = (int)gridDim.x;
-  const Place place{rank, gridDim.x, rank, ctas, (a.nchunks - rank + ctas - 1) / ctas, nullptr};
+  const Place place{rank, gridDim.x, rank, ctas, (a.nchunks - rank + ctas - 1) / ctas, nullptr, nullptr};
   cluster_arrive();  // every CTA's shared memory is there before the first store into it
   cluster_wait();
   resident_solve<true>(a, teams, place, smem);
@@ -502,7 +503,8 @@ __global__ void __launch_bounds__(32 * kMinWarps, 1) k_pg_resident_cluster(PGArg
 
 // A batch: every CTA works through its own list of jobs, a job being its part in one problem (the chunks rank,
 // rank + ctas, ...). The lists hold the problems in one global order, so a CTA waits in a problem's barriers only for
-// CTAs that are at this problem or at earlier ones.
+// CTAs that are at this problem or at earlier ones. The wait for earlier ones is as long as their solves are: it ends in
+// a timeout only when no CTA of the launch passes a barrier for the length of the limit (mono[nproblems] counts them).
 __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1)
     k_pg_resident_batch(PGBatchArgs ba, const int* job_ptr, const ResidentJob* jobs, unsigned long long* mono, int teams) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -530,7 +532,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps * kMaxTeams, 1)
     }
     __syncthreads();
     const int mine = a.nchunks > job.rank ? (a.nchunks - job.rank + job.ctas - 1) / job.ctas : 0;
-    const Place place{job.rank, (unsigned)job.ctas, job.rank, job.ctas, mine, nullptr};
+    const Place place{job.rank, (unsigned)job.ctas, job.rank, job.ctas, mine, nullptr, mono + ba.nproblems};
     resident_solve<false>(a, teams, place, smem);
     // the best iterate over the initial one, by the lanes that stored it
     const int warp = threadIdx.x >> 5, i = 32 * (job.rank + (warp / kTeamWarps) * job.ctas) + (threadIdx.x & 31);

@@ -277,6 +277,10 @@ struct ResidentReduce {
   const int C;
   double* stripes;  // 32 shared doubles
   const int lane, warp, nwarps;
+  // CTAs that share a problem may still be at others when this one arrives first: a counter that every CTA advances at
+  // every barrier of every problem (null where all CTAs start together). While it moves, the wait of the first barrier
+  // does not count as a hang; past it all CTAs are here and the limit holds as it is.
+  unsigned long long* progress = nullptr;
   unsigned phase = 0;  // barriers passed
   __device__ double* sums() const { return csum + (size_t)(phase & 1u) * 4 * C; }
   // v: quantity q of chunk c, in every lane
@@ -295,7 +299,10 @@ struct ResidentReduce {
     bool ok = true;
     __syncthreads();
     if (warp == nwarps - 1) side();
-    if (mb.parties > 1u && threadIdx.x == 0) ok = flat_wait(mb, phase);
+    if (threadIdx.x == 0) {
+      if (progress) red_add_relaxed_u64(progress, 1ull);
+      if (mb.parties > 1u) ok = flat_wait(mb, phase, phase == 0 ? progress : nullptr);
+    }
     return __syncthreads_and(ok) != 0;
   }
   __device__ bool sync() {
