@@ -16,6 +16,7 @@
 // maximum and the skip counters.
 #include "internal.h"
 #include "soc_device.cuh"
+#include "warp_wait.cuh"
 
 namespace bogus_gpu {
 
@@ -184,14 +185,11 @@ __global__ void __launch_bounds__(32 * kGSFlowWarps, 2) k_gs_flow(GSArgs a, int 
         if (idled && ++idle > 1) {
           __nanosleep(40);
           if ((idle & 63u) == 0) {
-            bool stop = ld_relaxed_i32(a.status) != 0;
             const unsigned long long now = global_timer_ns();
             if (t0 == 0) t0 = now;
-            else if (now - t0 > wait_limit_ns()) {
-              if (lane == 0) atomicCAS(a.status, 0, (int)BOGUS_GPU_TIMEOUT);
-              stop = true;
-            }
-            if (__any_sync(0xffffffffu, stop)) return;
+            if (warp_gives_up(now - t0 > wait_limit_ns(), ld_relaxed_i32(a.status) != 0, lane, a.status,
+                              (int)BOGUS_GPU_TIMEOUT))
+              return;
           }
         }
       }

@@ -51,6 +51,20 @@ inline double shfl(double v, int src) {
   return r;
 }
 
+inline unsigned __ballot_sync(unsigned, bool on) {
+  sim::warp->swap[sim::lane] = on;
+  __syncwarp();
+  unsigned m = 0;
+  for (int l = 0; l < 32; ++l) m |= (sim::warp->swap[l] != 0.0 ? 1u : 0u) << l;
+  __syncwarp();
+  return m;
+}
+inline bool __any_sync(unsigned mask, bool on) { return __ballot_sync(mask, on) != 0; }
+inline int atomicCAS(int* p, int expected, int v) {
+  std::atomic_ref<int>(*p).compare_exchange_strong(expected, v);
+  return expected;
+}
+
 namespace bogus_gpu {
 inline void store_cluster(const double* p, int rank, double v) {
   sim::cluster->cta[rank]->smem[p - sim::cta->smem] = v;
@@ -64,6 +78,7 @@ inline double warp_sum_butterfly(double v) {
 }  // namespace bogus_gpu
 
 #include "cluster_reduce.cuh"
+#include "warp_wait.cuh"
 
 using namespace bogus_gpu;
 
@@ -119,6 +134,16 @@ int hw_cluster_reduce(int C, int rounds) {
     }
   });
   return wrong;
+}
+
+// A warp's wait with the lanes of `late` past the limit and those of `stopped` told to stop, *status as given; returns
+// whether every lane (1), no lane (0) or only some (-1) gave up.
+int hw_warp_gives_up(unsigned late, unsigned stopped, int* status) {
+  std::atomic<int> gave{0};
+  run_cluster(1, 1, [&](int, int, int l) {
+    gave += warp_gives_up((late >> l) & 1u, (stopped >> l) & 1u, l, status, 5) ? 1 : 0;
+  });
+  return gave == 32 ? 1 : gave == 0 ? 0 : -1;
 }
 
 }  // extern "C"
