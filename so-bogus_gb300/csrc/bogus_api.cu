@@ -12,6 +12,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -3102,6 +3103,25 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
     if (int e = check_finite(f, (size_t)nb * d, "f")) return e;
   if (int e = ensure_body_lists(h)) return e;
   cudaStream_t s = h->stream;
+  // W's blocks are counted in ints: a body with some 46 000 contacts alone passes them. The pairs of contacts per body
+  // bound the count (a pair that shares two bodies twice); only where they pass it are the rows' own lengths added up.
+  {
+    const auto too_many = [n](long long lower) { return 2 * lower - n > INT_MAX; };
+    long long pairs = 0;
+    for (int k = 0; k < nb; ++k) {
+      const long long m = h->h_bptr[k + 1] - h->h_bptr[k];
+      pairs += m * (m + 1) / 2;
+    }
+    if (too_many(pairs)) {
+      std::vector<int> row(n);
+      BG_CUDA(h->pat_upper.ensure(n));
+      BG_CUDA(launch_lower_count(n, h->cb.p, h->bptr.p, h->bent.p, h->pat_upper.p, s));
+      BG_CUDA(cudaMemcpyAsync(row.data(), h->pat_upper.p, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
+      BG_CUDA(cudaStreamSynchronize(s));
+      if (too_many(std::accumulate(row.begin(), row.end(), 0ll)))
+        return fail(BOGUS_GPU_BAD_INPUT, "W would have more than 2^31 - 1 blocks");
+    }
+  }
   auto up = [&](void* dst, const void* src, size_t bytes) {
     return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess;
   };
