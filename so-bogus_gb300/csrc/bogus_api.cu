@@ -29,11 +29,13 @@ cudaError_t launch_assembly_T(int n, int ndof, const double* minv, const int* cb
                               cudaStream_t s);
 cudaError_t launch_assembly_slots(int n, int d, const int* cb, const int* objA, const double* HA, const double* HB,
                                   double* H, cudaStream_t s);
-cudaError_t launch_lower_count(int n, const int* cb, const int* bptr, const int* bent, int* count, cudaStream_t s);
-cudaError_t launch_lower_fill(int n, const int* cb, const int* bptr, const int* bent, const int* rowptr, int* row,
-                              int* col, cudaStream_t s);
-cudaError_t launch_assembly_W(int nlow, int ndof, const int* row, const int* col, const int* cb, const double* H,
-                              const double* T, double* val, cudaStream_t s);
+cudaError_t launch_row_count(int n, const int* cb, const int* bptr, const int* bent, int* lower, int* full,
+                             cudaStream_t s);
+cudaError_t launch_row_fill(int n, const int* cb, const int* bptr, const int* bent, const int* lptr, int* lrow,
+                            int* lcol, const int* fptr, int* fcol, cudaStream_t s);
+cudaError_t launch_assembly_W(int nlow, int ndof, const int* lptr, const int* row, const int* col, const int* fptr,
+                              const int* fcol, const int* cb, const double* H, const double* T, double* lval,
+                              double* fval, cudaStream_t s);
 cudaError_t launch_assembly_b(int n, int nbodies, int ndof, const double* minv, const double* f, const int* cb,
                               const double* H, const double* w, double* mf, double* b, cudaStream_t s);
 
@@ -3103,22 +3105,25 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
     if (int e = check_finite(f, (size_t)nb * d, "f")) return e;
   if (int e = ensure_body_lists(h)) return e;
   cudaStream_t s = h->stream;
+  BG_CUDA(h->pat_upper.ensure(n > 0 ? n : 1));
+  BG_CUDA(h->pat_cursor.ensure(n > 0 ? n : 1));
+  int* const lower_len = h->pat_upper.p;
+  int* const full_len = h->pat_cursor.p;
+  BG_CUDA(cudaEventRecord(h->ev0, s));
+  BG_CUDA(launch_row_count(n, h->cb.p, h->bptr.p, h->bent.p, lower_len, full_len, s));
   // W's blocks are counted in ints: a body with some 46 000 contacts alone passes them. The pairs of contacts per body
   // bound the count (a pair that shares two bodies twice); only where they pass it are the rows' own lengths added up.
   {
-    const auto too_many = [n](long long lower) { return 2 * lower - n > INT_MAX; };
     long long pairs = 0;
     for (int k = 0; k < nb; ++k) {
       const long long m = h->h_bptr[k + 1] - h->h_bptr[k];
-      pairs += m * (m + 1) / 2;
+      pairs += m * m;
     }
-    if (too_many(pairs)) {
+    if (pairs > INT_MAX) {
       std::vector<int> row(n);
-      BG_CUDA(h->pat_upper.ensure(n));
-      BG_CUDA(launch_lower_count(n, h->cb.p, h->bptr.p, h->bent.p, h->pat_upper.p, s));
-      BG_CUDA(cudaMemcpyAsync(row.data(), h->pat_upper.p, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
+      BG_CUDA(cudaMemcpyAsync(row.data(), full_len, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
       BG_CUDA(cudaStreamSynchronize(s));
-      if (too_many(std::accumulate(row.begin(), row.end(), 0ll)))
+      if (std::accumulate(row.begin(), row.end(), 0ll) > INT_MAX)
         return fail(BOGUS_GPU_BAD_INPUT, "W would have more than 2^31 - 1 blocks");
     }
   }
@@ -3128,8 +3133,7 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
   // the pattern of the lower triangle (the staging set of the lower-triangle buffers, as in set_dual_lower)
   const int nx = 1 - h->low_cur;
   BG_CUDA(h->low_rowptr[nx].ensure(n + 1));
-  BG_CUDA(h->pat_upper.ensure(n > 0 ? n : 1));
-  BG_CUDA(h->pat_cursor.ensure(n > 0 ? n : 1));
+  BG_CUDA(h->asm_row.ensure(n > 0 ? n : 1));
   BG_CUDA(h->diag.ensure(n));
   BG_CUDA(h->b.ensure(3 * (size_t)n));
   BG_CUDA(h->mu.ensure(n));
@@ -3149,9 +3153,8 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
     BG_CUDA(cudaMemsetAsync(h->low_rowptr[nx].p, 0, sizeof(int), s));
     BG_CUDA(cudaMemsetAsync(h->rowptr.p, 0, sizeof(int), s));
   }
-  BG_CUDA(cudaEventRecord(h->ev0, s));
-  BG_CUDA(launch_lower_count(n, h->cb.p, h->bptr.p, h->bent.p, h->pat_upper.p, s));
-  BG_CUDA(launch_prefix_sum(n, h->pat_upper.p, h->pat_cursor.p, h->low_rowptr[nx].p, s));
+  BG_CUDA(launch_prefix_sum(n, lower_len, h->asm_row.p, h->low_rowptr[nx].p, s));
+  BG_CUDA(launch_prefix_sum(n, full_len, h->asm_row.p, h->rowptr.p, s));
   int nlow = 0;
   BG_CUDA(cudaMemcpyAsync(&nlow, h->low_rowptr[nx].p + n, sizeof(int), cudaMemcpyDeviceToHost, s));
   BG_CUDA(launch_assembly_T(n, d, h->minv.p, h->cb.p, h->H.p, h->T.p, s));
@@ -3163,14 +3166,12 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
   BG_CUDA(h->low_col[nx].ensure(nlow > 0 ? nlow : 1));
   BG_CUDA(h->low_val[nx].ensure(9 * (size_t)(nlow > 0 ? nlow : 1)));
   BG_CUDA(h->asm_row.ensure(nlow > 0 ? nlow : 1));
-  BG_CUDA(h->full_src.ensure(nnz > 0 ? nnz : 1));
   BG_CUDA(h->col.ensure(nnz));
   BG_CUDA(h->val.ensure(9 * (size_t)nnz));
-  BG_CUDA(launch_lower_fill(n, h->cb.p, h->bptr.p, h->bent.p, h->low_rowptr[nx].p, h->asm_row.p, h->low_col[nx].p, s));
-  BG_CUDA(launch_assembly_W(nlow, d, h->asm_row.p, h->low_col[nx].p, h->cb.p, h->H.p, h->T.p, h->low_val[nx].p, s));
-  BG_CUDA(launch_full_pattern(n, h->low_rowptr[nx].p, h->low_col[nx].p, h->pat_upper.p, h->pat_cursor.p, h->rowptr.p,
-                              h->col.p, h->full_src.p, s));
-  BG_CUDA(launch_expand_lower(nnz, h->full_src.p, h->low_val[nx].p, h->val.p, s));
+  BG_CUDA(launch_row_fill(n, h->cb.p, h->bptr.p, h->bent.p, h->low_rowptr[nx].p, h->asm_row.p, h->low_col[nx].p,
+                          h->rowptr.p, h->col.p, s));
+  BG_CUDA(launch_assembly_W(nlow, d, h->low_rowptr[nx].p, h->asm_row.p, h->low_col[nx].p, h->rowptr.p, h->col.p, h->cb.p,
+                            h->H.p, h->T.p, h->low_val[nx].p, h->val.p, s));
   BG_CUDA(cudaEventRecord(h->ev1, s));
   h->W.n = n;
   h->W.nnzb = nnz;
@@ -3181,7 +3182,7 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
   BG_CUDA(launch_diag_and_scaling(h->W, h->scaling.p, s));
   BG_CUDA(cudaStreamSynchronize(s));
   BG_CUDA(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
-  h->last_launches = 15;
+  h->last_launches = 7 + 2 * (n > 1024 ? 3 : 1);
   // the host copy of the lower triangle is downloaded when first needed (ensure_host_lower)
   h->low_cur = nx;
   h->host_lower_valid = false;
