@@ -166,9 +166,13 @@ struct bogus_gpu_problem {
   DevBuf<int> chunk_order;  // chunks by decreasing segment length (ticket order of the persistent solvers)
   std::vector<int> h_chunk_order;  // the same on the host
   std::vector<int> h_chunk_seg;    // S of every chunk
-  // per-CTA chunk lists of the single-problem kernel for a grid of cta_grid CTAs (0: none built)
-  DevBuf<int> cta_ptr, cta_list;
-  int cta_grid = 0;
+  // per-CTA chunk lists by grid (0: none built): a problem's kernels use up to three (resident, FP64, FP32), a refined
+  // solve two of them in turn
+  struct CtaLists {
+    int grid = 0;
+    DevBuf<int> ptr, list;
+  } cta_lists[3];
+  int cta_next = 0;  // the set that a fourth grid replaces
   DevBuf<int> icol;
   DevBuf<double> ival;
   // FP32 copies of W (interleaved), b, mu, scalings and FP32 work (mixed precision), valid while W is unchanged
@@ -500,7 +504,7 @@ int ensure_pg_work(bogus_gpu_problem* h, unsigned max_iters) {
 
 int ensure_chunks(bogus_gpu_problem* h);
 int ensure_interleaved(bogus_gpu_problem* h);
-int ensure_cta_lists(bogus_gpu_problem* h, int G);
+int ensure_cta_lists(bogus_gpu_problem* h, int G, const int** ptr, const int** list);
 int ensure_incidence(bogus_gpu_problem* h);
 
 // Algorithmic bytes and W passes of one persistent solve from its phase counters. A W pass reads nnzb blocks
@@ -650,9 +654,7 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
   }
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
   a.flat = !sc && a.nchunks <= kFlatChunks;
-  if (int e = ensure_cta_lists(h, grid)) return e;
-  a.cta_ptr = h->cta_ptr.p;
-  a.cta_list = h->cta_list.p;
+  if (int e = ensure_cta_lists(h, grid, &a.cta_ptr, &a.cta_list)) return e;
   BG_CUDA(cudaEventRecord(h->ev0, h->stream));
   BG_CUDA(cluster    ? launch_pg_resident_cluster(a, rs.longest, h->stream)
           : resident ? launch_pg_resident(a, grid, rs.teams, rs.steps, h->stream)
@@ -705,8 +707,16 @@ int run_pg(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* residual
 // CTAs') are equal to within about one chunk; each CTA's warps share its list dynamically. A phase then
 // ends with every SM at about the same time instead of each SM finishing the chunks it happened to hold when
 // a global ticket pool ran out. Which warp handles a chunk does not change any result.
-int ensure_cta_lists(bogus_gpu_problem* h, int G) {
-  if (h->cta_grid == G) return BOGUS_GPU_OK;
+int ensure_cta_lists(bogus_gpu_problem* h, int G, const int** ptr, const int** chunks) {
+  for (auto& t : h->cta_lists)
+    if (t.grid == G) {
+      *ptr = t.ptr.p;
+      *chunks = t.list.p;
+      return BOGUS_GPU_OK;
+    }
+  auto& t = h->cta_lists[h->cta_next];
+  h->cta_next = (h->cta_next + 1) % 3;
+  t.grid = 0;
   const int C = (int)h->h_chunk_order.size();
   std::vector<int> cnt(G + 1, 0), owner(C);
   for (int k = 0; k < C; ++k) {
@@ -717,13 +727,14 @@ int ensure_cta_lists(bogus_gpu_problem* h, int G) {
   for (int b = 0; b < G; ++b) cnt[b + 1] += cnt[b];
   std::vector<int> list(C > 0 ? C : 1), fill(cnt.begin(), cnt.end() - 1);
   for (int k = 0; k < C; ++k) list[fill[owner[k]]++] = h->h_chunk_order[k];
-  BG_CUDA(h->cta_ptr.ensure(G + 1));
-  BG_CUDA(h->cta_list.ensure(C > 0 ? C : 1));
-  BG_CUDA(cudaMemcpyAsync(h->cta_ptr.p, cnt.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice, h->stream));
-  BG_CUDA(cudaMemcpyAsync(h->cta_list.p, list.data(), sizeof(int) * (C > 0 ? C : 1), cudaMemcpyHostToDevice,
-                          h->stream));
+  BG_CUDA(t.ptr.ensure(G + 1));
+  BG_CUDA(t.list.ensure(C > 0 ? C : 1));
+  BG_CUDA(cudaMemcpyAsync(t.ptr.p, cnt.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice, h->stream));
+  BG_CUDA(cudaMemcpyAsync(t.list.p, list.data(), sizeof(int) * (C > 0 ? C : 1), cudaMemcpyHostToDevice, h->stream));
   BG_CUDA(cudaStreamSynchronize(h->stream));
-  h->cta_grid = G;
+  t.grid = G;
+  *ptr = t.ptr.p;
+  *chunks = t.list.p;
   return BOGUS_GPU_OK;
 }
 
@@ -744,7 +755,7 @@ int ensure_chunks(bogus_gpu_problem* h) {
   }
   const std::vector<int>& seg = h->h_chunk_seg;
   std::stable_sort(h->h_chunk_order.begin(), h->h_chunk_order.end(), [&](int x, int y) { return seg[x] > seg[y]; });
-  h->cta_grid = 0;
+  for (auto& t : h->cta_lists) t.grid = 0;
   h->chunks_valid = true;
   return BOGUS_GPU_OK;
 }
@@ -867,9 +878,7 @@ int run_pg_mixed(bogus_gpu_problem* h, const bogus_gpu_pg_options* o, double* re
   const int grid = resident ? rs.ctas : pg_grid(h->device, true, a.nchunks);
   if (grid <= 0) return fail(BOGUS_GPU_CUDA_ERROR, "cooperative occupancy query failed");
   a.flat = a.nchunks <= kFlatChunks;
-  if (int e = ensure_cta_lists(h, grid)) return e;
-  a.cta_ptr = h->cta_ptr.p;
-  a.cta_list = h->cta_list.p;
+  if (int e = ensure_cta_lists(h, grid, &a.cta_ptr, &a.cta_list)) return e;
   BG_CUDA(cudaEventRecord(h->ev0, s));
   BG_CUDA(resident ? launch_pg_resident32(a, grid, rs.teams, rs.steps, s) : launch_pg_persistent(a, grid, s));
   BG_CUDA(cudaEventRecord(h->ev1, s));
@@ -1189,8 +1198,10 @@ int bogus_gpu_destroy(bogus_gpu_problem* h) {
     b->release();
   h->slot0.release();
   h->chunk_order.release();
-  h->cta_ptr.release();
-  h->cta_list.release();
+  for (auto& t : h->cta_lists) {
+    t.ptr.release();
+    t.list.release();
+  }
   h->icol.release();
   h->ival.release();
   for (auto* b : {&h->a_prox, &h->a_f, &h->a_w, &h->a_mu, &h->a_invmu, &h->a_x, &h->a_r, &h->a_ut, &h->a_z, &h->a_zacc,
@@ -2539,10 +2550,8 @@ int run_adjoint(bogus_gpu_problem* h, const bogus_gpu_adjoint_options* o, double
   a.val = h->W.val;
   a.col = h->W.col;
   if (resident) {
-    if (int e = ensure_cta_lists(h, rs.ctas)) return e;
+    if (int e = ensure_cta_lists(h, rs.ctas, &a.cta_ptr, &a.cta_list)) return e;
     BG_CUDA(h->adj_G.ensure(4 * (size_t)n));
-    a.cta_ptr = h->cta_ptr.p;
-    a.cta_list = h->cta_list.p;
     a.G = h->adj_G.p;
   } else {
     if (int e = ensure_interleaved(h)) return e;
