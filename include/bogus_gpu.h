@@ -231,7 +231,7 @@ int bogus_gpu_solve_gs(bogus_gpu_problem* h, const bogus_gpu_gs_options* opts, d
  * assembled with bogus_gpu_assemble_dual). contact_ptr has nproblems + 1 entries, from 0 to n. */
 int bogus_gpu_set_batch(bogus_gpu_problem* h, int nproblems, const int* contact_ptr);
 
-/* Solves every problem of the batch in one persistent launch (one CTA per problem, largest first). Each
+/* Solves every problem of the batch in one persistent launch (launch shapes below, largest problem first). Each
  * problem gets exactly the result DualFrictionProblem::solveWith(ProjectedGradient&, r) gives for it alone
  * (same iterates, residual and iteration count). r: all problems, contact-major, in/out; residuals and iters
  * hold one entry per problem (NULL allowed). Returns BOGUS_GPU_NOT_CONVERGED if any problem did not converge. */
@@ -243,7 +243,11 @@ int bogus_gpu_solve_pg_batch_device(bogus_gpu_problem* h, const bogus_gpu_pg_opt
 
 /* Launch shape of the batched solves. schedule 0: one CTA per problem, at most ctas_per_sm resident CTAs per SM;
  * schedule 1: teams of team_size CTAs per problem (a cooperative launch), at most ctas_per_sm CTAs per SM. Every
- * shape gives the same results bit for bit: each problem's reductions follow its fixed 32-contact chunk order. */
+ * shape gives the same results bit for bit: each problem's reductions follow its fixed 32-contact chunk order.
+ * The resident form is no shape of these: one CTA per SM, each with a list of problems or parts of problems fixed by
+ * bogus_gpu_set_batch, W in shared memory. An FP64 batch (without momentum_by_linearity) whose problems fit runs in it
+ * in place of the rule's shape where it is estimated to end earlier, unless a shape is forced, tuning is on or the
+ * call is captured; the results are the same bit for bit. */
 typedef struct bogus_gpu_batch_shape {
   int schedule;
   int ctas_per_sm;
@@ -255,11 +259,12 @@ typedef struct bogus_gpu_batch_shape {
  * each run capped at 30 iterations from the same starting iterate, timed with CUDA events) and keeps the fastest,
  * which later solves reuse; the choice is also cached for the process by device, precision and the batch's size
  * class (problems, largest problem, total 32-contact chunks). 0 (default): a fixed rule (one CTA per problem when
- * there are at least half as many problems as resident CTAs, else teams). */
+ * there are at least half as many problems as resident CTAs, else teams), or the resident form. */
 int bogus_gpu_set_batch_tuning(bogus_gpu_problem* h, int on);
 /* Forces the shape of the following batched solves (NULL: back to tuning or the rule). */
 int bogus_gpu_set_batch_shape(bogus_gpu_problem* h, const bogus_gpu_batch_shape* shape);
-/* The shape of the last batched launch. */
+/* The shape of the last batched launch; where the resident form ran, the rule's shape that it took the place of (forcing
+ * it gives the same results, as any shape does). */
 int bogus_gpu_get_batch_shape(const bogus_gpu_problem* h, bogus_gpu_batch_shape* shape);
 /* The tuner's last measurements: *count shapes and their times in ms (pass NULL arrays to get the count). */
 int bogus_gpu_get_batch_tuning_log(const bogus_gpu_problem* h, bogus_gpu_batch_shape* shapes, double* ms, int* count);

@@ -819,7 +819,8 @@ class DualFrictionProblem:
         _check(lib().bogus_gpu_set_batch_shape(self._h, C.byref(sh)), False)
 
     def batchShape(self) -> tuple:
-        """(schedule, ctas_per_sm, team_size) of the last batched launch."""
+        """(schedule, ctas_per_sm, team_size) of the last batched launch; where the form with W in shared memory ran, the
+        rule's shape that it took the place of."""
         sh = BatchShape()
         _check(lib().bogus_gpu_get_batch_shape(self._h, C.byref(sh)), False)
         return sh.schedule, sh.ctas_per_sm, sh.team_size
