@@ -48,6 +48,10 @@ struct ClusterReduce {
     if ((lane & 15) < parties) store_cluster(sums() + (q + (lane >> 4)) * C + c, lane & 15, v);
   }
   __device__ void put(int q, int c, double v) { put_total(q, c, warp_sum_butterfly(v)); }
+  // With a NaN among the values the lanes' maxima differ (a sum is NaN in all of them): every CTA gets the first lane's, as
+  // the kernels that store it once do. CTAs with different totals would take different branches, and one that ends while
+  // another still writes to its shared memory faults the launch.
+  __device__ void put_max(int q, int c, double v) { put_total(q, c, __shfl_sync(0xffffffffu, warp_max_butterfly(v), 0)); }
   // The last warp, which has no chunk, prepares the next decision (side) before it arrives: the barrier orders arrivals
   // only, so what it wrote after its own would not be there for warp 0. Nothing in the phase before the barrier reads or
   // writes what side writes, and nothing but the decision before that phase writes what it reads.

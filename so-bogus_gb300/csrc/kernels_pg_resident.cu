@@ -254,8 +254,8 @@ __device__ __forceinline__ void resident_solve(const PGArgs& a, int teams, const
       }
     }
     if (role == 0) {
-      v = a.use_inf ? warp_max_butterfly(v) : warp_sum_butterfly(v);
-      red.put_total(0, c, v);
+      if (a.use_inf) red.put_max(0, c, v);
+      else put(0, v);
     } else if (role == (spg ? 1 : 2)) {
       put(1, v);
     }

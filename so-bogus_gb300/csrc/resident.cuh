@@ -283,7 +283,7 @@ struct ResidentReduce {
   unsigned long long* progress = nullptr;
   unsigned phase = 0;  // barriers passed
   __device__ double* sums() const { return csum + (size_t)(phase & 1u) * 4 * C; }
-  // v: quantity q of chunk c, in every lane
+  // v: quantity q of chunk c, in lane 0
   __device__ void put_total(int q, int c, double v) {
     if (lane == 0) sums()[q * C + c] = v;
   }
@@ -293,6 +293,7 @@ struct ResidentReduce {
   }
   // sum of v over the warp as chunk c's value of quantity q
   __device__ void put(int q, int c, double v) { put_total(q, c, warp_sum_butterfly(v)); }
+  __device__ void put_max(int q, int c, double v) { put_total(q, c, warp_max_butterfly(v)); }
   // The last warp prepares the next decision (side) while thread 0 waits for the other CTAs.
   template <class Side>
   __device__ bool arrive_and_wait(Side&& side) {

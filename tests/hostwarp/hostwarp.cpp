@@ -8,6 +8,7 @@
 #include <memory>
 #include <optional>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #define __device__
@@ -59,6 +60,7 @@ inline unsigned __ballot_sync(unsigned, bool on) {
   __syncwarp();
   return m;
 }
+inline double __shfl_sync(unsigned, double v, int src) { return shfl(v, src); }
 inline bool __any_sync(unsigned mask, bool on) { return __ballot_sync(mask, on) != 0; }
 inline int atomicCAS(int* p, int expected, int v) {
   std::atomic_ref<int>(*p).compare_exchange_strong(expected, v);
@@ -73,6 +75,13 @@ inline void cluster_arrive() { sim::token.emplace(sim::cluster->all.arrive()); }
 inline void cluster_wait() { sim::cluster->all.wait(std::move(*sim::token)); }
 inline double warp_sum_butterfly(double v) {
   for (int off = 16; off >= 1; off >>= 1) v = v + shfl(v, sim::lane ^ off);
+  return v;
+}
+inline double warp_max_butterfly(double v) {
+  for (int off = 16; off >= 1; off >>= 1) {
+    const double o = shfl(v, sim::lane ^ off);
+    v = (v < o) ? o : v;
+  }
   return v;
 }
 }  // namespace bogus_gpu
@@ -134,6 +143,17 @@ int hw_cluster_reduce(int C, int rounds) {
     }
   });
   return wrong;
+}
+
+// One maximum over two chunks of 32 values, one chunk per CTA of a cluster of two; the decision's total in each CTA.
+void hw_cluster_max(const double* values, double* totals) {
+  run_cluster(2, 2, [&](int r, int w, int l) {
+    ClusterReduce red{sim::cta->smem + 64, 2, sim::cta->smem, l, w, 2, 2};
+    if (w == 0) red.put_max(0, r, values[32 * r + l]);
+    red.reduce(2, 1u, [] {}, [&](double total) {
+      if (l == 0) totals[r] = total;
+    });
+  });
 }
 
 // A warp's wait with the lanes of `late` past the limit and those of `stopped` told to stop, *status as given; returns

@@ -4,6 +4,7 @@ import ctypes
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -34,3 +35,28 @@ def test_a_warp_that_gives_up_says_why(hostwarp, late, stopped, before):
     gave = hostwarp.hw_warp_gives_up(ctypes.c_uint(late), ctypes.c_uint(stopped), ctypes.byref(status))
     assert gave == (1 if late or stopped else 0)
     assert status.value == (before or (5 if late else 0))
+
+
+@pytest.mark.parametrize("at", [[], [0], [1], [17, 40], [0, 32], [33], list(range(64))])
+def test_every_cta_of_a_cluster_sees_the_same_maximum(hostwarp, at):
+    """A maximum over values with NaN among them depends on the lane that holds it; the CTAs of a cluster have to take one
+    lane's, the first as the other kernels do, or their decisions part."""
+    values = np.linspace(1.0, 2.0, 64)
+    values[at] = np.nan
+    totals = np.full(2, 7.0)
+    hostwarp.hw_cluster_max(values.ctypes.data_as(ctypes.c_void_p), totals.ctypes.data_as(ctypes.c_void_p))
+    assert np.array_equal(totals[:1], totals[1:], equal_nan=True)
+
+    def butterfly(v):
+        for off in (16, 8, 4, 2, 1):
+            o = v[np.arange(32) ^ off]
+            v = np.where(v < o, o, v)
+        return v[0]
+
+    # two chunks, a stripe each: 0, then the chunk's maximum where it is not below; the stripes left to right
+    total = None
+    for s in range(8):
+        v = butterfly(values[32 * s:32 * s + 32]) if s < 2 else 0.0
+        v = 0.0 if v < 0.0 else v
+        total = v if total is None else total if v < total else v
+    assert np.array_equal(totals[0], total, equal_nan=True)
