@@ -145,6 +145,7 @@ struct bogus_gpu_problem {
   // copied to host_lower when first needed; work of the device-side expansion
   bool low_pending = false;
   int low_cur = 0;
+  int low_nnz = 0;  // blocks of the pending lower triangle
   // DualFrictionProblem::applyPermutation: contact k of the stored problem is contact perm[k] of the caller's
   bool permuted = false;
   std::vector<int> perm, inv_perm;
@@ -365,6 +366,7 @@ int set_dual_lower(bogus_gpu_problem* h, int n, const int* rowptr, const int* co
   if (bad) return fail(BOGUS_GPU_NONFINITE, "non-finite block value");
   // the staged upload becomes the problem
   h->low_cur = nx;
+  h->low_nnz = nlow;
   const int nnz = 2 * nlow - check[1];
   BG_CUDA(h->rowptr.ensure(n + 1));
   BG_CUDA(h->col.ensure(nnz));
@@ -416,10 +418,9 @@ int ensure_host_lower(bogus_gpu_problem* h) {
   HostBSR& l = h->host_lower;
   const int n = l.n;
   cudaStream_t s = h->stream;
+  const int nlow = h->low_nnz;
   l.rowptr.resize(n + 1);
   BG_CUDA(cudaMemcpyAsync(l.rowptr.data(), h->low_rowptr[h->low_cur].p, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, s));
-  BG_CUDA(cudaStreamSynchronize(s));
-  const int nlow = l.rowptr[n];
   l.col.resize(nlow);
   l.val.resize(9 * (size_t)nlow);
   if (nlow) {
@@ -2801,8 +2802,9 @@ int bogus_gpu_add_compliance(bogus_gpu_problem* h, const double* c) {
   DevBuf<double> dc;
   BG_CUDA(dc.ensure(n > 0 ? n : 1));
   if (n) BG_CUDA(cudaMemcpyAsync(dc.p, c, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
-  if (h->low_pending)  // the host copy of the lower triangle takes the same diagonal terms
-    if (int e = ensure_host_lower(h)) return e;
+  // the lower triangle takes the same diagonal terms: the device's where the host has no copy yet, else the host's (below)
+  if (h->low_pending)
+    BG_CUDA(launch_add_lower_diagonal(n, h->low_rowptr[h->low_cur].p, dc.p, h->low_val[h->low_cur].p, h->stream));
   BG_CUDA(launch_add_diagonal(h->W, dc.p, h->stream));
   BG_CUDA(launch_diag_and_scaling(h->W, h->scaling.p, h->stream));
   BG_CUDA(cudaStreamSynchronize(h->stream));
@@ -3196,6 +3198,7 @@ int bogus_gpu_assemble_dual(bogus_gpu_problem* h, const double* f, const double*
   h->last_launches = 7 + 2 * (n > 1024 ? 3 : 1);
   // the host copy of the lower triangle is downloaded when first needed (ensure_host_lower)
   h->low_cur = nx;
+  h->low_nnz = nlow;
   h->host_lower_valid = false;
   h->low_pending = true;
   h->host_lower.n = n;

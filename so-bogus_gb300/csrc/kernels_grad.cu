@@ -91,6 +91,22 @@ cudaError_t launch_add_diagonal(const DevBSR& W, const double* c, cudaStream_t s
   return cudaGetLastError();
 }
 
+// The same on a lower triangle, whose rows end with their diagonal blocks.
+__global__ void k_add_lower_diagonal(int n, const int* __restrict__ rowptr, const double* __restrict__ c, double* val) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double* B = val + 9 * (size_t)(rowptr[i + 1] - 1);
+  B[0] = B[0] + c[i];
+  B[4] = B[4] + c[i];
+  B[8] = B[8] + c[i];
+}
+
+cudaError_t launch_add_lower_diagonal(int n, const int* rowptr, const double* c, double* val, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  k_add_lower_diagonal<<<(n + 127) / 128, 128, 0, s>>>(n, rowptr, c, val);
+  return cudaGetLastError();
+}
+
 }  // namespace bogus_gpu
 
 // ---- MecheFrictionProblem (Interfaces/MecheInterface.cpp) -----------------------------------------------
