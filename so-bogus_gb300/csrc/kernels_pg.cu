@@ -4,9 +4,10 @@
 // Work split: warp w of the grid owns the 32-contact chunks w, w + W, w + 2W, ... in every phase, lane l
 // contact 32c + l. A phase is one pass over the contacts (row-local vector work) or over W (SpMV with the
 // row-local work fused into its epilogue). Global dot products are reduced in the canonical order: a
-// butterfly per chunk inside the warp, then the 8-stripe combination run by the last CTA to reach the
-// grid barrier, which publishes the scalars; every CTA then takes the same line-search / momentum
-// decisions on identical values. Waits are bounded (grid_barrier), so a fault elsewhere ends the kernel
+// butterfly per chunk inside the warp, then the 8-stripe combination. Up to kFlatChunks chunks every CTA runs it
+// itself once all have arrived (flat_barrier, flat_combine); beyond, the last CTAs to reach the barrier take a stripe
+// each and the last of those publishes the scalars (mono_barrier_combine). Either way every CTA takes the same
+// line-search / momentum decisions on identical values. Waits are bounded, so a fault elsewhere ends the kernel
 // with BOGUS_GPU_TIMEOUT instead of a hang.
 //
 // Phases of one APGD iteration (reference line numbers in ProjectedGradient.impl.hpp):
